@@ -31,6 +31,7 @@ struct GemmCall {
   bool accumulate;
   float alpha;
   int force_bn;  // 0 = rule, else 128, 192 or 256
+  int force_pair;  // with force_bn: 1 = CTA pairs on 256 x force_bn tiles, 0 = one CTA per 128-row tile
   int split_k;   // K-split of the tail wave's tiles: 0 = rule, 1 = never, n = exactly n
   // 0 = plain outputs leave through TMA stores staged in shared memory when the output's base
   // and pitch allow it; -1 = always the per-thread row stores

@@ -45,7 +45,7 @@ Tensor status_tensor_op() { return status_tensor(); }
 void gemm(const Tensor& a, const Tensor& b, Tensor out, bool a_mn, bool b_mn,
           const c10::optional<Tensor>& bias, const c10::optional<Tensor>& residual,
           bool accumulate, double alpha, int64_t force_bn, int64_t split_k,
-          bool staged_store) {
+          bool staged_store, bool force_pair) {
   need(a, at::kBFloat16, "a");
   need(b, at::kBFloat16, "b");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && out.dim() == 2, "gemm operands must be 2-D");
@@ -71,6 +71,7 @@ void gemm(const Tensor& a, const Tensor& b, Tensor out, bool a_mn, bool b_mn,
   TORCH_CHECK(c.out_fp32 || out.scalar_type() == at::kBFloat16, "gemm out must be fp32 or bf16");
   c.accumulate = accumulate;
   c.alpha = static_cast<float>(alpha);
+  c.force_pair = force_pair ? 1 : 0;
   c.force_bn = static_cast<int>(force_bn);
   c.split_k = static_cast<int>(split_k);
   c.staged_store = staged_store ? 0 : -1;
@@ -862,7 +863,8 @@ TORCH_LIBRARY(stb, m) {
   m.def("status_reset", &status_reset);
   m.def("status_tensor", &status_tensor_op);
   m.def("gemm(Tensor a, Tensor b, Tensor out, bool a_mn, bool b_mn, Tensor? bias, Tensor? residual, "
-        "bool accumulate, float alpha, int force_bn, int split_k=0, bool staged_store=True) -> ()",
+        "bool accumulate, float alpha, int force_bn, int split_k=0, bool staged_store=True, "
+        "bool force_pair=False) -> ()",
         &gemm);
   m.def("gemm_scatter", &gemm_scatter);
   m.def("gemm_seq_pull", &gemm_seq_pull);

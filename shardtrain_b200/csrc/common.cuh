@@ -108,33 +108,139 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// CLUSTER: some of the arrivals come from the other CTA of a pair
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
+  if constexpr (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 // Bounded wait: false (and the status word set) once the time budget is spent, or as soon as the
 // status word shows that something else already failed.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code) {
   for (uint32_t i = 0; i < kFastPolls; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
   }
   const uint64_t t0 = global_ns();
   for (;;) {
     for (uint32_t i = 0; i < 256; ++i) {
-      if (mbar_try_wait(bar, parity)) return true;
+      if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     }
     if (status_failed(status)) return false;
     if (global_ns() - t0 > kWaitBudgetNs) break;
   }
   if (status != nullptr) atomicCAS(status, kOk, code);
   return false;
+}
+
+// Warp form of mbar_wait for the warps that issue TMA copies and MMAs: all 32 lanes call it and all
+// get the same answer, so the warp stays converged and may go on to elect a lane.
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, int code) {
+  for (uint32_t i = 0; i < kFastPolls; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait<CLUSTER>(bar, parity))) return true;
+  }
+  const uint64_t t0 = global_ns();
+  for (;;) {
+    for (uint32_t i = 0; i < 256; ++i) {
+      if (__all_sync(0xffffffffu, mbar_try_wait<CLUSTER>(bar, parity))) return true;
+    }
+    if (__any_sync(0xffffffffu, status_failed(status))) return false;
+    if (__any_sync(0xffffffffu, global_ns() - t0 > kWaitBudgetNs)) break;
+  }
+  if (status != nullptr) atomicCAS(status, kOk, code);
+  return false;
+}
+
+// ----------------------------------------------------------------------------- CTA pairs
+// Helpers for kernels launched as clusters of two CTAs that share one tensor-core tile
+// (tcgen05 cta_group::2).  Rank 0 of the pair issues the MMAs and owns the barriers they wait on.
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// shared::cluster address of `p` (an address of this CTA's shared memory) in the CTA of rank `rank`
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+// CTA-pair form of kernel_should_skip: both CTAs of the pair return the same answer (a status word
+// that changes between their reads must not let one of them wait for the other).
+__device__ __forceinline__ bool pair_should_skip(const int* status) {
+  __shared__ uint32_t skip;
+  if (threadIdx.x == 0) skip = status_failed(status) ? 1u : 0u;
+  cluster_sync();
+  uint32_t theirs;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];"
+               : "=r"(theirs) : "r"(cluster_addr(&skip, cluster_rank() ^ 1u)) : "memory");
+  const bool out = (skip | theirs) != 0;
+  cluster_sync();      // the peer has read this CTA's word: either may leave from here on
+  return out;
+}
+// TMA load into this CTA's shared memory that completes on a barrier of either CTA of the pair
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map,
+                                                 uint32_t cluster_bar, int32_t x, int32_t y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                   smem_u32(smem_result)),
+               "r"(ncols)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
+               : "memory");
+}
+// The barrier at this offset in BOTH CTAs of the pair arrives once the MMAs issued so far are done.
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
+}
+// One MMA over the pair: each CTA holds half the rows of A and D and half the rows (columns of the
+// result) of B; issued by rank 0 only.
+__device__ __forceinline__ void tc_mma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
+                                                uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
 
 // ----------------------------------------------------------------------------- TMA

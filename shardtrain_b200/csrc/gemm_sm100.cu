@@ -128,8 +128,8 @@ namespace {
 
 // How the tail wave of `tiles` tiles is cut along K (see GemmSplit).  `want`: 0 = rule, 1 = never,
 // n > 1 = exactly n (tests).  Returns the split factor and fills full / kb_per.
-int plan_split(int tiles, int num_kb, int want, int* full, int* kb_per) {
-  const int sms = sm_count();
+// `sms`: CTAs (or CTA pairs) of the persistent grid.
+int plan_split(int sms, int tiles, int num_kb, int want, int* full, int* kb_per) {
   *full = (tiles / sms) * sms;
   const int rem = tiles - *full;
   *kb_per = num_kb;
@@ -202,7 +202,7 @@ cudaError_t pull_flags(cudaStream_t stream, uint32_t** flags, uint32_t* epoch) {
   return cudaSuccess;
 }
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, bool PAIR>
 cudaError_t launch_variant(const GemmCall& c, int* status, cudaStream_t stream) {
   CUtensorMap ta, tb;
   bool ok;
@@ -211,7 +211,8 @@ cudaError_t launch_variant(const GemmCall& c, int* status, cudaStream_t stream) 
   else
     ok = make_bf16_tensor_map(&ta, c.a, c.K, c.M, c.lda, 64, 64);
   if (!B_MN)
-    ok = ok && make_bf16_tensor_map(&tb, c.b, c.N, c.K, c.ldb, 64, c.gated_inter > 0 ? BN / 2 : BN);
+    ok = ok && make_bf16_tensor_map(&tb, c.b, c.N, c.K, c.ldb, 64,
+                                   PAIR || c.gated_inter > 0 ? BN / 2 : BN);
   else
     ok = ok && make_bf16_tensor_map(&tb, c.b, c.K, c.N, c.ldb, 64, 64);
   if (!ok) return cudaErrorInvalidValue;
@@ -259,13 +260,15 @@ cudaError_t launch_variant(const GemmCall& c, int* status, cudaStream_t stream) 
       tc = tc_up = tc_h = ta;
   }
 
-  constexpr int smem = GemmSmem<BN>::kTotal;
-  const int m_tiles = (c.M + kGemmBM - 1) / kGemmBM;
+  constexpr int smem = GemmSmem<BN, B_MN, PAIR>::kTotal;
+  constexpr int tile_m = PAIR ? 2 * kGemmBM : kGemmBM;
+  const int workers = PAIR ? sm_count() / 2 : sm_count();
+  const int m_tiles = (c.M + tile_m - 1) / tile_m;
   const int n_tiles = c.gated_inter > 0 ? (c.gated_inter + BN / 2 - 1) / (BN / 2) : (c.N + BN - 1) / BN;
   const int tiles = m_tiles * n_tiles;
   const int num_kb = (c.K + kGemmBK - 1) / kGemmBK;
   GemmSplit sp{};
-  sp.split = plan_split(tiles, num_kb, c.gated_inter > 0 ? 1 : c.split_k, &sp.full_tiles,
+  sp.split = plan_split(workers, tiles, num_kb, c.gated_inter > 0 ? 1 : c.split_k, &sp.full_tiles,
                         &sp.kb_per_split);
   if (sp.split > 1) {
     SplitBuffers buffers;
@@ -277,8 +280,8 @@ cudaError_t launch_variant(const GemmCall& c, int* status, cudaStream_t stream) 
     sp.full_tiles = tiles;
   }
   sp.total_units = sp.full_tiles + (tiles - sp.full_tiles) * sp.split;
-  const int grid = std::min(sp.total_units, sm_count());   // persistent: one CTA per SM
-  if constexpr (!A_MN) {
+  const int grid = std::min(sp.total_units, workers) * (PAIR ? 2 : 1);   // persistent: one CTA per SM
+  if constexpr (!A_MN && !PAIR) {
     if (c.pull_degree > 1) {
       GemmPull pull{};
       for (int i = 0; i < c.pull_degree; ++i) pull.peers[i] = c.pull_peers[i];
@@ -303,7 +306,12 @@ cudaError_t launch_variant(const GemmCall& c, int* status, cudaStream_t stream) 
       return cudaGetLastError();
     }
   }
-  auto kernel = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN>;
+  auto kernel = [] {
+    if constexpr (PAIR)
+      return gemm_pair_bf16_tcgen05_kernel<BN, A_MN, B_MN>;
+    else
+      return gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN>;
+  }();
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [&] {
@@ -316,17 +324,105 @@ cudaError_t launch_variant(const GemmCall& c, int* status, cudaStream_t stream) 
   return cudaGetLastError();
 }
 
-template <int BN>
+template <int BN, bool PAIR>
 cudaError_t dispatch_major(const GemmCall& c, int* status, cudaStream_t stream) {
-  if (!c.a_mn && !c.b_mn) return launch_variant<BN, false, false>(c, status, stream);
-  if (!c.a_mn && c.b_mn) return launch_variant<BN, false, true>(c, status, stream);
-  if (c.a_mn && c.b_mn) return launch_variant<BN, true, true>(c, status, stream);
-  return launch_variant<BN, true, false>(c, status, stream);
+  if (!c.a_mn && !c.b_mn) return launch_variant<BN, false, false, PAIR>(c, status, stream);
+  if (!c.a_mn && c.b_mn) return launch_variant<BN, false, true, PAIR>(c, status, stream);
+  if (c.a_mn && c.b_mn) return launch_variant<BN, true, true, PAIR>(c, status, stream);
+  return launch_variant<BN, true, false, PAIR>(c, status, stream);
+}
+
+// Tile shape and tail split of one GEMM.
+struct TileChoice {
+  int bn = 0;
+  bool pair = false;
+  int split = 1;     // as GemmCall::split_k
+};
+
+// Clocks of one 64-wide k-block, measured on B200 over 8192 x 8192 x {1536, 8192} (the MMAs alone
+// need 2 BN):
+//     BN                      128    192    256
+//     pair, 256-row tile      349    435    518
+//     one CTA, 128-row tile   384    475    565
+double kblock_clocks(bool pair, int bn) { return pair ? 180.0 + 1.32 * bn : 204.0 + 1.41 * bn; }
+
+int tiles_of(const GemmCall& c, bool pair, int bn) {
+  const int m_tiles = (c.M + (pair ? 255 : 127)) / (pair ? 256 : 128);
+  return m_tiles * (c.gated_inter > 0 ? (c.gated_inter + bn / 2 - 1) / (bn / 2) : (c.N + bn - 1) / bn);
+}
+
+// Estimated time, in SM clocks, of a persistent kernel: waves of tiles x (k-blocks x clocks of one
+// + a constant), the tail wave shortened when its tiles are cut along K (parking and re-reading the
+// partial tiles costs 1000 + 24 BN split), and about 2500 more for a pair's cluster start and syncs.
+double estimate(const GemmCall& c, bool pair, int bn, int want_split) {
+  const int workers = pair ? sm_count() / 2 : sm_count();
+  if (workers < 1) return 1e30;
+  const int num_kb = (c.K + kGemmBK - 1) / kGemmBK;
+  const int tiles = tiles_of(c, pair, bn);
+  int full, kb_per;
+  const int split = plan_split(workers, tiles, num_kb, want_split, &full, &kb_per);
+  const double per_kb = kblock_clocks(pair, bn);
+  double cost = (pair ? 2500.0 : 0.0) + (full / workers) * (num_kb * per_kb + 400.0);
+  if (tiles > full) cost += kb_per * per_kb + 400.0 + (split > 1 ? 1000.0 + 24.0 * bn * split : 0.0);
+  return cost;
+}
+
+TileChoice choose_tile(const GemmCall& c) {
+  const int sms = sm_count();
+  const int num_kb = (c.K + kGemmBK - 1) / kGemmBK;
+  const int want = c.gated_inter > 0 ? 1 : c.split_k;
+  const bool may_pair = c.pull_degree <= 1;
+  TileChoice best;
+  // Which elements are summed in several K ranges (and in how many) is settled on 128-row tiles
+  // alone: the width whose waves x (128 + BN) is smallest, the tail wave counting 1 / split.  It
+  // decides the bits of the result, so it does not depend on the kernel that then runs.
+  double least = -1.0;
+  for (int cand : {256, 192, 128}) {
+    if (c.gated_inter > 0 && cand != 256) continue;
+    const int tiles = tiles_of(c, false, cand);
+    int full, kb_per;
+    const int split = plan_split(sms, tiles, num_kb, want, &full, &kb_per);
+    double waves = full / sms;
+    if (tiles > full) waves += 1.0 / split + (split > 1 ? 0.06 : 0.0);
+    const double cost = waves * (kGemmBM + cand);
+    if (least < 0 || cost < least) {
+      least = cost;
+      best.bn = cand;
+      best.split = split;
+    }
+  }
+  if (best.split > 1) {
+    // Pairs walk the same tiles two rows at a time (see GROUP in the kernel), so with an even number
+    // of 128-row tiles (and of SMs) the same elements fall into the same K ranges: 4096 x 1536 x
+    // 17920 in 165 us by pairs against 172 us, 512 x 1536 x 8960 in 33 us by single CTAs against 35.
+    const bool even = ((c.M + kGemmBM - 1) / kGemmBM) % 2 == 0 && sms % 2 == 0;
+    best.pair = may_pair && even &&
+                estimate(c, true, best.bn, best.split) < estimate(c, false, best.bn, best.split);
+    return best;
+  }
+  // Unsplit sums are the same whatever the tile: take the fastest.  A pair does twice the rows in
+  // less time per k-block but has half as many workers: single CTAs stay the better ones where
+  // there are few tiles (512 x 1536 x 1536: 19.4 us against 20.5 us; 4096 x 17920 x 1536 the other
+  // way: 152 us against 171 us).  Over 36 shapes of 512 to 8192 rows the estimate's choice is 1.5 %
+  // behind the best one on average, 8 % at worst.
+  double cost = -1.0;
+  for (int pair = 0; pair <= (may_pair ? 1 : 0); ++pair)
+    for (int cand : {256, 192, 128}) {
+      if (c.gated_inter > 0 && cand != 256) continue;
+      const double e = estimate(c, pair != 0, cand, 1);
+      if (cost < 0 || e < cost) {
+        cost = e;
+        best.bn = cand;
+        best.pair = pair != 0;
+      }
+    }
+  return best;
 }
 
 }  // namespace
 
-cudaError_t launch_gemm_bf16(const GemmCall& c, int* status, cudaStream_t stream) {
+cudaError_t launch_gemm_bf16(const GemmCall& call, int* status, cudaStream_t stream) {
+  GemmCall c = call;
   if (c.M <= 0 || c.N <= 0 || c.K <= 0) return cudaErrorInvalidValue;
   // TMA needs 16-byte aligned bases and strides; the vectorised epilogue needs N % 8 == 0.
   auto aligned16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
@@ -363,36 +459,26 @@ cudaError_t launch_gemm_bf16(const GemmCall& c, int* status, cudaStream_t stream
         c.residual != nullptr || c.scatter_degree > 1 || c.gated_out == nullptr ||
         !aligned16(c.gated_out) || c.N != 2 * c.gated_inter || c.gated_inter % 8)
       return cudaErrorInvalidValue;
-    return dispatch_major<256>(c, status, stream);
   }
-  int bn = c.force_bn;
-  if (bn == 0) {
-    // Persistent kernel, one CTA per SM: the run time is (waves of tiles) x (time of one tile).
-    // Measured on B200, a k-block of a 128 x BN tile is bound by the shared-memory operand reads
-    // of the MMAs, i.e. its time goes with 128 + BN, not with BN; the tail wave counts 1/split
-    // when its tiles are cut along K.  Pick the width with the smallest product.
-    const int sms = sm_count();
-    const int m_tiles = (c.M + kGemmBM - 1) / kGemmBM;
-    const int num_kb = (c.K + kGemmBK - 1) / kGemmBK;
-    double best = -1.0;
-    for (int cand : {256, 192, 128}) {
-      const int tiles = m_tiles * ((c.N + cand - 1) / cand);
-      int full, kb_per;
-      const int split = plan_split(tiles, num_kb, c.split_k, &full, &kb_per);
-      // whole waves + the tail wave (shortened by its K split, plus the cost of parking and
-      // re-reading the partial tiles)
-      double waves = full / sms;
-      if (tiles > full) waves += 1.0 / split + (split > 1 ? 0.06 : 0.0);
-      const double cost = waves * (kGemmBM + cand);
-      if (best < 0 || cost < best) {
-        best = cost;
-        bn = cand;
-      }
-    }
+  TileChoice t;
+  if (c.force_bn != 0) {
+    t.bn = c.force_bn;
+    t.pair = c.force_pair != 0;
+    if (t.pair && c.pull_degree > 1) return cudaErrorInvalidValue;
+  } else {
+    t = choose_tile(c);
+    c.split_k = t.split;
   }
-  if (bn == 256) return dispatch_major<256>(c, status, stream);
-  if (bn == 192) return dispatch_major<192>(c, status, stream);
-  if (bn == 128) return dispatch_major<128>(c, status, stream);
+  if (c.gated_inter > 0 && t.bn != 256) return cudaErrorInvalidValue;
+  if (t.pair) {
+    if (t.bn == 256) return dispatch_major<256, true>(c, status, stream);
+    if (t.bn == 192) return dispatch_major<192, true>(c, status, stream);
+    if (t.bn == 128) return dispatch_major<128, true>(c, status, stream);
+  } else {
+    if (t.bn == 256) return dispatch_major<256, false>(c, status, stream);
+    if (t.bn == 192) return dispatch_major<192, false>(c, status, stream);
+    if (t.bn == 128) return dispatch_major<128, false>(c, status, stream);
+  }
   return cudaErrorInvalidValue;
 }
 

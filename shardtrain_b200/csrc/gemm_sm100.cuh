@@ -98,11 +98,18 @@ constexpr int kGemmBM = 128;
 constexpr int kGemmBK = 64;
 constexpr int kGemmThreads = 192;
 
-template <int BN>
+// PAIR: two CTAs of a cluster share a 256 x BN tile (tcgen05 cta_group::2).  Each stages its own 128
+// rows of A and half of B's rows, so a k-block costs a CTA 128 + BN / 2 operand rows of shared
+// memory instead of 128 + BN.
+template <int BN, bool B_MN, bool PAIR>
 struct GemmSmem {
   static constexpr int kABytes = kGemmBM * kGemmBK * 2;
-  static constexpr int kBBytes = BN * kGemmBK * 2;
-  static constexpr int kStages = (BN == 256) ? 4 : (BN == 192 ? 5 : 6);
+  // rows of B a CTA stages; an MN-major B arrives in 64-wide chunks (192 / 2 = 96 takes two)
+  static constexpr int kBRows = PAIR ? BN / 2 : BN;
+  static constexpr int kBLoad = B_MN ? (kBRows + 63) / 64 * 64 : kBRows;
+  static constexpr int kBBytes = kBLoad * kGemmBK * 2;
+  static constexpr int kStages = PAIR ? (BN == 256 ? 6 : (BN == 192 ? 6 : 8))
+                                      : (BN == 256) ? 4 : (BN == 192 ? 5 : 6);
   // TMEM allocations are powers of two: two 192-column accumulators live in a 512-column grant
   static constexpr int kTmemCols = (2 * BN <= 256) ? 256 : 512;
   static constexpr int kStageBytes = kABytes + kBBytes;
@@ -112,13 +119,13 @@ struct GemmSmem {
   // (the staging area sits right after the operand tiles, so it is 1 KB aligned as the 128B
   // swizzle of the TMA stores needs; two buffers per warp where shared memory allows)
   static constexpr int kBarrierBytes = 256;
-  static constexpr int kStoreBufs = (BN == 192) ? 1 : 2;
+  static constexpr int kStoreBufs = (BN == 192 && !PAIR) ? 1 : 2;
   static constexpr int kScatterStageBytes = 4 * kStoreBufs * 4096;
   static constexpr int kTotal = kStages * kStageBytes + 1024 + kBarrierBytes + kScatterStageBytes;
   static_assert(kTotal <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
 };
 
-template <int BN, bool A_MN, bool B_MN, bool PULL>
+template <int BN, bool A_MN, bool B_MN, bool PULL, bool PAIR>
 __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
                                                        const CUtensorMap& tma_b,
                                                        const CUtensorMap& tma_c,
@@ -130,11 +137,16 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
   // Persistent: each CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...  The accumulator is
   // double buffered in TMEM (2 x BN columns) so the epilogue of one tile overlaps the MMAs of the
   // next; the shared-memory operand pipeline runs across tile boundaries without draining.
-  using S = GemmSmem<BN>;
+  using S = GemmSmem<BN, B_MN, PAIR>;
+  static_assert(!(PULL && PAIR), "the pulling GEMM runs one CTA per tile");
   constexpr int STAGES = S::kStages;
   // an earlier kernel recorded a failure (a peer that never signalled, a wait that expired): the
   // operands may be stale, skip the work -- uniformly, before any barrier or TMEM exists
-  if (kernel_should_skip(status)) return;
+  if (PAIR ? pair_should_skip(status) : kernel_should_skip(status)) return;
+  // position in the pair, and the index / stride of the CTA (or pair) over the work units
+  const int rank = PAIR ? static_cast<int>(cluster_rank()) : 0;
+  const int first_unit = PAIR ? blockIdx.x / 2 : blockIdx.x;
+  const int unit_stride = PAIR ? gridDim.x / 2 : gridDim.x;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -143,19 +155,22 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(store_stage + S::kScatterStageBytes);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* acc_full = empty_bar + STAGES;   // [2]
-  uint64_t* acc_empty = acc_full + 2;        // [2], 128 arrivals each
+  uint64_t* acc_empty = acc_full + 2;        // [2], 128 arrivals each (pair: 256, on rank 0)
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int m_tiles = (M + kGemmBM - 1) / kGemmBM;
+  constexpr int kTileM = PAIR ? 2 * kGemmBM : kGemmBM;
+  const int m_tiles = (M + kTileM - 1) / kTileM;
   const bool gated = ep.gated_inter > 0;
   const int tile_cols = gated ? BN / 2 : BN;          // output columns (per half) covered by a tile
   const int n_span = gated ? ep.gated_inter : N;
   const int n_tiles = (n_span + tile_cols - 1) / tile_cols;
   const int num_kb = (K + kGemmBK - 1) / kGemmBK;
-  constexpr int GROUP = 8;
+  // rows of tiles walked before the next column of tiles; with a K split a pair walks as many rows
+  // as single CTAs do, so that the same elements land in the split tail
+  const int GROUP = PAIR && sp.split > 1 ? 4 : 8;
   const int group_span = GROUP * n_tiles;
 
   // Grouped rasterisation: walk up to 8 M-tiles before moving to the next N-tile so that the
@@ -175,7 +190,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
   auto tile_origin = [&](int tile, int& m0, int& n0) {
     const int first_m = (tile / group_span) * GROUP;
     const int gm = min(m_tiles - first_m, GROUP);
-    m0 = (first_m + (tile % group_span) % gm) * kGemmBM;
+    m0 = (first_m + (tile % group_span) % gm) * kTileM + rank * kGemmBM;   // this CTA's rows
     n0 = ((tile % group_span) / gm) * tile_cols;
   };
 
@@ -186,7 +201,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], 128);
+      mbar_init(&acc_empty[b], PAIR ? 256 : 128);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -202,21 +217,45 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
     }
   }
   if (warp == 1) {
-    tmem_alloc(tmem_ptr, S::kTmemCols);
-    tmem_relinquish();
+    if constexpr (PAIR) {
+      tmem_alloc_pair(tmem_ptr, S::kTmemCols);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_ptr, S::kTmemCols);
+      tmem_relinquish();
+    }
   }
   tc_fence_before_sync();
-  __syncthreads();
+  if constexpr (PAIR)
+    cluster_sync();      // both CTAs' barriers exist before either signals the other's
+  else
+    __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr;
+  // the barriers of rank 0 that both CTAs of a pair signal
+  auto leader_bar = [&](uint64_t* bar) { return PAIR ? cluster_addr(bar, 0) : smem_u32(bar); };
+  auto load = [&](void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
+    if constexpr (PAIR)
+      tma_load_2d_pair(dst, map, leader_bar(bar), x, y);
+    else
+      tma_load_2d(dst, map, bar, x, y);
+  };
+  // an epilogue thread hands an accumulator buffer back to the MMA warp
+  auto release_acc = [&](uint64_t* bar) {
+    if constexpr (PAIR)
+      mbar_arrive_cluster(leader_bar(bar));
+    else
+      mbar_arrive(bar);
+  };
 
   if (warp == 0) {
-    if (lane == 0) {
+    // as for the MMAs below: the warp stays together and one elected lane issues the copies
+    {
       int it = 0;  // k-blocks issued so far, across tiles
       bool ok = true;
       uint64_t ready_tiles = 0;   // PULL: row tiles of A whose groups were all seen landed
       (void)ready_tiles;
-      for (int unit = blockIdx.x; unit < sp.total_units && ok; unit += gridDim.x) {
+      for (int unit = first_unit; unit < sp.total_units && ok; unit += unit_stride) {
         int tile, kb0, kb1, part, m0, n0;
         unit_work(unit, tile, kb0, kb1, part);
         tile_origin(tile, m0, n0);
@@ -243,9 +282,10 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
               bool all = true;
 #pragma unroll
               for (int g = 0; g < kGemmBM / kPullRows; ++g) all = all && seen[g] == pull.epoch;
-              if (all) break;
+              if (__all_sync(0xffffffffu, all)) break;
               if ((spin & 63u) == 63u &&
-                  (status_failed(status) || global_ns() - t0 > kWaitBudgetNs)) {
+                  __any_sync(0xffffffffu,
+                             status_failed(status) || global_ns() - t0 > kWaitBudgetNs)) {
                 if (status != nullptr) atomicCAS(status, kOk, kErrPullWait);
                 *abort_flag = 1;
                 ok = false;
@@ -263,53 +303,75 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&empty_bar[s], ph ^ 1, status, kErrProducerEmptyWait)) {
+          if (!mbar_wait_warp(&empty_bar[s], ph ^ 1, status, kErrProducerEmptyWait)) {
             *abort_flag = 1;
             ok = false;
             break;
           }
           uint8_t* sa = tiles + s * S::kStageBytes;
           uint8_t* sb = sa + S::kABytes;
-          mbar_expect_tx(&full_bar[s], S::kStageBytes);
-          if constexpr (!A_MN) {
-            tma_load_2d(sa, &tma_a, &full_bar[s], kb * kGemmBK, m0);
-          } else {
-#pragma unroll
-            for (int c = 0; c < kGemmBM / 64; ++c)
-              tma_load_2d(sa + c * 8192, &tma_a, &full_bar[s], m0 + c * 64, kb * kGemmBK);
-          }
-          if constexpr (!B_MN) {
-            if (gated) {   // box of BN / 2 rows: gate rows, then the matching up rows
-              tma_load_2d(sb, &tma_b, &full_bar[s], kb * kGemmBK, n0);
-              tma_load_2d(sb + (BN / 2) * 128, &tma_b, &full_bar[s], kb * kGemmBK,
-                          ep.gated_inter + n0);
+          // a pair's stage is complete when both CTAs' halves have landed (rank 0's barrier)
+          if (elect_one()) {
+            if (rank == 0) mbar_expect_tx(&full_bar[s], (PAIR ? 2 : 1) * S::kStageBytes);
+            if constexpr (!A_MN) {
+              load(sa, &tma_a, &full_bar[s], kb * kGemmBK, m0);
             } else {
-              tma_load_2d(sb, &tma_b, &full_bar[s], kb * kGemmBK, n0);
-            }
-          } else {
 #pragma unroll
-            for (int c = 0; c < BN / 64; ++c)
-              tma_load_2d(sb + c * 8192, &tma_b, &full_bar[s], n0 + c * 64, kb * kGemmBK);
+              for (int c = 0; c < kGemmBM / 64; ++c)
+                load(sa + c * 8192, &tma_a, &full_bar[s], m0 + c * 64, kb * kGemmBK);
+            }
+            if constexpr (!B_MN) {
+              if (gated) {   // box of BN / 2 rows: gate rows, then the matching up rows
+                if constexpr (PAIR) {
+                  load(sb, &tma_b, &full_bar[s], kb * kGemmBK, (rank ? ep.gated_inter : 0) + n0);
+                } else {
+                  load(sb, &tma_b, &full_bar[s], kb * kGemmBK, n0);
+                  load(sb + (BN / 2) * 128, &tma_b, &full_bar[s], kb * kGemmBK, ep.gated_inter + n0);
+                }
+              } else {
+                load(sb, &tma_b, &full_bar[s], kb * kGemmBK, n0 + rank * S::kBRows);
+              }
+            } else {
+#pragma unroll
+              for (int c = 0; c < S::kBLoad / 64; ++c)
+                load(sb + c * 8192, &tma_b, &full_bar[s], n0 + rank * S::kBRows + c * 64, kb * kGemmBK);
+            }
           }
+          __syncwarp();
         }
       }
       // Error path only: wait (bounded) for copies this thread issued that nobody consumed.
-      if (*abort_flag) {
+      // (Pair: the copies of rank 1 complete on rank 0's barriers, which it cannot wait on; it
+      // stays for a millisecond, and the pair leaves together, see the end.)
+      const bool aborted = __any_sync(0xffffffffu, *abort_flag != 0);
+      if (aborted && rank == 0) {
         for (int k = max(0, it - STAGES); k < it; ++k)
-          mbar_wait(&full_bar[k % STAGES], (k / STAGES) & 1, status, kErrDrainWait);
+          mbar_wait_warp(&full_bar[k % STAGES], (k / STAGES) & 1, status, kErrDrainWait);
+      } else if (aborted) {
+        const uint64_t t0 = global_ns();
+        while (global_ns() - t0 < 1000000ull) __nanosleep(1000);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(kGemmBM, BN, A_MN, B_MN);
+    // The whole warp walks the loop and one elected lane issues: everything the MMAs take is then
+    // warp-uniform and sits in uniform registers.  (With the loop inside `if (lane == 0)` an MMA
+    // took about 136 clocks to issue whatever its width, so a 128-wide tile ran no faster than a
+    // 256-wide one.)
+    if (rank == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(kTileM, BN, A_MN, B_MN);
+      // K-major: the 16-element K slice is 32 bytes further along each 128-byte row.  MN-major: the
+      // slice is 16 K-rows (two 8-row swizzle atoms, 1024 B apart) further on; 64-wide MN chunks sit
+      // 8192 B apart (the leading-dimension byte offset).
+      const uint64_t desc_a0 = make_smem_desc_sw128(smem_u32(tiles), A_MN ? 8192 : 16, 1024);
+      const uint64_t desc_b0 = make_smem_desc_sw128(smem_u32(tiles) + S::kABytes, B_MN ? 8192 : 16, 1024);
       int it = 0, local = 0;
       bool ok = true;
-      for (int unit = blockIdx.x; unit < sp.total_units && ok; unit += gridDim.x, ++local) {
+      for (int unit = first_unit; unit < sp.total_units && ok; unit += unit_stride, ++local) {
         int tile, kb0, kb1, part;
         unit_work(unit, tile, kb0, kb1, part);
         const int ab = local & 1;
         // the epilogue must have drained this accumulator buffer (two tiles ago)
-        if (!mbar_wait(&acc_empty[ab], ((local >> 1) & 1) ^ 1, status, kErrMmaFullWait)) {
+        if (!mbar_wait_warp<PAIR>(&acc_empty[ab], ((local >> 1) & 1) ^ 1, status, kErrMmaFullWait)) {
           *abort_flag = 1;
           break;
         }
@@ -318,28 +380,35 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&full_bar[s], ph, status, kErrMmaFullWait)) {
+          if (!mbar_wait_warp(&full_bar[s], ph, status, kErrMmaFullWait)) {
             *abort_flag = 1;
             ok = false;
             break;
           }
           tc_fence_after_sync();
-          const uint32_t a_base = smem_u32(tiles + s * S::kStageBytes);
-          const uint32_t b_base = a_base + S::kABytes;
+          // descriptors hold addresses in 16-byte units (below 2^14, so the sums never carry)
+          const uint64_t da_s = desc_a0 + s * (S::kStageBytes >> 4);
+          const uint64_t db_s = desc_b0 + s * (S::kStageBytes >> 4);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kGemmBK / 16; ++k) {
-            // K-major: the 16-element K slice is 32 bytes further along each 128-byte row.
-            // MN-major: the slice is 16 K-rows (two 8-row swizzle atoms, 1024 B apart) further
-            // on; 64-wide MN chunks sit 8192 B apart (the leading-dimension byte offset).
-            const uint64_t da = A_MN ? make_smem_desc_sw128(a_base + k * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(a_base + k * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc_sw128(b_base + k * 2048, 8192, 1024)
-                                     : make_smem_desc_sw128(b_base + k * 32, 16, 1024);
-            tc_mma_f16(tmem_d, da, db, idesc, ((kb - kb0) | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < kGemmBK / 16; ++k) {
+              const uint64_t da = da_s + k * ((A_MN ? 2048 : 32) >> 4);
+              const uint64_t db = db_s + k * ((B_MN ? 2048 : 32) >> 4);
+              const uint32_t acc = ((kb - kb0) | k) != 0 ? 1u : 0u;
+              if constexpr (PAIR)
+                tc_mma_f16_pair(tmem_d, da, db, idesc, acc);
+              else
+                tc_mma_f16(tmem_d, da, db, idesc, acc);
+            }
+            // frees the stage (in both CTAs of a pair) once these MMAs have read it
+            if constexpr (PAIR) tc_commit_pair(&empty_bar[s]); else tc_commit(&empty_bar[s]);
           }
-          tc_commit(&empty_bar[s]);  // frees the stage once these MMAs have read it
+          __syncwarp();
         }
-        tc_commit(&acc_full[ab]);
+        if (elect_one()) {
+          if constexpr (PAIR) tc_commit_pair(&acc_full[ab]); else tc_commit(&acc_full[ab]);
+        }
+        __syncwarp();
       }
     }
   } else if (PULL && warp >= 6) {
@@ -392,11 +461,26 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
     int sbuf = 0;          // staged store: which of this warp's staging buffers is written next
     bool ok = true;
     int* last_flag = reinterpret_cast<int*>(tmem_ptr + 2);   // shared: "this CTA reduces the tile"
-    for (int unit = blockIdx.x; unit < sp.total_units; unit += gridDim.x, ++local) {
+    for (int unit = first_unit; unit < sp.total_units; unit += unit_stride, ++local) {
       int tile, kb0, kb1, part, m0, n0;
       unit_work(unit, tile, kb0, kb1, part);
       tile_origin(tile, m0, n0);
       const int ab = local & 1;
+      // fp32 residual rows of the staged store are read one 32-column chunk ahead of the chunk that
+      // is being stored, the first one while the tile's MMAs still run: loaded where they are used,
+      // their latency came on top of every chunk.
+      const bool ahead = ep.staged_store && ep.out_fp32 && ep.residual != nullptr;
+      float4 res_next[8];
+      auto fetch_residual = [&](int c) {
+        const int64_t gr = static_cast<int64_t>(m0) + row;
+        const int col = n0 + c * 32;
+        if (!ahead || gr >= M) return;
+        const float* rs = reinterpret_cast<const float*>(ep.residual) + gr * ep.ldo + col;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (col + 4 * j < N) res_next[j] = *reinterpret_cast<const float4*>(rs + 4 * j);
+      };
+      fetch_residual(0);
       if (ok) ok = mbar_wait(&acc_full[ab], (local >> 1) & 1, status, kErrEpilogueAccumWait);
       tc_fence_after_sync();
       const uint32_t tmem_d = tmem_base + ab * BN;
@@ -482,14 +566,15 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
           }
           uint8_t* stage = store_stage + (q * S::kStoreBufs + sbuf) * 4096;
           if (ep.out_fp32) {
-            if (ep.residual != nullptr && row_ok) {
-              const float* rs = reinterpret_cast<const float*>(ep.residual) + g_row * ep.ldo + col0;
+            if (ahead) {
+              if (row_ok) {
 #pragma unroll
-              for (int i = 0; i < 32; i += 4) {
-                if (col0 + i >= N) break;
-                const float4 y = *reinterpret_cast<const float4*>(rs + i);
-                v[i] += y.x; v[i + 1] += y.y; v[i + 2] += y.z; v[i + 3] += y.w;
+                for (int j = 0; j < 8; ++j) {
+                  v[4 * j] += res_next[j].x; v[4 * j + 1] += res_next[j].y;
+                  v[4 * j + 2] += res_next[j].z; v[4 * j + 3] += res_next[j].w;
+                }
               }
+              if (c + 1 < BN / 32) fetch_residual(c + 1);
             }
             // the store that last read this buffer must have finished reading it
             if (lane == 0) bulk_wait_group_read<S::kStoreBufs - 1>();
@@ -674,7 +759,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
           }
         }
         tc_fence_before_sync();
-        mbar_arrive(&acc_empty[ab]);
+        release_acc(&acc_empty[ab]);
         continue;
       }
       if (part < 0) {
@@ -686,7 +771,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
           emit(r, c);
         }
         tc_fence_before_sync();
-        mbar_arrive(&acc_empty[ab]);   // TMEM reads complete: hand the buffer back to the MMA warp
+        release_acc(&acc_empty[ab]);   // TMEM reads complete: hand the buffer back to the MMA warp
         continue;
       }
       // ---- K-split unit: park the raw partial tile, the last arrival reduces
@@ -695,7 +780,8 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
       // and when reducing; the thread that reduces a row is the one that owns it in every unit.
       const int rem_tile = tile - sp.full_tiles;
       constexpr int64_t kTileFloats = static_cast<int64_t>(kGemmBM) * BN;
-      float* mine = sp.workspace + (static_cast<int64_t>(rem_tile) * sp.split + part) * kTileFloats +
+      const int slab = PAIR ? rem_tile * 2 + rank : rem_tile;   // a pair's halves reduce separately
+      float* mine = sp.workspace + (static_cast<int64_t>(slab) * sp.split + part) * kTileFloats +
                     row * 4;
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
@@ -708,18 +794,18 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
               make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
       }
       tc_fence_before_sync();
-      mbar_arrive(&acc_empty[ab]);
+      release_acc(&acc_empty[ab]);
       __threadfence();                              // partial tile visible before the count
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (threadIdx.x == 64) {
-        const int seen = atomicAdd(sp.counters + rem_tile, 1);
+        const int seen = atomicAdd(sp.counters + slab, 1);
         *last_flag = (seen == sp.split - 1) ? 1 : 0;
-        if (seen == sp.split - 1) sp.counters[rem_tile] = 0;   // ready for the next launch
+        if (seen == sp.split - 1) sp.counters[slab] = 0;   // ready for the next launch
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (*last_flag == 0) continue;
       __threadfence();
-      const float* first = sp.workspace + static_cast<int64_t>(rem_tile) * sp.split * kTileFloats +
+      const float* first = sp.workspace + static_cast<int64_t>(slab) * sp.split * kTileFloats +
                            row * 4;
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
@@ -746,10 +832,16 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
   }
 
   tc_fence_before_sync();
-  __syncthreads();
+  if constexpr (PAIR)
+    cluster_sync();      // neither CTA leaves while the other still signals it or reads its operands
+  else
+    __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, S::kTmemCols);
+    if constexpr (PAIR)
+      tmem_dealloc_pair(tmem_base, S::kTmemCols);
+    else
+      tmem_dealloc(tmem_base, S::kTmemCols);
   }
 }
 
@@ -761,8 +853,21 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
                          const __grid_constant__ CUtensorMap tma_c_up,
                          const __grid_constant__ CUtensorMap tma_c_h, GemmEpilogue ep, GemmSplit sp,
                          int M, int N, int K, int* __restrict__ status) {
-  gemm_bf16_tcgen05_body<BN, A_MN, B_MN, false>(tma_a, tma_b, tma_c, tma_c_up, tma_c_h, ep, sp,
+  gemm_bf16_tcgen05_body<BN, A_MN, B_MN, false, false>(tma_a, tma_b, tma_c, tma_c_up, tma_c_h, ep, sp,
                                                 GemmPull{}, M, N, K, status);
+}
+
+// The same GEMM with pairs of CTAs on 256 x BN tiles.
+template <int BN, bool A_MN, bool B_MN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+gemm_pair_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
+                              const __grid_constant__ CUtensorMap tma_b,
+                              const __grid_constant__ CUtensorMap tma_c,
+                              const __grid_constant__ CUtensorMap tma_c_up,
+                              const __grid_constant__ CUtensorMap tma_c_h, GemmEpilogue ep,
+                              GemmSplit sp, int M, int N, int K, int* __restrict__ status) {
+  gemm_bf16_tcgen05_body<BN, A_MN, B_MN, false, true>(tma_a, tma_b, tma_c, tma_c_up, tma_c_h, ep, sp,
+                                                      GemmPull{}, M, N, K, status);
 }
 
 // The same GEMM with four more warps that pull the A operand from its owners (see GemmPull).
@@ -775,7 +880,7 @@ gemm_pull_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
                               const __grid_constant__ CUtensorMap tma_c_h, GemmEpilogue ep,
                               GemmSplit sp, GemmPull pull, int M, int N, int K,
                               int* __restrict__ status) {
-  gemm_bf16_tcgen05_body<BN, false, B_MN, true>(tma_a, tma_b, tma_c, tma_c_up, tma_c_h, ep, sp, pull,
+  gemm_bf16_tcgen05_body<BN, false, B_MN, true, false>(tma_a, tma_b, tma_c, tma_c_up, tma_c_h, ep, sp, pull,
                                                 M, N, K, status);
 }
 

@@ -1,0 +1,61 @@
+"""GEMM with pairs of CTAs on 256-row tiles: edges of tiles, every operand order, K splits."""
+
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from shardtrain_b200 import ops as ops_module
+
+    return ops_module.load()
+
+
+CASES = [
+    # M, N, K, a_mn, b_mn, out_fp32, bias, residual, tile width, split
+    (8, 8, 8, False, False, True, False, False, 256, 1),         # one corner of one tile
+    (128, 256, 64, False, False, False, True, False, 256, 1),    # the second CTA's rows are all past M
+    (257, 264, 72, False, False, True, True, True, 256, 1),      # one row / one column group over a tile
+    (256, 192, 512, False, False, False, False, True, 192, 1),
+    (520, 200, 136, False, True, True, False, False, 192, 1),    # MN-major B: 96 columns in two chunks
+    (520, 392, 136, True, True, True, False, False, 192, 1),
+    (264, 136, 200, True, True, True, False, False, 128, 1),
+    (384, 128, 328, False, True, False, False, False, 128, 1),
+    (264, 520, 64, True, False, True, False, False, 256, 1),
+    (2048, 2560, 192, False, False, True, False, True, 256, 1),  # 80 tiles: several per pair
+    (512, 1536, 1096, False, True, True, False, False, 256, 4),  # tail tiles cut along K
+    (300, 584, 1104, False, False, False, True, True, 128, 3),
+    (640, 520, 1104, True, True, True, False, False, 192, 2),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=["x".join(map(str, c[:3])) + f"_{int(c[3])}{int(c[4])}_{c[8]}s{c[9]}"
+                                             for c in CASES])
+def test_pair_gemm_matches_reference_and_stays_inside_the_output(ops, case):
+    M, N, K, a_mn, b_mn, out_fp32, bias, residual, bn, split = case
+    torch.manual_seed(2)
+    a = torch.randn((K, M) if a_mn else (M, K), device=DEV).bfloat16()
+    b = torch.randn((K, N) if b_mn else (N, K), device=DEV).bfloat16()
+    dtype = torch.float32 if out_fp32 else torch.bfloat16
+    bias_t = torch.randn(N, device=DEV) if bias else None
+    res = torch.randn(M, N + 8, device=DEV).to(dtype)[:, :N] if residual else None
+    plane = torch.full((M + 3, N + 8), 7.0, device=DEV, dtype=dtype)
+    out = plane[:M, :N]
+    ops.gemm(a, b, out, a_mn, b_mn, bias_t, res, False, 1.0, bn, split, True, True)
+    want = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    want = want + (bias_t if bias else 0) + (res.double() if residual else 0)
+    # products of bf16 values are exact in fp32; K roundings of 2^-24 on partial sums of size up to
+    # a few sqrt(K), and one output rounding
+    bound = 2.0 ** -24 * math.sqrt(K) * K * 0.5 + 1e-6
+    if not out_fp32:
+        bound = bound + want.abs() * 2.0 ** -8
+    assert torch.all((out.double() - want).abs() <= bound)
+    assert torch.all(plane[M:] == 7.0) and torch.all(plane[:, N:] == 7.0)
+    again = torch.empty_like(plane)
+    ops.gemm(a, b, again[:M, :N], a_mn, b_mn, bias_t, res, False, 1.0, bn, split, True, True)
+    assert torch.equal(again[:M, :N], out)      # split sums run in index order
