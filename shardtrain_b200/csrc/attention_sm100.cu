@@ -2,15 +2,17 @@
 // kernels (dK/dV per key block, dQ per query block).  All five/seven matrix products run on
 // tcgen05 with accumulators in TMEM; Q/K/V/dO tiles arrive by TMA from the packed, rope-applied
 // qkv buffer; the softmax warps read scores from TMEM with tcgen05.ld and hand P / dS back to the
-// tensor core through 128-byte-swizzled shared memory.  No S x S matrix ever reaches global
-// memory (the reference materialises it: src/sharded_runtime/models/qwen2.py:247-257).
+// tensor core as TMEM operands.  No S x S matrix ever reaches global memory (the reference materialises it: src/sharded_runtime/models/qwen2.py:247-257).
 //
 // Tile = 128 x 128 (rows x head_dim or rows x rows) bf16, held as two 64-column halves of 16 KB
 // (128 rows x 128 bytes, TMA SWIZZLE_128B).  The same tile serves as a K-major operand (reduction
 // over its columns) or an MN-major operand (reduction over its rows); only the descriptor differs.
 //
-// CTA = 6 warps: 0 = TMA producer, 1 = MMA issuer / TMEM owner, 2..5 = softmax (one row each).
+// Warp 0 = TMA producer, warp 1 = MMA issuer / TMEM owner, the others = softmax: 4 warps with a row
+// per thread forward, 8 warps with half a row per thread backward.
 // Every mbarrier wait is bounded; on expiry the status word is set and the roles fall through.
+#include <type_traits>
+
 #include "api.h"
 #include "common.cuh"
 
@@ -25,7 +27,8 @@ constexpr int kD = 128;          // head dim
 constexpr int kBlk = 128;        // rows per tile
 constexpr int kHalf = 16384;     // bytes of one 64-column half tile
 constexpr int kTile = 2 * kHalf;
-constexpr int kThreads = 192;
+constexpr int kFwdThreads = 192;     // producer, MMA and 4 softmax warps (one row per thread)
+constexpr int kBwdThreads = 320;     // producer, MMA and 8 softmax warps (half a row per thread)
 
 // k-th 16-wide reduction slice of a tile used K-major (reduce over columns).
 __device__ __forceinline__ uint64_t desc_k(uint32_t tile, int kk) {
@@ -36,17 +39,26 @@ __device__ __forceinline__ uint64_t desc_mn(uint32_t tile, int kk) {
   return make_smem_desc_sw128(tile + kk * 2048, kHalf, 1024);
 }
 
-// D[128x128] (+)= A * B over a 128-long reduction: 8 MMAs of K = 16.
-template <bool A_MN, bool B_MN>
-__device__ __forceinline__ void mma_128(uint32_t tmem_d, uint32_t a_tile, uint32_t b_tile,
-                                        bool accumulate) {
-  constexpr uint32_t idesc = make_idesc_bf16(128, 128, A_MN, B_MN);
+// The MMAs below are issued by a warp that stays converged, one elected lane doing the work: then
+// addresses and descriptors are warp-uniform.  (Issued inside `if (lane == 0)` an MMA cost about 136
+// clocks whatever its size.)
+
+// D[128x128] = A B^T over a 128-long reduction, both tiles K-major: 8 MMAs of K = 16.
+__device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint32_t a_tile, uint32_t b_tile) {
+  constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, false);
 #pragma unroll
-  for (int kk = 0; kk < 8; ++kk) {
-    const uint64_t da = A_MN ? desc_mn(a_tile, kk) : desc_k(a_tile, kk);
-    const uint64_t db = B_MN ? desc_mn(b_tile, kk) : desc_k(b_tile, kk);
-    tc_mma_f16(tmem_d, da, db, idesc, (accumulate || kk > 0) ? 1u : 0u);
-  }
+  for (int kk = 0; kk < 8; ++kk)
+    tc_mma_f16(tmem_d, desc_k(a_tile, kk), desc_k(b_tile, kk), idesc, kk > 0 ? 1u : 0u);
+}
+// D[128x128] (+)= A B with A (bf16, 128 x 128) in TMEM and B MN-major in shared memory.  The first
+// 64 columns of A are packed at tmem_a, the last 64 at tmem_a + second_half.
+__device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t second_half,
+                                       uint32_t b_tile, bool accumulate) {
+  constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, true);
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk)
+    tc_mma_f16_ts(tmem_d, tmem_a + (kk >> 2) * second_half + (kk & 3) * 8, desc_mn(b_tile, kk), idesc,
+                  (accumulate || kk > 0) ? 1u : 0u);
 }
 
 // TMA: one 128x128 tile = two boxes of 64 columns.
@@ -56,13 +68,42 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
   tma_load_2d(dst + kHalf, map, bar, col + 64, row);
 }
 
-// Store 8 bf16 values (columns c8*8 .. +7 of row r) into a swizzled K-major tile.
-__device__ __forceinline__ void store_row8(uint8_t* tile, int r, int c8, uint4 v) {
-  const int half = c8 >> 3, chunk = c8 & 7;
-  *reinterpret_cast<uint4*>(tile + half * kHalf + r * 128 + ((chunk ^ (r & 7)) << 4)) = v;
-}
+// Writes this warp's 32 x 128 bf16 block through shared memory: row `lane` is stored swizzled at
+// stage + lane * 256 (8 KB per warp) by put, then leaves as whole 256-byte rows.
+struct RowStager {
+  uint8_t* stage;
+  int lane;
+  __device__ __forceinline__ void put(int c16, uint4 v) const {   // 16-byte piece c16 (0..15) of the row
+    *reinterpret_cast<uint4*>(stage + lane * 256 + ((c16 ^ (lane & 7)) << 4)) = v;
+  }
+  // rows row0 .. row0 + n_rows - 1 of the block go to base + row * pitch elements
+  __device__ __forceinline__ void flush(__nv_bfloat16* base, int64_t pitch, int n_rows) const {
+    __syncwarp();
+    const int piece = lane & 15;
+#pragma unroll 4
+    for (int r = lane >> 4; r < n_rows; r += 2)
+      *reinterpret_cast<uint4*>(base + r * pitch + piece * 8) =
+          *reinterpret_cast<const uint4*>(stage + r * 256 + ((piece ^ (r & 7)) << 4));
+    __syncwarp();
+  }
+};
 
-__device__ __forceinline__ void softmax_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ uint4 pack8(const uint32_t* v, float scale) {
+  uint4 pk;
+  pk.x = pack_bf16x2(__uint_as_float(v[0]) * scale, __uint_as_float(v[1]) * scale);
+  pk.y = pack_bf16x2(__uint_as_float(v[2]) * scale, __uint_as_float(v[3]) * scale);
+  pk.z = pack_bf16x2(__uint_as_float(v[4]) * scale, __uint_as_float(v[5]) * scale);
+  pk.w = pack_bf16x2(__uint_as_float(v[6]) * scale, __uint_as_float(v[7]) * scale);
+  return pk;
+}
+__device__ __forceinline__ uint4 pack8(const uint32_t* v) {
+  uint4 pk;
+  pk.x = pack_bf16x2(__uint_as_float(v[0]), __uint_as_float(v[1]));
+  pk.y = pack_bf16x2(__uint_as_float(v[2]), __uint_as_float(v[3]));
+  pk.z = pack_bf16x2(__uint_as_float(v[4]), __uint_as_float(v[5]));
+  pk.w = pack_bf16x2(__uint_as_float(v[6]), __uint_as_float(v[7]));
+  return pk;
+}
 
 struct FwdParams {
   __nv_bfloat16* out;
@@ -97,106 +138,108 @@ __device__ __forceinline__ void load_key_bits(const uint32_t* bits, int pitch, c
   }
 }
 
-// smem: Q tile | K,V x 2 stages | P tile | barriers
-constexpr int kFwdSmem = kTile + 4 * kTile + kTile + 1024 + 256;
+// Forward: one CTA per (query block, head, sample), two CTAs per SM.  The chain of a key block is
+//   S = Q K^T -> softmax -> O += P V,
+// serial inside a CTA; the second CTA of the SM fills the gaps (tensor pipe under the other's
+// exponentials and the other way round).  To fit twice, a CTA keeps S and O in 256 TMEM columns,
+// with P (bf16) written over the S it came from and read by the MMA as a TMEM operand, and one
+// stage each of K and V: 97 KB of shared memory.  CTAs start with the longest rows of blocks, so
+// the short ones fill the last wave.  Bound by the exponentials (1024 clocks a block) and the
+// softmax's issue slots.
+// Measured on B200 (12 heads): 1 x 8192, causal, 1576 us before (one CTA per SM, MMAs issued from
+// one lane, P through shared memory) and 311 us now; 8 x 512: 100 and 35 us.
+// smem: Q | K | V | barriers
+constexpr int kFwdSmem = 3 * kTile + 1024 + 128;
 
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kFwdThreads, 2)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
   if (kernel_should_skip(p.status)) return;   // an earlier kernel already failed
   extern __shared__ uint8_t raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sQ = smem;
-  uint8_t* sKV = sQ + kTile;          // stage s: K at sKV + s*2*kTile, V right after
-  uint8_t* sP = sKV + 4 * kTile;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + kTile);
-  uint64_t* q_full = bars;            // 1
-  uint64_t* kv_full = bars + 1;       // 2
-  uint64_t* kv_empty = bars + 3;      // 2
-  uint64_t* s_full = bars + 5;        // 2: scores are double buffered in TMEM
-  uint64_t* p_full = bars + 7;        // 1 (128 arrivals)
-  uint64_t* o_done = bars + 8;        // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+  uint8_t* sK = sQ + kTile;
+  uint8_t* sV = sK + kTile;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + kTile);
+  uint64_t* q_full = bars;
+  uint64_t* k_full = bars + 1;
+  uint64_t* k_empty = bars + 2;
+  uint64_t* v_full = bars + 3;
+  uint64_t* v_empty = bars + 4;
+  uint64_t* s_full = bars + 5;
+  uint64_t* p_full = bars + 6;        // 128 arrivals
+  uint64_t* o_done = bars + 7;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qb = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int nblk = (p.seq + kBlk - 1) / kBlk;
+  const int qb = nblk - 1 - static_cast<int>(blockIdx.x) / (p.hq * p.batch);
+  const int hb = static_cast<int>(blockIdx.x) % (p.hq * p.batch);
+  const int h = hb % p.hq, b = hb / p.hq;
   const int hk = h / (p.hq / p.hkv);
   const int n_kv = qb + 1;  // causal: key blocks 0..qb
   const int row0 = b * p.seq;
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&kv_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
-    }
-    mbar_init(&s_full[0], 1);
-    mbar_init(&s_full[1], 1);
-    mbar_init(p_full, 128);
-    mbar_init(o_done, 1);
+    for (int i = 0; i < 8; ++i) mbar_init(bars + i, i == 6 ? 128 : 1);
     fence_barrier_init();
     fence_proxy_async();
     prefetch_tensormap(&map);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
+    tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  // S(j) lives in columns (j & 1) * 128: Q K^T of key block j + 1 is issued before the softmax of
-  // block j has finished, so the tensor pipe works under the softmax instead of after it
-  const uint32_t tS0 = tmem, tO = tmem + 256;
+  const uint32_t tS = tmem, tO = tmem + 128;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, kTile);
       load_tile(sQ, &map, q_full, h * kD, row0 + qb * kBlk);
-      for (int j = 0; j < n_kv; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait(&kv_empty[s], ((j >> 1) & 1) ^ 1, p.status, kErrAttnWait)) break;
-        uint8_t* k_dst = sKV + s * 2 * kTile;
-        mbar_expect_tx(&kv_full[s], 2 * kTile);
-        load_tile(k_dst, &map, &kv_full[s], (p.hq + hk) * kD, row0 + j * kBlk);
-        load_tile(k_dst + kTile, &map, &kv_full[s], (p.hq + p.hkv + hk) * kD, row0 + j * kBlk);
+    }
+    __syncwarp();
+    for (int j = 0; j < n_kv; ++j) {
+      if (!mbar_wait_warp(k_empty, (j & 1) ^ 1, p.status, kErrAttnWait)) break;
+      if (elect_one()) {
+        mbar_expect_tx(k_full, kTile);
+        load_tile(sK, &map, k_full, (p.hq + hk) * kD, row0 + j * kBlk);
       }
+      __syncwarp();
+      if (!mbar_wait_warp(v_empty, (j & 1) ^ 1, p.status, kErrAttnWait)) break;
+      if (elect_one()) {
+        mbar_expect_tx(v_full, kTile);
+        load_tile(sV, &map, v_full, (p.hq + p.hkv + hk) * kD, row0 + j * kBlk);
+      }
+      __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = mbar_wait(q_full, 0, p.status, kErrAttnWait);
-      if (ok) ok = mbar_wait(&kv_full[0], 0, p.status, kErrAttnWait);
-      if (ok) {
-        tc_fence_after_sync();
-        mma_128<false, false>(tS0, smem_u32(sQ), smem_u32(sKV), false);          // S(0) = Q K_0^T
-        tc_commit(&s_full[0]);
+    const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV);
+    bool ok = mbar_wait_warp(q_full, 0, p.status, kErrAttnWait);
+    for (int j = 0; j < n_kv && ok; ++j) {
+      // S(j) may overwrite P(j-1): MMAs run in issue order, so P V of block j-1 has read it
+      ok = mbar_wait_warp(k_full, j & 1, p.status, kErrAttnWait);
+      if (!ok) break;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        mma_ss(tS, aQ, aK);                                          // S = Q K^T
+        tc_commit(k_empty);
+        tc_commit(s_full);
       }
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int s = j & 1;
-        const uint32_t k_tile = smem_u32(sKV + s * 2 * kTile);
-        if (j + 1 < n_kv) {
-          // S(j+1) into the other score buffer: its last reader, the softmax of block j-1,
-          // finished before p_full(j-1), which this thread has already waited for
-          const int s1 = (j + 1) & 1;
-          ok = mbar_wait(&kv_full[s1], ((j + 1) >> 1) & 1, p.status, kErrAttnWait);
-          if (!ok) break;
-          tc_fence_after_sync();
-          mma_128<false, false>(tS0 + s1 * 128, smem_u32(sQ), smem_u32(sKV + s1 * 2 * kTile), false);
-          tc_commit(&s_full[s1]);
-        }
-        ok = mbar_wait(p_full, j & 1, p.status, kErrAttnWait);       // P in smem, O rescaled
-        if (!ok) break;
-        tc_fence_after_sync();
-        mma_128<false, true>(tO, smem_u32(sP), k_tile + kTile, j > 0);  // O += P V
-        tc_commit(&kv_empty[s]);
-        tc_commit(o_done);
+      __syncwarp();
+      ok = mbar_wait_warp(p_full, j & 1, p.status, kErrAttnWait) &&  // P in TMEM, O rescaled
+           mbar_wait_warp(v_full, j & 1, p.status, kErrAttnWait);
+      if (!ok) break;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        mma_ts(tO, tS, 32, aV, j > 0);                               // O += P V
+        tc_commit(v_empty);
+        if (j + 1 == n_kv) tc_commit(o_done);
       }
-      if (!ok) {  // let the softmax warps fall through their bounded waits quickly
-        tc_commit(&s_full[0]);
-        tc_commit(&s_full[1]);
-        tc_commit(o_done);
-      }
+      __syncwarp();
     }
   } else {
     const int q = warp & 3;
@@ -206,110 +249,115 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < n_kv && ok; ++j) {
-      ok = mbar_wait(&s_full[j & 1], (j >> 1) & 1, p.status, kErrAttnWait);
-      if (!ok) break;
-      tc_fence_after_sync();
-      const uint32_t tS = tS0 + (j & 1) * 128;
-      const bool diag = (j == qb);
-      // the whole score row (128 fp32) is read from TMEM once and kept in registers: four loads in
-      // flight, one wait, no second pass over TMEM for the exponentials
-      uint32_t sv[128];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld_32x32(tS + lane_base + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&sv[c * 32]));
-      tmem_ld_wait();
-      // the block's 128 key-mask bits: one 16-byte load per thread (same address for the whole
-      // warp), and a block with every key visible takes the mask-free path
+      // the block's 128 key-mask bits (one 16-byte load, the same address for the whole warp), cut
+      // at the diagonal; a block with every key visible takes the mask-free path
       uint32_t mw[4];
       load_key_bits(p.key_bits, p.bits_pitch, p.key_mask, p.seq, b, j, mw);
-      const bool all_on = (mw[0] & mw[1] & mw[2] & mw[3]) == 0xffffffffu;
-      const bool plain = !diag && all_on;     // every key of the block is visible
-      float mx = -INFINITY;
+      const bool plain = j != qb && (mw[0] & mw[1] & mw[2] & mw[3]) == 0xffffffffu;
+      if (j == qb) {
 #pragma unroll
-      for (int i = 0; i < 128; ++i) {
-        const int kv = j * kBlk + i;
-        const bool keep = plain || ((!diag || kv <= q_idx) && ((mw[i >> 5] >> (i & 31)) & 1u));
-        const float x = keep ? __uint_as_float(sv[i]) * p.scale : -INFINITY;
-        sv[i] = __float_as_uint(x);
-        mx = fmaxf(mx, x);
-      }
-      const float m_new = fmaxf(m, mx);
-      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-      const float alpha = (m == -INFINITY) ? 0.f : __expf(m - m_use);
-      // probabilities, rounded to bf16 and packed (masked scores are -inf: exp gives 0); kept in
-      // registers until the previous P V has released the shared-memory P tile
-      float sum = 0.f;
-      uint32_t pk[64];
-#pragma unroll
-      for (int i = 0; i < 128; i += 2) {
-        const float x0 = __uint_as_float(sv[i]), x1 = __uint_as_float(sv[i + 1]);
-        float e0 = (x0 == -INFINITY) ? 0.f : __expf(x0 - m_use);
-        float e1 = (x1 == -INFINITY) ? 0.f : __expf(x1 - m_use);
-        // sum what the tensor core will see (bf16-rounded), as the normaliser
-        e0 = __bfloat162float(__float2bfloat16(e0));
-        e1 = __bfloat162float(__float2bfloat16(e1));
-        sum += e0 + e1;
-        pk[i >> 1] = pack_bf16x2(e0, e1);
-      }
-      if (j > 0) {
-        // previous P V finished (o_done), so O may be rescaled in place and P overwritten; the
-        // score registers are dead by now, so the whole O row (128 fp32) fits in registers
-        ok = mbar_wait(o_done, (j - 1) & 1, p.status, kErrAttnWait);
-        tc_fence_after_sync();
-        if (__any_sync(0xffffffffu, alpha != 1.f)) {
-          uint32_t ov[128];
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            tmem_ld_32x32(tO + lane_base + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&ov[c * 32]));
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 128; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            tmem_st_32x32(tO + lane_base + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&ov[c * 32]));
-          tmem_st_wait();
+        for (int c = 0; c < 4; ++c) {
+          const int n = r + 1 - c * 32;          // keys c*32 .. of this row up to its own position
+          mw[c] &= n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u);
         }
       }
+      ok = __all_sync(0xffffffffu, mbar_wait(s_full, j & 1, p.status, kErrAttnWait));
+      if (!ok) break;
+      tc_fence_after_sync();                      // also: P V of block j-1 is done (issue order)
+      float alpha = 1.f, sum = 0.f;
+      auto block = [&](auto masked) {
+        constexpr bool kMasked = decltype(masked)::value;
+        float mx = -INFINITY;
 #pragma unroll
-      for (int g = 0; g < 16; ++g)
-        store_row8(sP, r, g, make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]));
+        for (int g = 0; g < 2; ++g) {
+          uint32_t s[64];
+          tmem_ld_32x32(tS + lane_base + g * 64, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
+          tmem_ld_32x32(tS + lane_base + g * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&s[32]));
+          tmem_ld_wait();
+          float part[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains of maxima
+#pragma unroll
+          for (int i = 0; i < 64; ++i) {
+            float x = __uint_as_float(s[i]) * p.scale;
+            if (kMasked) x = ((mw[g * 2 + (i >> 5)] >> (i & 31)) & 1u) ? x : -INFINITY;
+            part[i & 3] = fmaxf(part[i & 3], x);
+          }
+          mx = fmaxf(mx, fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3])));
+        }
+        const float m_new = fmaxf(m, mx);
+        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+        alpha = (m == -INFINITY) ? 0.f : __expf(m - m_use);
+        m = m_new;
+        // probabilities, rounded to bf16: what the tensor core will see is also what is summed
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t s[32], pk[16];
+          tmem_ld_32x32(tS + lane_base + c * 32, s);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            float x0 = __uint_as_float(s[i]) * p.scale, x1 = __uint_as_float(s[i + 1]) * p.scale;
+            if (kMasked) {
+              x0 = ((mw[c] >> i) & 1u) ? x0 : -INFINITY;            // exp gives 0
+              x1 = ((mw[c] >> (i + 1)) & 1u) ? x1 : -INFINITY;
+            }
+            // (rounded product minus m_use: no multiply-add, so both paths round alike)
+            const uint32_t e = pack_bf16x2(__expf(__fadd_rn(x0, -m_use)), __expf(__fadd_rn(x1, -m_use)));
+            pk[i >> 1] = e;
+            sum += __uint_as_float(e << 16) + __uint_as_float(e & 0xffff0000u);
+          }
+          // columns 16 c .. of S, read above, make room for P
+          tmem_st_32x16(tS + lane_base + c * 16, pk);
+        }
+      };
+      if (plain)
+        block(std::false_type{});
+      else
+        block(std::true_type{});
+      if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+          uint32_t o[64];
+          tmem_ld_32x32(tO + lane_base + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&o[0]));
+          tmem_ld_32x32(tO + lane_base + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&o[32]));
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 64; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st_32x32(tO + lane_base + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&o[0]));
+          tmem_st_32x32(tO + lane_base + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&o[32]));
+        }
+      }
       l = l * alpha + sum;
-      m = m_new;
+      tmem_st_wait();
       tc_fence_before_sync();
-      fence_proxy_async();   // generic-proxy writes of P must be visible to the MMA's async proxy
       mbar_arrive(p_full);
     }
-    // epilogue: O / l -> bf16
-    if (ok) ok = mbar_wait(o_done, (n_kv - 1) & 1, p.status, kErrAttnWait);
+    // epilogue: O / l -> bf16, through the Q tile (every S = Q K^T is done with it)
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(o_done, 0, p.status, kErrAttnWait));
     tc_fence_after_sync();
     const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
-    const bool store = ok && q_idx < p.seq;
-    __nv_bfloat16* orow = p.out + (static_cast<int64_t>(row0 + q_idx) * p.hq + h) * kD;
+    const RowStager rows{sQ + q * 8192, lane};
 #pragma unroll 1
     for (int c = 0; c < 4; ++c) {
       uint32_t v[32];
       tmem_ld_32x32(tO + lane_base + c * 32, v);
       tmem_ld_wait();
-      if (store) {
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 pk;
-          pk.x = pack_bf16x2(__uint_as_float(v[8 * g]) * inv_l, __uint_as_float(v[8 * g + 1]) * inv_l);
-          pk.y = pack_bf16x2(__uint_as_float(v[8 * g + 2]) * inv_l, __uint_as_float(v[8 * g + 3]) * inv_l);
-          pk.z = pack_bf16x2(__uint_as_float(v[8 * g + 4]) * inv_l, __uint_as_float(v[8 * g + 5]) * inv_l);
-          pk.w = pack_bf16x2(__uint_as_float(v[8 * g + 6]) * inv_l, __uint_as_float(v[8 * g + 7]) * inv_l);
-          *reinterpret_cast<uint4*>(orow + c * 32 + g * 8) = pk;
-        }
-      }
+      for (int g = 0; g < 4; ++g) rows.put(c * 4 + g, pack8(&v[8 * g], inv_l));
     }
-    if (store)
-      p.lse[(static_cast<int64_t>(b) * p.hq + h) * p.seq + q_idx] = (l > 0.f) ? m + __logf(l) : 0.f;
+    const int first = qb * kBlk + q * 32;
+    if (ok) {
+      rows.flush(p.out + (static_cast<int64_t>(row0 + first) * p.hq + h) * kD,
+                 static_cast<int64_t>(p.hq) * kD, min(32, p.seq - first));
+      if (q_idx < p.seq)
+        p.lse[(static_cast<int64_t>(b) * p.hq + h) * p.seq + q_idx] = (l > 0.f) ? m + __logf(l) : 0.f;
+    }
   }
 
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem, 512);
+    tmem_dealloc(tmem, 256);
   }
 }
 
@@ -355,10 +403,17 @@ struct BwdParams {
 // ---------------------------------------------------------------------------- dQ
 // One CTA per (query block, query head, batch).  Per key block j <= i:
 //   S = Q K^T, dP = dO V^T  ->  dS = P * (dP - delta) * scale  ->  dQ += dS K.
-// smem: Q | dO | K | V | dS | barriers
-constexpr int kDqSmem = 5 * kTile + 1024 + 256;
+// S is double buffered in TMEM and dS (bf16) is written over the S it came from, each half row into
+// its own 64 columns, and read by the MMA as a TMEM operand.  While the softmax warps work on block
+// j, S(j+1) runs; when they are done, dP(j+1) goes first and dQ += dS(j) K(j) and S(j+2) run under
+// the softmax of block j+1, so the chain of a block is dP and half a row of exponentials per
+// thread.  K has three stages (K(j) is held until dQ), V two.
+// Measured on B200 inside a training step (12 heads): 1 x 8192: 764 us before (serial chain, one
+// thread per row, MMAs issued from one lane) and 371 us now; 8 x 512: 51 and 38 us.
+// smem: Q | dO | K x 3 | V x 2 | barriers
+constexpr int kDqSmem = 7 * kTile + 1024 + 256;
 
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kBwdThreads, 1)
 attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
                     const __grid_constant__ CUtensorMap map_do, BwdParams p) {
   if (kernel_should_skip(p.status)) return;   // an earlier kernel already failed
@@ -367,31 +422,34 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sQ = smem;
   uint8_t* sdO = sQ + kTile;
-  uint8_t* sK = sdO + kTile;
-  uint8_t* sV = sK + kTile;
-  uint8_t* sdS = sV + kTile;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sdS + kTile);
+  uint8_t* sK = sdO + kTile;          // 3 stages
+  uint8_t* sV = sK + 3 * kTile;       // 2 stages
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * kTile);
   uint64_t* q_full = bars;
-  uint64_t* kv_full = bars + 1;
-  uint64_t* kv_empty = bars + 2;
-  uint64_t* sdp_full = bars + 3;
-  uint64_t* ds_full = bars + 4;   // 128 arrivals
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
+  uint64_t* sdp_full = bars + 1;
+  uint64_t* ds_full = bars + 2;   // 256 arrivals
+  uint64_t* dq_done = bars + 3;
+  uint64_t* k_full = bars + 4;    // 3
+  uint64_t* k_empty = bars + 7;   // 3
+  uint64_t* v_full = bars + 10;   // 2
+  uint64_t* v_empty = bars + 12;  // 2
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qb = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int nblk = (p.seq + kBlk - 1) / kBlk;
+  const int qb = nblk - 1 - static_cast<int>(blockIdx.x) / (p.hq * p.batch);   // long rows first
+  const int hb = static_cast<int>(blockIdx.x) % (p.hq * p.batch);
+  const int h = hb % p.hq, b = hb / p.hq;
   const int hk = h / (p.hq / p.hkv);
   const int n_kv = qb + 1;
   const int row0 = b * p.seq;
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    mbar_init(kv_full, 1);
-    mbar_init(kv_empty, 1);
-    mbar_init(sdp_full, 1);
-    mbar_init(ds_full, 128);
+    for (int i = 0; i < 14; ++i) mbar_init(bars + i, i == 2 ? 256 : 1);
     fence_barrier_init();
     fence_proxy_async();
+    prefetch_tensormap(&map_qkv);
+    prefetch_tensormap(&map_do);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -401,40 +459,69 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tS = tmem, tdP = tmem + 128, tdQ = tmem + 256;
+  const uint32_t tS = tmem, tdP = tmem + 256, tdQ = tmem + 384;   // S: two buffers
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, 2 * kTile);
       load_tile(sQ, &map_qkv, q_full, h * kD, row0 + qb * kBlk);
       load_tile(sdO, &map_do, q_full, h * kD, row0 + qb * kBlk);
-      for (int j = 0; j < n_kv; ++j) {
-        if (!mbar_wait(kv_empty, (j & 1) ^ 1, p.status, kErrAttnWait)) break;
-        mbar_expect_tx(kv_full, 2 * kTile);
-        load_tile(sK, &map_qkv, kv_full, (p.hq + hk) * kD, row0 + j * kBlk);
-        load_tile(sV, &map_qkv, kv_full, (p.hq + p.hkv + hk) * kD, row0 + j * kBlk);
+    }
+    __syncwarp();
+    for (int j = 0; j < n_kv; ++j) {
+      const int ks = j % 3, vs = j & 1;
+      if (!mbar_wait_warp(&k_empty[ks], ((j / 3) & 1) ^ 1, p.status, kErrAttnWait)) break;
+      if (elect_one()) {
+        mbar_expect_tx(&k_full[ks], kTile);
+        load_tile(sK + ks * kTile, &map_qkv, &k_full[ks], (p.hq + hk) * kD, row0 + j * kBlk);
       }
+      __syncwarp();
+      if (!mbar_wait_warp(&v_empty[vs], ((j >> 1) & 1) ^ 1, p.status, kErrAttnWait)) break;
+      if (elect_one()) {
+        mbar_expect_tx(&v_full[vs], kTile);
+        load_tile(sV + vs * kTile, &map_qkv, &v_full[vs], (p.hq + p.hkv + hk) * kD, row0 + j * kBlk);
+      }
+      __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = mbar_wait(q_full, 0, p.status, kErrAttnWait);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        ok = mbar_wait(kv_full, j & 1, p.status, kErrAttnWait);
-        if (!ok) break;
-        tc_fence_after_sync();
-        mma_128<false, false>(tS, smem_u32(sQ), smem_u32(sK), false);    // S  = Q  K^T
-        mma_128<false, false>(tdP, smem_u32(sdO), smem_u32(sV), false);  // dP = dO V^T
+    const uint32_t aQ = smem_u32(sQ), adO = smem_u32(sdO), aK = smem_u32(sK), aV = smem_u32(sV);
+    auto scores = [&](int j) {        // S(j) = Q K(j)^T
+      if (!mbar_wait_warp(&k_full[j % 3], (j / 3) & 1, p.status, kErrAttnWait)) return false;
+      tc_fence_after_sync();
+      if (elect_one()) mma_ss(tS + (j & 1) * 128, aQ, aK + (j % 3) * kTile);
+      __syncwarp();
+      return true;
+    };
+    auto dprobs = [&](int j) {        // dP(j) = dO V(j)^T; with it S(j), issued earlier, is complete too
+      if (!mbar_wait_warp(&v_full[j & 1], (j >> 1) & 1, p.status, kErrAttnWait)) return false;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        mma_ss(tdP, adO, aV + (j & 1) * kTile);
+        tc_commit(&v_empty[j & 1]);
         tc_commit(sdp_full);
-        ok = mbar_wait(ds_full, j & 1, p.status, kErrAttnWait);
-        if (!ok) break;
-        tc_fence_after_sync();
-        mma_128<false, true>(tdQ, smem_u32(sdS), smem_u32(sK), j > 0);   // dQ += dS K
-        tc_commit(kv_empty);
       }
-      if (!ok) tc_commit(sdp_full);
+      __syncwarp();
+      return true;
+    };
+    bool ok = mbar_wait_warp(q_full, 0, p.status, kErrAttnWait);
+    ok = ok && scores(0) && dprobs(0);
+    if (ok && n_kv > 1) ok = scores(1);
+    for (int j = 0; j < n_kv && ok; ++j) {
+      ok = mbar_wait_warp(ds_full, j & 1, p.status, kErrAttnWait);   // dS(j) written, dP(j) read
+      if (!ok) break;
+      tc_fence_after_sync();
+      if (j + 1 < n_kv) ok = dprobs(j + 1);
+      if (!ok) break;
+      if (elect_one()) {
+        mma_ts(tdQ, tS + (j & 1) * 128, 64, aK + (j % 3) * kTile, j > 0);   // dQ += dS K
+        tc_commit(&k_empty[j % 3]);
+        if (j + 1 == n_kv) tc_commit(dq_done);
+      }
+      __syncwarp();
+      if (j + 2 < n_kv) ok = scores(j + 2);     // over dS(j), which the MMA before has read
     }
   } else {
-    const int q = warp & 3;
+    const int q = warp & 3, half = (warp - 2) >> 2;   // rows 32 q .., columns 64 half ..
     const int r = q * 32 + lane;
     const int q_idx = qb * kBlk + r;
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
@@ -443,61 +530,68 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
     const float lse = p.lse[stat], dlt = p.delta[stat];
     bool ok = true;
     for (int j = 0; j < n_kv && ok; ++j) {
-      ok = mbar_wait(sdp_full, j & 1, p.status, kErrAttnWait);
-      if (!ok) break;
-      tc_fence_after_sync();
-      const bool diag = (j == qb);
       uint32_t mw[4];
       load_key_bits(p.key_bits, p.bits_pitch, p.key_mask, p.seq, b, j, mw);
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t s[32], d[32];
-        tmem_ld_32x32(tS + lane_base + c * 32, s);
-        tmem_ld_32x32(tdP + lane_base + c * 32, d);
-        tmem_ld_wait();
-        float ds[32];
-        const uint32_t word = mw[c];
+      uint32_t word[2];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int kv = j * kBlk + c * 32 + i;
-          const bool keep = q_ok && (!diag || kv <= q_idx) && ((word >> i) & 1u);
-          const float pr = keep ? __expf(__uint_as_float(s[i]) * p.scale - lse) : 0.f;
-          ds[i] = pr * (__uint_as_float(d[i]) - dlt) * p.scale;
+      for (int c = 0; c < 2; ++c) {
+        word[c] = half ? mw[2 + c] : mw[c];
+        if (j == qb) {
+          const int n = r + 1 - (half * 64 + c * 32);
+          word[c] &= n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u);
         }
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 pk;
-          pk.x = pack_bf16x2(ds[8 * g], ds[8 * g + 1]);
-          pk.y = pack_bf16x2(ds[8 * g + 2], ds[8 * g + 3]);
-          pk.z = pack_bf16x2(ds[8 * g + 4], ds[8 * g + 5]);
-          pk.w = pack_bf16x2(ds[8 * g + 6], ds[8 * g + 7]);
-          store_row8(sdS, r, c * 4 + g, pk);
-        }
+        if (!q_ok) word[c] = 0;
       }
+      ok = __all_sync(0xffffffffu, mbar_wait(sdp_full, j & 1, p.status, kErrAttnWait));
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint32_t tSj = tS + (j & 1) * 128 + lane_base + half * 64;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t s[32], d[32], pk[16];
+        tmem_ld_32x32(tSj + c * 32, s);
+        tmem_ld_32x32(tdP + lane_base + half * 64 + c * 32, d);
+        tmem_ld_wait();
+        const bool all_on = __all_sync(0xffffffffu, word[c] == 0xffffffffu);
+        float ds[32];
+        if (all_on) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float pr = __expf(__uint_as_float(s[i]) * p.scale - lse);
+            ds[i] = pr * (__uint_as_float(d[i]) - dlt) * p.scale;
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float pr =
+                ((word[c] >> i) & 1u) ? __expf(__uint_as_float(s[i]) * p.scale - lse) : 0.f;
+            ds[i] = pr * (__uint_as_float(d[i]) - dlt) * p.scale;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(ds[2 * i], ds[2 * i + 1]);
+        tmem_st_32x16(tSj + c * 16, pk);
+      }
+      tmem_st_wait();
       tc_fence_before_sync();
-      fence_proxy_async();
       mbar_arrive(ds_full);
     }
-    // dQ is complete once the last dS K product has retired (kv_empty's last phase)
-    if (ok) ok = mbar_wait(kv_empty, (n_kv - 1) & 1, p.status, kErrAttnWait);
+    // dQ is complete; it leaves through the K stages, which nothing reads any more
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(dq_done, 0, p.status, kErrAttnWait));
     tc_fence_after_sync();
-    __nv_bfloat16* drow = p.dqkv + static_cast<int64_t>(row0 + q_idx) * (p.hq + 2 * p.hkv) * kD + h * kD;
+    if (half == 0) {
+      const RowStager rows{sK + q * 8192, lane};
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
-      uint32_t v[32];
-      tmem_ld_32x32(tdQ + lane_base + c * 32, v);
-      tmem_ld_wait();
-      if (ok && q_ok) {
+      for (int c = 0; c < 4; ++c) {
+        uint32_t v[32];
+        tmem_ld_32x32(tdQ + lane_base + c * 32, v);
+        tmem_ld_wait();
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 pk;
-          pk.x = pack_bf16x2(__uint_as_float(v[8 * g]), __uint_as_float(v[8 * g + 1]));
-          pk.y = pack_bf16x2(__uint_as_float(v[8 * g + 2]), __uint_as_float(v[8 * g + 3]));
-          pk.z = pack_bf16x2(__uint_as_float(v[8 * g + 4]), __uint_as_float(v[8 * g + 5]));
-          pk.w = pack_bf16x2(__uint_as_float(v[8 * g + 6]), __uint_as_float(v[8 * g + 7]));
-          *reinterpret_cast<uint4*>(drow + c * 32 + g * 8) = pk;
-        }
+        for (int g = 0; g < 4; ++g) rows.put(c * 4 + g, pack8(&v[8 * g]));
       }
+      const int first = qb * kBlk + q * 32;
+      const int64_t width = static_cast<int64_t>(p.hq + 2 * p.hkv) * kD;
+      if (ok) rows.flush(p.dqkv + static_cast<int64_t>(row0 + first) * width + h * kD, width, min(32, p.seq - first));
     }
   }
   tc_fence_before_sync();
@@ -514,13 +608,20 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
 // With parts == 1 the CTA owns the whole group and writes bf16 dK / dV; with parts > 1 (small
 // batches would otherwise leave most SMs idle) each part writes an fp32 partial plane and
 // attention_dkv_finish_kernel adds the planes in a fixed order.
-// Scores are formed transposed (rows = keys): S^T = K Q^T, dP^T = V dO^T, so each softmax thread
-// owns one key row and writes P^T / dS^T rows directly as K-major operands of
+// Scores are formed transposed (rows = keys): S^T = K Q^T, dP^T = V dO^T, so a softmax thread owns
+// half a key row and P^T / dS^T rows are K-major operands of
 //   dV += P^T dO,   dK += dS^T Q.
-// smem: K | V | Q | dO | P^T | dS^T | lse[128] delta[128] | barriers
-constexpr int kDkvSmem = 6 * kTile + 1024 + 1024 + 256;
+// P^T and dS^T (bf16) are written over the S^T and dP^T they came from, each half row into its own 64
+// columns, and read by the MMAs from TMEM.  The two chains S^T -> P^T -> dV and dP^T -> dS^T -> dK
+// hand over separately: while the softmax warps take exponentials of block t+1, dK(t) and dP^T(t+1)
+// run, and while they form dS^T(t+1), dV(t+1) and S^T(t+2) run.  Q and dO have two stages.
+// Bound by the four products (2048 clocks a block).
+// Measured on B200 inside a training step (12 heads, 2 kv heads): 1 x 8192: 1188 us before (serial
+// chain, P^T and dS^T through shared memory, one thread per row) and 507 us now; 8 x 512: 80 and 42 us.
+// smem: K | V | (Q, dO) x 2 | (lse[128], delta[128]) x 2 | barriers
+constexpr int kDkvSmem = 6 * kTile + 2048 + 1024 + 256;
 
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kBwdThreads, 1)
 attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
                      const __grid_constant__ CUtensorMap map_do, BwdParams p) {
   if (kernel_should_skip(p.status)) return;   // an earlier kernel already failed
@@ -529,38 +630,38 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sK = smem;
   uint8_t* sV = sK + kTile;
-  uint8_t* sQ = sV + kTile;
-  uint8_t* sdO = sQ + kTile;
-  uint8_t* sPT = sdO + kTile;
-  uint8_t* sdST = sPT + kTile;
-  float* s_lse = reinterpret_cast<float*>(sdST + kTile);
-  float* s_dlt = s_lse + 128;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_dlt + 128);
+  uint8_t* sQ = sV + kTile;                     // stage s: Q at sQ + s * 2 * kTile, dO right after
+  float* s_stat = reinterpret_cast<float*>(sQ + 4 * kTile);   // buffer s: lse at s * 256, delta + 128
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_stat + 512);
   uint64_t* kv_full = bars;
-  uint64_t* q_full = bars + 1;
-  uint64_t* q_empty = bars + 2;
-  uint64_t* st_full = bars + 3;
-  uint64_t* pt_full = bars + 4;   // 128 arrivals
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
+  uint64_t* s_full = bars + 1;
+  uint64_t* dp_full = bars + 2;
+  uint64_t* pt_full = bars + 3;   // 256 arrivals
+  uint64_t* ds_full = bars + 4;   // 256 arrivals
+  uint64_t* done = bars + 5;
+  uint64_t* q_full = bars + 6;    // 2
+  uint64_t* q_empty = bars + 8;   // 2
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kb = blockIdx.x, hk = blockIdx.y / p.parts, part = blockIdx.y % p.parts, b = blockIdx.z;
+  const int n_q = (p.seq + kBlk - 1) / kBlk;
+  const int kb = static_cast<int>(blockIdx.x) / (p.hkv * p.parts * p.batch);   // long loops first
+  const int rest = static_cast<int>(blockIdx.x) % (p.hkv * p.parts * p.batch);
+  const int b = rest / (p.hkv * p.parts);
+  const int hk = rest % (p.hkv * p.parts) / p.parts, part = rest % p.parts;
   const int group = p.hq / p.hkv;
   const int heads_here = group / p.parts;   // parts divides group (checked on the host)
   const int head0 = hk * group + part * heads_here;
-  const int n_q = (p.seq + kBlk - 1) / kBlk;
   const int per_head = n_q - kb;          // query blocks kb .. n_q-1
   const int iters = heads_here * per_head;
   const int row0 = b * p.seq;
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
-    mbar_init(q_full, 1);
-    mbar_init(q_empty, 1);
-    mbar_init(st_full, 1);
-    mbar_init(pt_full, 128);
+    for (int i = 0; i < 10; ++i) mbar_init(bars + i, i == 3 || i == 4 ? 256 : 1);
     fence_barrier_init();
     fence_proxy_async();
+    prefetch_tensormap(&map_qkv);
+    prefetch_tensormap(&map_do);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -573,40 +674,70 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
   const uint32_t tST = tmem, tdPT = tmem + 128, tdV = tmem + 256, tdK = tmem + 384;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * kTile);
       load_tile(sK, &map_qkv, kv_full, (p.hq + hk) * kD, row0 + kb * kBlk);
       load_tile(sV, &map_qkv, kv_full, (p.hq + p.hkv + hk) * kD, row0 + kb * kBlk);
-      for (int t = 0; t < iters; ++t) {
-        const int h = head0 + t / per_head;
-        const int i = kb + t % per_head;
-        if (!mbar_wait(q_empty, (t & 1) ^ 1, p.status, kErrAttnWait)) break;
-        mbar_expect_tx(q_full, 2 * kTile);
-        load_tile(sQ, &map_qkv, q_full, h * kD, row0 + i * kBlk);
-        load_tile(sdO, &map_do, q_full, h * kD, row0 + i * kBlk);
+    }
+    __syncwarp();
+    for (int t = 0; t < iters; ++t) {
+      const int h = head0 + t / per_head;
+      const int i = kb + t % per_head;
+      const int s = t & 1;
+      if (!mbar_wait_warp(&q_empty[s], ((t >> 1) & 1) ^ 1, p.status, kErrAttnWait)) break;
+      if (elect_one()) {
+        mbar_expect_tx(&q_full[s], 2 * kTile);
+        load_tile(sQ + s * 2 * kTile, &map_qkv, &q_full[s], h * kD, row0 + i * kBlk);
+        load_tile(sQ + s * 2 * kTile + kTile, &map_do, &q_full[s], h * kD, row0 + i * kBlk);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = mbar_wait(kv_full, 0, p.status, kErrAttnWait);
-      for (int t = 0; t < iters && ok; ++t) {
-        ok = mbar_wait(q_full, t & 1, p.status, kErrAttnWait);
-        if (!ok) break;
-        tc_fence_after_sync();
-        mma_128<false, false>(tST, smem_u32(sK), smem_u32(sQ), false);    // S^T  = K Q^T
-        mma_128<false, false>(tdPT, smem_u32(sV), smem_u32(sdO), false);  // dP^T = V dO^T
-        tc_commit(st_full);
-        ok = mbar_wait(pt_full, t & 1, p.status, kErrAttnWait);
-        if (!ok) break;
-        tc_fence_after_sync();
-        mma_128<false, true>(tdV, smem_u32(sPT), smem_u32(sdO), t > 0);   // dV += P^T dO
-        mma_128<false, true>(tdK, smem_u32(sdST), smem_u32(sQ), t > 0);   // dK += dS^T Q
-        tc_commit(q_empty);
+    const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ);
+    bool ok = mbar_wait_warp(kv_full, 0, p.status, kErrAttnWait) &&
+              mbar_wait_warp(&q_full[0], 0, p.status, kErrAttnWait);
+    if (ok) {
+      tc_fence_after_sync();
+      if (elect_one()) {
+        mma_ss(tST, aK, aQ);                      // S^T  = K Q^T
+        tc_commit(s_full);
+        mma_ss(tdPT, aV, aQ + kTile);             // dP^T = V dO^T
+        tc_commit(dp_full);
       }
-      if (!ok) tc_commit(st_full);
+      __syncwarp();
+    }
+    for (int t = 0; t < iters && ok; ++t) {
+      const uint32_t q_t = aQ + (t & 1) * 2 * kTile, q_n = aQ + ((t + 1) & 1) * 2 * kTile;
+      const bool more = t + 1 < iters;
+      ok = mbar_wait_warp(pt_full, t & 1, p.status, kErrAttnWait);
+      if (ok && more) ok = mbar_wait_warp(&q_full[(t + 1) & 1], ((t + 1) >> 1) & 1, p.status, kErrAttnWait);
+      if (!ok) break;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        mma_ts(tdV, tST, 64, q_t + kTile, t > 0);           // dV += P^T dO
+        if (more) {
+          mma_ss(tST, aK, q_n);                             // S^T(t+1), over the P^T just read
+          tc_commit(s_full);
+        }
+      }
+      __syncwarp();
+      ok = mbar_wait_warp(ds_full, t & 1, p.status, kErrAttnWait);
+      if (!ok) break;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        mma_ts(tdK, tdPT, 64, q_t, t > 0);                  // dK += dS^T Q
+        tc_commit(&q_empty[t & 1]);
+        if (more) {
+          mma_ss(tdPT, aV, q_n + kTile);                    // dP^T(t+1), over the dS^T just read
+          tc_commit(dp_full);
+        } else {
+          tc_commit(done);
+        }
+      }
+      __syncwarp();
     }
   } else {
-    const int q = warp & 3;
+    const int q = warp & 3, half = (warp - 2) >> 2;
     const int r = q * 32 + lane;              // key row inside the tile
     const int kv_idx = kb * kBlk + r;
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
@@ -615,99 +746,125 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
       kv_ok = (p.key_bits[static_cast<int64_t>(b) * p.bits_pitch + (kv_idx >> 5)] >> (kv_idx & 31)) & 1u;
     else if (kv_ok && p.key_mask != nullptr)
       kv_ok = p.key_mask[b * p.seq + kv_idx] != 0;
+    // this thread's share of a query block's statistics: lse (half 0) or delta (half 1) of query r
+    const float* stats = half ? p.delta : p.lse;
+    auto stat_of = [&](int t) {
+      const int h = head0 + t / per_head;
+      const int qi = (kb + t % per_head) * kBlk + r;
+      return stats[(static_cast<int64_t>(b) * p.hq + h) * p.seq + min(qi, p.seq - 1)];
+    };
+    float* mine = s_stat + half * 128 + r;
+    mine[0] = stat_of(0);
+    asm volatile("bar.sync 1, 256;" ::: "memory");
     bool ok = true;
     for (int t = 0; t < iters; ++t) {
-      const int h = head0 + t / per_head;
-      const int i = kb + t % per_head;
-      softmax_bar();  // everyone finished reading the previous block's lse / delta
-      {
-        const int qi = i * kBlk + r;
-        const int64_t stat = (static_cast<int64_t>(b) * p.hq + h) * p.seq + min(qi, p.seq - 1);
-        s_lse[r] = p.lse[stat];
-        s_dlt[r] = p.delta[stat];
+      const float next = t + 1 < iters ? stat_of(t + 1) : 0.f;
+      const float* lse = s_stat + (t & 1) * 256 + half * 64;
+      const float* dlt = lse + 128;
+      const int q0 = (kb + t % per_head) * kBlk + half * 64;   // first query of this half
+      // queries from the key's own position to the end of the sequence, as bits
+      uint32_t word[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int from = kv_idx - (q0 + c * 32), to = p.seq - (q0 + c * 32);
+        uint32_t w = kv_ok ? 0xffffffffu : 0u;
+        if (from > 0) w = from >= 32 ? 0u : w & (0xffffffffu << from);
+        if (to < 32) w = to <= 0 ? 0u : w & ((1u << to) - 1u);
+        word[c] = w;
       }
-      softmax_bar();
       // after a failed wait the loop keeps its shape (no early exit) so that every thread
-      // still reaches the named barriers above the same number of times
-      if (ok) ok = mbar_wait(st_full, t & 1, p.status, kErrAttnWait);
+      // still reaches the named barrier below the same number of times
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(s_full, t & 1, p.status, kErrAttnWait));
       tc_fence_after_sync();
+      float pr[64];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t s[32], pk[16];
+        tmem_ld_32x32(tST + lane_base + half * 64 + c * 32, s);
+        tmem_ld_wait();
+        const bool all_on = __all_sync(0xffffffffu, word[c] == 0xffffffffu);
+#pragma unroll
+        for (int x = 0; x < 32; x += 4) {
+          const float4 l4 = *reinterpret_cast<const float4*>(lse + c * 32 + x);
+          const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            pr[c * 32 + x + u] = __expf(__uint_as_float(s[x + u]) * p.scale - lv[u]);
+        }
+        if (!all_on) {
+#pragma unroll
+          for (int x = 0; x < 32; ++x) pr[c * 32 + x] = ((word[c] >> x) & 1u) ? pr[c * 32 + x] : 0.f;
+        }
+#pragma unroll
+        for (int x = 0; x < 16; ++x) pk[x] = pack_bf16x2(pr[c * 32 + 2 * x], pr[c * 32 + 2 * x + 1]);
+        tmem_st_32x16(tST + lane_base + half * 64 + c * 16, pk);
+      }
+      tmem_st_wait();
+      tc_fence_before_sync();
+      mbar_arrive(pt_full);
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(dp_full, t & 1, p.status, kErrAttnWait));
+      tc_fence_after_sync();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t d[32], pk[16];
+        tmem_ld_32x32(tdPT + lane_base + half * 64 + c * 32, d);
+        tmem_ld_wait();
+#pragma unroll
+        for (int x = 0; x < 32; x += 4) {
+          const float4 d4 = *reinterpret_cast<const float4*>(dlt + c * 32 + x);
+          const float dv[4] = {d4.x, d4.y, d4.z, d4.w};
+          float ds[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            ds[u] = pr[c * 32 + x + u] * (__uint_as_float(d[x + u]) - dv[u]) * p.scale;
+          pk[x >> 1] = pack_bf16x2(ds[0], ds[1]);
+          pk[(x >> 1) + 1] = pack_bf16x2(ds[2], ds[3]);
+        }
+        tmem_st_32x16(tdPT + lane_base + half * 64 + c * 16, pk);
+      }
+      tmem_st_wait();
+      tc_fence_before_sync();
+      mbar_arrive(ds_full);
+      // the other buffer's readers (iteration t - 1) passed the last barrier
+      mine[((t + 1) & 1) * 256] = next;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(done, 0, p.status, kErrAttnWait));
+    tc_fence_after_sync();
+    // half 0 writes dK, half 1 dV
+    const int first = kb * kBlk + q * 32;
+    const uint32_t acc = half ? tdV : tdK;
+    if (p.parts > 1) {
+      const int64_t pwidth = static_cast<int64_t>(2 * p.hkv) * kD;
+      float* row = p.dkv_part + (static_cast<int64_t>(part) * p.batch * p.seq + row0 + kv_idx) * pwidth +
+                   (half * p.hkv + hk) * kD;
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
-        uint32_t s[32], d[32];
-        tmem_ld_32x32(tST + lane_base + c * 32, s);
-        tmem_ld_32x32(tdPT + lane_base + c * 32, d);
+        uint32_t v[32];
+        tmem_ld_32x32(acc + lane_base + c * 32, v);
         tmem_ld_wait();
-        float pt[32], ds[32];
+        if (ok && kv_idx < p.seq) {
 #pragma unroll
-        for (int x = 0; x < 32; ++x) {
-          const int col = c * 32 + x;
-          const int qi = i * kBlk + col;
-          const bool keep = kv_ok && qi < p.seq && qi >= kv_idx;
-          const float pr = keep ? __expf(__uint_as_float(s[x]) * p.scale - s_lse[col]) : 0.f;
-          pt[x] = pr;
-          ds[x] = pr * (__uint_as_float(d[x]) - s_dlt[col]) * p.scale;
-        }
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 a, e;
-          a.x = pack_bf16x2(pt[8 * g], pt[8 * g + 1]);
-          a.y = pack_bf16x2(pt[8 * g + 2], pt[8 * g + 3]);
-          a.z = pack_bf16x2(pt[8 * g + 4], pt[8 * g + 5]);
-          a.w = pack_bf16x2(pt[8 * g + 6], pt[8 * g + 7]);
-          e.x = pack_bf16x2(ds[8 * g], ds[8 * g + 1]);
-          e.y = pack_bf16x2(ds[8 * g + 2], ds[8 * g + 3]);
-          e.z = pack_bf16x2(ds[8 * g + 4], ds[8 * g + 5]);
-          e.w = pack_bf16x2(ds[8 * g + 6], ds[8 * g + 7]);
-          store_row8(sPT, r, c * 4 + g, a);
-          store_row8(sdST, r, c * 4 + g, e);
+          for (int g = 0; g < 8; ++g)
+            *reinterpret_cast<uint4*>(row + c * 32 + g * 4) =
+                make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
         }
       }
-      tc_fence_before_sync();
-      fence_proxy_async();
-      mbar_arrive(pt_full);
-    }
-    if (ok) ok = mbar_wait(q_empty, (iters - 1) & 1, p.status, kErrAttnWait);
-    tc_fence_after_sync();
-    const int64_t width = static_cast<int64_t>(p.hq + 2 * p.hkv) * kD;
-    __nv_bfloat16* krow = p.dqkv + (row0 + kv_idx) * width + (p.hq + hk) * kD;
-    __nv_bfloat16* vrow = krow + p.hkv * kD;
-    const bool store = ok && kv_idx < p.seq;
-    const int64_t pwidth = static_cast<int64_t>(2 * p.hkv) * kD;
-    float* pk_row = p.parts > 1
-                        ? p.dkv_part + (static_cast<int64_t>(part) * p.batch * p.seq + row0 + kv_idx) * pwidth +
-                              hk * kD
-                        : nullptr;
+    } else {
+      // through the Q / dO stages, which nothing reads any more
+      const RowStager rows{sQ + (half * 4 + q) * 8192, lane};
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
-      uint32_t dk[32], dv[32];
-      tmem_ld_32x32(tdK + lane_base + c * 32, dk);
-      tmem_ld_32x32(tdV + lane_base + c * 32, dv);
-      tmem_ld_wait();
-      if (store && p.parts > 1) {
-        float* pv_row = pk_row + p.hkv * kD;
+      for (int c = 0; c < 4; ++c) {
+        uint32_t v[32];
+        tmem_ld_32x32(acc + lane_base + c * 32, v);
+        tmem_ld_wait();
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          *reinterpret_cast<uint4*>(pk_row + c * 32 + g * 4) =
-              make_uint4(dk[4 * g], dk[4 * g + 1], dk[4 * g + 2], dk[4 * g + 3]);
-          *reinterpret_cast<uint4*>(pv_row + c * 32 + g * 4) =
-              make_uint4(dv[4 * g], dv[4 * g + 1], dv[4 * g + 2], dv[4 * g + 3]);
-        }
-      } else if (store) {
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 a, e;
-          a.x = pack_bf16x2(__uint_as_float(dk[8 * g]), __uint_as_float(dk[8 * g + 1]));
-          a.y = pack_bf16x2(__uint_as_float(dk[8 * g + 2]), __uint_as_float(dk[8 * g + 3]));
-          a.z = pack_bf16x2(__uint_as_float(dk[8 * g + 4]), __uint_as_float(dk[8 * g + 5]));
-          a.w = pack_bf16x2(__uint_as_float(dk[8 * g + 6]), __uint_as_float(dk[8 * g + 7]));
-          e.x = pack_bf16x2(__uint_as_float(dv[8 * g]), __uint_as_float(dv[8 * g + 1]));
-          e.y = pack_bf16x2(__uint_as_float(dv[8 * g + 2]), __uint_as_float(dv[8 * g + 3]));
-          e.z = pack_bf16x2(__uint_as_float(dv[8 * g + 4]), __uint_as_float(dv[8 * g + 5]));
-          e.w = pack_bf16x2(__uint_as_float(dv[8 * g + 6]), __uint_as_float(dv[8 * g + 7]));
-          *reinterpret_cast<uint4*>(krow + c * 32 + g * 8) = a;
-          *reinterpret_cast<uint4*>(vrow + c * 32 + g * 8) = e;
-        }
+        for (int g = 0; g < 4; ++g) rows.put(c * 4 + g, pack8(&v[8 * g]));
       }
+      const int64_t width = static_cast<int64_t>(p.hq + 2 * p.hkv) * kD;
+      if (ok)
+        rows.flush(p.dqkv + static_cast<int64_t>(row0 + first) * width + (p.hq + half * p.hkv + hk) * kD,
+                   width, min(32, p.seq - first));
     }
   }
   tc_fence_before_sync();
@@ -766,8 +923,8 @@ cudaError_t launch_attention_fwd(const AttnCall& c, int* status, cudaStream_t s)
     return cudaErrorInvalidValue;
   FwdParams p{reinterpret_cast<__nv_bfloat16*>(c.out), c.lse, c.key_mask, c.batch, c.seq, c.hq,
               c.hkv, c.scale, status, c.key_bits, c.key_bits_pitch};
-  dim3 grid((c.seq + kBlk - 1) / kBlk, c.hq, c.batch);
-  attention_fwd_kernel<<<grid, kThreads, kFwdSmem, s>>>(map, p);
+  const int64_t grid = static_cast<int64_t>((c.seq + kBlk - 1) / kBlk) * c.hq * c.batch;
+  attention_fwd_kernel<<<static_cast<unsigned>(grid), kFwdThreads, kFwdSmem, s>>>(map, p);
   count_launch();
   return cudaGetLastError();
 }
@@ -804,10 +961,11 @@ cudaError_t launch_attention_bwd(const AttnBwdCall& c, int* status, cudaStream_t
   BwdParams p{c.lse, c.delta, reinterpret_cast<__nv_bfloat16*>(c.dqkv), c.key_mask, c.batch, c.seq,
               c.hq, c.hkv, c.scale, status, parts > 1 ? c.dkv_accum : nullptr, parts,
               c.key_bits, c.key_bits_pitch};
-  attention_dkv_kernel<<<dim3(nblk, c.hkv * parts, c.batch), kThreads, kDkvSmem, s>>>(map_qkv,
-                                                                                     map_do, p);
+  attention_dkv_kernel<<<static_cast<unsigned>(static_cast<int64_t>(nblk) * c.hkv * parts * c.batch),
+                         kBwdThreads, kDkvSmem, s>>>(map_qkv, map_do, p);
   count_launch();
-  attention_dq_kernel<<<dim3(nblk, c.hq, c.batch), kThreads, kDqSmem, s>>>(map_qkv, map_do, p);
+  attention_dq_kernel<<<static_cast<unsigned>(static_cast<int64_t>(nblk) * c.hq * c.batch), kBwdThreads,
+                        kDqSmem, s>>>(map_qkv, map_do, p);
   count_launch();
   if (parts > 1) {
     const int64_t work = rows * (2 * c.hkv * kD / 8);
