@@ -240,7 +240,7 @@ cudaError_t launch_variant(const GemmCall& c, int* status, cudaStream_t stream) 
   // half cannot spill into the up half) and `gated_out`.
   CUtensorMap tc = ta, tc_up = ta, tc_h = ta;
   ep.staged_store = 0;
-  if (c.staged_store >= 0 && ep.scatter_degree == 0 && !c.accumulate &&
+  if (c.staged_store >= 0 && ep.scatter_degree == 0 &&
       (c.ldo * (c.out_fp32 ? 4 : 2)) % 16 == 0) {
     bool made;
     if (ep.gated_inter > 0) {

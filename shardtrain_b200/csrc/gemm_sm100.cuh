@@ -45,8 +45,9 @@ struct GemmEpilogue {
   int scatter_broadcast;
   // Staged store: the epilogue warps transpose each 32-row band through 128B-swizzled shared
   // memory and hand whole 32 x 128-byte boxes to TMA stores (`tma_c`), instead of every thread
-  // storing 16-byte pieces of its own row.  Set by the launcher for plain bf16 / fp32 outputs
-  // (no scatter, no gating, no accumulate) whose base and pitch TMA accepts.
+  // storing 16-byte pieces of its own row.  Set by the launcher for outputs that are not scattered
+  // and whose base and pitch TMA accepts; an accumulating GEMM's boxes are added to the output in
+  // L2 (cp.reduce) instead of being read back by the epilogue warps.
   int staged_store;
 };
 
@@ -586,7 +587,10 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) {
-              tma_store_2d(&tma_c, stage, col0, band_row);
+              if (ep.accumulate)
+                tma_reduce_add_2d(&tma_c, stage, col0, band_row);
+              else
+                tma_store_2d(&tma_c, stage, col0, band_row);
               bulk_commit_group();
             }
             sbuf = (sbuf + 1) % S::kStoreBufs;

@@ -132,8 +132,9 @@ struct Gemm {
     ok(stb::launch_gemm_allgather(c, status, stream), "gemm all-gather");
   }
   // `pull`: `a` is the local buffer that the GEMM first fills from the peers' sequence slices
+  // `accumulate`: add to the fp32 output instead of storing it
   void run(const Tensor& a, const Tensor& b, Tensor& out, bool a_mn, bool b_mn, const float* bias,
-           const Tensor* residual, const SeqPull& pull = SeqPull{}) const {
+           const Tensor* residual, const SeqPull& pull = SeqPull{}, bool accumulate = false) const {
     stb::GemmCall c{};
     set_pull(c, pull, a.stride(0));
     c.M = static_cast<int>(a_mn ? a.size(1) : a.size(0));
@@ -148,7 +149,7 @@ struct Gemm {
     c.a_mn = a_mn;
     c.b_mn = b_mn;
     c.out_fp32 = out.scalar_type() == at::kFloat;
-    c.accumulate = false;
+    c.accumulate = accumulate;
     c.alpha = 1.f;
     c.force_bn = 0;
     c.bias = bias;
@@ -571,6 +572,7 @@ BackwardScratch& shared_backward_scratch(const Tensor& like, int64_t B, int64_t 
 }
 
 // Gradient views (down, gate_up, ln2, o, bias, qkv, ln1) point into the unit's gradient slot.
+// `accumulate`: the slot is the gradient arena itself and already holds earlier micro-steps' sums.
 Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1, const Tensor& h1,
                       const Tensor& qkv, const Tensor& attn, const Tensor& lse, const Tensor& x_mid,
                       const Tensor& inv2, const Tensor& h2, const Tensor& gu, const Tensor& hm,
@@ -579,7 +581,8 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
                       const Tensor& ln2, Tensor g_down, Tensor g_gate_up, Tensor g_ln2, Tensor g_o,
                       Tensor g_bias, Tensor g_qkv, Tensor g_ln1, const Tensor& cos, const Tensor& sin,
                       const c10::optional<Tensor>& positions, const c10::optional<Tensor>& mask,
-                      Tensor status, int64_t B, int64_t S, int64_t hq, int64_t hkv, bool replay) {
+                      Tensor status, int64_t B, int64_t S, int64_t hq, int64_t hkv, bool replay,
+                      bool accumulate) {
   const int64_t M = B * S, H = x2.size(1), D = 128;
   const int64_t W = (hq + 2 * hkv) * D, inter = w_down.size(1);
   auto f32 = x2.options().dtype(at::kFloat);
@@ -598,18 +601,18 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
   auto launch = [&](std::vector<Tensor>& b) {
     Tensor& dx = b[0];
     ok(stb::launch_cast_f32_to_bf16(d_out.data_ptr<float>(), t.d_out_b.data_ptr(), M * H, st), "cast");
-    g.run(t.d_out_b, hm, g_down, true, true, nullptr, nullptr);                 // dW down
+    g.run(t.d_out_b, hm, g_down, true, true, nullptr, nullptr, SeqPull{}, accumulate);                 // dW down
     g.run(t.d_out_b, w_down, t.d_hm, false, true, nullptr, nullptr);            // dX down
     ok(stb::launch_swiglu_bwd(t.d_hm.data_ptr(), gu.data_ptr(), t.d_gu.data_ptr(), M, inter, st), "swiglu_bwd");
-    g.run(t.d_gu, h2, g_gate_up, true, true, nullptr, nullptr);                 // dW gate|up
+    g.run(t.d_gu, h2, g_gate_up, true, true, nullptr, nullptr, SeqPull{}, accumulate);                 // dW gate|up
     g.run(t.d_gu, w_gu, t.d_h2, false, true, nullptr, nullptr);                 // dX gate|up
     ok(stb::launch_rmsnorm_bwd(t.d_h2.data_ptr<float>(), x_mid.data_ptr<float>(), ln2.data_ptr<float>(),
                                inv2.data_ptr<float>(), d_out.data_ptr<float>(), t.d_mid.data_ptr<float>(),
                                t.partial.data_ptr<float>(), kNormPartialRows, M, H, st), "rmsnorm_bwd");
     ok(stb::launch_colsum_f32(t.partial.data_ptr<float>(), g_ln2.data_ptr<float>(), kNormPartialRows, H,
-                              false, st), "colsum");
+                              accumulate, st), "colsum");
     ok(stb::launch_cast_f32_to_bf16(t.d_mid.data_ptr<float>(), t.d_mid_b.data_ptr(), M * H, st), "cast");
-    g.run(t.d_mid_b, attn, g_o, true, true, nullptr, nullptr);                  // dW o
+    g.run(t.d_mid_b, attn, g_o, true, true, nullptr, nullptr, SeqPull{}, accumulate);                  // dW o
     g.run(t.d_mid_b, w_o, t.d_attn, false, true, nullptr, nullptr);             // dX o
     stb::AttnBwdCall bc{};
     bc.qkv = qkv.data_ptr();
@@ -631,15 +634,15 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
     ok(stb::launch_attention_bwd(bc, g.status, st), "attention_bwd");
     ok(stb::launch_rope(t.d_qkv.data_ptr(), cos.data_ptr<float>(), sin.data_ptr<float>(), pos, M, S, hq,
                         hkv, D, true, st), "rope inverse");
-    ok(stb::launch_colsum_bf16(t.d_qkv.data_ptr(), W, g_bias.data_ptr<float>(), M, W, false,
+    ok(stb::launch_colsum_bf16(t.d_qkv.data_ptr(), W, g_bias.data_ptr<float>(), M, W, accumulate,
                                t.bias_partial.data_ptr<float>(), 64, st), "bias colsum");
-    g.run(t.d_qkv, h1, g_qkv, true, true, nullptr, nullptr);                    // dW q|k|v
+    g.run(t.d_qkv, h1, g_qkv, true, true, nullptr, nullptr, SeqPull{}, accumulate);                    // dW q|k|v
     g.run(t.d_qkv, w_qkv, t.d_h1, false, true, nullptr, nullptr);               // dX q|k|v
     ok(stb::launch_rmsnorm_bwd(t.d_h1.data_ptr<float>(), x2.data_ptr<float>(), ln1.data_ptr<float>(),
                                inv1.data_ptr<float>(), t.d_mid.data_ptr<float>(), dx.data_ptr<float>(),
                                t.partial.data_ptr<float>(), kNormPartialRows, M, H, st), "rmsnorm_bwd");
     ok(stb::launch_colsum_f32(t.partial.data_ptr<float>(), g_ln1.data_ptr<float>(), kNormPartialRows, H,
-                              false, st), "colsum");
+                              accumulate, st), "colsum");
   };
   if (!replay) {
     std::vector<Tensor> b = alloc();
@@ -650,7 +653,7 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
   k.tag(2).t(d_out).t(x2).t(inv1).t(h1).t(qkv).t(attn).t(lse).t(x_mid).t(inv2).t(h2).t(gu).t(hm)
       .t(w_qkv).t(w_o).t(w_gu).t(w_down).t(ln1).t(ln2).t(g_down).t(g_gate_up).t(g_ln2).t(g_o)
       .t(g_bias).t(g_qkv).t(g_ln1).t(cos).t(sin).t(positions).t(mask).t(status).i(B).i(S).i(hq)
-      .i(hkv).i(H).i(inter).i(static_cast<int64_t>(reinterpret_cast<uintptr_t>(st)));
+      .i(hkv).i(H).i(inter).i(accumulate).i(static_cast<int64_t>(reinterpret_cast<uintptr_t>(st)));
   return replay_cache().run(std::move(k.v), st, alloc, launch)[0];
 }
 

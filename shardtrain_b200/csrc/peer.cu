@@ -164,7 +164,7 @@ __global__ void gather_params_kernel(PeerPtrs shards, ShadowPtrs shadows, int us
 // reduce-scatter (src/sharded_runtime/runtime/materializer.py:228-233).
 template <bool ADAMW>
 __global__ void reduce_scatter_kernel(PeerPtrs full, int degree, int rank, int tp, int tp_rank,
-                                      SegTable tab, float* __restrict__ gshard,
+                                      SegTable tab, float* gshard /* may be the slot itself */,
                                       float* __restrict__ p, float* __restrict__ m,
                                       float* __restrict__ v, float split_scale, float rep_scale,
                                       int accumulate, AdamWArgs a, int* __restrict__ flags,
@@ -185,6 +185,9 @@ __global__ void reduce_scatter_kernel(PeerPtrs full, int degree, int rank, int t
   const int64_t lo = static_cast<int64_t>(rank) * sg.q;
   const int64_t valid = max(static_cast<int64_t>(0), min(sg.q, sg.numel - lo));
   const bool vec = (sg.q % 4 == 0) && (sg.shard_off % 4 == 0) && (sg.full_off % 4 == 0);
+  // a single member whose gradients were written straight into its shard: nothing to store
+  const bool in_place = n_src == 1 && scale == 1.f && !accumulate &&
+                        full.p[offset] + sg.full_off + lo == gshard + sg.shard_off;
   const float step_size = ADAMW ? a.lr / a.bias_correction1 : 0.f;
   const float inv_bc2_sqrt = ADAMW ? rsqrtf(a.bias_correction2) : 0.f;
   // the gradient check rides along: flags[0] = a non-finite reduced gradient was written,
@@ -233,7 +236,7 @@ __global__ void reduce_scatter_kernel(PeerPtrs full, int degree, int rank, int t
           const float4 o = *reinterpret_cast<const float4*>(gshard + e);
           g.x += o.x; g.y += o.y; g.z += o.z; g.w += o.w;
         }
-        *reinterpret_cast<float4*>(gshard + e) = g;   // padding stays exactly zero: acc is 0 there
+        if (!in_place) *reinterpret_cast<float4*>(gshard + e) = g;   // padding stays exactly zero: acc is 0 there
         bad |= !(isfinite(g.x) && isfinite(g.y) && isfinite(g.z) && isfinite(g.w));
         if (i + 3 >= valid) {
           const float* gp = &g.x;
@@ -267,7 +270,7 @@ __global__ void reduce_scatter_kernel(PeerPtrs full, int degree, int rank, int t
         const int64_t e = sg.shard_off + i;
         float g = acc[0] * scale;
         if (accumulate) g += gshard[e];
-        gshard[e] = g;
+        if (!in_place) gshard[e] = g;
         bad |= !isfinite(g);
         if (i >= valid && g != 0.f) pad_bad = 1;
         if (ADAMW) {

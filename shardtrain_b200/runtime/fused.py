@@ -35,6 +35,11 @@ _LAYER_ORDER = ("q_proj.weight", "k_proj.weight", "v_proj.weight", "o_proj.weigh
                 "q_proj.bias", "k_proj.bias", "v_proj.bias",
                 "input_layernorm.weight", "post_attention_layernorm.weight")
 
+# pairs of parameters whose gradients one kernel writes as one matrix or vector
+_FUSED_NEIGHBOURS = (("q_proj.weight", "k_proj.weight"), ("k_proj.weight", "v_proj.weight"),
+                     ("gate_proj.weight", "up_proj.weight"), ("q_proj.bias", "k_proj.bias"),
+                     ("k_proj.bias", "v_proj.bias"))
+
 
 def _up(value, multiple):
     return -(-value // multiple) * multiple
@@ -69,6 +74,9 @@ class UnitPlan:
     last_reader: object = None                        # event after the buffers' last consumer
     fwd: dict = field(default_factory=dict)           # fused operand views (built on first use)
     gslots: dict = field(default_factory=dict)        # id(slot) -> fused gradient views
+    # a single member (no FSDP or TP peers): the unit's window of the gradient arena, into which
+    # the backward writes (first micro-step) or adds (later ones) its gradients
+    arena_slot: "GradSlot | None" = None
 
     def views(self, full_bf16, full_fp32):
         out = {}
@@ -289,11 +297,17 @@ class FusedExecutor:
                        else self._shadow_buffer.owner.view(torch.bfloat16)[:total])
         self.shadow_peer_ptrs = list(self._shadow_buffer.ptrs)
         self._shadow_stale = True
-        largest = 0
+        largest = ring_units = 0
         token_pool = torch.zeros(64 * max(1, len(rt.units)), dtype=torch.float32, device=rt.device)
         for unit in rt.units:
             plan = mat.plans[unit.unit_id] = build_plan(unit)
-            largest = max(largest, plan.grad_numel)
+            if self._gradients_in_arena(unit, plan):
+                lo, hi = rt.plan.unit_ranges[unit.unit_id]
+                window = self.grad.narrow(0, lo, hi - lo)
+                plan.arena_slot = GradSlot(window, [window.data_ptr()])
+            else:
+                largest = max(largest, plan.grad_numel)
+                ring_units += 1
             if self._alias_shadow(unit, plan):
                 # FSDP degree 1: a "gathered" matrix is the shard itself, and the shadow arena
                 # already holds it in bf16 at the offsets the kernels want -- the unit's weight
@@ -315,12 +329,38 @@ class FusedExecutor:
         # axis) -- with TP the slots are shared by the whole mesh and a multicast sum would add
         # the other TP coordinates' gradients of TP-split parameters
         want_nvls = (rt.nvls != "off" and self.tp_degree == 1 and self.peer.degree > 1)
-        self.ring = GradRing(self.reduce_peer, self.ops, _up(largest, 4), count=4,
+        self.ring = GradRing(self.reduce_peer, self.ops, _up(largest, 4), count=4 if ring_units else 0,
                              multicast=want_nvls)
         self.nvls_active = all(slot.multicast_ptr for slot in self.ring.slots) and want_nvls
         mat.bind(self.ops, self)
         ranges = rt.padding_ranges or [(0, 0)]
         self._pad_ranges = torch.tensor(ranges, dtype=torch.int64, device=rt.device).reshape(-1)
+
+    def _gradients_in_arena(self, unit, plan) -> bool:
+        """Single member: "reducing" a full gradient would only copy it into (or add it to) the
+        arena, so the backward writes there itself -- 8 (store) to 12 (add) bytes of memory traffic
+        per parameter and micro-step less, and no ring of slots.  True (and the plan's gradient
+        offsets are the arena's) when the fused gradient views are contiguous in the arena too."""
+        if self.reduce_peer.degree != 1:
+            return False
+        lo = self.runtime.plan.unit_ranges[unit.unit_id][0]
+        at = {h.spec.param_id: h.arena_offset - lo for h in unit.handles}
+        if any(o % 4 or h.spec.fsdp_shard_numel != h.spec.numel
+               for h, o in zip(unit.handles, at.values())) or lo % 4:
+            return False
+        for first, second in zip(plan.names, plan.names[1:]):
+            fused = any(first.endswith(a) and second.endswith(b) for a, b in _FUSED_NEIGHBOURS)
+            if fused and at[second] != at[first] + math.prod(plan.shapes[first]):
+                return False
+        plan.grad_offsets = at
+        plan.reduce_table = segment_table([self.runtime.registry[n] for n in plan.names], at, set(),
+                                          mark_replicated=True)
+        return True
+
+    def accumulates(self, unit) -> bool:
+        """Does this micro-step's backward add to gradients that the unit's slot already holds?"""
+        plan = self.runtime.materializer.plans[unit.unit_id]
+        return plan.arena_slot is not None and not self.runtime.first_commit(unit)
 
     def _alias_shadow(self, unit, plan) -> bool:
         """True when the unit's bf16 matrices sit in the shard arena exactly as in its fused
@@ -380,7 +420,8 @@ class FusedExecutor:
 
     def acquire_grad_slot(self, unit):
         if getattr(unit, "grad_slot", None) is None:
-            unit.grad_slot = self.ring.acquire(unit.unit_id, self.runtime.comm.current_stream())
+            own = self.runtime.materializer.plans[unit.unit_id].arena_slot
+            unit.grad_slot = own if own is not None else self.ring.acquire(unit.unit_id, self.runtime.comm.current_stream())
         return unit.grad_slot
 
     def grad_slot(self, unit):
@@ -390,7 +431,8 @@ class FusedExecutor:
         return slot
 
     def grad_slot_issued(self, unit, slot, ticket):
-        self.ring.issued(slot, ticket.ready_event)
+        if self.runtime.materializer.plans[unit.unit_id].arena_slot is None:
+            self.ring.issued(slot, ticket.ready_event)
         unit.grad_slot = None
 
     def layer_operands(self, plan, index):
@@ -635,7 +677,7 @@ class FusedEmbeddingFn(torch.autograd.Function):
         fresh = getattr(unit, "grad_slot", None) is None
         slot = ex.acquire_grad_slot(unit)
         dw = plan.grad_view(slot.local, name)
-        if fresh:
+        if fresh and not ex.accumulates(unit):
             dw.zero_()  # untied: nothing wrote the slot yet; tied: the head's dW is already there
         pad = ex.cfg.pad_token_id
         ex.ops.embedding_scatter_add(grad.reshape(-1, grad.shape[-1]).contiguous(),
@@ -678,7 +720,7 @@ class FusedNormFn(torch.autograd.Function):
         partial = ex.scratch("norm_partial", (592, x2.shape[1]), torch.float32)
         ex.ops.rmsnorm_bwd(dy, x2, weight, inv, None, dx, partial)
         dw = plan.grad_view(slot.local, name)
-        ex.ops.colsum_f32(partial, dw, False)
+        ex.ops.colsum_f32(partial, dw, ex.accumulates(unit))
         return dx.view(ctx.shape), ex.token_grad, None, None
 
 
@@ -726,7 +768,7 @@ class FusedHeadLossFn(torch.autograd.Function):
         plan = ex.runtime.materializer.plans[unit.unit_id]
         slot = ex.acquire_grad_slot(unit)
         dw = plan.grad_view(slot.local, name)
-        ops.gemm(logits, hidden2, dw, True, True, None, None, False, 1.0, 0)
+        ops.gemm(logits, hidden2, dw, True, True, None, None, ex.accumulates(unit), 1.0, 0)
         dx = torch.empty(hidden2.shape, dtype=torch.float32, device=hidden2.device)
         ops.gemm(logits, weight, dx, False, True, None, None, False, 1.0, 0)
         ex._head_dx = dx
@@ -842,7 +884,7 @@ class FusedLayerFn(torch.autograd.Function):
         dx = ops.layer_backward(
             d_out, x2, inv1, h1, qkv, attn, lse, x_mid, inv2, h2, gu, hm, w_qkv, w_o, w_gu, w_down, ln1,
             ln2, gv["down"], gv["gate_up"], gv["ln2"], gv["o"], gv["bias"], gv["qkv"], gv["ln1"], cos,
-            sin, positions, ctx.mask, ex.status, B, S, hq, hkv, ctx.replay)
+            sin, positions, ctx.mask, ex.status, B, S, hq, hkv, ctx.replay, ex.accumulates(unit))
         ex._forward_open.discard(index)
         return (dx.view(B, S, H), None, None, None, None, None, *([ex.token_grad] * len(plan.names)))
 

@@ -363,17 +363,24 @@ class PeerMaterializer:
         # NVLS: the switch adds the members' slots (only when the ring got multicast addresses)
         multicast = slot.multicast_ptr if getattr(arenas, "nvls_active", False) else 0
 
+        # A single member's gradients are in the arena already (see FusedExecutor): nothing moves, and
+        # what is left, the check of the sums and AdamW, belongs to the last micro-step.
+        in_arena = plan.arena_slot is not None
+
         def launch():
+            if in_arena and not runtime.last_microstep:
+                return
             arenas.reduce_peer.barrier("fsdp_rs")     # no-op for a single member
             if fuse_adamw:
                 hp = runtime.fused_optimizer_args()
                 self.ops.reduce_scatter_adamw(
                     slot.peer_ptrs, self.rank, plan.reduce_table, arenas.grad, arenas.param,
-                    arenas.exp_avg, arenas.exp_avg_sq, 1.0 / self.degree, not first, *hp,
+                    arenas.exp_avg, arenas.exp_avg_sq, 1.0 / self.degree, not first and not in_arena, *hp,
                     arenas.check_flags, *tp, arenas.shadow, multicast)
             else:
                 self.ops.reduce_scatter(slot.peer_ptrs, self.rank, plan.reduce_table, arenas.grad,
-                                        1.0 / self.degree, not first, arenas.check_flags, *tp,
+                                        1.0 / self.degree, not first and not in_arena,
+                                        arenas.check_flags, *tp,
                                         multicast)
 
         comm = self.comm
