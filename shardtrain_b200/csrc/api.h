@@ -73,7 +73,7 @@ cudaError_t launch_slot_sum_rmsnorm(const float* slots, int n_slots, int64_t slo
 // dx_out = dres_in (optional) + rmsnorm backward of dy ; dw_partial [blocks, cols]
 cudaError_t launch_rmsnorm_bwd(const float* dy, const float* x, const float* w, const float* inv,
                                const float* dres_in, float* dx_out, float* dw_partial,
-                               int partial_rows, int rows, int cols, cudaStream_t s);
+                               int partial_rows, int rows, int cols, cudaStream_t s, void* dx_bf16 = nullptr);
 cudaError_t launch_colsum_f32(const float* partial, float* out, int rows, int cols,
                               bool accumulate, cudaStream_t s);
 cudaError_t launch_colsum_bf16(const void* x, int64_t ldx, float* out, int rows, int cols,

@@ -266,7 +266,8 @@ void slot_sum_rmsnorm(const Tensor& slots, const c10::optional<Tensor>& residual
 }
 
 void rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& inv,
-                 const c10::optional<Tensor>& dres, Tensor dx, Tensor dw_partial) {
+                 const c10::optional<Tensor>& dres, Tensor dx, Tensor dw_partial,
+                 const c10::optional<Tensor>& dx_bf16) {
   need(dy, at::kFloat, "dy");
   need(x, at::kFloat, "x");
   need(dx, at::kFloat, "dx");
@@ -275,11 +276,16 @@ void rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tenso
   const int rows = static_cast<int>(x.numel() / cols);
   TORCH_CHECK(dy.is_contiguous() && x.is_contiguous() && dx.is_contiguous());
   TORCH_CHECK(dw_partial.dim() == 2 && dw_partial.size(1) == cols && dw_partial.is_contiguous());
+  if (dx_bf16.has_value()) {
+    need(*dx_bf16, at::kBFloat16, "dx_bf16");
+    TORCH_CHECK(dx_bf16->numel() == dx.numel() && dx_bf16->is_contiguous());
+  }
   check(stb::launch_rmsnorm_bwd(dy.data_ptr<float>(), x.data_ptr<float>(), w.data_ptr<float>(),
                                 inv.data_ptr<float>(),
                                 dres.has_value() ? dres->data_ptr<float>() : nullptr,
                                 dx.data_ptr<float>(), dw_partial.data_ptr<float>(),
-                                static_cast<int>(dw_partial.size(0)), rows, cols, cur_stream()),
+                                static_cast<int>(dw_partial.size(0)), rows, cols, cur_stream(),
+                                dx_bf16.has_value() ? dx_bf16->data_ptr() : nullptr),
         "rmsnorm_bwd");
 }
 
@@ -872,7 +878,8 @@ TORCH_LIBRARY(stb, m) {
   m.def("gemm_broadcast", &gemm_broadcast);
   m.def("slot_sum_rmsnorm", &slot_sum_rmsnorm);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
-  m.def("rmsnorm_bwd", &rmsnorm_bwd);
+  m.def("rmsnorm_bwd(Tensor dy, Tensor x, Tensor w, Tensor inv, Tensor? dres, Tensor(a!) dx, "
+        "Tensor(b!) dw_partial, Tensor(c!)? dx_bf16=None) -> ()", &rmsnorm_bwd);
   m.def("colsum_f32", &colsum_f32);
   m.def("colsum_bf16", &colsum_bf16);
   m.def("rope", &rope);

@@ -124,11 +124,13 @@ __global__ void slot_sum_rmsnorm_kernel(const float* __restrict__ slots, int n_s
   }
 }
 
-// dx = inv * (g*w - x * inv^2 * mean(g*w*x)) (+ incoming residual gradient);
-// d(weight) partial per CTA = sum over its rows of g * (x*inv).  Rows are strided over CTAs.
+// dx = inv * (g*w - x * inv^2 * mean(g*w*x)) (+ incoming residual gradient), and optionally a bf16
+// copy of it; d(weight) partial per CTA = sum over its rows of g * (x*inv).  Rows are strided over
+// CTAs; thread t owns columns 4 t + 1024 k, whatever the width.
 __global__ void rmsnorm_bwd_kernel(const float* __restrict__ dy, const float* __restrict__ x,
                                    const float* __restrict__ w, const float* __restrict__ inv,
                                    const float* __restrict__ dres, float* __restrict__ dx,
+                                   __nv_bfloat16* __restrict__ dx_bf16,
                                    float* __restrict__ dw_partial, int rows, int cols) {
   extern __shared__ float sm[];  // cols floats of dw accumulation + 32 for reductions
   float* dw_acc = sm;
@@ -162,6 +164,12 @@ __global__ void rmsnorm_bwd_kernel(const float* __restrict__ dy, const float* __
         o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w;
       }
       *reinterpret_cast<float4*>(dx + row * cols + c) = o;
+      if (dx_bf16 != nullptr) {
+        uint2 pk;
+        pk.x = pack2(o.x, o.y);
+        pk.y = pack2(o.z, o.w);
+        *reinterpret_cast<uint2*>(dx_bf16 + row * cols + c) = pk;
+      }
       // each thread owns fixed columns across rows, so no race on dw_acc
       dw_acc[c] += gv.x * xv.x * iv;
       dw_acc[c + 1] += gv.y * xv.y * iv;
@@ -174,6 +182,104 @@ __global__ void rmsnorm_bwd_kernel(const float* __restrict__ dy, const float* __
     dw_partial[static_cast<int64_t>(blockIdx.x) * cols + c] = dw_acc[c];
 }
 
+// The same for up to 1024 K columns with everything a thread needs of a row in registers: x and dy are
+// read once, the next row's are on their way while this row is reduced (K <= 2), d(weight) never
+// leaves the registers, and a row costs one block barrier instead of two.  The sums run in the same
+// order, so the results have the same bits.  The general kernel above was bound by its chain of load
+// -> reduction -> load per row: 35 us at 4096 x 1536, 107 us at 8192 x 3584; now 31 and 92 us.
+template <int K>
+__global__ void __launch_bounds__(256, 4)
+rmsnorm_bwd_rows_kernel(const float* __restrict__ dy, const float* __restrict__ x,
+                        const float* __restrict__ w, const float* __restrict__ inv,
+                        const float* __restrict__ dres, float* __restrict__ dx,
+                        __nv_bfloat16* __restrict__ dx_bf16, float* __restrict__ dw_partial,
+                        int rows, int cols) {
+  constexpr bool kAhead = K <= 2;
+  __shared__ float red[2][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c0 = threadIdx.x * 4;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 acc[K], xv[K], gv[K], xn[kAhead ? K : 1], gn[kAhead ? K : 1];
+#pragma unroll
+  for (int k = 0; k < K; ++k) acc[k] = zero;
+  auto load = [&](int64_t row, float4* xs, float4* gs) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int c = c0 + k * 1024;
+      xs[k] = gs[k] = zero;
+      if (c < cols) {
+        xs[k] = *reinterpret_cast<const float4*>(x + row * cols + c);
+        gs[k] = *reinterpret_cast<const float4*>(dy + row * cols + c);
+      }
+    }
+  };
+  if (blockIdx.x < rows) load(blockIdx.x, xv, gv);
+  int parity = 0;
+  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, parity ^= 1) {
+    const int64_t next = row + gridDim.x;
+    if constexpr (kAhead) {
+      if (next < rows) load(next, xn, gn);
+    }
+    const float iv = inv[row];
+    float dot = 0.f;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int c = c0 + k * 1024;
+      if (c < cols) {
+        const float4 wv = *reinterpret_cast<const float4*>(w + c);
+        dot += gv[k].x * wv.x * xv[k].x + gv[k].y * wv.y * xv[k].y + gv[k].z * wv.z * xv[k].z +
+               gv[k].w * wv.w * xv[k].w;
+      }
+    }
+    dot = warp_sum(dot);
+    if (lane == 0) red[parity][warp] = dot;
+    __syncthreads();           // (the buffer's readers of two rows ago passed the barrier in between)
+    dot = warp_sum(lane < 8 ? red[parity][lane] : 0.f);
+    const float coef = iv * iv * dot / cols;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int c = c0 + k * 1024;
+      if (c >= cols) continue;
+      const float4 wv = *reinterpret_cast<const float4*>(w + c);
+      float4 o;
+      o.x = iv * (gv[k].x * wv.x - xv[k].x * coef);
+      o.y = iv * (gv[k].y * wv.y - xv[k].y * coef);
+      o.z = iv * (gv[k].z * wv.z - xv[k].z * coef);
+      o.w = iv * (gv[k].w * wv.w - xv[k].w * coef);
+      if (dres != nullptr) {
+        const float4 r = *reinterpret_cast<const float4*>(dres + row * cols + c);
+        o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w;
+      }
+      *reinterpret_cast<float4*>(dx + row * cols + c) = o;
+      if (dx_bf16 != nullptr) {
+        uint2 pk;
+        pk.x = pack2(o.x, o.y);
+        pk.y = pack2(o.z, o.w);
+        *reinterpret_cast<uint2*>(dx_bf16 + row * cols + c) = pk;
+      }
+      acc[k].x += gv[k].x * xv[k].x * iv;
+      acc[k].y += gv[k].y * xv[k].y * iv;
+      acc[k].z += gv[k].z * xv[k].z * iv;
+      acc[k].w += gv[k].w * xv[k].w * iv;
+    }
+    if constexpr (kAhead) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        xv[k] = xn[k];
+        gv[k] = gn[k];
+      }
+    } else {
+      if (next < rows) load(next, xv, gv);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int c = c0 + k * 1024;
+    if (c < cols)
+      *reinterpret_cast<float4*>(dw_partial + static_cast<int64_t>(blockIdx.x) * cols + c) = acc[k];
+  }
+}
+
 // out[c] (+)= sum_r partial[r, c]; deterministic order.
 // out[c] = sum_r partial[r, c].  A CTA covers 32 columns with 8 row groups (blockDim 32 x 8): the
 // groups stride over the rows, then combine through shared memory in a fixed order.
@@ -182,8 +288,17 @@ __global__ void colsum_f32_kernel(const float* __restrict__ partial, float* __re
   __shared__ float part[8][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
-  if (c < cols)
-    for (int r = threadIdx.y; r < rows; r += 8) s += partial[static_cast<int64_t>(r) * cols + c];
+  if (c < cols) {
+    for (int r = threadIdx.y; r < rows; r += 8 * 16) {   // 16 loads in flight, added in row order
+      float v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (r + u * 8 < rows) v[u] = partial[static_cast<int64_t>(r + u * 8) * cols + c];
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (r + u * 8 < rows) s += v[u];
+    }
+  }
   part[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
   if (threadIdx.y == 0 && c < cols) {
@@ -200,10 +315,21 @@ __global__ void colsum_bf16_partial_kernel(const __nv_bfloat16* __restrict__ x, 
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
   if (c >= cols) return;
   float s0 = 0.f, s1 = 0.f;
-  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
-    const float2 v = unpack2(*reinterpret_cast<const uint32_t*>(x + r * ldx + c));
-    s0 += v.x;
-    s1 += v.y;
+  // 16 loads in flight, added in row order (one at a time cost a round trip per row: 40 us at 4096 x
+  // 2048 with the final sum, 17 us now)
+  const int step = gridDim.y;
+  for (int r = blockIdx.y; r < rows; r += step * 16) {
+    uint32_t v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+      if (r + u * step < rows) v[u] = *reinterpret_cast<const uint32_t*>(x + (r + u * step) * ldx + c);
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+      if (r + u * step < rows) {
+        const float2 f = unpack2(v[u]);
+        s0 += f.x;
+        s1 += f.y;
+      }
   }
   scratch[static_cast<int64_t>(blockIdx.y) * cols + c] = s0;
   scratch[static_cast<int64_t>(blockIdx.y) * cols + c + 1] = s1;
@@ -213,32 +339,63 @@ __global__ void colsum_bf16_partial_kernel(const __nv_bfloat16* __restrict__ x, 
 // rotate_half form: out[i] = x[i]*cos - x[i+d/2]*sin ; out[i+d/2] = x[i+d/2]*cos + x[i]*sin.
 // Applied in place to the q and k heads of the packed qkv rows; `inverse` flips the sign of sin
 // (the backward pass is the transposed rotation).
+// V elements of each half per thread: 8 (16-byte accesses) where d and the base allow it, else 2.
+template <int V>
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, const int* __restrict__ positions,
                             int rows, int seq, int hq, int hkv, int d, int inverse) {
   const int half = d / 2;
   const int heads = hq + hkv;
-  const int pairs_per_row = heads * (half / 2);  // two (i, i+half) pairs per thread
+  const int per_head = half / V, per_row = heads * per_head;
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= static_cast<int64_t>(rows) * pairs_per_row) return;
-  const int row = static_cast<int>(idx / pairs_per_row);
-  const int rem = static_cast<int>(idx % pairs_per_row);
-  const int head = rem / (half / 2);
-  const int i = (rem % (half / 2)) * 2;
+  if (idx >= static_cast<int64_t>(rows) * per_row) return;
+  const int row = static_cast<int>(idx / per_row);
+  const int rem = static_cast<int>(idx - static_cast<int64_t>(row) * per_row);
+  const int head = rem / per_head;
+  const int i = (rem - head * per_head) * V;
   const int pos = positions ? positions[row] : (row % seq);
   const int64_t stride = static_cast<int64_t>(hq + 2 * hkv) * d;
-  __nv_bfloat16* base = qkv + row * stride + static_cast<int64_t>(head) * d;
-  const float2 lo = unpack2(*reinterpret_cast<uint32_t*>(base + i));
-  const float2 hi = unpack2(*reinterpret_cast<uint32_t*>(base + i + half));
-  const float c0 = cos_t[pos * half + i], c1 = cos_t[pos * half + i + 1];
-  float s0 = sin_t[pos * half + i], s1 = sin_t[pos * half + i + 1];
-  if (inverse) {
-    s0 = -s0;
-    s1 = -s1;
+  __nv_bfloat16* base = qkv + row * stride + static_cast<int64_t>(head) * d + i;
+  uint32_t lo[V / 2], hi[V / 2];
+  float cv[V], sv[V];
+  if constexpr (V == 8) {
+    *reinterpret_cast<uint4*>(lo) = *reinterpret_cast<const uint4*>(base);
+    *reinterpret_cast<uint4*>(hi) = *reinterpret_cast<const uint4*>(base + half);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      *reinterpret_cast<float4*>(cv + 4 * j) =
+          *reinterpret_cast<const float4*>(cos_t + static_cast<int64_t>(pos) * half + i + 4 * j);
+      *reinterpret_cast<float4*>(sv + 4 * j) =
+          *reinterpret_cast<const float4*>(sin_t + static_cast<int64_t>(pos) * half + i + 4 * j);
+    }
+  } else {
+    lo[0] = *reinterpret_cast<const uint32_t*>(base);
+    hi[0] = *reinterpret_cast<const uint32_t*>(base + half);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      cv[j] = cos_t[static_cast<int64_t>(pos) * half + i + j];
+      sv[j] = sin_t[static_cast<int64_t>(pos) * half + i + j];
+    }
   }
-  *reinterpret_cast<uint32_t*>(base + i) = pack2(lo.x * c0 - hi.x * s0, lo.y * c1 - hi.y * s1);
-  *reinterpret_cast<uint32_t*>(base + i + half) =
-      pack2(hi.x * c0 + lo.x * s0, hi.y * c1 + lo.y * s1);
+#pragma unroll
+  for (int j = 0; j < V / 2; ++j) {
+    const float2 l = unpack2(lo[j]), h = unpack2(hi[j]);
+    const float c0 = cv[2 * j], c1 = cv[2 * j + 1];
+    float s0 = sv[2 * j], s1 = sv[2 * j + 1];
+    if (inverse) {
+      s0 = -s0;
+      s1 = -s1;
+    }
+    lo[j] = pack2(l.x * c0 - h.x * s0, l.y * c1 - h.y * s1);
+    hi[j] = pack2(h.x * c0 + l.x * s0, h.y * c1 + l.y * s1);
+  }
+  if constexpr (V == 8) {
+    *reinterpret_cast<uint4*>(base) = *reinterpret_cast<const uint4*>(lo);
+    *reinterpret_cast<uint4*>(base + half) = *reinterpret_cast<const uint4*>(hi);
+  } else {
+    *reinterpret_cast<uint32_t*>(base) = lo[0];
+    *reinterpret_cast<uint32_t*>(base + half) = hi[0];
+  }
 }
 
 // ------------------------------------------------------------------ SwiGLU
@@ -466,9 +623,17 @@ __global__ void adamw_kernel(float* __restrict__ p, const float* __restrict__ g,
 
 __global__ void sgd_kernel(float* __restrict__ p, const float* __restrict__ g, int64_t n,
                            float lr) {
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    p[i] -= lr * g[i];
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const bool wide = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g)) & 15) == 0;
+  const int64_t n4 = wide ? n / 4 : 0;     // 16-byte pieces, then the rest one by one
+  for (int64_t i = first; i < n4; i += stride) {
+    float4 a = reinterpret_cast<const float4*>(p)[i];
+    const float4 b = reinterpret_cast<const float4*>(g)[i];
+    a.x -= lr * b.x; a.y -= lr * b.y; a.z -= lr * b.z; a.w -= lr * b.w;
+    reinterpret_cast<float4*>(p)[i] = a;
+  }
+  for (int64_t i = n4 * 4 + first; i < n; i += stride) p[i] -= lr * g[i];
 }
 
 // flags[0]: non-finite gradient seen; flags[1]: non-zero value inside a padding range.
@@ -568,12 +733,30 @@ cudaError_t launch_slot_sum_rmsnorm(const float* slots, int n_slots, int64_t slo
 
 cudaError_t launch_rmsnorm_bwd(const float* dy, const float* x, const float* w, const float* inv,
                                const float* dres_in, float* dx_out, float* dw_partial,
-                               int partial_rows, int rows, int cols, cudaStream_t s) {
+                               int partial_rows, int rows, int cols, cudaStream_t s, void* dx_bf16) {
   if (cols % 4 || partial_rows < 1) return cudaErrorInvalidValue;
-  const int threads = 256;
-  const size_t smem = (cols + 32) * sizeof(float);
-  rmsnorm_bwd_kernel<<<partial_rows, threads, smem, s>>>(dy, x, w, inv, dres_in, dx_out,
-                                                         dw_partial, rows, cols);
+  __nv_bfloat16* copy = reinterpret_cast<__nv_bfloat16*>(dx_bf16);
+  switch ((cols + 1023) / 1024) {
+    case 1:
+      rmsnorm_bwd_rows_kernel<1><<<partial_rows, 256, 0, s>>>(dy, x, w, inv, dres_in, dx_out, copy,
+                                                              dw_partial, rows, cols);
+      break;
+    case 2:
+      rmsnorm_bwd_rows_kernel<2><<<partial_rows, 256, 0, s>>>(dy, x, w, inv, dres_in, dx_out, copy,
+                                                              dw_partial, rows, cols);
+      break;
+    case 3:
+      rmsnorm_bwd_rows_kernel<3><<<partial_rows, 256, 0, s>>>(dy, x, w, inv, dres_in, dx_out, copy,
+                                                              dw_partial, rows, cols);
+      break;
+    case 4:
+      rmsnorm_bwd_rows_kernel<4><<<partial_rows, 256, 0, s>>>(dy, x, w, inv, dres_in, dx_out, copy,
+                                                              dw_partial, rows, cols);
+      break;
+    default:     // wider rows than the registers hold
+      rmsnorm_bwd_kernel<<<partial_rows, 256, (cols + 32) * sizeof(float), s>>>(
+          dy, x, w, inv, dres_in, dx_out, copy, dw_partial, rows, cols);
+  }
   count_launch();
   return cudaGetLastError();
 }
@@ -601,9 +784,18 @@ cudaError_t launch_colsum_bf16(const void* x, int64_t ldx, float* out, int rows,
 cudaError_t launch_rope(void* qkv, const float* cos, const float* sin, const int* positions,
                         int rows, int seq, int hq, int hkv, int d, bool inverse, cudaStream_t s) {
   if (d % 4) return cudaErrorInvalidValue;
-  const int64_t work = static_cast<int64_t>(rows) * (hq + hkv) * (d / 4);
-  rope_kernel<<<static_cast<int>((work + 255) / 256), 256, 0, s>>>(
-      reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions, rows, seq, hq, hkv, d, inverse);
+  // 16-byte accesses need whole 8-element pieces of each half and aligned bases (4096 x 14 heads of
+  // 128: 16 us with 4-byte accesses, 12 us with 16-byte ones; 8192 x 32 heads: 51 and 31 us)
+  const bool wide = d % 16 == 0 && ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(cos) |
+                                     reinterpret_cast<uintptr_t>(sin)) & 15) == 0;
+  const int64_t work = static_cast<int64_t>(rows) * (hq + hkv) * (d / (wide ? 16 : 4));
+  const int grid = static_cast<int>((work + 255) / 256);
+  if (wide)
+    rope_kernel<8><<<grid, 256, 0, s>>>(reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions, rows,
+                                        seq, hq, hkv, d, inverse);
+  else
+    rope_kernel<2><<<grid, 256, 0, s>>>(reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions, rows,
+                                        seq, hq, hkv, d, inverse);
   count_launch();
   return cudaGetLastError();
 }
@@ -680,7 +872,7 @@ cudaError_t launch_adamw(float* p, const float* g, float* m, float* v, int64_t n
 }
 
 cudaError_t launch_sgd(float* p, const float* g, int64_t n, float lr, cudaStream_t s) {
-  sgd_kernel<<<grid_for(n, 256, sm_count() * 16), 256, 0, s>>>(p, g, n, lr);
+  sgd_kernel<<<grid_for(n / 4 + 1, 256, sm_count() * 16), 256, 0, s>>>(p, g, n, lr);
   count_launch();
   return cudaGetLastError();
 }

@@ -608,10 +608,10 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
     g.run(t.d_gu, w_gu, t.d_h2, false, true, nullptr, nullptr);                 // dX gate|up
     ok(stb::launch_rmsnorm_bwd(t.d_h2.data_ptr<float>(), x_mid.data_ptr<float>(), ln2.data_ptr<float>(),
                                inv2.data_ptr<float>(), d_out.data_ptr<float>(), t.d_mid.data_ptr<float>(),
-                               t.partial.data_ptr<float>(), kNormPartialRows, M, H, st), "rmsnorm_bwd");
+                               t.partial.data_ptr<float>(), kNormPartialRows, M, H, st,
+                               t.d_mid_b.data_ptr()), "rmsnorm_bwd");
     ok(stb::launch_colsum_f32(t.partial.data_ptr<float>(), g_ln2.data_ptr<float>(), kNormPartialRows, H,
                               accumulate, st), "colsum");
-    ok(stb::launch_cast_f32_to_bf16(t.d_mid.data_ptr<float>(), t.d_mid_b.data_ptr(), M * H, st), "cast");
     g.run(t.d_mid_b, attn, g_o, true, true, nullptr, nullptr, SeqPull{}, accumulate);                  // dW o
     g.run(t.d_mid_b, w_o, t.d_attn, false, true, nullptr, nullptr);             // dX o
     stb::AttnBwdCall bc{};
