@@ -1,5 +1,5 @@
 // Native executor of one Qwen2 decoder layer: the whole forward (10 or 11 launches) or backward
-// (26 launches) sequence is issued from C++ in one call, so the host cost per layer is a few
+// (about 20 launches) sequence is issued from C++ in one call, so the host cost per layer is a few
 // microseconds per launch instead of a Python round trip per kernel.  The math and the launch
 // order are those documented in shardtrain_b200/runtime/fused.py (FusedLayerFn); this file only
 // moves the sequencing off the interpreter.
@@ -280,7 +280,7 @@ SpLink make_link(cudaStream_t st, int* status, c10::ArrayRef<int64_t> pads, int6
 // too keep their addresses.  A sequence is therefore keyed by EVERYTHING its kernels receive
 // (every pointer, pitch and scalar, the stream); the first time a key is seen the sequence is
 // launched kernel by kernel into buffers that the cache entry owns, the second time it is
-// captured into a graph, and from then on one cudaGraphLaunch replaces the 10 or 26 launches.
+// captured into a graph, and from then on one cudaGraphLaunch replaces the 10 or 20 launches.
 // Any difference in the key (another input address, another mask, another shape) is simply a
 // different entry; nothing is ever replayed against arguments it was not captured with.
 //

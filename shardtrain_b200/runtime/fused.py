@@ -880,7 +880,7 @@ class FusedLayerFn(torch.autograd.Function):
             tp.epochs["sp_ag"] = epoch + 2
             return (dx.view(B, S, H), None, None, None, None, None,
                     *([ex.token_grad] * len(plan.names)))
-        # the 26 launches of the backward run from C++ (csrc/layer_executor.cpp)
+        # the launches of the backward (about 20) run from C++ (csrc/layer_executor.cpp)
         dx = ops.layer_backward(
             d_out, x2, inv1, h1, qkv, attn, lse, x_mid, inv2, h2, gu, hm, w_qkv, w_o, w_gu, w_down, ln1,
             ln2, gv["down"], gv["gate_up"], gv["ln2"], gv["o"], gv["bias"], gv["qkv"], gv["ln1"], cos,

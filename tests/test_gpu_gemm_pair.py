@@ -59,3 +59,23 @@ def test_pair_gemm_matches_reference_and_stays_inside_the_output(ops, case):
     again = torch.empty_like(plane)
     ops.gemm(a, b, again[:M, :N], a_mn, b_mn, bias_t, res, False, 1.0, bn, split, True, True)
     assert torch.equal(again[:M, :N], out)      # split sums run in index order
+
+
+@pytest.mark.parametrize("shape", [(512, 1536, 8960, False, False), (1024, 1536, 4096, False, True),
+                                   (1536, 1536, 4096, True, True), (777, 1536, 8960, False, False),
+                                   (4096, 1536, 512, False, True), (1554, 2048, 1536, False, False),
+                                   (16, 264, 72, False, False)],
+                         ids=lambda s: "x".join(map(str, s[:3])) + f"_{int(s[3])}{int(s[4])}")
+def test_automatic_choice_has_the_bits_of_single_ctas(ops, shape):
+    """Whatever kernel runs, the elements summed in several K ranges are those that 128-row tiles of
+    one of the three widths would cut."""
+    M, N, K, a_mn, b_mn = shape
+    torch.manual_seed(4)
+    a = torch.randn((K, M) if a_mn else (M, K), device=DEV).bfloat16()
+    b = torch.randn((K, N) if b_mn else (N, K), device=DEV).bfloat16()
+    outs = []
+    for bn in (0, 256, 192, 128):
+        out = torch.empty(M, N, device=DEV)
+        ops.gemm(a, b, out, a_mn, b_mn, None, None, False, 1.0, bn)
+        outs.append(out)
+    assert any(torch.equal(outs[0], o) for o in outs[1:])
