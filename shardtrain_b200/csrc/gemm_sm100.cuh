@@ -12,6 +12,7 @@
 // the epilogue (warp w reads TMEM lanes 32*(w%4)..+31, as the hardware requires).
 #pragma once
 #include "common.cuh"
+#include "pipeline_tail.h"
 
 namespace stb {
 
@@ -340,6 +341,17 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
           }
           __syncwarp();
         }
+      }
+      // Pair: rank 0's commits arrive at the empty barriers of both CTAs, and no later barrier tells
+      // that they have (a commit's arrival is ordered behind its MMAs, not behind other commits').
+      // Each CTA sees its own last ones in before the pair parts.  The epilogue is draining the last
+      // tile meanwhile, so the wait costs nothing.
+      if constexpr (PAIR) {
+        if (ok)
+          ring_tail(it, STAGES, [&](int s, int parity) {
+            if (ok) ok = mbar_wait_warp(&empty_bar[s], parity, status, kErrDrainWait);
+          });
+        if (!ok) *abort_flag = 1;
       }
       // Error path only: wait (bounded) for copies this thread issued that nobody consumed.
       // (Pair: the copies of rank 1 complete on rank 0's barriers, which it cannot wait on; it
@@ -837,7 +849,8 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
 
   tc_fence_before_sync();
   if constexpr (PAIR)
-    cluster_sync();      // neither CTA leaves while the other still signals it or reads its operands
+    cluster_sync();      // no thread of the other CTA signals this one or issues for it any more; what is
+                         // asynchronous (copies, commits) was waited for above
   else
     __syncthreads();
   if (warp == 1) {
