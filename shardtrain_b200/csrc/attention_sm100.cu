@@ -10,7 +10,9 @@
 //
 // Warp 0 = TMA producer, warp 1 = MMA issuer / TMEM owner, the others = softmax: 4 warps with a row
 // per thread forward, 8 warps with half a row per thread backward.
-// Every mbarrier wait is bounded; on expiry the status word is set and the roles fall through.
+// Every mbarrier wait is bounded; on expiry the status word is set and the roles fall through.  Whether
+// they do or not, the producer and the MMA warp leave only after the copies and commits that they issued
+// have landed.
 #include <type_traits>
 
 #include "api.h"
@@ -105,6 +107,21 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* v) {
   return pk;
 }
 
+// The last uses of a ring of barriers (see ring_tail) have ended.
+__device__ __forceinline__ void drain_ring(uint64_t* bars, int count, int stages, uint64_t deadline,
+                                           int* status) {
+  ring_tail(count, stages, [&](int s, int parity) { mbar_drain(&bars[s], parity, deadline, status); });
+}
+// End of the MMA warp: every MMA issued so far is over, committed or not.  Returns the deadline for
+// what is left to wait for, the arrivals of the earlier commits.
+__device__ __forceinline__ uint64_t mmas_idle(uint64_t* idle, int* status) {
+  if (elect_one()) tc_commit(idle);
+  __syncwarp();
+  const uint64_t deadline = drain_deadline();
+  mbar_drain(idle, 0, deadline, status);
+  return deadline;
+}
+
 struct FwdParams {
   __nv_bfloat16* out;
   float* lse;
@@ -169,7 +186,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
   uint64_t* s_full = bars + 5;
   uint64_t* p_full = bars + 6;        // 128 arrivals
   uint64_t* o_done = bars + 7;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint64_t* idle = bars + 8;          // every MMA is over
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nblk = (p.seq + kBlk - 1) / kBlk;
@@ -181,7 +199,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
   const int row0 = b * p.seq;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 8; ++i) mbar_init(bars + i, i == 6 ? 128 : 1);
+    for (int i = 0; i < 9; ++i) mbar_init(bars + i, i == 6 ? 128 : 1);
     fence_barrier_init();
     fence_proxy_async();
     prefetch_tensormap(&map);
@@ -202,6 +220,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
       load_tile(sQ, &map, q_full, h * kD, row0 + qb * kBlk);
     }
     __syncwarp();
+    int k_loads = 0, v_loads = 0;
     for (int j = 0; j < n_kv; ++j) {
       if (!mbar_wait_warp(k_empty, (j & 1) ^ 1, p.status, kErrAttnWait)) break;
       if (elect_one()) {
@@ -209,16 +228,23 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
         load_tile(sK, &map, k_full, (p.hq + hk) * kD, row0 + j * kBlk);
       }
       __syncwarp();
+      ++k_loads;
       if (!mbar_wait_warp(v_empty, (j & 1) ^ 1, p.status, kErrAttnWait)) break;
       if (elect_one()) {
         mbar_expect_tx(v_full, kTile);
         load_tile(sV, &map, v_full, (p.hq + p.hkv + hk) * kD, row0 + j * kBlk);
       }
       __syncwarp();
+      ++v_loads;
     }
+    const uint64_t deadline = drain_deadline();
+    drain_ring(q_full, 1, 1, deadline, p.status);
+    drain_ring(k_full, k_loads, 1, deadline, p.status);
+    drain_ring(v_full, v_loads, 1, deadline, p.status);
   } else if (warp == 1) {
     const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV);
     bool ok = mbar_wait_warp(q_full, 0, p.status, kErrAttnWait);
+    int s_done = 0, pv_done = 0;
     for (int j = 0; j < n_kv && ok; ++j) {
       // S(j) may overwrite P(j-1): MMAs run in issue order, so P V of block j-1 has read it
       ok = mbar_wait_warp(k_full, j & 1, p.status, kErrAttnWait);
@@ -230,6 +256,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
         tc_commit(s_full);
       }
       __syncwarp();
+      ++s_done;
       ok = mbar_wait_warp(p_full, j & 1, p.status, kErrAttnWait) &&  // P in TMEM, O rescaled
            mbar_wait_warp(v_full, j & 1, p.status, kErrAttnWait);
       if (!ok) break;
@@ -240,7 +267,13 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
         if (j + 1 == n_kv) tc_commit(o_done);
       }
       __syncwarp();
+      ++pv_done;
     }
+    const uint64_t deadline = mmas_idle(idle, p.status);
+    drain_ring(k_empty, s_done, 1, deadline, p.status);
+    drain_ring(s_full, s_done, 1, deadline, p.status);
+    drain_ring(v_empty, pv_done, 1, deadline, p.status);
+    drain_ring(o_done, pv_done == n_kv, 1, deadline, p.status);
   } else {
     const int q = warp & 3;
     const int r = q * 32 + lane;                 // row inside the tile
@@ -433,7 +466,8 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
   uint64_t* k_empty = bars + 7;   // 3
   uint64_t* v_full = bars + 10;   // 2
   uint64_t* v_empty = bars + 12;  // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* idle = bars + 14;     // every MMA is over
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nblk = (p.seq + kBlk - 1) / kBlk;
@@ -445,7 +479,7 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
   const int row0 = b * p.seq;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 14; ++i) mbar_init(bars + i, i == 2 ? 256 : 1);
+    for (int i = 0; i < 15; ++i) mbar_init(bars + i, i == 2 ? 256 : 1);
     fence_barrier_init();
     fence_proxy_async();
     prefetch_tensormap(&map_qkv);
@@ -468,6 +502,7 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
       load_tile(sdO, &map_do, q_full, h * kD, row0 + qb * kBlk);
     }
     __syncwarp();
+    int k_loads = 0, v_loads = 0;
     for (int j = 0; j < n_kv; ++j) {
       const int ks = j % 3, vs = j & 1;
       if (!mbar_wait_warp(&k_empty[ks], ((j / 3) & 1) ^ 1, p.status, kErrAttnWait)) break;
@@ -476,13 +511,19 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
         load_tile(sK + ks * kTile, &map_qkv, &k_full[ks], (p.hq + hk) * kD, row0 + j * kBlk);
       }
       __syncwarp();
+      ++k_loads;
       if (!mbar_wait_warp(&v_empty[vs], ((j >> 1) & 1) ^ 1, p.status, kErrAttnWait)) break;
       if (elect_one()) {
         mbar_expect_tx(&v_full[vs], kTile);
         load_tile(sV + vs * kTile, &map_qkv, &v_full[vs], (p.hq + p.hkv + hk) * kD, row0 + j * kBlk);
       }
       __syncwarp();
+      ++v_loads;
     }
+    const uint64_t deadline = drain_deadline();
+    drain_ring(q_full, 1, 1, deadline, p.status);
+    drain_ring(k_full, k_loads, 3, deadline, p.status);
+    drain_ring(v_full, v_loads, 2, deadline, p.status);
   } else if (warp == 1) {
     const uint32_t aQ = smem_u32(sQ), adO = smem_u32(sdO), aK = smem_u32(sK), aV = smem_u32(sV);
     auto scores = [&](int j) {        // S(j) = Q K(j)^T
@@ -492,6 +533,7 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
       __syncwarp();
       return true;
     };
+    int dp_done = 0, dq_count = 0;
     auto dprobs = [&](int j) {        // dP(j) = dO V(j)^T; with it S(j), issued earlier, is complete too
       if (!mbar_wait_warp(&v_full[j & 1], (j >> 1) & 1, p.status, kErrAttnWait)) return false;
       tc_fence_after_sync();
@@ -501,6 +543,7 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
         tc_commit(sdp_full);
       }
       __syncwarp();
+      ++dp_done;
       return true;
     };
     bool ok = mbar_wait_warp(q_full, 0, p.status, kErrAttnWait);
@@ -518,8 +561,14 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
         if (j + 1 == n_kv) tc_commit(dq_done);
       }
       __syncwarp();
+      ++dq_count;
       if (j + 2 < n_kv) ok = scores(j + 2);     // over dS(j), which the MMA before has read
     }
+    const uint64_t deadline = mmas_idle(idle, p.status);
+    drain_ring(v_empty, dp_done, 2, deadline, p.status);
+    drain_ring(sdp_full, dp_done, 1, deadline, p.status);
+    drain_ring(k_empty, dq_count, 3, deadline, p.status);
+    drain_ring(dq_done, dq_count == n_kv, 1, deadline, p.status);
   } else {
     const int q = warp & 3, half = (warp - 2) >> 2;   // rows 32 q .., columns 64 half ..
     const int r = q * 32 + lane;
@@ -641,7 +690,8 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
   uint64_t* done = bars + 5;
   uint64_t* q_full = bars + 6;    // 2
   uint64_t* q_empty = bars + 8;   // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint64_t* idle = bars + 10;     // every MMA is over
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_q = (p.seq + kBlk - 1) / kBlk;
@@ -657,7 +707,7 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
   const int row0 = b * p.seq;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 10; ++i) mbar_init(bars + i, i == 3 || i == 4 ? 256 : 1);
+    for (int i = 0; i < 11; ++i) mbar_init(bars + i, i == 3 || i == 4 ? 256 : 1);
     fence_barrier_init();
     fence_proxy_async();
     prefetch_tensormap(&map_qkv);
@@ -680,6 +730,7 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
       load_tile(sV, &map_qkv, kv_full, (p.hq + p.hkv + hk) * kD, row0 + kb * kBlk);
     }
     __syncwarp();
+    int loads = 0;
     for (int t = 0; t < iters; ++t) {
       const int h = head0 + t / per_head;
       const int i = kb + t % per_head;
@@ -691,11 +742,16 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
         load_tile(sQ + s * 2 * kTile + kTile, &map_do, &q_full[s], h * kD, row0 + i * kBlk);
       }
       __syncwarp();
+      ++loads;
     }
+    const uint64_t deadline = drain_deadline();
+    drain_ring(kv_full, 1, 1, deadline, p.status);
+    drain_ring(q_full, loads, 2, deadline, p.status);
   } else if (warp == 1) {
     const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ);
     bool ok = mbar_wait_warp(kv_full, 0, p.status, kErrAttnWait) &&
               mbar_wait_warp(&q_full[0], 0, p.status, kErrAttnWait);
+    int s_done = 0, dp_done = 0, dk_done = 0;
     if (ok) {
       tc_fence_after_sync();
       if (elect_one()) {
@@ -705,6 +761,7 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
         tc_commit(dp_full);
       }
       __syncwarp();
+      s_done = dp_done = 1;
     }
     for (int t = 0; t < iters && ok; ++t) {
       const uint32_t q_t = aQ + (t & 1) * 2 * kTile, q_n = aQ + ((t + 1) & 1) * 2 * kTile;
@@ -721,6 +778,7 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
         }
       }
       __syncwarp();
+      s_done += more;
       ok = mbar_wait_warp(ds_full, t & 1, p.status, kErrAttnWait);
       if (!ok) break;
       tc_fence_after_sync();
@@ -735,7 +793,14 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
         }
       }
       __syncwarp();
+      ++dk_done;
+      dp_done += more;
     }
+    const uint64_t deadline = mmas_idle(idle, p.status);
+    drain_ring(s_full, s_done, 1, deadline, p.status);
+    drain_ring(dp_full, dp_done, 1, deadline, p.status);
+    drain_ring(q_empty, dk_done, 2, deadline, p.status);
+    drain_ring(done, dk_done == iters, 1, deadline, p.status);
   } else {
     const int q = warp & 3, half = (warp - 2) >> 2;
     const int r = q * 32 + lane;              // key row inside the tile

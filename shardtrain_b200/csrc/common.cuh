@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "pipeline_tail.h"
+
 namespace stb {
 
 // Status codes written to the status word (first writer wins).
@@ -168,6 +170,20 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, i
   return false;
 }
 
+// Wait for what is still in flight when a kernel leaves: it ends with the barrier's phase or at
+// `deadline` (see drain_deadline), whatever the status word says.  (mbar_wait gives up as soon as a
+// failure is on record, which is the very case in which copies and MMAs are left in flight.)
+__device__ __forceinline__ uint64_t drain_deadline() { return global_ns() + kWaitBudgetNs; }
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity, uint64_t deadline, int* status) {
+  for (;;) {
+    for (uint32_t i = 0; i < 256; ++i) {
+      if (mbar_try_wait(bar, parity)) return;
+    }
+    if (global_ns() > deadline) break;
+  }
+  if (status != nullptr) atomicCAS(status, kOk, kErrDrainWait);
+}
+
 // ----------------------------------------------------------------------------- CTA pairs
 // Helpers for kernels launched as clusters of two CTAs that share one tensor-core tile
 // (tcgen05 cta_group::2).  Rank 0 of the pair issues the MMAs and owns the barriers they wait on.
@@ -177,6 +193,7 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   return r;
 }
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();      // (the aligned forms want a converged warp)
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // shared::cluster address of `p` (an address of this CTA's shared memory) in the CTA of rank `rank`
@@ -187,6 +204,14 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t cluster_addr, uint32_t value) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(value) : "memory");
+}
+// Takes `bytes` off what the barrier's phase still expects: copies that were announced and will not come.
+__device__ __forceinline__ void mbar_complete_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
+               : "memory");
 }
 // CTA-pair form of kernel_should_skip: both CTAs of the pair return the same answer (a status word
 // that changes between their reads must not let one of them wait for the other).

@@ -194,7 +194,6 @@ gemm_allgather_kernel(const __grid_constant__ CUtensorMap tma_a,
   uint64_t* acc_full = a_empty + kAStages;     // [1]
   uint64_t* acc_empty = acc_full + 1;          // [1], 128 arrivals
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 1);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
   SegShared* segs = reinterpret_cast<SegShared*>(tmem_ptr + 4);   // 4 x 40 bytes, 16-byte aligned
 
   const int warp = threadIdx.x >> 5;
@@ -218,7 +217,6 @@ gemm_allgather_kernel(const __grid_constant__ CUtensorMap tma_a,
     }
     mbar_init(acc_full, 1);
     mbar_init(acc_empty, kProducers);
-    *abort_flag = 0;
     int first = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -262,7 +260,6 @@ gemm_allgather_kernel(const __grid_constant__ CUtensorMap tma_a,
               const int s = it % kAStages;
               if (!mbar_wait(&a_empty[s], ((it / kAStages) & 1) ^ 1, p.status,
                              kErrProducerEmptyWait)) {
-                *abort_flag = 1;
                 ok = false;
                 break;
               }
@@ -272,41 +269,32 @@ gemm_allgather_kernel(const __grid_constant__ CUtensorMap tma_a,
           }
         }
       }
-      if (*abort_flag) {   // error path only: drain the copies nobody consumed
-        for (int k = max(0, it - kAStages); k < it; ++k)
-          mbar_wait(&a_full[k % kAStages], (k / kAStages) & 1, p.status, kErrDrainWait);
-      }
+      // (the MMAs have waited for these copies, unless something failed)
+      const uint64_t deadline = drain_deadline();
+      ring_tail(it, kAStages, [&](int s, int parity) { mbar_drain(&a_full[s], parity, deadline, p.status); });
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(kBM, BN, false, false);
-      int ita = 0, itb = 0, round = 0;
+      int ita = 0, itb = 0, round = 0;     // stages and accumulator rounds committed so far
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        for (int pass = 0; pass < passes && ok; ++pass, ++round) {
+        for (int pass = 0; pass < passes; ++pass, ++round) {
           const int m_count = min(p.mt, m_tiles - pass * p.mt);
           // the epilogue of the previous round must have drained the accumulators
-          if (!mbar_wait(acc_empty, (round & 1) ^ 1, p.status, kErrMmaFullWait)) {
-            *abort_flag = 1;
-            break;
-          }
+          ok = mbar_wait(acc_empty, (round & 1) ^ 1, p.status, kErrMmaFullWait);
+          if (!ok) break;
           tc_fence_after_sync();
-          for (int kb = 0; kb < num_kb && ok; ++kb, ++itb) {
+          for (int kb = 0; kb < num_kb; ++kb, ++itb) {
             const int sb = itb % NB;
-            if (!mbar_wait(&b_full[sb], (itb / NB) & 1, p.status, kErrMmaFullWait)) {
-              *abort_flag = 1;
-              ok = false;
-              break;
-            }
+            ok = mbar_wait(&b_full[sb], (itb / NB) & 1, p.status, kErrMmaFullWait);
+            if (!ok) break;
             const uint32_t b_base = smem_u32(b_tiles + sb * S::kBTile);
             for (int m = 0; m < m_count; ++m, ++ita) {
               const int sa = ita % kAStages;
-              if (!mbar_wait(&a_full[sa], (ita / kAStages) & 1, p.status, kErrMmaFullWait)) {
-                *abort_flag = 1;
-                ok = false;
-                break;
-              }
+              ok = mbar_wait(&a_full[sa], (ita / kAStages) & 1, p.status, kErrMmaFullWait);
+              if (!ok) break;
               tc_fence_after_sync();
               const uint32_t a_base = smem_u32(a_tiles + sa * kATile);
 #pragma unroll
@@ -317,11 +305,18 @@ gemm_allgather_kernel(const __grid_constant__ CUtensorMap tma_a,
               }
               tc_commit(&a_empty[sa]);
             }
-            if (ok) tc_commit(&b_empty[sb]);   // the weight stage is free once these MMAs read it
+            if (!ok) break;
+            tc_commit(&b_empty[sb]);   // the weight stage is free once these MMAs read it
           }
-          if (ok) tc_commit(acc_full);
+          if (!ok) break;
+          tc_commit(acc_full);
         }
       }
+      // the commits' arrivals are in, and with them the MMAs are over
+      const uint64_t deadline = drain_deadline();
+      ring_tail(ita, kAStages, [&](int s, int parity) { mbar_drain(&a_empty[s], parity, deadline, p.status); });
+      ring_tail(itb, NB, [&](int s, int parity) { mbar_drain(&b_empty[s], parity, deadline, p.status); });
+      ring_tail(round, 1, [&](int, int parity) { mbar_drain(acc_full, parity, deadline, p.status); });
     }
   } else {
     // ------------------------------------------------------------ weight producers, then epilogue
@@ -408,7 +403,6 @@ gemm_allgather_kernel(const __grid_constant__ CUtensorMap tma_a,
           const int kb = (step + rot) % num_kb;
           const int sb = itb % NB;
           if (!mbar_wait(&b_empty[sb], ((itb / NB) & 1) ^ 1, p.status, kErrProducerEmptyWait)) {
-            *abort_flag = 1;
             ok = false;
             break;
           }

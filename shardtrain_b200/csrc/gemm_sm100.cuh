@@ -12,7 +12,6 @@
 // the epilogue (warp w reads TMEM lanes 32*(w%4)..+31, as the hardware requires).
 #pragma once
 #include "common.cuh"
-#include "pipeline_tail.h"
 
 namespace stb {
 
@@ -159,7 +158,14 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
   uint64_t* acc_full = empty_bar + STAGES;   // [2]
   uint64_t* acc_empty = acc_full + 2;        // [2], 128 arrivals each (pair: 256, on rank 0)
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  // [0] tmem_ptr, [1] a wait of the pair failed, [2] split reduction, then what a pair that gave up
+  // has in flight: k-blocks loaded by this CTA and (on rank 0) by the other one, k-blocks and tiles
+  // committed (on rank 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
+  volatile int* loads = abort_flag + 2;
+  volatile int* peer_loads = abort_flag + 3;
+  volatile int* peer_kblocks = abort_flag + 4;
+  volatile int* peer_tiles = abort_flag + 5;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -205,7 +211,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], PAIR ? 256 : 128);
     }
-    *abort_flag = 0;
+    for (int i = 0; i < 6; ++i) abort_flag[i] = 0;
     fence_barrier_init();
     fence_proxy_async();
     prefetch_tensormap(&tma_a);
@@ -241,6 +247,14 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
       tma_load_2d_pair(dst, map, leader_bar(bar), x, y);
     else
       tma_load_2d(dst, map, bar, x, y);
+  };
+  // A role of a pair leaves its loop early: both CTAs learn of it at the barrier they part at.  (A
+  // single CTA needs no flag: its warps wait for what they themselves have in flight.)
+  auto give_up = [&] {
+    if constexpr (PAIR) {
+      *abort_flag = 1;
+      st_cluster(cluster_addr(const_cast<int*>(abort_flag), rank ^ 1), 1u);
+    }
   };
   // an epilogue thread hands an accumulator buffer back to the MMA warp
   auto release_acc = [&](uint64_t* bar) {
@@ -289,7 +303,6 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
                   __any_sync(0xffffffffu,
                              status_failed(status) || global_ns() - t0 > kWaitBudgetNs)) {
                 if (status != nullptr) atomicCAS(status, kOk, kErrPullWait);
-                *abort_flag = 1;
                 ok = false;
                 break;
               }
@@ -306,7 +319,6 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait_warp(&empty_bar[s], ph ^ 1, status, kErrProducerEmptyWait)) {
-            *abort_flag = 1;
             ok = false;
             break;
           }
@@ -342,27 +354,24 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
           __syncwarp();
         }
       }
-      // Pair: rank 0's commits arrive at the empty barriers of both CTAs, and no later barrier tells
-      // that they have (a commit's arrival is ordered behind its MMAs, not behind other commits').
-      // Each CTA sees its own last ones in before the pair parts.  The epilogue is draining the last
-      // tile meanwhile, so the wait costs nothing.
       if constexpr (PAIR) {
-        if (ok)
+        // Rank 0's commits arrive at the empty barriers of both CTAs, and no later barrier tells that
+        // they have (a commit's arrival is ordered behind its MMAs, not behind other commits').  Each
+        // CTA sees its own last ones in before the pair parts: rank 1 here, rank 0 in its MMA warp.
+        // The epilogue is draining the last tile meanwhile, so the wait costs nothing.
+        if (ok && rank == 1)
           ring_tail(it, STAGES, [&](int s, int parity) {
             if (ok) ok = mbar_wait_warp(&empty_bar[s], parity, status, kErrDrainWait);
           });
-        if (!ok) *abort_flag = 1;
-      }
-      // Error path only: wait (bounded) for copies this thread issued that nobody consumed.
-      // (Pair: the copies of rank 1 complete on rank 0's barriers, which it cannot wait on; it
-      // stays for a millisecond, and the pair leaves together, see the end.)
-      const bool aborted = __any_sync(0xffffffffu, *abort_flag != 0);
-      if (aborted && rank == 0) {
-        for (int k = max(0, it - STAGES); k < it; ++k)
-          mbar_wait_warp(&full_bar[k % STAGES], (k / STAGES) & 1, status, kErrDrainWait);
-      } else if (aborted) {
-        const uint64_t t0 = global_ns();
-        while (global_ns() - t0 < 1000000ull) __nanosleep(1000);
+        if (!ok) give_up();
+        if (lane == 0) {
+          *loads = it;
+          if (rank == 1) st_cluster(cluster_addr(const_cast<int*>(peer_loads), 0), it);
+        }
+      } else {
+        // (the MMAs have waited for these copies, unless something failed)
+        const uint64_t deadline = drain_deadline();
+        ring_tail(it, STAGES, [&](int s, int parity) { mbar_drain(&full_bar[s], parity, deadline, status); });
       }
     }
   } else if (warp == 1) {
@@ -377,27 +386,22 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
       // 8192 B apart (the leading-dimension byte offset).
       const uint64_t desc_a0 = make_smem_desc_sw128(smem_u32(tiles), A_MN ? 8192 : 16, 1024);
       const uint64_t desc_b0 = make_smem_desc_sw128(smem_u32(tiles) + S::kABytes, B_MN ? 8192 : 16, 1024);
-      int it = 0, local = 0;
+      int it = 0, local = 0;      // k-blocks and tiles committed so far
       bool ok = true;
-      for (int unit = first_unit; unit < sp.total_units && ok; unit += unit_stride, ++local) {
+      for (int unit = first_unit; unit < sp.total_units; unit += unit_stride, ++local) {
         int tile, kb0, kb1, part;
         unit_work(unit, tile, kb0, kb1, part);
         const int ab = local & 1;
         // the epilogue must have drained this accumulator buffer (two tiles ago)
-        if (!mbar_wait_warp<PAIR>(&acc_empty[ab], ((local >> 1) & 1) ^ 1, status, kErrMmaFullWait)) {
-          *abort_flag = 1;
-          break;
-        }
+        ok = mbar_wait_warp<PAIR>(&acc_empty[ab], ((local >> 1) & 1) ^ 1, status, kErrMmaFullWait);
+        if (!ok) break;
         tc_fence_after_sync();
         const uint32_t tmem_d = tmem_base + ab * BN;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait_warp(&full_bar[s], ph, status, kErrMmaFullWait)) {
-            *abort_flag = 1;
-            ok = false;
-            break;
-          }
+          ok = mbar_wait_warp(&full_bar[s], ph, status, kErrMmaFullWait);
+          if (!ok) break;
           tc_fence_after_sync();
           // descriptors hold addresses in 16-byte units (below 2^14, so the sums never carry)
           const uint64_t da_s = desc_a0 + s * (S::kStageBytes >> 4);
@@ -418,11 +422,23 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
           }
           __syncwarp();
         }
+        if (!ok) break;
         if (elect_one()) {
           if constexpr (PAIR) tc_commit_pair(&acc_full[ab]); else tc_commit(&acc_full[ab]);
         }
         __syncwarp();
       }
+      if constexpr (PAIR) {
+        if (!ok) give_up();
+        if (lane == 0) {
+          st_cluster(cluster_addr(const_cast<int*>(peer_kblocks), 1), it);
+          st_cluster(cluster_addr(const_cast<int*>(peer_tiles), 1), local);
+        }
+      }
+      // the commits' arrivals are in, and with them the MMAs are over
+      const uint64_t deadline = drain_deadline();
+      ring_tail(it, STAGES, [&](int s, int parity) { mbar_drain(&empty_bar[s], parity, deadline, status); });
+      ring_tail(local, 2, [&](int b, int parity) { mbar_drain(&acc_full[b], parity, deadline, status); });
     }
   } else if (PULL && warp >= 6) {
     // Pull warps: copy groups of rows of A from their owners into the local buffer, lowest groups
@@ -494,7 +510,10 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
           if (col + 4 * j < N) res_next[j] = *reinterpret_cast<const float4*>(rs + 4 * j);
       };
       fetch_residual(0);
-      if (ok) ok = mbar_wait(&acc_full[ab], (local >> 1) & 1, status, kErrEpilogueAccumWait);
+      if (ok) {
+        ok = mbar_wait(&acc_full[ab], (local >> 1) & 1, status, kErrEpilogueAccumWait);
+        if (!ok) give_up();
+      }
       tc_fence_after_sync();
       const uint32_t tmem_d = tmem_base + ab * BN;
       const int64_t g_row = static_cast<int64_t>(m0) + row;
@@ -848,11 +867,37 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
   }
 
   tc_fence_before_sync();
-  if constexpr (PAIR)
+  if constexpr (PAIR) {
     cluster_sync();      // no thread of the other CTA signals this one or issues for it any more; what is
                          // asynchronous (copies, commits) was waited for above
-  else
+    if (*abort_flag != 0) {      // ... unless a role gave up: the same answer in both CTAs
+      if (warp == 0) {
+        const uint64_t deadline = drain_deadline();
+        auto wait_for = [&](uint64_t* bars) {
+          return [=](int i, int parity) { mbar_drain(&bars[i], parity, deadline, status); };
+        };
+        if (rank == 0) {
+          pair_copies_tail(
+              *loads, *peer_loads, STAGES,
+              [&](int s) {
+                if (lane == 0) mbar_expect_tx(&full_bar[s], S::kStageBytes);
+                __syncwarp();
+              },
+              [&](int s) {
+                if (lane == 0) mbar_complete_tx(&full_bar[s], S::kStageBytes);
+                __syncwarp();
+              },
+              wait_for(full_bar));
+        } else {
+          ring_tail(*peer_kblocks, STAGES, wait_for(empty_bar));
+          ring_tail(*peer_tiles, 2, wait_for(acc_full));
+        }
+      }
+      cluster_sync();
+    }
+  } else {
     __syncthreads();
+  }
   if (warp == 1) {
     tc_fence_after_sync();
     if constexpr (PAIR)

@@ -22,4 +22,22 @@ STB_HD void ring_tail(int count, int stages, Wait wait) {
   for (int k = count > stages ? count - stages : 0; k < count; ++k) wait(k % stages, (k / stages) & 1);
 }
 
+// The copies of a CTA pair.  Both CTAs load half of each k-block into a stage of their own and both
+// halves complete on rank 0's barrier, whose phase expects the two together.  When a pair gives up, its
+// ranks may have issued different numbers of k-blocks (never more than `stages` apart: a stage is
+// filled again only after both halves were used).  Rank 0 makes its barriers expect what was really
+// issued, then waits for it: expect(barrier) stands in for its own share of a block that only rank 1
+// loads, forgive(barrier) takes back rank 1's half of a block that only rank 0 loads.
+template <typename Expect, typename Forgive, typename Wait>
+STB_HD void pair_copies_tail(int mine, int theirs, int stages, Expect expect, Forgive forgive, Wait wait) {
+  const int most = mine > theirs ? mine : theirs;
+  for (int k = most > stages ? most - stages : 0; k < most; ++k) {
+    if (k >= mine)
+      expect(k % stages);
+    else if (k >= theirs)
+      forgive(k % stages);
+    wait(k % stages, (k / stages) & 1);
+  }
+}
+
 }  // namespace stb

@@ -79,3 +79,30 @@ def test_automatic_choice_has_the_bits_of_single_ctas(ops, shape):
         ops.gemm(a, b, out, a_mn, b_mn, None, None, False, 1.0, bn)
         outs.append(out)
     assert any(torch.equal(outs[0], o) for o in outs[1:])
+
+
+@pytest.mark.parametrize("pair", [True, False])
+def test_a_failure_on_record_ends_a_running_gemm(ops, pair):
+    """Another kernel records a failure while a long GEMM runs.  Its roles give up one after the other, in
+    whatever state their pipelines are; the kernel waits for the copies and MMAs it has in flight and
+    returns, and the next launch finds barriers, TMEM and tile counters in order."""
+    torch.manual_seed(6)
+    side, code = torch.cuda.Stream(), torch.full((1,), 7, dtype=torch.int32).pin_memory()
+    x, w = torch.randn(512, 4096, device=DEV).bfloat16(), torch.randn(1536, 4096, device=DEV).bfloat16()
+    want = torch.empty(512, 1536, device=DEV)
+    ops.gemm(x, w, want, False, False, None, None, False, 1.0, 256, 4, True, pair)
+    a = torch.randn(2048, 1 << 17, device=DEV).bfloat16()
+    out = torch.empty(2048, 2048, device=DEV)
+    torch.cuda.synchronize()
+    assert ops.status_read() == 0
+    for _ in range(3):
+        ops.gemm(a, a, out, False, False, None, None, False, 1.0, 128, 1, True, pair)     # about 1 ms each
+    with torch.cuda.stream(side):
+        ops.status_tensor()[:1].copy_(code, non_blocking=True)
+    torch.cuda.synchronize()
+    assert ops.status_read() == 7
+    ops.status_reset()
+    got = torch.empty_like(want)
+    ops.gemm(x, w, got, False, False, None, None, False, 1.0, 256, 4, True, pair)
+    assert ops.status_read() == 0
+    assert torch.equal(got, want)

@@ -71,3 +71,74 @@ def run_model(tmp_path, source):
 
 def test_a_pipeline_leaves_no_arrival_behind(tmp_path):
     run_model(tmp_path, MODEL)
+
+
+PAIR_MODEL = r"""
+#include <cstdio>
+#include <random>
+#include <vector>
+#include "pipeline_tail.h"
+
+// One arrival per phase; a phase ends once it has arrived and the announced bytes have come (which may
+// happen before they are announced).
+struct Barrier {
+  int phase = 0, arrivals = 0;
+  long tx = 0;
+  void settle() { if (arrivals == 1 && tx == 0) { ++phase; arrivals = 0; } }
+  void expect(long bytes) { tx += bytes; ++arrivals; settle(); }
+  void complete(long bytes) { tx -= bytes; settle(); }
+  bool ended(int parity) const { return (phase & 1) != parity; }
+};
+struct Copy { int block, rank; };
+constexpr long kHalf = 3;
+
+int give_up(int stages, int consumed, int mine, int theirs, bool fix, std::mt19937& rng) {
+  std::vector<Barrier> full(stages);
+  std::vector<Copy> flying;
+  auto land = [&](size_t i) {
+    full[flying[i].block % stages].complete(kHalf);
+    flying.erase(flying.begin() + i);
+  };
+  for (int k = 0; k < (mine > theirs ? mine : theirs); ++k) {
+    for (int rank = 0; rank < 2; ++rank)
+      if (k < (rank ? theirs : mine)) flying.push_back({k, rank});
+    if (k < mine) full[k % stages].expect(2 * kHalf);
+    if (k < consumed)                               // the MMAs took block k before its stage was reused
+      while (!flying.empty() && flying.front().block <= k) land(0);
+  }
+  while (!flying.empty() && rng() % 4) land(rng() % flying.size());
+  bool ok = true;
+  auto wait = [&](int s, int parity) {
+    while (ok && !full[s].ended(parity)) {
+      if (flying.empty()) ok = false; else land(rng() % flying.size());
+    }
+  };
+  if (fix)
+    stb::pair_copies_tail(mine, theirs, stages, [&](int s) { full[s].expect(kHalf); },
+                          [&](int s) { full[s].complete(kHalf); }, wait);
+  else
+    stb::ring_tail(mine, stages, wait);
+  return ok ? static_cast<int>(flying.size()) : -1;
+}
+
+int main() {
+  std::mt19937 rng(11);
+  int wrong_without = 0;
+  for (int stages : {1, 2, 3, 6, 8})
+    for (int consumed = 0; consumed <= 2 * stages + 1; ++consumed)
+      for (int mine = consumed; mine <= consumed + stages; ++mine)
+        for (int theirs = consumed; theirs <= consumed + stages; ++theirs)
+          for (int trial = 0; trial < 40; ++trial) {
+            const int left = give_up(stages, consumed, mine, theirs, true, rng);
+            if (left != 0)
+              return std::printf("stages %d consumed %d loads %d %d: %d\n", stages, consumed, mine, theirs, left), 1;
+            wrong_without += give_up(stages, consumed, mine, theirs, false, rng) != 0;
+          }
+  if (wrong_without == 0) return std::printf("the model never leaves early\n"), 1;
+  return 0;
+}
+"""
+
+
+def test_a_pair_that_gives_up_waits_for_what_each_rank_issued(tmp_path):
+    run_model(tmp_path, PAIR_MODEL)
