@@ -734,9 +734,13 @@ cudaError_t launch_slot_sum_rmsnorm(const float* slots, int n_slots, int64_t slo
 cudaError_t launch_rmsnorm_bwd(const float* dy, const float* x, const float* w, const float* inv,
                                const float* dres_in, float* dx_out, float* dw_partial,
                                int partial_rows, int rows, int cols, cudaStream_t s, void* dx_bf16) {
-  if (cols % 4 || partial_rows < 1) return cudaErrorInvalidValue;
+  // the bf16 copy leaves in 8-byte pieces
+  if (cols % 4 || partial_rows < 1 || (reinterpret_cast<uintptr_t>(dx_bf16) & 7))
+    return cudaErrorInvalidValue;
   __nv_bfloat16* copy = reinterpret_cast<__nv_bfloat16*>(dx_bf16);
-  switch ((cols + 1023) / 1024) {
+  // the row kernels write d(weight) in 16-byte pieces; the general one takes any float address
+  const bool wide = (reinterpret_cast<uintptr_t>(dw_partial) & 15) == 0;
+  switch (wide ? (cols + 1023) / 1024 : 0) {
     case 1:
       rmsnorm_bwd_rows_kernel<1><<<partial_rows, 256, 0, s>>>(dy, x, w, inv, dres_in, dx_out, copy,
                                                               dw_partial, rows, cols);
@@ -753,7 +757,7 @@ cudaError_t launch_rmsnorm_bwd(const float* dy, const float* x, const float* w, 
       rmsnorm_bwd_rows_kernel<4><<<partial_rows, 256, 0, s>>>(dy, x, w, inv, dres_in, dx_out, copy,
                                                               dw_partial, rows, cols);
       break;
-    default:     // wider rows than the registers hold
+    default:     // wider rows than the registers hold, or partial sums off a 16-byte boundary
       rmsnorm_bwd_kernel<<<partial_rows, 256, (cols + 32) * sizeof(float), s>>>(
           dy, x, w, inv, dres_in, dx_out, copy, dw_partial, rows, cols);
   }

@@ -83,3 +83,27 @@ def test_column_sums(ops, rows):
     total = base.clone()
     ops.colsum_bf16(xb, total, True, scratch)
     assert torch.all((total.double() - base.double() - xb.double().sum(0)).abs() <= bound + 2.0 ** -22 * base.abs())
+
+
+@pytest.mark.parametrize("cols", [260, 1536, 4096])
+@pytest.mark.parametrize("shift", [1, 2, 3])             # floats off a 16-byte boundary
+def test_rmsnorm_backward_takes_partial_sums_at_any_address(ops, cols, shift):
+    rows, parts = 37, 8
+    torch.manual_seed(cols)
+    dy, x, w = torch.randn(rows, cols, device=DEV), torch.randn(rows, cols, device=DEV), torch.randn(cols, device=DEV)
+    inv = torch.rsqrt(x.square().mean(-1) + 1e-6)
+    flat = torch.full((parts * cols + 8,), 7.0, device=DEV)
+    partial, aligned = flat[shift:shift + parts * cols].view(parts, cols), torch.empty(parts, cols, device=DEV)
+    dx, want = torch.empty_like(x), torch.empty_like(x)
+    ops.rmsnorm_bwd(dy, x, w, inv, None, dx, partial)
+    ops.rmsnorm_bwd(dy, x, w, inv, None, want, aligned)
+    assert torch.equal(dx, want) and torch.equal(partial, aligned)       # both kernels sum in the same order
+    assert torch.all(flat[:shift] == 7.0) and torch.all(flat[shift + parts * cols:] == 7.0)
+
+
+def test_rmsnorm_backward_refuses_a_copy_off_an_8_byte_boundary(ops):
+    x, w = torch.randn(4, 64, device=DEV), torch.randn(64, device=DEV)
+    copy = torch.empty(4 * 64 + 2, device=DEV, dtype=torch.bfloat16)[2:].view(4, 64)
+    with pytest.raises(RuntimeError, match="rmsnorm_bwd"):
+        ops.rmsnorm_bwd(x, x, w, torch.ones(4, device=DEV), None, torch.empty_like(x), torch.empty(2, 64, device=DEV),
+                        copy)
