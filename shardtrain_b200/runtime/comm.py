@@ -510,7 +510,11 @@ class CommunicationCoordinator:
         `after_streams` and for each event in `after_events`.  The ticket's `ready_event` is
         recorded behind the kernels.  Ordering between GPUs is carried by flags in peer memory,
         so neither policy adds edges here; the per-communicator sequence is still recorded.
+        `launch` None: the data is where it belongs already.  The ticket keeps its place in the
+        sequence and its event, and the log says that nothing ran (`launched` false, no elements).
         """
+        if launch is None:
+            numel = 0
         _, members, _ = self._describe_group(group)
         seq = self.sequence.get(pg_id, 0)
         if self.expected_sequence is not None:
@@ -533,7 +537,7 @@ class CommunicationCoordinator:
                 self.event("collective_issue", op_id=ticket.op_id, pg_id=pg_id, pg_seq=seq, kind=kind,
                            numel=numel, dtype="torch.float32", op_kind=kind, pg_local_seq=seq,
                            group_members=list(members), group_role=ticket.group_role,
-                           issue_stream=channel, backend="peer_kernel",
+                           issue_stream=channel, backend="peer_kernel", launched=launch is not None,
                            output_buffer_ids=[l.buffer_id for l in leases])
             for name in after_streams:
                 produced = torch.cuda.Event()
@@ -544,8 +548,9 @@ class CommunicationCoordinator:
                                     consumer="collective_input", wait_stream=channel, producer_stream=name)
             for event in after_events:
                 stream.wait_event(event)
-            with StreamScope(self, stream):
-                launch()
+            if launch is not None:
+                with StreamScope(self, stream):
+                    launch()
             if self.diagnostics_enabled:
                 self.event("work_issued", op_id=ticket.op_id, work_issued=False, issue_stream=channel)
             ticket.ready_event = torch.cuda.Event()

@@ -368,8 +368,6 @@ class PeerMaterializer:
         in_arena = plan.arena_slot is not None
 
         def launch():
-            if in_arena and not runtime.last_microstep:
-                return
             arenas.reduce_peer.barrier("fsdp_rs")     # no-op for a single member
             if fuse_adamw:
                 hp = runtime.fused_optimizer_args()
@@ -386,7 +384,8 @@ class PeerMaterializer:
         comm = self.comm
         ticket = comm.issue_kernel(
             "fsdp_grad", "fsdp_rs_accumulate_adamw" if fuse_adamw else "fsdp_rs_accumulate",
-            self.group, launch, channel="fsdp_rs", after_streams=("compute",),
+            self.group, None if in_arena and not runtime.last_microstep else launch,
+            channel="fsdp_rs", after_streams=("compute",),
             numel=plan.grad_numel, group_role="main_gradient_bucket")
         if not runtime.async_grad_rs:
             comm.consume(ticket, consumer="main_gradient_bucket")

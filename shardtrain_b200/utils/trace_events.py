@@ -22,7 +22,7 @@ from shardtrain_b200.utils.audit import read_events
 INSTANTS = {"step_end", "optimizer_ready", "prefetch_boundary", "parameter_shards_ready",
             "backward_prefetch_token", "runtime_failed"}
 KEEP = ("step_id", "unit_id", "phase", "kind", "numel", "dtype", "pg_id", "pg_local_seq", "group_role",
-        "group_members", "dependency_type", "target_unit", "scheduling_boundary", "reason")
+        "group_members", "launched", "dependency_type", "target_unit", "scheduling_boundary", "reason")
 
 
 def _args(row: dict) -> dict:

@@ -183,3 +183,43 @@ def test_reduce_rejects_a_missing_gradient():
     unit = SimpleNamespace(runtime=SimpleNamespace(), unit_id=3, handles=[SimpleNamespace(spec=spec)])
     with pytest.raises(RuntimeError, match="Missing full parameter gradient U3"):
         Materializer(None, comm).reduce(unit, [None])
+
+
+def test_the_log_of_a_single_member_tells_which_micro_steps_launch_a_reduction(monkeypatch):
+    """Without peers the gradients of a unit are in the arena already: earlier micro-steps launch
+    nothing, and the log must not show a reduction or a payload for them; the last one checks (and
+    updates) and logs what it went over."""
+    from types import SimpleNamespace
+
+    from shardtrain_b200.runtime.materializer import PeerMaterializer
+
+    monkeypatch.setattr(torch.cuda, "Event", lambda: SimpleNamespace(record=lambda stream: None))
+    monkeypatch.setattr(torch.cuda, "set_stream", lambda stream: None)
+    comm = CommunicationCoordinator("cpu")
+    stream = SimpleNamespace(cuda_stream=1, wait_event=lambda event: None)
+    comm.streams = {"fsdp_rs": stream, "compute": stream}
+    monkeypatch.setattr(comm, "current_stream", lambda: stream)
+    launches = []
+    slot = SimpleNamespace(multicast_ptr=0, peer_ptrs=[0])
+    runtime = SimpleNamespace(
+        sp=False, async_grad_rs=True, last_microstep=False, first_commit=lambda unit: True,
+        fused_optimizer_armed=lambda unit: False, mark_committed=lambda handle, ticket: None,
+        fused=SimpleNamespace(grad_slot=lambda unit: slot, grad_slot_issued=lambda *a: None))
+    unit = SimpleNamespace(runtime=runtime, unit_id=0,
+                           handles=[SimpleNamespace(spec=SimpleNamespace(param_id="w"))])
+    mat = PeerMaterializer(None, comm, None)
+    mat.plans[0] = SimpleNamespace(arena_slot=slot, reduce_table=None, grad_numel=12, shard_numel=12)
+    mat.bind(SimpleNamespace(reduce_scatter=lambda *a: launches.append(a)),
+             SimpleNamespace(tp_degree=1, tp_rank=0, grad=None, check_flags=None,
+                             reduce_peer=SimpleNamespace(barrier=lambda name: None)))
+    for last in (False, True):
+        runtime.last_microstep = last
+        mat.reduce(unit, [torch.zeros(1)])
+    rows = [e for e in comm.events if e["event_type"] == "collective_issue"]
+    assert [(r["launched"], r["numel"]) for r in rows] == [(False, 0), (True, 12)]
+    assert len(launches) == 1 and [t.pg_local_seq for t in comm.tickets] == [0, 1]
+    mat.plans[0].arena_slot = None          # peers: every micro-step reduces
+    runtime.last_microstep = False
+    mat.reduce(unit, [torch.zeros(1)])
+    row = [e for e in comm.events if e["event_type"] == "collective_issue"][-1]
+    assert (row["launched"], row["numel"], len(launches)) == (True, 12, 2)
