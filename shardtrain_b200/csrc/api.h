@@ -31,7 +31,7 @@ struct GemmCall {
   bool accumulate;
   float alpha;
   int force_bn;  // 0 = rule, else 128, 192 or 256
-  int force_pair;  // with force_bn: 1 = CTA pairs on 256 x force_bn tiles, 0 = one CTA per 128-row tile
+  int force_pair;  // 1 = CTA pairs on 256-row tiles; 0 = one CTA per 128-row tile (without force_bn: rule)
   int split_k;   // K-split of the tail wave's tiles: 0 = rule, 1 = never, n = exactly n
   // 0 = plain outputs leave through TMA stores staged in shared memory when the output's base
   // and pitch allow it; -1 = always the per-thread row stores
@@ -61,6 +61,14 @@ struct GemmCall {
   int64_t pull_src_ld;
 };
 cudaError_t launch_gemm_bf16(const GemmCall& c, int* status, cudaStream_t stream);
+// What launch_gemm_bf16 runs for this call (only sizes and options count): tile width, CTA pairs or
+// single CTAs, K ranges per tile of the last wave.
+struct GemmTile {
+  int bn = 0;
+  bool pair = false;
+  int split = 1;     // as GemmCall::split_k
+};
+GemmTile gemm_tile(const GemmCall& c);
 
 // ------------------------------------------------------------------ elementwise (elementwise.cu)
 cudaError_t launch_rmsnorm_fwd(const float* x, const float* w, void* y, float* inv, int rows,

@@ -178,6 +178,20 @@ void gemm_scatter(const Tensor& a, const Tensor& b, c10::ArrayRef<int64_t> dest_
   check(stb::launch_gemm_bf16(c, status_ptr(), cur_stream()), "gemm_scatter");
 }
 
+// {tile width, CTA pairs?, K ranges per tile of the last wave} that `gemm` (or, with gated_inter,
+// `gemm_swiglu`) runs for these sizes
+std::vector<int64_t> gemm_tile(int64_t m, int64_t n, int64_t k, int64_t gated_inter, bool force_pair) {
+  TORCH_CHECK(m > 0 && n > 0 && k > 0 && gated_inter >= 0, "gemm_tile: sizes");
+  stb::GemmCall c{};
+  c.M = static_cast<int>(m);
+  c.N = static_cast<int>(n);
+  c.K = static_cast<int>(k);
+  c.gated_inter = static_cast<int>(gated_inter);
+  c.force_pair = force_pair ? 1 : 0;
+  const stb::GemmTile t = stb::gemm_tile(c);
+  return {t.bn, t.pair ? 1 : 0, t.split};
+}
+
 // gate|up projection with the SwiGLU epilogue: gu [M, 2*inter] and h = silu(gate) * up [M, inter]
 void gemm_swiglu(const Tensor& a, const Tensor& w_gu, Tensor gu, Tensor h) {
   need(a, at::kBFloat16, "a");
@@ -872,6 +886,7 @@ TORCH_LIBRARY(stb, m) {
         "bool accumulate, float alpha, int force_bn, int split_k=0, bool staged_store=True, "
         "bool force_pair=False) -> ()",
         &gemm);
+  m.def("gemm_tile(int m, int n, int k, int gated_inter=0, bool force_pair=False) -> int[]", &gemm_tile);
   m.def("gemm_scatter", &gemm_scatter);
   m.def("gemm_seq_pull", &gemm_seq_pull);
   m.def("gemm_swiglu", &gemm_swiglu);

@@ -332,13 +332,6 @@ cudaError_t dispatch_major(const GemmCall& c, int* status, cudaStream_t stream) 
   return launch_variant<BN, true, false, PAIR>(c, status, stream);
 }
 
-// Tile shape and tail split of one GEMM.
-struct TileChoice {
-  int bn = 0;
-  bool pair = false;
-  int split = 1;     // as GemmCall::split_k
-};
-
 // Clocks of one 64-wide k-block, measured on B200 over 8192 x 8192 x {1536, 8192} (the MMAs alone
 // need 2 BN):
 //     BN                      128    192    256
@@ -367,12 +360,28 @@ double estimate(const GemmCall& c, bool pair, int bn, int want_split) {
   return cost;
 }
 
-TileChoice choose_tile(const GemmCall& c) {
+GemmTile choose_tile(const GemmCall& c) {
   const int sms = sm_count();
   const int num_kb = (c.K + kGemmBK - 1) / kGemmBK;
   const int want = c.gated_inter > 0 ? 1 : c.split_k;
   const bool may_pair = c.pull_degree <= 1;
-  TileChoice best;
+  GemmTile best;
+  if (c.force_pair) {      // the caller wants pairs: the width that is fastest for them
+    if (sms < 2) return best;      // (no width: refused)
+    double cost = -1.0;
+    for (int cand : {256, 192, 128}) {
+      if (c.gated_inter > 0 && cand != 256) continue;
+      const double e = estimate(c, true, cand, want);
+      if (cost < 0 || e < cost) {
+        int full, kb_per;
+        cost = e;
+        best.bn = cand;
+        best.pair = true;
+        best.split = plan_split(sms / 2, tiles_of(c, true, cand), num_kb, want, &full, &kb_per);
+      }
+    }
+    return best;
+  }
   // Which elements are summed in several K ranges (and in how many) is settled on 128-row tiles
   // alone: the width whose waves x (128 + BN) is smallest, the tail wave counting 1 / split.  It
   // decides the bits of the result, so it does not depend on the kernel that then runs.
@@ -421,6 +430,15 @@ TileChoice choose_tile(const GemmCall& c) {
 
 }  // namespace
 
+GemmTile gemm_tile(const GemmCall& c) {
+  if (c.force_bn == 0) return choose_tile(c);
+  GemmTile t;
+  t.bn = c.force_bn;
+  t.pair = c.force_pair != 0;
+  t.split = c.split_k;
+  return t;
+}
+
 cudaError_t launch_gemm_bf16(const GemmCall& call, int* status, cudaStream_t stream) {
   GemmCall c = call;
   if (c.M <= 0 || c.N <= 0 || c.K <= 0) return cudaErrorInvalidValue;
@@ -460,15 +478,9 @@ cudaError_t launch_gemm_bf16(const GemmCall& call, int* status, cudaStream_t str
         !aligned16(c.gated_out) || c.N != 2 * c.gated_inter || c.gated_inter % 8)
       return cudaErrorInvalidValue;
   }
-  TileChoice t;
-  if (c.force_bn != 0) {
-    t.bn = c.force_bn;
-    t.pair = c.force_pair != 0;
-    if (t.pair && c.pull_degree > 1) return cudaErrorInvalidValue;
-  } else {
-    t = choose_tile(c);
-    c.split_k = t.split;
-  }
+  const GemmTile t = gemm_tile(c);
+  if (t.pair && c.pull_degree > 1) return cudaErrorInvalidValue;
+  c.split_k = t.split;
   if (c.gated_inter > 0 && t.bn != 256) return cudaErrorInvalidValue;
   if (t.pair) {
     if (t.bn == 256) return dispatch_major<256, true>(c, status, stream);

@@ -106,3 +106,21 @@ def test_a_failure_on_record_ends_a_running_gemm(ops, pair):
     ops.gemm(x, w, got, False, False, None, None, False, 1.0, 256, 4, True, pair)
     assert ops.status_read() == 0
     assert torch.equal(got, want)
+
+
+def test_forced_pairs_run_as_pairs_whatever_the_width(ops):
+    """`force_pair` without a width used to run whatever the rule picked."""
+    M, N, K = 300, 520, 200
+    assert ops.gemm_tile(M, N, K)[1] == 0                       # the rule takes single CTAs here
+    bn, pair, split = ops.gemm_tile(M, N, K, 0, True)
+    assert pair == 1 and bn in (128, 192, 256) and split == 1
+    torch.manual_seed(3)
+    a, b = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16()
+    outs = []
+    for width in (0, bn):
+        out = torch.empty(M, N, device=DEV)
+        ops.gemm(a, b, out, False, False, None, None, False, 1.0, width, 0, True, True)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    _, pair, split = ops.gemm_tile(512, 1536, 8960, 0, True)    # too few tiles for 74 pairs: cut along K
+    assert pair == 1 and split > 1
