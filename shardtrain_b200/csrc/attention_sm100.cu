@@ -107,19 +107,10 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* v) {
   return pk;
 }
 
-// The last uses of a ring of barriers (see ring_tail) have ended.
-__device__ __forceinline__ void drain_ring(uint64_t* bars, int count, int stages, uint64_t deadline,
-                                           int* status) {
-  ring_tail(count, stages, [&](int s, int parity) { mbar_drain(&bars[s], parity, deadline, status); });
-}
-// End of the MMA warp: every MMA issued so far is over, committed or not.  Returns the deadline for
-// what is left to wait for, the arrivals of the earlier commits.
-__device__ __forceinline__ uint64_t mmas_idle(uint64_t* idle, int* status) {
+// End of the MMA warp: one more commit, behind every MMA issued so far, committed or not.
+__device__ __forceinline__ void commit_all(uint64_t* idle) {
   if (elect_one()) tc_commit(idle);
   __syncwarp();
-  const uint64_t deadline = drain_deadline();
-  mbar_drain(idle, 0, deadline, status);
-  return deadline;
 }
 
 struct FwdParams {
@@ -237,10 +228,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
       __syncwarp();
       ++v_loads;
     }
-    const uint64_t deadline = drain_deadline();
-    drain_ring(q_full, 1, 1, deadline, p.status);
-    drain_ring(k_full, k_loads, 1, deadline, p.status);
-    drain_ring(v_full, v_loads, 1, deadline, p.status);
+    // q_full, k_full, -, v_full
+    mbar_drain(bars + lane, lane == 0 ? 1 : lane == 1 ? k_loads : lane == 3 ? v_loads : 0, p.status);
   } else if (warp == 1) {
     const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV);
     bool ok = mbar_wait_warp(q_full, 0, p.status, kErrAttnWait);
@@ -269,11 +258,10 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
       __syncwarp();
       ++pv_done;
     }
-    const uint64_t deadline = mmas_idle(idle, p.status);
-    drain_ring(k_empty, s_done, 1, deadline, p.status);
-    drain_ring(s_full, s_done, 1, deadline, p.status);
-    drain_ring(v_empty, pv_done, 1, deadline, p.status);
-    drain_ring(o_done, pv_done == n_kv, 1, deadline, p.status);
+    commit_all(idle);
+    // k_empty, s_full; v_empty; o_done; idle
+    mbar_drain(bars + lane, lane == 2 || lane == 5 ? s_done : lane == 4 ? pv_done
+                            : lane == 7 ? pv_done == n_kv : lane == 8, p.status);
   } else {
     const int q = warp & 3;
     const int r = q * 32 + lane;                 // row inside the tile
@@ -520,10 +508,9 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
       __syncwarp();
       ++v_loads;
     }
-    const uint64_t deadline = drain_deadline();
-    drain_ring(q_full, 1, 1, deadline, p.status);
-    drain_ring(k_full, k_loads, 3, deadline, p.status);
-    drain_ring(v_full, v_loads, 2, deadline, p.status);
+    // q_full; k_full[3]; v_full[2]
+    mbar_drain(bars + lane, lane == 0 ? 1 : lane >= 4 && lane < 7 ? ring_uses(k_loads, 3, lane - 4)
+                            : lane == 10 || lane == 11 ? ring_uses(v_loads, 2, lane - 10) : 0, p.status);
   } else if (warp == 1) {
     const uint32_t aQ = smem_u32(sQ), adO = smem_u32(sdO), aK = smem_u32(sK), aV = smem_u32(sV);
     auto scores = [&](int j) {        // S(j) = Q K(j)^T
@@ -564,11 +551,11 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
       ++dq_count;
       if (j + 2 < n_kv) ok = scores(j + 2);     // over dS(j), which the MMA before has read
     }
-    const uint64_t deadline = mmas_idle(idle, p.status);
-    drain_ring(v_empty, dp_done, 2, deadline, p.status);
-    drain_ring(sdp_full, dp_done, 1, deadline, p.status);
-    drain_ring(k_empty, dq_count, 3, deadline, p.status);
-    drain_ring(dq_done, dq_count == n_kv, 1, deadline, p.status);
+    commit_all(idle);
+    // sdp_full; dq_done; k_empty[3]; v_empty[2]; idle
+    mbar_drain(bars + lane, lane == 1 ? dp_done : lane == 3 ? dq_count == n_kv
+                            : lane >= 7 && lane < 10 ? ring_uses(dq_count, 3, lane - 7)
+                            : lane == 12 || lane == 13 ? ring_uses(dp_done, 2, lane - 12) : lane == 14, p.status);
   } else {
     const int q = warp & 3, half = (warp - 2) >> 2;   // rows 32 q .., columns 64 half ..
     const int r = q * 32 + lane;
@@ -744,9 +731,8 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
       __syncwarp();
       ++loads;
     }
-    const uint64_t deadline = drain_deadline();
-    drain_ring(kv_full, 1, 1, deadline, p.status);
-    drain_ring(q_full, loads, 2, deadline, p.status);
+    // kv_full; q_full[2]
+    mbar_drain(bars + lane, lane == 0 ? 1 : lane == 6 || lane == 7 ? ring_uses(loads, 2, lane - 6) : 0, p.status);
   } else if (warp == 1) {
     const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ);
     bool ok = mbar_wait_warp(kv_full, 0, p.status, kErrAttnWait) &&
@@ -796,11 +782,10 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
       ++dk_done;
       dp_done += more;
     }
-    const uint64_t deadline = mmas_idle(idle, p.status);
-    drain_ring(s_full, s_done, 1, deadline, p.status);
-    drain_ring(dp_full, dp_done, 1, deadline, p.status);
-    drain_ring(q_empty, dk_done, 2, deadline, p.status);
-    drain_ring(done, dk_done == iters, 1, deadline, p.status);
+    commit_all(idle);
+    // s_full; dp_full; done; q_empty[2]; idle
+    mbar_drain(bars + lane, lane == 1 ? s_done : lane == 2 ? dp_done : lane == 5 ? dk_done == iters
+                            : lane == 8 || lane == 9 ? ring_uses(dk_done, 2, lane - 8) : lane == 10, p.status);
   } else {
     const int q = warp & 3, half = (warp - 2) >> 2;
     const int r = q * 32 + lane;              // key row inside the tile

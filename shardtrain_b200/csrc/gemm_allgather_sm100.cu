@@ -246,8 +246,8 @@ gemm_allgather_kernel(const __grid_constant__ CUtensorMap tma_a,
 
   if (warp == 0) {
     // ------------------------------------------------------------ A: TMA from local memory
+    int it = 0;
     if (lane == 0) {
-      int it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         const int rot = k_rotation(tile, num_kb);
@@ -269,15 +269,15 @@ gemm_allgather_kernel(const __grid_constant__ CUtensorMap tma_a,
           }
         }
       }
-      // (the MMAs have waited for these copies, unless something failed)
-      const uint64_t deadline = drain_deadline();
-      ring_tail(it, kAStages, [&](int s, int parity) { mbar_drain(&a_full[s], parity, deadline, p.status); });
     }
+    // (the MMAs have waited for these copies, unless something failed)
+    it = __shfl_sync(0xffffffffu, it, 0);
+    mbar_drain(&a_full[lane], lane < kAStages ? ring_uses(it, kAStages, lane) : 0, p.status);
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
+    int ita = 0, itb = 0, round = 0;       // stages and accumulator rounds committed so far
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(kBM, BN, false, false);
-      int ita = 0, itb = 0, round = 0;     // stages and accumulator rounds committed so far
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         for (int pass = 0; pass < passes; ++pass, ++round) {
@@ -312,12 +312,21 @@ gemm_allgather_kernel(const __grid_constant__ CUtensorMap tma_a,
           tc_commit(acc_full);
         }
       }
-      // the commits' arrivals are in, and with them the MMAs are over
-      const uint64_t deadline = drain_deadline();
-      ring_tail(ita, kAStages, [&](int s, int parity) { mbar_drain(&a_empty[s], parity, deadline, p.status); });
-      ring_tail(itb, NB, [&](int s, int parity) { mbar_drain(&b_empty[s], parity, deadline, p.status); });
-      ring_tail(round, 1, [&](int, int parity) { mbar_drain(acc_full, parity, deadline, p.status); });
     }
+    // the commits' arrivals are in, and with them the MMAs are over
+    ita = __shfl_sync(0xffffffffu, ita, 0);
+    itb = __shfl_sync(0xffffffffu, itb, 0);
+    round = __shfl_sync(0xffffffffu, round, 0);
+    uint64_t* bar = acc_full;
+    int uses = lane == 0 ? round : 0;
+    if (lane >= 1 && lane < 1 + kAStages) {
+      bar = &a_empty[lane - 1];
+      uses = ring_uses(ita, kAStages, lane - 1);
+    } else if (lane >= 16 && lane < 16 + NB) {
+      bar = &b_empty[lane - 16];
+      uses = ring_uses(itb, NB, lane - 16);
+    }
+    mbar_drain(bar, uses, p.status);
   } else {
     // ------------------------------------------------------------ weight producers, then epilogue
     const int t = threadIdx.x - 64;          // 0..127

@@ -257,6 +257,12 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
     }
   };
   // an epilogue thread hands an accumulator buffer back to the MMA warp
+  // phases that the commits of `kblocks` k-blocks and `tiles` tiles end on barrier `lane` of the row
+  // empty_bar[STAGES], acc_full[2]
+  auto committed = [&](int kblocks, int tiles) {
+    if (lane < STAGES) return ring_uses(kblocks, STAGES, lane);
+    return lane < STAGES + 2 ? ring_uses(tiles, 2, lane - STAGES) : 0;
+  };
   auto release_acc = [&](uint64_t* bar) {
     if constexpr (PAIR)
       mbar_arrive_cluster(leader_bar(bar));
@@ -360,9 +366,8 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
         // CTA sees its own last ones in before the pair parts: rank 1 here, rank 0 in its MMA warp.
         // The epilogue is draining the last tile meanwhile, so the wait costs nothing.
         if (ok && rank == 1)
-          ring_tail(it, STAGES, [&](int s, int parity) {
-            if (ok) ok = mbar_wait_warp(&empty_bar[s], parity, status, kErrDrainWait);
-          });
+          for (int k = max(0, it - STAGES); k < it && ok; ++k)
+            ok = mbar_wait_warp(&empty_bar[k % STAGES], (k / STAGES) & 1, status, kErrDrainWait);
         if (!ok) give_up();
         if (lane == 0) {
           *loads = it;
@@ -370,8 +375,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
         }
       } else {
         // (the MMAs have waited for these copies, unless something failed)
-        const uint64_t deadline = drain_deadline();
-        ring_tail(it, STAGES, [&](int s, int parity) { mbar_drain(&full_bar[s], parity, deadline, status); });
+        mbar_drain(&full_bar[lane], lane < STAGES ? ring_uses(it, STAGES, lane) : 0, status);
       }
     }
   } else if (warp == 1) {
@@ -436,9 +440,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
         }
       }
       // the commits' arrivals are in, and with them the MMAs are over
-      const uint64_t deadline = drain_deadline();
-      ring_tail(it, STAGES, [&](int s, int parity) { mbar_drain(&empty_bar[s], parity, deadline, status); });
-      ring_tail(local, 2, [&](int b, int parity) { mbar_drain(&acc_full[b], parity, deadline, status); });
+      mbar_drain(&empty_bar[lane], committed(it, local), status);
     }
   } else if (PULL && warp >= 6) {
     // Pull warps: copy groups of rows of A from their owners into the local buffer, lowest groups
@@ -872,25 +874,14 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
                          // asynchronous (copies, commits) was waited for above
     if (*abort_flag != 0) {      // ... unless a role gave up: the same answer in both CTAs
       if (warp == 0) {
-        const uint64_t deadline = drain_deadline();
-        auto wait_for = [&](uint64_t* bars) {
-          return [=](int i, int parity) { mbar_drain(&bars[i], parity, deadline, status); };
-        };
         if (rank == 0) {
-          pair_copies_tail(
-              *loads, *peer_loads, STAGES,
-              [&](int s) {
-                if (lane == 0) mbar_expect_tx(&full_bar[s], S::kStageBytes);
-                __syncwarp();
-              },
-              [&](int s) {
-                if (lane == 0) mbar_complete_tx(&full_bar[s], S::kStageBytes);
-                __syncwarp();
-              },
-              wait_for(full_bar));
+          PairStage stage{};
+          if (lane < STAGES) stage = pair_stage(*loads, *peer_loads, STAGES, lane);
+          if (stage.expect) mbar_expect_tx(&full_bar[lane], S::kStageBytes);
+          if (stage.forgive) mbar_complete_tx(&full_bar[lane], S::kStageBytes);
+          mbar_drain(&full_bar[lane], stage.uses, status);
         } else {
-          ring_tail(*peer_kblocks, STAGES, wait_for(empty_bar));
-          ring_tail(*peer_tiles, 2, wait_for(acc_full));
+          mbar_drain(&empty_bar[lane], committed(*peer_kblocks, *peer_tiles), status);
         }
       }
       cluster_sync();

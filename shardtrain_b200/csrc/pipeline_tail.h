@@ -14,30 +14,24 @@
 
 namespace stb {
 
-// A ring of `stages` barriers of which use k ends phase k / stages of barrier k % stages: after
-// `count` uses, wait(barrier, parity) is called for the last use of every barrier that had one.
-// (The uses before those have ended: a barrier's next use waits for its last one.)
-template <typename Wait>
-STB_HD void ring_tail(int count, int stages, Wait wait) {
-  for (int k = count > stages ? count - stages : 0; k < count; ++k) wait(k % stages, (k / stages) & 1);
-}
+// A ring of `stages` barriers of which use k ends a phase of barrier k % stages: how many phases of
+// barrier `s` the first `count` uses end.  (Waiting for the last of them is enough: a barrier's next use
+// waits for the one before.)
+STB_HD int ring_uses(int count, int stages, int s) { return count > s ? (count - s - 1) / stages + 1 : 0; }
 
 // The copies of a CTA pair.  Both CTAs load half of each k-block into a stage of their own and both
 // halves complete on rank 0's barrier, whose phase expects the two together.  When a pair gives up, its
 // ranks may have issued different numbers of k-blocks (never more than `stages` apart: a stage is
 // filled again only after both halves were used).  Rank 0 makes its barriers expect what was really
-// issued, then waits for it: expect(barrier) stands in for its own share of a block that only rank 1
-// loads, forgive(barrier) takes back rank 1's half of a block that only rank 0 loads.
-template <typename Expect, typename Forgive, typename Wait>
-STB_HD void pair_copies_tail(int mine, int theirs, int stages, Expect expect, Forgive forgive, Wait wait) {
-  const int most = mine > theirs ? mine : theirs;
-  for (int k = most > stages ? most - stages : 0; k < most; ++k) {
-    if (k >= mine)
-      expect(k % stages);
-    else if (k >= theirs)
-      forgive(k % stages);
-    wait(k % stages, (k / stages) & 1);
-  }
+// issued, then waits for it.
+struct PairStage {
+  int uses;       // phases of rank 0's barrier to wait for
+  bool expect;    // rank 1 has loaded a block that rank 0 has not: stand in for rank 0's arrival
+  bool forgive;   // rank 0 has loaded a block that rank 1 has not: take rank 1's half back
+};
+STB_HD PairStage pair_stage(int mine, int theirs, int stages, int s) {
+  const int a = ring_uses(mine, stages, s), b = ring_uses(theirs, stages, s);
+  return PairStage{a > b ? a : b, b > a, a > b};
 }
 
 }  // namespace stb

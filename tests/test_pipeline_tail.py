@@ -40,7 +40,10 @@ int leave(int count, int stages, bool tail, std::mt19937& rng) {
     if (rng() % 2 && !ring.pending.empty()) ring.land(rng() % ring.pending.size());
   }
   bool ok = true;
-  if (tail) stb::ring_tail(count, stages, [&](int s, int parity) { ok = ok && wait(s, parity); });
+  for (int s = 0; tail && s < stages; ++s) {
+    const int uses = stb::ring_uses(count, stages, s);
+    if (uses > 0) ok = ok && wait(s, (uses - 1) & 1);
+  }
   return ok ? static_cast<int>(ring.pending.size()) : -1;
 }
 
@@ -113,11 +116,13 @@ int give_up(int stages, int consumed, int mine, int theirs, bool fix, std::mt199
       if (flying.empty()) ok = false; else land(rng() % flying.size());
     }
   };
-  if (fix)
-    stb::pair_copies_tail(mine, theirs, stages, [&](int s) { full[s].expect(kHalf); },
-                          [&](int s) { full[s].complete(kHalf); }, wait);
-  else
-    stb::ring_tail(mine, stages, wait);
+  for (int s = 0; s < stages; ++s) {
+    stb::PairStage stage = stb::pair_stage(mine, theirs, stages, s);
+    if (!fix) stage = {stb::ring_uses(mine, stages, s), false, false};
+    if (stage.expect) full[s].expect(kHalf);
+    if (stage.forgive) full[s].complete(kHalf);
+    if (stage.uses > 0) wait(s, (stage.uses - 1) & 1);
+  }
   return ok ? static_cast<int>(flying.size()) : -1;
 }
 
