@@ -2,7 +2,8 @@
 // kernels (dK/dV per key block, dQ per query block).  All five/seven matrix products run on
 // tcgen05 with accumulators in TMEM; Q/K/V/dO tiles arrive by TMA from the packed, rope-applied
 // qkv buffer; the softmax warps read scores from TMEM with tcgen05.ld and hand P / dS back to the
-// tensor core as TMEM operands.  No S x S matrix ever reaches global memory (the reference materialises it: src/sharded_runtime/models/qwen2.py:247-257).
+// tensor core as TMEM operands.  No S x S matrix ever reaches global memory (the reference materialises
+// it: src/sharded_runtime/models/qwen2.py:247-257).
 //
 // Tile = 128 x 128 (rows x head_dim or rows x rows) bf16, held as two 64-column halves of 16 KB
 // (128 rows x 128 bytes, TMA SWIZZLE_128B).  The same tile serves as a K-major operand (reduction
@@ -43,7 +44,8 @@ __device__ __forceinline__ uint64_t desc_mn(uint32_t tile, int kk) {
 
 // The MMAs below are issued by a warp that stays converged, one elected lane doing the work: then
 // addresses and descriptors are warp-uniform.  (Issued inside `if (lane == 0)` an MMA cost about 136
-// clocks whatever its size.)
+// clocks whatever its size.)  Where an MMA overwrites columns of TMEM that the one before it reads as its
+// A operand, the kernels take it that MMAs issued by one thread run in that order.
 
 // D[128x128] = A B^T over a 128-long reduction, both tiles K-major: 8 MMAs of K = 16.
 __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint32_t a_tile, uint32_t b_tile) {
@@ -152,10 +154,13 @@ __device__ __forceinline__ void load_key_bits(const uint32_t* bits, int pitch, c
 // exponentials and the other way round).  To fit twice, a CTA keeps S and O in 256 TMEM columns,
 // with P (bf16) written over the S it came from and read by the MMA as a TMEM operand, and one
 // stage each of K and V: 97 KB of shared memory.  CTAs start with the longest rows of blocks, so
-// the short ones fill the last wave.  Bound by the exponentials (1024 clocks a block) and the
-// softmax's issue slots.
+// the short ones fill the last wave.
+// Bound by the latency of the chain, not by a pipe: at 2 x 2048 (12 heads) the tensor pipe is active
+// 24 % of the cycles, the exponentials' unit 24 %, issue slots are used to 35 %, and warps mostly wait
+// for TMEM loads and barriers.  At 1 x 8192 a block takes 2300 to 3200 clocks of an SM (1.4 to 1.965
+// GHz); its exponentials need 1024, its products 1024.
 // Measured on B200 (12 heads): 1 x 8192, causal, 1576 us before (one CTA per SM, MMAs issued from
-// one lane, P through shared memory) and 311 us now; 8 x 512: 100 and 35 us.
+// one lane, P through shared memory) and 274 us now; 8 x 512: 100 and 33 us.
 // smem: Q | K | V | barriers
 constexpr int kFwdSmem = 3 * kTile + 1024 + 128;
 
@@ -429,6 +434,9 @@ struct BwdParams {
 // j, S(j+1) runs; when they are done, dP(j+1) goes first and dQ += dS(j) K(j) and S(j+2) run under
 // the softmax of block j+1, so the chain of a block is dP and half a row of exponentials per
 // thread.  K has three stages (K(j) is held until dQ), V two.
+// The chain is still what bounds it: at 2 x 2048 (12 heads) the tensor pipe is active 34 % of the cycles,
+// the exponentials' unit 23 %, issue slots are used to 28 %.  At 1 x 8192 a block takes 3100 to 4300
+// clocks (1.4 to 1.965 GHz); its products need 1536.
 // Measured on B200 inside a training step (12 heads): 1 x 8192: 764 us before (serial chain, one
 // thread per row, MMAs issued from one lane) and 371 us now; 8 x 512: 51 and 38 us.
 // smem: Q | dO | K x 3 | V x 2 | barriers
@@ -627,7 +635,9 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
       }
       const int first = qb * kBlk + q * 32;
       const int64_t width = static_cast<int64_t>(p.hq + 2 * p.hkv) * kD;
-      if (ok) rows.flush(p.dqkv + static_cast<int64_t>(row0 + first) * width + h * kD, width, min(32, p.seq - first));
+      if (ok)
+        rows.flush(p.dqkv + static_cast<int64_t>(row0 + first) * width + h * kD, width,
+                   min(32, p.seq - first));
     }
   }
   tc_fence_before_sync();
@@ -651,7 +661,10 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
 // columns, and read by the MMAs from TMEM.  The two chains S^T -> P^T -> dV and dP^T -> dS^T -> dK
 // hand over separately: while the softmax warps take exponentials of block t+1, dK(t) and dP^T(t+1)
 // run, and while they form dS^T(t+1), dV(t+1) and S^T(t+2) run.  Q and dO have two stages.
-// Bound by the four products (2048 clocks a block).
+// Bound by the chain of hand-overs and by the grid: at 2 x 2048 (12 heads, 2 kv heads) the tensor pipe is
+// active 39 % of the cycles, issue slots are used to 29 %, and SMs are busy for 87 to 149 thousand cycles
+// (mean 115): the CTAs of the first key blocks are the longest.  At 1 x 8192 a block takes 4200 to
+// 5900 clocks (1.4 to 1.965 GHz); its products need 2048.
 // Measured on B200 inside a training step (12 heads, 2 kv heads): 1 x 8192: 1188 us before (serial
 // chain, P^T and dS^T through shared memory, one thread per row) and 507 us now; 8 x 512: 80 and 42 us.
 // smem: K | V | (Q, dO) x 2 | (lse[128], delta[128]) x 2 | barriers

@@ -8,8 +8,9 @@
 // (K,K), (K,MN) and (MN,MN).  This replaces the reference's F.linear / `@` call sites
 // (src/sharded_runtime/runtime/qwen2_operators.py:55-64, 78-96, 122-125, 138-143).
 //
-// CTA = 6 warps: warp 0 issues TMA, warp 1 owns TMEM and issues MMAs (one lane), warps 2..5 are
-// the epilogue (warp w reads TMEM lanes 32*(w%4)..+31, as the hardware requires).
+// CTA = 6 warps: warp 0 issues TMA, warp 1 owns TMEM and issues MMAs (both stay converged and elect the
+// issuing lane), warps 2..5 are the epilogue (warp w reads TMEM lanes 32*(w%4)..+31, as the hardware
+// requires).
 #pragma once
 #include "common.cuh"
 
@@ -256,13 +257,13 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
       st_cluster(cluster_addr(const_cast<int*>(abort_flag), rank ^ 1), 1u);
     }
   };
-  // an epilogue thread hands an accumulator buffer back to the MMA warp
   // phases that the commits of `kblocks` k-blocks and `tiles` tiles end on barrier `lane` of the row
   // empty_bar[STAGES], acc_full[2]
   auto committed = [&](int kblocks, int tiles) {
     if (lane < STAGES) return ring_uses(kblocks, STAGES, lane);
     return lane < STAGES + 2 ? ring_uses(tiles, 2, lane - STAGES) : 0;
   };
+  // an epilogue thread hands an accumulator buffer back to the MMA warp
   auto release_acc = [&](uint64_t* bar) {
     if constexpr (PAIR)
       mbar_arrive_cluster(leader_bar(bar));

@@ -275,9 +275,10 @@ SpLink make_link(cudaStream_t st, int* status, c10::ArrayRef<int64_t> pads, int6
 // Replay of launch sequences (CUDA graphs).
 //
 // A training step presents every decoder layer with the same addresses, shapes and scalars as the
-// step before: the weights live in per-unit buffers allocated once, the gradient slots rotate with
-// a period that divides the step, and the activations a layer produces are owned here, so they
-// too keep their addresses.  A sequence is therefore keyed by EVERYTHING its kernels receive
+// step before: the weights live in per-unit buffers allocated once, the gradient slots are windows of
+// the gradient arena (a single member; the key then says whether they are stored to or added to) or
+// rotate with a period that divides the step, and the activations a layer produces are owned here, so
+// they too keep their addresses.  A sequence is therefore keyed by EVERYTHING its kernels receive
 // (every pointer, pitch and scalar, the stream); the first time a key is seen the sequence is
 // launched kernel by kernel into buffers that the cache entry owns, the second time it is
 // captured into a graph, and from then on one cudaGraphLaunch replaces the 10 or 20 launches.
@@ -601,10 +602,11 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
   auto launch = [&](std::vector<Tensor>& b) {
     Tensor& dx = b[0];
     ok(stb::launch_cast_f32_to_bf16(d_out.data_ptr<float>(), t.d_out_b.data_ptr(), M * H, st), "cast");
-    g.run(t.d_out_b, hm, g_down, true, true, nullptr, nullptr, SeqPull{}, accumulate);                 // dW down
+    g.run(t.d_out_b, hm, g_down, true, true, nullptr, nullptr, SeqPull{}, accumulate);   // dW down
     g.run(t.d_out_b, w_down, t.d_hm, false, true, nullptr, nullptr);            // dX down
-    ok(stb::launch_swiglu_bwd(t.d_hm.data_ptr(), gu.data_ptr(), t.d_gu.data_ptr(), M, inter, st), "swiglu_bwd");
-    g.run(t.d_gu, h2, g_gate_up, true, true, nullptr, nullptr, SeqPull{}, accumulate);                 // dW gate|up
+    ok(stb::launch_swiglu_bwd(t.d_hm.data_ptr(), gu.data_ptr(), t.d_gu.data_ptr(), M, inter, st),
+       "swiglu_bwd");
+    g.run(t.d_gu, h2, g_gate_up, true, true, nullptr, nullptr, SeqPull{}, accumulate);   // dW gate|up
     g.run(t.d_gu, w_gu, t.d_h2, false, true, nullptr, nullptr);                 // dX gate|up
     ok(stb::launch_rmsnorm_bwd(t.d_h2.data_ptr<float>(), x_mid.data_ptr<float>(), ln2.data_ptr<float>(),
                                inv2.data_ptr<float>(), d_out.data_ptr<float>(), t.d_mid.data_ptr<float>(),
@@ -612,7 +614,7 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
                                t.d_mid_b.data_ptr()), "rmsnorm_bwd");
     ok(stb::launch_colsum_f32(t.partial.data_ptr<float>(), g_ln2.data_ptr<float>(), kNormPartialRows, H,
                               accumulate, st), "colsum");
-    g.run(t.d_mid_b, attn, g_o, true, true, nullptr, nullptr, SeqPull{}, accumulate);                  // dW o
+    g.run(t.d_mid_b, attn, g_o, true, true, nullptr, nullptr, SeqPull{}, accumulate);    // dW o
     g.run(t.d_mid_b, w_o, t.d_attn, false, true, nullptr, nullptr);             // dX o
     stb::AttnBwdCall bc{};
     bc.qkv = qkv.data_ptr();
@@ -636,7 +638,7 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
                         hkv, D, true, st), "rope inverse");
     ok(stb::launch_colsum_bf16(t.d_qkv.data_ptr(), W, g_bias.data_ptr<float>(), M, W, accumulate,
                                t.bias_partial.data_ptr<float>(), 64, st), "bias colsum");
-    g.run(t.d_qkv, h1, g_qkv, true, true, nullptr, nullptr, SeqPull{}, accumulate);                    // dW q|k|v
+    g.run(t.d_qkv, h1, g_qkv, true, true, nullptr, nullptr, SeqPull{}, accumulate);      // dW q|k|v
     g.run(t.d_qkv, w_qkv, t.d_h1, false, true, nullptr, nullptr);               // dX q|k|v
     ok(stb::launch_rmsnorm_bwd(t.d_h1.data_ptr<float>(), x2.data_ptr<float>(), ln1.data_ptr<float>(),
                                inv1.data_ptr<float>(), t.d_mid.data_ptr<float>(), dx.data_ptr<float>(),

@@ -421,7 +421,8 @@ class FusedExecutor:
     def acquire_grad_slot(self, unit):
         if getattr(unit, "grad_slot", None) is None:
             own = self.runtime.materializer.plans[unit.unit_id].arena_slot
-            unit.grad_slot = own if own is not None else self.ring.acquire(unit.unit_id, self.runtime.comm.current_stream())
+            unit.grad_slot = own if own is not None else self.ring.acquire(
+                unit.unit_id, self.runtime.comm.current_stream())
         return unit.grad_slot
 
     def grad_slot(self, unit):

@@ -83,7 +83,8 @@ class QwenTrainer:
         """1 if every rank's gradients (and the loss) are finite, as an int32 device tensor."""
         runtime = self.runtime
         if runtime.fused is not None:
-            # written by the gradient-check kernel of every micro-step
+            # written by the kernels that reduce or check gradients; a single member's check the sums
+            # of all micro-steps, once, in the last one (what is not finite stays so when added to)
             finite = runtime.fused._flags[0].eq(0).to(torch.int32)
         else:
             finite = torch.isfinite(runtime.grad_arena).all().to(torch.int32)
