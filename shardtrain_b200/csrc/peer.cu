@@ -156,31 +156,63 @@ __global__ void gather_params_kernel(PeerPtrs shards, ShadowPtrs shadows, int us
   }
 }
 
+// Gradient reduction (+ AdamW).  Bound by memory: with AdamW 30 bytes per element (gradient read; p, m,
+// v read and written; bf16 shadow written).  It runs on its own stream under the backward, which sets its
+// shape.  A CTA takes ONE tile and leaves: a kernel of the compute stream (higher priority) that needs
+// whole SMs can be placed only when the CTAs in its way have left, and with CTAs that lived for a sixth
+// of the sweep every layer's gate|up dW GEMM (pairs of CTAs) stood still for that long -- 65 us at the
+// 1.5B widths, 380 us twice a layer at the 7B widths.  A thread keeps 128 bytes of loads in flight, the
+// first of them issued before the status word is known.  Alone, in place: 46.8 M elements 217 us (6470
+// GB/s; 248 us before), 233 M 1038 us (1187), the check alone 33 us (84); tiles of 2048 and 8192
+// elements ran the training steps no faster.
+constexpr int kRsThreads = 256;
+constexpr int kRsGroups = 2;                                     // float4 groups a thread loads at once
+constexpr int kRsRound = kRsThreads * 4 * kRsGroups;
+constexpr int kRsTile = 2 * kRsRound;                            // 4096 elements
+struct RsTable {
+  SegmentDesc s[kMaxSegs];
+  int first[kMaxSegs + 1];                                       // first tile of each segment
+  int n;
+};
+
+__device__ __forceinline__ void adamw_update(float& p, float& m, float& v, float g, const AdamWArgs& a,
+                                             float step_size, float inv_bc2_sqrt) {
+  const float gr = g * a.grad_scale;
+  p *= 1.f - a.lr * a.weight_decay;
+  m = a.beta1 * m + (1.f - a.beta1) * gr;
+  v = a.beta2 * v + (1.f - a.beta2) * gr * gr;
+  p -= step_size * m / (sqrtf(v) * inv_bc2_sqrt + a.eps);
+}
+
 // Rank `rank` owns elements [rank*q, rank*q + q) of each segment (zero beyond numel).
 // With a tensor-parallel axis (tp > 1) `full` lists the gradient slots of the whole mesh in rank
 // order (index f * tp + t).  A TP-split parameter is summed over the F ranks of this rank's TP
 // coordinate; a TP-replicated one (segment flag `pad`) over all F * tp ranks, scaled by
 // rep_scale -- the T-way sum that the reference issues as a separate all-reduce after its
 // reduce-scatter (src/sharded_runtime/runtime/materializer.py:228-233).
-template <bool ADAMW>
-__global__ void reduce_scatter_kernel(PeerPtrs full, int degree, int rank, int tp, int tp_rank,
-                                      SegTable tab, float* gshard /* may be the slot itself */,
-                                      float* __restrict__ p, float* __restrict__ m,
-                                      float* __restrict__ v, float split_scale, float rep_scale,
-                                      int accumulate, AdamWArgs a, int* __restrict__ flags,
-                                      __nv_bfloat16* __restrict__ shadow, const int* status,
-                                      const float* __restrict__ multicast) {
+// LOCAL: a single member (degree * tp == 1), plain loads.
+template <bool ADAMW, bool LOCAL>
+__global__ void __launch_bounds__(kRsThreads, 4)
+    reduce_scatter_kernel(PeerPtrs full, int degree, int rank, int tp, int tp_rank, RsTable tab,
+                          float* gshard /* may be the slot itself */, float* __restrict__ p,
+                          float* __restrict__ m, float* __restrict__ v, float split_scale,
+                          float rep_scale, int accumulate, AdamWArgs a, int* __restrict__ flags,
+                          __nv_bfloat16* __restrict__ shadow, const int* status,
+                          const float* __restrict__ multicast) {
   // A failure recorded earlier (a peer that never signalled) means the slots may hold stale
-  // data: neither the gradient shard nor, with ADAMW, the parameters are touched.
-  if (kernel_should_skip(status)) return;
-  const SegmentDesc sg = tab.s[blockIdx.y];
-  const bool replicated = tp > 1 && sg.pad != 0;
-  const int n_src = replicated ? degree * tp : degree;
+  // data: neither the gradient shard nor, with ADAMW, the parameters are touched.  (Every thread asks
+  // for itself, nothing below needs them to agree.)
+  const bool skip = status_failed(status);
+  int seg = 0;
+  while (seg + 1 < tab.n && static_cast<int>(blockIdx.x) >= tab.first[seg + 1]) ++seg;
+  const SegmentDesc& sg = tab.s[seg];
+  const bool replicated = !LOCAL && tp > 1 && sg.pad != 0;
+  const int n_src = LOCAL ? 1 : replicated ? degree * tp : degree;
   // replicated segments use one fixed summation order so every TP replica computes bit-identical
   // shard gradients (and updates); split segments rotate the order to spread the load
   const int first = replicated ? 0 : rank;
   const int stride = replicated ? 1 : tp;
-  const int offset = replicated ? 0 : tp_rank;
+  const int offset = LOCAL || replicated ? 0 : tp_rank;
   const float scale = replicated ? rep_scale : split_scale;
   const int64_t lo = static_cast<int64_t>(rank) * sg.q;
   const int64_t valid = max(static_cast<int64_t>(0), min(sg.q, sg.numel - lo));
@@ -193,93 +225,114 @@ __global__ void reduce_scatter_kernel(PeerPtrs full, int degree, int rank, int t
   // the gradient check rides along: flags[0] = a non-finite reduced gradient was written,
   // flags[1] = a padding element of the shard is not exactly zero
   int bad = 0, pad_bad = 0;
-  for (int64_t chunk = blockIdx.x; chunk * kChunk < sg.q; chunk += gridDim.x) {
-    const int64_t base = chunk * kChunk;
-    const int64_t end = min(base + kChunk, sg.q);
-    const int step = vec ? 4 : 1;
-    for (int64_t i = base + threadIdx.x * step; i < end; i += blockDim.x * step) {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      const int cnt = vec ? 4 : 1;
-      if (vec && i + 3 < valid && multicast != nullptr && !replicated) {
+  const int64_t base = static_cast<int64_t>(blockIdx.x - tab.first[seg]) * kRsTile;
+  const int64_t end = min(base + kRsTile, sg.q);
+  if (vec && base + kRsTile <= valid) {
+    // whole tile: 16-byte accesses, every load of a round in flight before the first use.  p, m and v
+    // stream past (nobody reads them again in this step): they should not push GEMM operands out of L2
+#pragma unroll 1
+    for (int64_t i = base + threadIdx.x * 4; i < base + kRsTile; i += kRsRound) {
+      const int64_t e = sg.shard_off + i;
+      float4 g[kRsGroups], pv[kRsGroups], mv[kRsGroups], vv[kRsGroups];
+      auto load_state = [&] {
+#pragma unroll
+        for (int u = 0; u < kRsGroups; ++u) {
+          pv[u] = __ldcs(reinterpret_cast<const float4*>(p + e + u * kRsThreads * 4));
+          mv[u] = __ldcs(reinterpret_cast<const float4*>(m + e + u * kRsThreads * 4));
+          vv[u] = __ldcs(reinterpret_cast<const float4*>(v + e + u * kRsThreads * 4));
+        }
+      };
+      if (ADAMW && LOCAL) load_state();
+      if (LOCAL) {
+        const float* src = full.p[0] + sg.full_off + i;
+#pragma unroll
+        for (int u = 0; u < kRsGroups; ++u)
+          g[u] = *reinterpret_cast<const float4*>(src + u * kRsThreads * 4);
+      } else if (multicast != nullptr && !replicated) {
         // NVLS: one load through the multicast address of the gradient slot; the NVSwitch reads
         // the same 16 bytes of every member's slot, adds them and returns the sum, so only
         // 1 / F of the gradient enters this GPU instead of (F - 1) / F
-        float4 t;
-        asm volatile("multimem.ld_reduce.relaxed.sys.global.add.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
-                     : "l"(multicast + sg.full_off + lo + i)
-                     : "memory");
-        acc[0] = t.x; acc[1] = t.y; acc[2] = t.z; acc[3] = t.w;
-      } else if (vec && i + 3 < valid) {
+#pragma unroll
+        for (int u = 0; u < kRsGroups; ++u)
+          asm volatile("multimem.ld_reduce.relaxed.sys.global.add.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(g[u].x), "=f"(g[u].y), "=f"(g[u].z), "=f"(g[u].w)
+                       : "l"(multicast + sg.full_off + lo + i + u * kRsThreads * 4)
+                       : "memory");
+      } else {
+#pragma unroll
+        for (int u = 0; u < kRsGroups; ++u) g[u] = make_float4(0.f, 0.f, 0.f, 0.f);
         // rotate the peer order by rank so the ranks do not all hit one peer at once
         for (int d = 0; d < n_src; ++d) {
           const int src = ((first + d) % n_src) * stride + offset;
-          const float4 t =
-              *reinterpret_cast<const float4*>(full.p[src] + sg.full_off + lo + i);
-          acc[0] += t.x; acc[1] += t.y; acc[2] += t.z; acc[3] += t.w;
-        }
-      } else {
-        for (int j = 0; j < cnt; ++j) {
-          if (i + j < valid) {
-            for (int d = 0; d < n_src; ++d) {
-              const int src = ((first + d) % n_src) * stride + offset;
-              acc[j] += full.p[src][sg.full_off + lo + i + j];
-            }
+          const float* from = full.p[src] + sg.full_off + lo + i;
+#pragma unroll
+          for (int u = 0; u < kRsGroups; ++u) {
+            const float4 t = *reinterpret_cast<const float4*>(from + u * kRsThreads * 4);
+            g[u].x += t.x; g[u].y += t.y; g[u].z += t.z; g[u].w += t.w;
           }
         }
       }
-      if (vec) {
-        // q % 4 == 0: the four elements are inside the shard; 16-byte accesses throughout
-        const int64_t e = sg.shard_off + i;
-        float4 g = make_float4(acc[0] * scale, acc[1] * scale, acc[2] * scale, acc[3] * scale);
-        if (accumulate) {
-          const float4 o = *reinterpret_cast<const float4*>(gshard + e);
-          g.x += o.x; g.y += o.y; g.z += o.z; g.w += o.w;
-        }
-        if (!in_place) *reinterpret_cast<float4*>(gshard + e) = g;   // padding stays exactly zero: acc is 0 there
-        bad |= !(isfinite(g.x) && isfinite(g.y) && isfinite(g.z) && isfinite(g.w));
-        if (i + 3 >= valid) {
-          const float* gp = &g.x;
-          for (int j = 0; j < 4; ++j)
-            if (i + j >= valid && gp[j] != 0.f) pad_bad = 1;
-        }
-        if (ADAMW) {
-          float4 pv = *reinterpret_cast<const float4*>(p + e);
-          float4 mv = *reinterpret_cast<const float4*>(m + e);
-          float4 vv = *reinterpret_cast<const float4*>(v + e);
-          float* pp = &pv.x; float* mp = &mv.x; float* vp = &vv.x; const float* gp = &g.x;
+      if (skip) return;
+      if (ADAMW && !LOCAL) load_state();       // (before the sum they would spill)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float gr = gp[j] * a.grad_scale;
-            pp[j] *= 1.f - a.lr * a.weight_decay;
-            mp[j] = a.beta1 * mp[j] + (1.f - a.beta1) * gr;
-            vp[j] = a.beta2 * vp[j] + (1.f - a.beta2) * gr * gr;
-            pp[j] -= step_size * mp[j] / (sqrtf(vp[j]) * inv_bc2_sqrt + a.eps);
-          }
-          *reinterpret_cast<float4*>(p + e) = pv;   // padding has p = g = m = v = 0 and stays 0
-          if (shadow != nullptr) {                   // compute-dtype copy for the next gather
-            uint2 pk;
-            pk.x = pk2(pv.x, pv.y);
-            pk.y = pk2(pv.z, pv.w);
-            *reinterpret_cast<uint2*>(shadow + e) = pk;
-          }
-          *reinterpret_cast<float4*>(m + e) = mv;
-          *reinterpret_cast<float4*>(v + e) = vv;
+      for (int u = 0; u < kRsGroups; ++u) {
+        const int64_t eu = e + u * kRsThreads * 4;
+        g[u].x *= scale; g[u].y *= scale; g[u].z *= scale; g[u].w *= scale;
+        if (accumulate) {
+          const float4 o = *reinterpret_cast<const float4*>(gshard + eu);
+          g[u].x += o.x; g[u].y += o.y; g[u].z += o.z; g[u].w += o.w;
         }
-      } else {
-        const int64_t e = sg.shard_off + i;
-        float g = acc[0] * scale;
-        if (accumulate) g += gshard[e];
-        if (!in_place) gshard[e] = g;
-        bad |= !isfinite(g);
-        if (i >= valid && g != 0.f) pad_bad = 1;
+        if (!in_place) *reinterpret_cast<float4*>(gshard + eu) = g[u];
+        bad |= !(isfinite(g[u].x) && isfinite(g[u].y) && isfinite(g[u].z) && isfinite(g[u].w));
         if (ADAMW) {
-          float pj = p[e] * (1.f - a.lr * a.weight_decay);
-          const float gr = g * a.grad_scale;
-          const float mj = a.beta1 * m[e] + (1.f - a.beta1) * gr;
-          const float vj = a.beta2 * v[e] + (1.f - a.beta2) * gr * gr;
-          pj -= step_size * mj / (sqrtf(vj) * inv_bc2_sqrt + a.eps);
-          p[e] = pj;
+          adamw_update(pv[u].x, mv[u].x, vv[u].x, g[u].x, a, step_size, inv_bc2_sqrt);
+          adamw_update(pv[u].y, mv[u].y, vv[u].y, g[u].y, a, step_size, inv_bc2_sqrt);
+          adamw_update(pv[u].z, mv[u].z, vv[u].z, g[u].z, a, step_size, inv_bc2_sqrt);
+          adamw_update(pv[u].w, mv[u].w, vv[u].w, g[u].w, a, step_size, inv_bc2_sqrt);
+          __stcs(reinterpret_cast<float4*>(p + eu), pv[u]);
+          __stcs(reinterpret_cast<float4*>(m + eu), mv[u]);
+          __stcs(reinterpret_cast<float4*>(v + eu), vv[u]);
+          if (shadow != nullptr)                     // compute-dtype copy for the next gather
+            *reinterpret_cast<uint2*>(shadow + eu) =
+                make_uint2(pk2(pv[u].x, pv[u].y), pk2(pv[u].z, pv[u].w));
+        }
+      }
+    }
+  } else {
+    // the last tile of a segment, or one that is not aligned
+    if (skip) return;
+    const int step = vec ? 4 : 1;
+    for (int64_t i = base + threadIdx.x * step; i < end; i += kRsThreads * step) {
+      const bool quad = vec && i + 3 < valid;
+#pragma unroll 1
+      for (int j = 0; j < step; ++j) {
+        const int64_t e = sg.shard_off + i + j;
+        float acc = 0.f;
+        if (i + j < valid) {
+          if (!LOCAL && quad && multicast != nullptr && !replicated) {
+            // the switch adds 16 bytes at a time; each of the four elements takes its own part
+            float4 t;
+            asm volatile("multimem.ld_reduce.relaxed.sys.global.add.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
+                         : "l"(multicast + sg.full_off + lo + i)
+                         : "memory");
+            acc = j == 0 ? t.x : j == 1 ? t.y : j == 2 ? t.z : t.w;
+          } else {
+            for (int d = 0; d < n_src; ++d) {
+              const int src = ((first + d) % n_src) * stride + offset;
+              acc += full.p[src][sg.full_off + lo + i + j];
+            }
+          }
+        }
+        float g = acc * scale;
+        if (accumulate) g += gshard[e];
+        if (!in_place) gshard[e] = g;              // padding stays exactly zero: acc is 0 there
+        bad |= !isfinite(g);
+        if (i + j >= valid && g != 0.f) pad_bad = 1;
+        if (ADAMW) {
+          float pj = p[e], mj = m[e], vj = v[e];
+          adamw_update(pj, mj, vj, g, a, step_size, inv_bc2_sqrt);
+          p[e] = pj;                               // padding has p = g = m = v = 0 and stays 0
           m[e] = mj;
           v[e] = vj;
           if (shadow != nullptr) shadow[e] = __float2bfloat16(pj);
@@ -287,7 +340,7 @@ __global__ void reduce_scatter_kernel(PeerPtrs full, int degree, int rank, int t
       }
     }
   }
-  if (flags != nullptr) {
+  if (flags != nullptr && __syncthreads_or(bad | pad_bad)) {
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&flags[0], 1);
     if (__syncthreads_or(pad_bad) && threadIdx.x == 0) atomicOr(&flags[1], 1);
   }
@@ -475,24 +528,37 @@ bool fill_table(SegTable* t, const SegmentDesc* segs, int n) {
 }
 
 int g_ctas_per_sm = 0;   // 0: read STB_COLLECTIVE_CTAS_PER_SM once (default below)
-int chunks_for(const SegmentDesc* segs, int n, bool per_shard) {
+int chunks_for(const SegmentDesc* segs, int n) {
   if (g_ctas_per_sm == 0) {
     const char* env = getenv("STB_COLLECTIVE_CTAS_PER_SM");
     g_ctas_per_sm = env != nullptr ? std::max(1, atoi(env)) : 48;   // measured: 8..48 equal, 4 slower
   }
   const int kCtasPerSm = g_ctas_per_sm;
-  // grid.x of a (chunks, segments) grid.  The kernels loop over chunks, so the grid only has to
-  // be large enough to keep the memory system busy; STB_COLLECTIVE_CTAS_PER_SM bounds the total
-  // (CTAs per SM over all segments).  The compute stream has the higher priority, so a larger
-  // grid does not keep GEMMs launched meanwhile from being placed.
+  // grid.x of the gather's (chunks, segments) grid.  The kernel loops over chunks, so the grid only
+  // has to be large enough to keep the memory system busy; STB_COLLECTIVE_CTAS_PER_SM bounds the total
+  // (CTAs per SM over all segments).
   int64_t most = 1;
   for (int i = 0; i < n; ++i) {
-    const int64_t len = per_shard ? segs[i].q : segs[i].numel;
-    most = std::max<int64_t>(most, (len + kChunk - 1) / kChunk);
+    most = std::max<int64_t>(most, (segs[i].numel + kChunk - 1) / kChunk);
   }
   const int64_t budget = std::max<int64_t>(1, (sm_count() * kCtasPerSm) / std::max(1, n));
   // and never more than four CTAs per SM for one segment: more only adds scheduling work
   return static_cast<int>(std::min<int64_t>({most, budget, static_cast<int64_t>(sm_count() * 4)}));
+}
+
+// One tile after the other over all segments; false when the table or the grid does not fit.
+bool fill_tiles(RsTable* t, const SegmentDesc* segs, int n) {
+  if (n < 1 || n > kMaxSegs) return false;
+  int64_t tiles = 0;
+  for (int i = 0; i < n; ++i) {
+    t->s[i] = segs[i];
+    t->first[i] = static_cast<int>(tiles);
+    tiles += (segs[i].q + kRsTile - 1) / kRsTile;
+    if (segs[i].q < 0 || tiles > INT32_MAX) return false;
+  }
+  t->first[n] = static_cast<int>(tiles);
+  t->n = n;
+  return true;
 }
 
 }  // namespace
@@ -511,7 +577,7 @@ cudaError_t launch_gather_params(PeerPtrs shards, int degree, const SegmentDesc*
         return cudaErrorInvalidValue;
       sh.p[i] = reinterpret_cast<const __nv_bfloat16*>(shadows[i]);
     }
-  dim3 grid(chunks_for(segs, n_segs, false), n_segs);
+  dim3 grid(chunks_for(segs, n_segs), n_segs);
   gather_params_kernel<<<grid, 256, 0, s>>>(shards, sh, shadows != nullptr ? 1 : 0, degree, tab,
                                             reinterpret_cast<__nv_bfloat16*>(full_bf16), full_fp32);
   count_launch();
@@ -529,12 +595,14 @@ cudaError_t launch_reduce_scatter_grads(PeerPtrs full_grads, int degree, int ran
                                         int* flags, cudaStream_t s, TpAxis tp, const int* status,
                                         const float* multicast) {
   (void)shard_total;
-  SegTable tab;
-  if (!valid_mesh(degree, rank, tp) || !fill_table(&tab, segs, n_segs) ||
+  RsTable tab;
+  if (!valid_mesh(degree, rank, tp) || !fill_tiles(&tab, segs, n_segs) ||
       (reinterpret_cast<uintptr_t>(multicast) & 15))
     return cudaErrorInvalidValue;
-  dim3 grid(chunks_for(segs, n_segs, true), n_segs);
-  reduce_scatter_kernel<false><<<grid, 256, 0, s>>>(
+  if (tab.first[n_segs] == 0) return cudaSuccess;
+  auto kernel = degree * tp.degree == 1 && multicast == nullptr ? reduce_scatter_kernel<false, true>
+                                                                : reduce_scatter_kernel<false, false>;
+  kernel<<<tab.first[n_segs], kRsThreads, 0, s>>>(
       full_grads, degree, rank, tp.degree, tp.rank, tab, grad_shard, nullptr, nullptr, nullptr,
       scale, tp.replicated_scale, accumulate ? 1 : 0, AdamWArgs{}, flags, nullptr, status,
       multicast);
@@ -549,12 +617,14 @@ cudaError_t launch_reduce_scatter_adamw(PeerPtrs full_grads, int degree, int ran
                                         cudaStream_t s, TpAxis tp, void* shadow, const int* status,
                                         const float* multicast) {
   (void)shard_total;
-  SegTable tab;
-  if (!valid_mesh(degree, rank, tp) || !fill_table(&tab, segs, n_segs) ||
+  RsTable tab;
+  if (!valid_mesh(degree, rank, tp) || !fill_tiles(&tab, segs, n_segs) ||
       (reinterpret_cast<uintptr_t>(multicast) & 15))
     return cudaErrorInvalidValue;
-  dim3 grid(chunks_for(segs, n_segs, true), n_segs);
-  reduce_scatter_kernel<true><<<grid, 256, 0, s>>>(
+  if (tab.first[n_segs] == 0) return cudaSuccess;
+  auto kernel = degree * tp.degree == 1 && multicast == nullptr ? reduce_scatter_kernel<true, true>
+                                                                : reduce_scatter_kernel<true, false>;
+  kernel<<<tab.first[n_segs], kRsThreads, 0, s>>>(
       full_grads, degree, rank, tp.degree, tp.rank, tab, grad_shard, p, m, v, scale,
       tp.replicated_scale, accumulate ? 1 : 0, a, flags,
       reinterpret_cast<__nv_bfloat16*>(shadow), status, multicast);
