@@ -98,7 +98,15 @@ constexpr int kPullBatch = 12;     // independent 16-byte loads per thread befor
 
 constexpr int kGemmBM = 128;
 constexpr int kGemmBK = 64;
-constexpr int kGemmThreads = 192;
+// Warpgroup 0: TMA producer (warp 0), MMA issue (warp 1), two warps that only keep the group whole.
+// Warpgroup 1: the epilogue.  A CTA starts with 168 registers a thread (`kGemmLaunchBound`: 65536 / 384)
+// and the groups then trade theirs for 88 and 248, which is what the epilogue needs.  An SM's registers are
+// four files of 16384; with 255 a thread two warps filled a file and NOTHING ran next to a GEMM, neither
+// the optimizer sweep of the other stream nor the first CTAs of the next kernel.
+constexpr int kGemmThreads = 256;
+constexpr int kGemmLaunchBound = 384;
+constexpr int kIssueRegs = 88, kEpilogueRegs = 248;
+static_assert((kIssueRegs + kEpilogueRegs) * 128 <= 168 * kGemmThreads, "more registers than the CTA has");
 
 // PAIR: two CTAs of a cluster share a 256 x BN tile (tcgen05 cta_group::2).  Each stages its own 128
 // rows of A and half of B's rows, so a k-block costs a CTA 128 + BN / 2 operand rows of shared
@@ -271,179 +279,183 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
       mbar_arrive(bar);
   };
 
-  if (warp == 0) {
-    // as for the MMAs below: the warp stays together and one elected lane issues the copies
-    {
-      int it = 0;  // k-blocks issued so far, across tiles
-      bool ok = true;
-      uint64_t ready_tiles = 0;   // PULL: row tiles of A whose groups were all seen landed
-      (void)ready_tiles;
-      for (int unit = first_unit; unit < sp.total_units && ok; unit += unit_stride) {
-        int tile, kb0, kb1, part, m0, n0;
-        unit_work(unit, tile, kb0, kb1, part);
-        tile_origin(tile, m0, n0);
-        if constexpr (PULL) {
-          // The rows m0 .. m0 + 127 of A must have landed in the local buffer.  All flags of the
-          // tile are read in one batch of independent relaxed loads (an acquire load per flag
-          // would serialise sixteen L2 round trips); one fence then orders the tile's TMA reads
-          // behind them.  Row tiles already seen complete are remembered.
-          const int m_tile = m0 / kGemmBM;
-          const bool known = m_tile < 64 && ((ready_tiles >> m_tile) & 1ull);
-          if (!known) {
-            const int g_first = m0 / kPullRows;
-            const int g_count = (min(M, m0 + kGemmBM) - 1) / kPullRows - g_first + 1;
-            const uint64_t t0 = global_ns();
-            for (uint32_t spin = 0;; ++spin) {
-              uint32_t seen[kGemmBM / kPullRows];
-#pragma unroll
-              for (int g = 0; g < kGemmBM / kPullRows; ++g) {
-                seen[g] = pull.epoch;
-                if (g < g_count)
-                  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
-                               : "=r"(seen[g]) : "l"(pull.flags + g_first + g) : "memory");
+  // (the pulling GEMM has a third warpgroup, which keeps what it was launched with: 168 a thread)
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
+    if (warp == 0) {
+      // as for the MMAs below: the warp stays together and one elected lane issues the copies
+      {
+        int it = 0;  // k-blocks issued so far, across tiles
+        bool ok = true;
+        uint64_t ready_tiles = 0;   // PULL: row tiles of A whose groups were all seen landed
+        (void)ready_tiles;
+        for (int unit = first_unit; unit < sp.total_units && ok; unit += unit_stride) {
+          int tile, kb0, kb1, part, m0, n0;
+          unit_work(unit, tile, kb0, kb1, part);
+          tile_origin(tile, m0, n0);
+          if constexpr (PULL) {
+            // The rows m0 .. m0 + 127 of A must have landed in the local buffer.  All flags of the
+            // tile are read in one batch of independent relaxed loads (an acquire load per flag
+            // would serialise sixteen L2 round trips); one fence then orders the tile's TMA reads
+            // behind them.  Row tiles already seen complete are remembered.
+            const int m_tile = m0 / kGemmBM;
+            const bool known = m_tile < 64 && ((ready_tiles >> m_tile) & 1ull);
+            if (!known) {
+              const int g_first = m0 / kPullRows;
+              const int g_count = (min(M, m0 + kGemmBM) - 1) / kPullRows - g_first + 1;
+              const uint64_t t0 = global_ns();
+              for (uint32_t spin = 0;; ++spin) {
+                uint32_t seen[kGemmBM / kPullRows];
+  #pragma unroll
+                for (int g = 0; g < kGemmBM / kPullRows; ++g) {
+                  seen[g] = pull.epoch;
+                  if (g < g_count)
+                    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
+                                 : "=r"(seen[g]) : "l"(pull.flags + g_first + g) : "memory");
+                }
+                bool all = true;
+  #pragma unroll
+                for (int g = 0; g < kGemmBM / kPullRows; ++g) all = all && seen[g] == pull.epoch;
+                if (__all_sync(0xffffffffu, all)) break;
+                if ((spin & 63u) == 63u &&
+                    __any_sync(0xffffffffu,
+                               status_failed(status) || global_ns() - t0 > kWaitBudgetNs)) {
+                  if (status != nullptr) atomicCAS(status, kOk, kErrPullWait);
+                  ok = false;
+                  break;
+                }
+                __nanosleep(32);
               }
-              bool all = true;
-#pragma unroll
-              for (int g = 0; g < kGemmBM / kPullRows; ++g) all = all && seen[g] == pull.epoch;
-              if (__all_sync(0xffffffffu, all)) break;
-              if ((spin & 63u) == 63u &&
-                  __any_sync(0xffffffffu,
-                             status_failed(status) || global_ns() - t0 > kWaitBudgetNs)) {
-                if (status != nullptr) atomicCAS(status, kOk, kErrPullWait);
-                ok = false;
-                break;
+              if (!ok) break;
+              if (m_tile < 64) ready_tiles |= 1ull << m_tile;
+              asm volatile("fence.acq_rel.gpu;" ::: "memory");
+              // generic-proxy stores of the pulling warps -> visible to the TMA (async proxy) reads
+              asm volatile("fence.proxy.async;" ::: "memory");
+            }
+          }
+          for (int kb = kb0; kb < kb1; ++kb, ++it) {
+            const int s = it % STAGES;
+            const uint32_t ph = (it / STAGES) & 1;
+            if (!mbar_wait_warp(&empty_bar[s], ph ^ 1, status, kErrProducerEmptyWait)) {
+              ok = false;
+              break;
+            }
+            uint8_t* sa = tiles + s * S::kStageBytes;
+            uint8_t* sb = sa + S::kABytes;
+            // a pair's stage is complete when both CTAs' halves have landed (rank 0's barrier)
+            if (elect_one()) {
+              if (rank == 0) mbar_expect_tx(&full_bar[s], (PAIR ? 2 : 1) * S::kStageBytes);
+              if constexpr (!A_MN) {
+                load(sa, &tma_a, &full_bar[s], kb * kGemmBK, m0);
+              } else {
+  #pragma unroll
+                for (int c = 0; c < kGemmBM / 64; ++c)
+                  load(sa + c * 8192, &tma_a, &full_bar[s], m0 + c * 64, kb * kGemmBK);
               }
-              __nanosleep(32);
-            }
-            if (!ok) break;
-            if (m_tile < 64) ready_tiles |= 1ull << m_tile;
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
-            // generic-proxy stores of the pulling warps -> visible to the TMA (async proxy) reads
-            asm volatile("fence.proxy.async;" ::: "memory");
-          }
-        }
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait_warp(&empty_bar[s], ph ^ 1, status, kErrProducerEmptyWait)) {
-            ok = false;
-            break;
-          }
-          uint8_t* sa = tiles + s * S::kStageBytes;
-          uint8_t* sb = sa + S::kABytes;
-          // a pair's stage is complete when both CTAs' halves have landed (rank 0's barrier)
-          if (elect_one()) {
-            if (rank == 0) mbar_expect_tx(&full_bar[s], (PAIR ? 2 : 1) * S::kStageBytes);
-            if constexpr (!A_MN) {
-              load(sa, &tma_a, &full_bar[s], kb * kGemmBK, m0);
-            } else {
-#pragma unroll
-              for (int c = 0; c < kGemmBM / 64; ++c)
-                load(sa + c * 8192, &tma_a, &full_bar[s], m0 + c * 64, kb * kGemmBK);
-            }
-            if constexpr (!B_MN) {
-              if (gated) {   // box of BN / 2 rows: gate rows, then the matching up rows
-                if constexpr (PAIR) {
-                  load(sb, &tma_b, &full_bar[s], kb * kGemmBK, (rank ? ep.gated_inter : 0) + n0);
+              if constexpr (!B_MN) {
+                if (gated) {   // box of BN / 2 rows: gate rows, then the matching up rows
+                  if constexpr (PAIR) {
+                    load(sb, &tma_b, &full_bar[s], kb * kGemmBK, (rank ? ep.gated_inter : 0) + n0);
+                  } else {
+                    load(sb, &tma_b, &full_bar[s], kb * kGemmBK, n0);
+                    load(sb + (BN / 2) * 128, &tma_b, &full_bar[s], kb * kGemmBK, ep.gated_inter + n0);
+                  }
                 } else {
-                  load(sb, &tma_b, &full_bar[s], kb * kGemmBK, n0);
-                  load(sb + (BN / 2) * 128, &tma_b, &full_bar[s], kb * kGemmBK, ep.gated_inter + n0);
+                  load(sb, &tma_b, &full_bar[s], kb * kGemmBK, n0 + rank * S::kBRows);
                 }
               } else {
-                load(sb, &tma_b, &full_bar[s], kb * kGemmBK, n0 + rank * S::kBRows);
+  #pragma unroll
+                for (int c = 0; c < S::kBLoad / 64; ++c)
+                  load(sb + c * 8192, &tma_b, &full_bar[s], n0 + rank * S::kBRows + c * 64, kb * kGemmBK);
               }
-            } else {
-#pragma unroll
-              for (int c = 0; c < S::kBLoad / 64; ++c)
-                load(sb + c * 8192, &tma_b, &full_bar[s], n0 + rank * S::kBRows + c * 64, kb * kGemmBK);
             }
+            __syncwarp();
           }
-          __syncwarp();
+        }
+        if constexpr (PAIR) {
+          // Rank 0's commits arrive at the empty barriers of both CTAs, and no later barrier tells that
+          // they have (a commit's arrival is ordered behind its MMAs, not behind other commits').  Each
+          // CTA sees its own last ones in before the pair parts: rank 1 here, rank 0 in its MMA warp.
+          // The epilogue is draining the last tile meanwhile, so the wait costs nothing.
+          if (ok && rank == 1)
+            for (int k = max(0, it - STAGES); k < it && ok; ++k)
+              ok = mbar_wait_warp(&empty_bar[k % STAGES], (k / STAGES) & 1, status, kErrDrainWait);
+          if (!ok) give_up();
+          if (lane == 0) {
+            *loads = it;
+            if (rank == 1) st_cluster(cluster_addr(const_cast<int*>(peer_loads), 0), it);
+          }
+        } else {
+          // (the MMAs have waited for these copies, unless something failed)
+          mbar_drain(&full_bar[lane], lane < STAGES ? ring_uses(it, STAGES, lane) : 0, status);
         }
       }
-      if constexpr (PAIR) {
-        // Rank 0's commits arrive at the empty barriers of both CTAs, and no later barrier tells that
-        // they have (a commit's arrival is ordered behind its MMAs, not behind other commits').  Each
-        // CTA sees its own last ones in before the pair parts: rank 1 here, rank 0 in its MMA warp.
-        // The epilogue is draining the last tile meanwhile, so the wait costs nothing.
-        if (ok && rank == 1)
-          for (int k = max(0, it - STAGES); k < it && ok; ++k)
-            ok = mbar_wait_warp(&empty_bar[k % STAGES], (k / STAGES) & 1, status, kErrDrainWait);
-        if (!ok) give_up();
-        if (lane == 0) {
-          *loads = it;
-          if (rank == 1) st_cluster(cluster_addr(const_cast<int*>(peer_loads), 0), it);
-        }
-      } else {
-        // (the MMAs have waited for these copies, unless something failed)
-        mbar_drain(&full_bar[lane], lane < STAGES ? ring_uses(it, STAGES, lane) : 0, status);
-      }
-    }
-  } else if (warp == 1) {
-    // The whole warp walks the loop and one elected lane issues: everything the MMAs take is then
-    // warp-uniform and sits in uniform registers.  (With the loop inside `if (lane == 0)` an MMA
-    // took about 136 clocks to issue whatever its width, so a 128-wide tile ran no faster than a
-    // 256-wide one.)
-    if (rank == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(kTileM, BN, A_MN, B_MN);
-      // K-major: the 16-element K slice is 32 bytes further along each 128-byte row.  MN-major: the
-      // slice is 16 K-rows (two 8-row swizzle atoms, 1024 B apart) further on; 64-wide MN chunks sit
-      // 8192 B apart (the leading-dimension byte offset).
-      const uint64_t desc_a0 = make_smem_desc_sw128(smem_u32(tiles), A_MN ? 8192 : 16, 1024);
-      const uint64_t desc_b0 = make_smem_desc_sw128(smem_u32(tiles) + S::kABytes, B_MN ? 8192 : 16, 1024);
-      int it = 0, local = 0;      // k-blocks and tiles committed so far
-      bool ok = true;
-      for (int unit = first_unit; unit < sp.total_units; unit += unit_stride, ++local) {
-        int tile, kb0, kb1, part;
-        unit_work(unit, tile, kb0, kb1, part);
-        const int ab = local & 1;
-        // the epilogue must have drained this accumulator buffer (two tiles ago)
-        ok = mbar_wait_warp<PAIR>(&acc_empty[ab], ((local >> 1) & 1) ^ 1, status, kErrMmaFullWait);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const uint32_t tmem_d = tmem_base + ab * BN;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          ok = mbar_wait_warp(&full_bar[s], ph, status, kErrMmaFullWait);
+    } else if (warp == 1) {
+      // The whole warp walks the loop and one elected lane issues: everything the MMAs take is then
+      // warp-uniform and sits in uniform registers.  (With the loop inside `if (lane == 0)` an MMA
+      // took about 136 clocks to issue whatever its width, so a 128-wide tile ran no faster than a
+      // 256-wide one.)
+      if (rank == 0) {
+        constexpr uint32_t idesc = make_idesc_bf16(kTileM, BN, A_MN, B_MN);
+        // K-major: the 16-element K slice is 32 bytes further along each 128-byte row.  MN-major: the
+        // slice is 16 K-rows (two 8-row swizzle atoms, 1024 B apart) further on; 64-wide MN chunks sit
+        // 8192 B apart (the leading-dimension byte offset).
+        const uint64_t desc_a0 = make_smem_desc_sw128(smem_u32(tiles), A_MN ? 8192 : 16, 1024);
+        const uint64_t desc_b0 = make_smem_desc_sw128(smem_u32(tiles) + S::kABytes, B_MN ? 8192 : 16, 1024);
+        int it = 0, local = 0;      // k-blocks and tiles committed so far
+        bool ok = true;
+        for (int unit = first_unit; unit < sp.total_units; unit += unit_stride, ++local) {
+          int tile, kb0, kb1, part;
+          unit_work(unit, tile, kb0, kb1, part);
+          const int ab = local & 1;
+          // the epilogue must have drained this accumulator buffer (two tiles ago)
+          ok = mbar_wait_warp<PAIR>(&acc_empty[ab], ((local >> 1) & 1) ^ 1, status, kErrMmaFullWait);
           if (!ok) break;
           tc_fence_after_sync();
-          // descriptors hold addresses in 16-byte units (below 2^14, so the sums never carry)
-          const uint64_t da_s = desc_a0 + s * (S::kStageBytes >> 4);
-          const uint64_t db_s = desc_b0 + s * (S::kStageBytes >> 4);
-          if (elect_one()) {
-#pragma unroll
-            for (int k = 0; k < kGemmBK / 16; ++k) {
-              const uint64_t da = da_s + k * ((A_MN ? 2048 : 32) >> 4);
-              const uint64_t db = db_s + k * ((B_MN ? 2048 : 32) >> 4);
-              const uint32_t acc = ((kb - kb0) | k) != 0 ? 1u : 0u;
-              if constexpr (PAIR)
-                tc_mma_f16_pair(tmem_d, da, db, idesc, acc);
-              else
-                tc_mma_f16(tmem_d, da, db, idesc, acc);
+          const uint32_t tmem_d = tmem_base + ab * BN;
+          for (int kb = kb0; kb < kb1; ++kb, ++it) {
+            const int s = it % STAGES;
+            const uint32_t ph = (it / STAGES) & 1;
+            ok = mbar_wait_warp(&full_bar[s], ph, status, kErrMmaFullWait);
+            if (!ok) break;
+            tc_fence_after_sync();
+            // descriptors hold addresses in 16-byte units (below 2^14, so the sums never carry)
+            const uint64_t da_s = desc_a0 + s * (S::kStageBytes >> 4);
+            const uint64_t db_s = desc_b0 + s * (S::kStageBytes >> 4);
+            if (elect_one()) {
+  #pragma unroll
+              for (int k = 0; k < kGemmBK / 16; ++k) {
+                const uint64_t da = da_s + k * ((A_MN ? 2048 : 32) >> 4);
+                const uint64_t db = db_s + k * ((B_MN ? 2048 : 32) >> 4);
+                const uint32_t acc = ((kb - kb0) | k) != 0 ? 1u : 0u;
+                if constexpr (PAIR)
+                  tc_mma_f16_pair(tmem_d, da, db, idesc, acc);
+                else
+                  tc_mma_f16(tmem_d, da, db, idesc, acc);
+              }
+              // frees the stage (in both CTAs of a pair) once these MMAs have read it
+              if constexpr (PAIR) tc_commit_pair(&empty_bar[s]); else tc_commit(&empty_bar[s]);
             }
-            // frees the stage (in both CTAs of a pair) once these MMAs have read it
-            if constexpr (PAIR) tc_commit_pair(&empty_bar[s]); else tc_commit(&empty_bar[s]);
+            __syncwarp();
+          }
+          if (!ok) break;
+          if (elect_one()) {
+            if constexpr (PAIR) tc_commit_pair(&acc_full[ab]); else tc_commit(&acc_full[ab]);
           }
           __syncwarp();
         }
-        if (!ok) break;
-        if (elect_one()) {
-          if constexpr (PAIR) tc_commit_pair(&acc_full[ab]); else tc_commit(&acc_full[ab]);
+        if constexpr (PAIR) {
+          if (!ok) give_up();
+          if (lane == 0) {
+            st_cluster(cluster_addr(const_cast<int*>(peer_kblocks), 1), it);
+            st_cluster(cluster_addr(const_cast<int*>(peer_tiles), 1), local);
+          }
         }
-        __syncwarp();
+        // the commits' arrivals are in, and with them the MMAs are over
+        mbar_drain(&empty_bar[lane], committed(it, local), status);
       }
-      if constexpr (PAIR) {
-        if (!ok) give_up();
-        if (lane == 0) {
-          st_cluster(cluster_addr(const_cast<int*>(peer_kblocks), 1), it);
-          st_cluster(cluster_addr(const_cast<int*>(peer_tiles), 1), local);
-        }
-      }
-      // the commits' arrivals are in, and with them the MMAs are over
-      mbar_drain(&empty_bar[lane], committed(it, local), status);
     }
-  } else if (PULL && warp >= 6) {
+  } else if (PULL && warp >= 8) {
     // Pull warps: copy groups of rows of A from their owners into the local buffer, lowest groups
     // first (the order in which the tiles of the first wave need them), then publish the flag.
     const int t = threadIdx.x - kGemmThreads;              // 0..127
@@ -487,6 +499,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
     }
   } else {
     // Epilogue: 4 warps x 32 lanes = the 128 accumulator rows.
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpilogueRegs));
     const int q = warp & 3;
     const int row = q * 32 + lane;
     int local = 0;
@@ -835,7 +848,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
       release_acc(&acc_empty[ab]);
       __threadfence();                              // partial tile visible before the count
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (threadIdx.x == 64) {
+      if (threadIdx.x == 128) {
         const int seen = atomicAdd(sp.counters + slab, 1);
         *last_flag = (seen == sp.split - 1) ? 1 : 0;
         if (seen == sp.split - 1) sp.counters[slab] = 0;   // ready for the next launch
@@ -900,7 +913,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
 }
 
 template <int BN, bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(kGemmLaunchBound, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
                          const __grid_constant__ CUtensorMap tma_b,
                          const __grid_constant__ CUtensorMap tma_c,
@@ -913,7 +926,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
 
 // The same GEMM with pairs of CTAs on 256 x BN tiles.
 template <int BN, bool A_MN, bool B_MN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmLaunchBound, 1)
 gemm_pair_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
                               const __grid_constant__ CUtensorMap tma_b,
                               const __grid_constant__ CUtensorMap tma_c,
