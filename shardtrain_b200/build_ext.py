@@ -18,7 +18,8 @@ OUT = ROOT / "_C.so"
 OBJ = ROOT / "csrc" / "build"
 
 CUDA_SOURCES = ["gemm_sm100.cu", "gemm_allgather_sm100.cu", "elementwise.cu", "peer.cu",
-                "attention_sm100.cu", "noalloc.cu"]
+                "attention_sm100.cu", "noalloc.cu", "portable.cu"]
+EXACT_MATH = {"portable.cu"}     # serves fp32 runs: the accurate exponential, division and square root
 CPP_SOURCES = ["bindings.cpp", "layer_executor.cpp"]
 NVCC_FLAGS = [
     "-gencode",
@@ -66,7 +67,8 @@ def build(verbose: bool = False) -> Path:
         if _newer(obj, [src, *headers]):
             if verbose:
                 print("nvcc", name, flush=True)
-            _run([nvcc, *NVCC_FLAGS, "-c", str(src), "-o", str(obj)], OBJ / (name + ".ptxas.log"))
+            flags = [f for f in NVCC_FLAGS if f != "--use_fast_math" or name not in EXACT_MATH]
+            _run([nvcc, *flags, "-c", str(src), "-o", str(obj)], OBJ / (name + ".ptxas.log"))
         objects.append(obj)
     includes = [f"-I{p}" for p in cpp_extension.include_paths(device_type="cuda")]
     defines = ["-D_GLIBCXX_USE_CXX11_ABI=1"]

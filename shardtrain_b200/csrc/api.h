@@ -186,6 +186,38 @@ cudaError_t launch_reduce_scatter_adamw(PeerPtrs full_grads, int degree, int ran
 // everything else keep the fixed-order peer loads.
 // `status` (both reductions): when the word already holds a failure code on entry the kernel
 // returns without touching gradients or parameters (the data it would reduce may be stale).
+// ------------------------------------------------------------------ portable executor (portable.cu)
+enum class ScalarKind { f32, f16, bf16 };
+struct HeadTensors { void* p[3]; };      // q, k, v
+constexpr int kPortableNormCols = 8192;  // 32 KB of column sums per CTA
+cudaError_t launch_portable_norm_fwd(const float* x, const float* w, float* out, float* inv, int64_t rows,
+                                     int cols, float eps, cudaStream_t s);
+// partial [parts, cols]: column sums of each CTA's rows (launch_colsum_f32 adds them up)
+cudaError_t launch_portable_norm_bwd(const float* g, const float* x, const float* inv, const float* w,
+                                     float* dx, float* partial, int parts, int64_t rows, int cols,
+                                     cudaStream_t s);
+// forward: [B, S, heads * d] -> [B, heads, S, d], q and k rotated; backward: the adjoint.  cos / sin
+// [batch_tables, S, d] with batch_tables 1 or B
+cudaError_t launch_portable_rotate(ScalarKind kind, HeadTensors in, HeadTensors out, const float* cos,
+                                   const float* sin, int batch_tables, int64_t batch, int seq, int hq,
+                                   int hkv, int d, bool backward, cudaStream_t s);
+// causal softmax over the last dimension of [rows, seq]; row r is query r % seq of sample
+// r / rows_per_batch; `mask` [B, seq] bytes or null; stats [rows, 2]
+cudaError_t launch_portable_softmax_fwd(ScalarKind kind, const void* scores, const uint8_t* mask, void* probs,
+                                        float* stats, int64_t rows, int64_t rows_per_batch, int seq,
+                                        float scale, cudaStream_t s);
+cudaError_t launch_portable_softmax_bwd(ScalarKind kind, const void* scores, const uint8_t* mask,
+                                        const float* stats, const void* dprobs, void* dscores, int64_t rows,
+                                        int64_t rows_per_batch, int seq, float scale, cudaStream_t s);
+cudaError_t launch_portable_swiglu_fwd(ScalarKind kind, const void* gate, const void* up, void* out,
+                                       int64_t n, cudaStream_t s);
+cudaError_t launch_portable_swiglu_bwd(ScalarKind kind, const void* grad, const void* gate, const void* up,
+                                       void* dgate, void* dup, int64_t n, cudaStream_t s);
+cudaError_t launch_portable_sum(ScalarKind kind, const void* a, const void* b, const void* c, float* out,
+                                int64_t n, cudaStream_t s);
+// table [n, 3]: {start in `packed`, length, offset in the arena}
+cudaError_t launch_portable_commit(const float* packed, const int64_t* table, int n_params, int64_t largest,
+                                   float* arena, bool accumulate, cudaStream_t s);
 // ------------------------------------------------------------------ all-gather -> GEMM (gemm_allgather_sm100.cu)
 // One FSDP-sharded parameter of the fused weight: `rows` consecutive rows of W, stored flat
 // ([rows * K] elements) and cut into F shards of q elements that sit at `shard_off` in every

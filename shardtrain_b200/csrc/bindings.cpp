@@ -476,6 +476,191 @@ void unpack_gathered(const Tensor& packed, int64_t slot, const Tensor& table, in
         "unpack_gathered");
 }
 
+// ---- portable executor (portable.cu).  Outputs are allocated here: a call is one trip from Python.
+stb::ScalarKind scalar_kind(const Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return stb::ScalarKind::f32;
+    case at::kHalf: return stb::ScalarKind::f16;
+    case at::kBFloat16: return stb::ScalarKind::bf16;
+    default: TORCH_CHECK(false, "portable kernels take fp32, fp16 or bf16");
+  }
+}
+void need_like(const Tensor& t, const Tensor& like) {
+  TORCH_CHECK(t.is_cuda() && t.is_contiguous() && t.scalar_type() == like.scalar_type() &&
+                  t.sizes() == like.sizes(), "portable kernels: operands must be contiguous and alike");
+}
+void need_f32(const Tensor& t, int64_t numel) {
+  TORCH_CHECK(t.is_cuda() && t.is_contiguous() && t.scalar_type() == at::kFloat && t.numel() == numel,
+              "portable kernels: a contiguous fp32 tensor of another length was expected");
+}
+
+std::tuple<Tensor, Tensor> portable_norm_fwd(const Tensor& x, const Tensor& w, double eps) {
+  const int64_t cols = x.size(-1), rows = x.numel() / std::max<int64_t>(cols, 1);
+  need_f32(x, rows * cols);
+  need_f32(w, cols);
+  const c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = at::empty_like(x), inv = at::empty({rows}, x.options());
+  check(stb::launch_portable_norm_fwd(x.data_ptr<float>(), w.data_ptr<float>(), out.data_ptr<float>(),
+                                      inv.data_ptr<float>(), rows, static_cast<int>(cols),
+                                      static_cast<float>(eps), cur_stream()), "portable_norm_fwd");
+  return {out, inv};
+}
+
+std::tuple<Tensor, Tensor> portable_norm_bwd(const Tensor& g, const Tensor& x, const Tensor& inv,
+                                             const Tensor& w) {
+  const int64_t cols = x.size(-1), rows = x.numel() / std::max<int64_t>(cols, 1);
+  need_f32(x, rows * cols);
+  need_like(g, x);
+  need_f32(inv, rows);
+  need_f32(w, cols);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int parts = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(rows, 2 * stb::sm_count())));
+  Tensor dx = at::empty_like(x), dw = at::empty({cols}, x.options());
+  Tensor partial = at::empty({parts, cols}, x.options());
+  check(stb::launch_portable_norm_bwd(g.data_ptr<float>(), x.data_ptr<float>(), inv.data_ptr<float>(),
+                                      w.data_ptr<float>(), dx.data_ptr<float>(), partial.data_ptr<float>(),
+                                      parts, rows, static_cast<int>(cols), cur_stream()),
+        "portable_norm_bwd");
+  check(stb::launch_colsum_f32(partial.data_ptr<float>(), dw.data_ptr<float>(), parts,
+                               static_cast<int>(cols), false, cur_stream()), "colsum_f32");
+  return {dx, dw};
+}
+
+// q [B, S, hq * d], k and v [B, S, hkv * d] -> [B, heads, S, d]
+std::tuple<Tensor, Tensor, Tensor> portable_rotate(const Tensor& q, const Tensor& k, const Tensor& v,
+                                                   const Tensor& cos, const Tensor& sin, int64_t d) {
+  TORCH_CHECK(q.dim() == 3 && k.dim() == 3 && d >= 2 && d % 2 == 0 && q.size(2) % d == 0 &&
+                  k.size(2) % d == 0 && q.size(0) == k.size(0) && q.size(1) == k.size(1),
+              "portable_rotate: [B, S, heads * d] expected");
+  need_like(q, q);
+  need_like(k, k);
+  need_like(v, k);
+  TORCH_CHECK(q.scalar_type() == k.scalar_type(), "portable_rotate: one dtype");
+  const int64_t B = q.size(0), S = q.size(1), hq = q.size(2) / d, hkv = k.size(2) / d;
+  TORCH_CHECK(cos.dim() == 3 && (cos.size(0) == 1 || cos.size(0) == B), "portable_rotate: tables");
+  need_f32(cos, cos.size(0) * S * d);
+  need_f32(sin, cos.numel());
+  const c10::cuda::CUDAGuard guard(q.device());
+  Tensor qo = at::empty({B, hq, S, d}, q.options()), ko = at::empty({B, hkv, S, d}, q.options());
+  Tensor vo = at::empty({B, hkv, S, d}, q.options());
+  check(stb::launch_portable_rotate(scalar_kind(q), {{q.data_ptr(), k.data_ptr(), v.data_ptr()}},
+                                    {{qo.data_ptr(), ko.data_ptr(), vo.data_ptr()}}, cos.data_ptr<float>(),
+                                    sin.data_ptr<float>(), static_cast<int>(cos.size(0)), B,
+                                    static_cast<int>(S), static_cast<int>(hq), static_cast<int>(hkv),
+                                    static_cast<int>(d), false, cur_stream()), "portable_rotate");
+  return {qo, ko, vo};
+}
+
+std::tuple<Tensor, Tensor, Tensor> portable_rotate_bwd(const Tensor& q, const Tensor& k, const Tensor& v,
+                                                       const Tensor& cos, const Tensor& sin) {
+  TORCH_CHECK(q.dim() == 4 && k.dim() == 4 && q.size(0) == k.size(0) && q.size(2) == k.size(2) &&
+                  q.size(3) == k.size(3) && q.scalar_type() == k.scalar_type(),
+              "portable_rotate_bwd: [B, heads, S, d] expected");
+  need_like(q, q);
+  need_like(k, k);
+  need_like(v, k);
+  const int64_t B = q.size(0), hq = q.size(1), hkv = k.size(1), S = q.size(2), d = q.size(3);
+  TORCH_CHECK(cos.dim() == 3 && (cos.size(0) == 1 || cos.size(0) == B), "portable_rotate_bwd: tables");
+  need_f32(cos, cos.size(0) * S * d);
+  need_f32(sin, cos.numel());
+  const c10::cuda::CUDAGuard guard(q.device());
+  Tensor qo = at::empty({B, S, hq * d}, q.options()), ko = at::empty({B, S, hkv * d}, q.options());
+  Tensor vo = at::empty({B, S, hkv * d}, q.options());
+  check(stb::launch_portable_rotate(scalar_kind(q), {{q.data_ptr(), k.data_ptr(), v.data_ptr()}},
+                                    {{qo.data_ptr(), ko.data_ptr(), vo.data_ptr()}}, cos.data_ptr<float>(),
+                                    sin.data_ptr<float>(), static_cast<int>(cos.size(0)), B,
+                                    static_cast<int>(S), static_cast<int>(hq), static_cast<int>(hkv),
+                                    static_cast<int>(d), true, cur_stream()), "portable_rotate_bwd");
+  return {qo, ko, vo};
+}
+
+const uint8_t* portable_mask(const c10::optional<Tensor>& mask, const Tensor& scores) {
+  if (!mask.has_value()) return nullptr;
+  TORCH_CHECK(mask->is_cuda() && mask->is_contiguous() && mask->element_size() == 1 && mask->dim() == 2 &&
+                  mask->size(0) == scores.size(0) && mask->size(1) == scores.size(-1),
+              "portable softmax: the mask is [B, S] bytes");
+  return static_cast<const uint8_t*>(mask->data_ptr());
+}
+// 1 / sqrt(d) as a division by sqrt(d) is carried out for a whole tensor
+float portable_scale(int64_t d) { return 1.f / static_cast<float>(std::sqrt(static_cast<double>(d))); }
+
+// scores [B, hkv, g * S, S] -> probabilities and the rows' {maximum, sum}
+std::tuple<Tensor, Tensor> portable_softmax(const Tensor& scores, const c10::optional<Tensor>& mask, int64_t d) {
+  need_like(scores, scores);
+  TORCH_CHECK(scores.dim() == 4 && scores.size(3) >= 1 && scores.size(2) % scores.size(3) == 0 && d >= 1,
+              "portable_softmax: [B, heads, g * S, S] expected");
+  const int64_t S = scores.size(3), rows = scores.numel() / S;
+  const c10::cuda::CUDAGuard guard(scores.device());
+  Tensor probs = at::empty_like(scores), stats = at::empty({rows, 2}, scores.options().dtype(at::kFloat));
+  check(stb::launch_portable_softmax_fwd(scalar_kind(scores), scores.data_ptr(), portable_mask(mask, scores),
+                                         probs.data_ptr(), stats.data_ptr<float>(), rows,
+                                         scores.size(1) * scores.size(2), static_cast<int>(S),
+                                         portable_scale(d), cur_stream()), "portable_softmax");
+  return {probs, stats};
+}
+
+Tensor portable_softmax_bwd(const Tensor& scores, const c10::optional<Tensor>& mask, const Tensor& stats,
+                            const Tensor& dprobs, int64_t d) {
+  need_like(scores, scores);
+  need_like(dprobs, scores);
+  TORCH_CHECK(scores.dim() == 4 && scores.size(3) >= 1 && d >= 1, "portable_softmax_bwd: scores");
+  const int64_t S = scores.size(3), rows = scores.numel() / S;
+  need_f32(stats, rows * 2);
+  const c10::cuda::CUDAGuard guard(scores.device());
+  Tensor out = at::empty_like(scores);
+  check(stb::launch_portable_softmax_bwd(scalar_kind(scores), scores.data_ptr(), portable_mask(mask, scores),
+                                         stats.data_ptr<float>(), dprobs.data_ptr(), out.data_ptr(), rows,
+                                         scores.size(1) * scores.size(2), static_cast<int>(S),
+                                         portable_scale(d), cur_stream()), "portable_softmax_bwd");
+  return out;
+}
+
+Tensor portable_swiglu(const Tensor& gate, const Tensor& up) {
+  need_like(gate, gate);
+  need_like(up, gate);
+  const c10::cuda::CUDAGuard guard(gate.device());
+  Tensor out = at::empty_like(gate);
+  check(stb::launch_portable_swiglu_fwd(scalar_kind(gate), gate.data_ptr(), up.data_ptr(), out.data_ptr(),
+                                        gate.numel(), cur_stream()), "portable_swiglu");
+  return out;
+}
+
+std::tuple<Tensor, Tensor> portable_swiglu_bwd(const Tensor& grad, const Tensor& gate, const Tensor& up) {
+  need_like(gate, gate);
+  need_like(up, gate);
+  need_like(grad, gate);
+  const c10::cuda::CUDAGuard guard(gate.device());
+  Tensor dgate = at::empty_like(gate), dup = at::empty_like(gate);
+  check(stb::launch_portable_swiglu_bwd(scalar_kind(gate), grad.data_ptr(), gate.data_ptr(), up.data_ptr(),
+                                        dgate.data_ptr(), dup.data_ptr(), gate.numel(), cur_stream()),
+        "portable_swiglu_bwd");
+  return {dgate, dup};
+}
+
+// fp32 sum of one to three tensors, in order
+Tensor portable_sum(const Tensor& a, const c10::optional<Tensor>& b, const c10::optional<Tensor>& c) {
+  need_like(a, a);
+  if (b.has_value()) need_like(*b, a);
+  if (c.has_value()) need_like(*c, a);
+  const c10::cuda::CUDAGuard guard(a.device());
+  Tensor out = at::empty(a.sizes(), a.options().dtype(at::kFloat));
+  check(stb::launch_portable_sum(scalar_kind(a), a.data_ptr(), b.has_value() ? b->data_ptr() : nullptr,
+                                 c.has_value() ? c->data_ptr() : nullptr, out.data_ptr<float>(), a.numel(),
+                                 cur_stream()), "portable_sum");
+  return out;
+}
+
+void portable_commit(const Tensor& packed, const Tensor& table, int64_t largest, Tensor arena, bool accumulate) {
+  need_f32(packed, packed.numel());
+  need_f32(arena, arena.numel());
+  need(table, at::kLong, "table");
+  TORCH_CHECK(table.dim() == 2 && table.size(1) == 3 && table.is_contiguous(), "table must be [n, 3]");
+  const c10::cuda::CUDAGuard guard(packed.device());
+  check(stb::launch_portable_commit(packed.data_ptr<float>(), table.data_ptr<int64_t>(),
+                                    static_cast<int>(table.size(0)), largest, arena.data_ptr<float>(),
+                                    accumulate, cur_stream()), "portable_commit");
+}
+
 void pack_gradients(const Tensor& grad_ptrs, const Tensor& table, int64_t degree, int64_t slot,
                     int64_t used, int64_t largest, Tensor packed) {
   need(grad_ptrs, at::kLong, "grad_ptrs");
@@ -935,6 +1120,16 @@ TORCH_LIBRARY(stb, m) {
   m.def("launch_count", &launch_count);
   m.def("unpack_gathered", &unpack_gathered);
   m.def("pack_gradients", &pack_gradients);
+  m.def("portable_norm_fwd", &portable_norm_fwd);
+  m.def("portable_norm_bwd", &portable_norm_bwd);
+  m.def("portable_rotate", &portable_rotate);
+  m.def("portable_rotate_bwd", &portable_rotate_bwd);
+  m.def("portable_softmax", &portable_softmax);
+  m.def("portable_softmax_bwd", &portable_softmax_bwd);
+  m.def("portable_swiglu", &portable_swiglu);
+  m.def("portable_swiglu_bwd", &portable_swiglu_bwd);
+  m.def("portable_sum", &portable_sum);
+  m.def("portable_commit", &portable_commit);
   m.def("enable_peer_access", &enable_peer_access);
   m.def("ipc_handle", &ipc_handle);
   m.def("ipc_open", &ipc_open);

@@ -17,7 +17,7 @@ _loaded = False
 
 
 def extension_path() -> str | None:
-    return str(_LIB) if _LIB.exists() else None
+    return str(_LIB) if _loaded or _LIB.exists() else None
 
 
 def available() -> bool:

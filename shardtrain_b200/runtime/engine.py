@@ -29,9 +29,12 @@ import torch
 import torch.distributed as dist
 from torch import nn
 
+from shardtrain_b200 import ops as ops_module
 from shardtrain_b200.runtime.bridge import PreBackward, UnitMaterialize
 from shardtrain_b200.runtime.comm import CommunicationCoordinator, RuntimeTPGroup
-from shardtrain_b200.runtime.layout import ArenaPlan, ParameterSpec, ShardedParameter, padding_ranges
+from shardtrain_b200.runtime.layout import (
+    ArenaPlan, ParameterSpec, ShardedParameter, commit_table, padding_ranges,
+)
 from shardtrain_b200.runtime.materializer import Materializer
 
 MATERIALIZED_WAITING = {"RESHARDED", "FWD_RETAINED", "FWD_MATERIALIZING", "BWD_MATERIALIZING"}
@@ -433,7 +436,7 @@ class ShardedRuntime:
     def first_commit(self, unit) -> bool:
         return unit.handles[0].grad_epoch != self.grad_epoch
 
-    def mark_committed(self, handle, ticket=None):
+    def mark_committed(self, handle, ticket=None, event=None):
         if handle.grad_step == self.step_id:
             raise RuntimeError(f"Repeated gradient commit {handle.spec.param_id}")
         handle.grad_step = self.step_id
@@ -441,9 +444,12 @@ class ShardedRuntime:
         if handle.local_shard.grad is None:
             handle.local_shard.grad = handle.grad_shard
         if self.comm.streams:
-            handle.grad_ready_event = ticket.ready_event if ticket is not None else torch.cuda.Event()
-            if ticket is None:
-                handle.grad_ready_event.record(self.comm.current_stream())
+            if ticket is not None:
+                event = ticket.ready_event
+            elif event is None:
+                event = torch.cuda.Event()
+                event.record(self.comm.current_stream())
+            handle.grad_ready_event = event
         self.comm.event("leaf_grad_committed", param_id=handle.spec.param_id,
                         unit_id=handle.spec.unit_id)
 
@@ -454,6 +460,22 @@ class ShardedRuntime:
         else:
             handle.grad_shard.add_(shard_grad)
         self.mark_committed(handle)
+
+    @torch.no_grad()
+    def commit_packed(self, unit, members, slot):
+        """The shard gradients of some of a unit's parameters (by index), packed in `slot` in that order,
+        with one kernel; False where they are not all at the same point of accumulation."""
+        handles = [unit.handles[i] for i in members]
+        fresh = {h.grad_epoch != self.grad_epoch for h in handles}
+        if len(fresh) != 1:
+            return False
+        table, largest = commit_table(unit, members, slot.device)
+        ops_module.load().portable_commit(slot, table, largest, self.grad_arena, not fresh.pop())
+        event = torch.cuda.Event()
+        event.record(self.comm.current_stream())
+        for handle in handles:
+            self.mark_committed(handle, event=event)
+        return True
 
     # ------------------------------------------------------------------ optimizer binding
     def bind_optimizer(self, optimizer):

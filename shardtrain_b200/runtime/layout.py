@@ -132,6 +132,11 @@ def copy_out(storage: Tensor, specs: Sequence[ParameterSpec], degree: int) -> di
     """Rank-major packed gather buffer -> one independent tensor per parameter, padding dropped.
     On a GPU one kernel launch writes all the unit's parameters into one flat buffer (the
     returned tensors are views of it); elsewhere one copy per parameter."""
+    return copy_out_flat(storage, specs, degree)[0]
+
+
+def copy_out_flat(storage: Tensor, specs: Sequence[ParameterSpec], degree: int):
+    """`copy_out` and the flat buffer that its tensors are views of (None: they are independent)."""
     starts, slot = offsets(specs)
     if storage.numel() != degree * slot:
         raise RuntimeError("Packed gather buffer has the wrong length")
@@ -142,7 +147,7 @@ def copy_out(storage: Tensor, specs: Sequence[ParameterSpec], degree: int) -> di
         flat = torch.empty(outs[-1], dtype=storage.dtype, device=storage.device)
         ops.load().unpack_gathered(storage.reshape(-1), slot, table, max(s.numel for s in specs), flat)
         return {spec.param_id: flat[off : off + spec.numel].view(spec.tp_local_shape)
-                for spec, off in zip(specs, outs)}
+                for spec, off in zip(specs, outs)}, flat
     by_rank = storage.view(degree, slot)
     result = {}
     for spec, start in zip(specs, starts):
@@ -150,7 +155,35 @@ def copy_out(storage: Tensor, specs: Sequence[ParameterSpec], degree: int) -> di
         # [degree, q] -> flat [degree*q]; the first numel elements are the parameter
         full = by_rank[:, start : start + q].reshape(-1)[: spec.numel].clone()
         result[spec.param_id] = full.view(spec.tp_local_shape)
-    return result
+    return result, None
+
+
+def shard_table(unit, device):
+    """Device table of the copy arena window -> slot of a unit's shards, {start in the window, q, q, start in
+    the slot} each, and the largest q; built once per unit."""
+    hit = unit.__dict__.get("_shard_table")
+    if hit is None:
+        starts, _ = offsets([h.spec for h in unit.handles])
+        lo = min(h.arena_offset for h in unit.handles)
+        rows = [[h.arena_offset - lo, h.spec.fsdp_shard_numel, h.spec.fsdp_shard_numel, at]
+                for h, at in zip(unit.handles, starts)]
+        hit = unit._shard_table = (torch.tensor(rows, dtype=torch.int64, device=device),
+                                   max(row[1] for row in rows))
+    return hit
+
+
+def commit_table(unit, members, device):
+    """Device table of the commit slot -> gradient arena of some of a unit's shards (by index), packed in
+    that order: {start in the slot, q, offset in the arena} each, and the largest q; built once."""
+    held = unit.__dict__.setdefault("_commit_tables", {})
+    hit = held.get(tuple(members))
+    if hit is None:
+        handles = [unit.handles[i] for i in members]
+        starts, _ = offsets([h.spec for h in handles])
+        rows = [[at, h.spec.fsdp_shard_numel, h.arena_offset] for h, at in zip(handles, starts)]
+        hit = held[tuple(members)] = (torch.tensor(rows, dtype=torch.int64, device=device),
+                                      max(row[1] for row in rows))
+    return hit
 
 
 def pack_gradients(grads: Sequence[Tensor], specs: Sequence[ParameterSpec], degree: int) -> Tensor:

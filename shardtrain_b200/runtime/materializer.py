@@ -23,7 +23,10 @@ from dataclasses import dataclass, field
 import torch
 import torch.distributed as dist
 
-from shardtrain_b200.runtime.layout import copy_out, offsets, pack_gradients
+from shardtrain_b200 import ops as ops_module
+from shardtrain_b200.runtime.layout import (
+    _native_packing, copy_out_flat, offsets, pack_gradients, shard_table,
+)
 
 
 @dataclass
@@ -70,8 +73,14 @@ class Materializer:
             lease = MaterializationLease(unit.unit_id, runtime.step_id, phase, unit.generation,
                                          self.comm.buffer(storage, "fsdp_ag"))
             mine = storage.narrow(0, self.rank * slot_len, slot_len)
-            for handle, start in zip(unit.handles, starts):
-                mine.narrow(0, start, handle.spec.fsdp_shard_numel).copy_(handle.local_shard)
+            if _native_packing(storage, specs) and runtime.param_arena is not None:
+                # one kernel instead of a copy per parameter
+                table, largest = shard_table(unit, storage.device)
+                lo, hi = runtime.plan.unit_ranges[unit.unit_id]
+                ops_module.load().unpack_gathered(runtime.param_arena[lo:hi], hi - lo, table, largest, mine)
+            else:
+                for handle, start in zip(unit.handles, starts):
+                    mine.narrow(0, start, handle.spec.fsdp_shard_numel).copy_(handle.local_shard)
             if self.degree > 1:
                 if self.backend == "nccl":
                     def operation(async_):
@@ -113,7 +122,8 @@ class Materializer:
         if lease.full_param_storages:
             raise RuntimeError(f"Duplicate copy-out U{unit.unit_id}")
         self._await_gather(unit, lease)
-        weights = copy_out(lease.ag_storage.tensor, [h.spec for h in unit.handles], self.degree)
+        weights, lease.extras["flat"] = copy_out_flat(
+            lease.ag_storage.tensor, [h.spec for h in unit.handles], self.degree)
         for name, weight in weights.items():
             lease.full_param_storages[name] = self.comm.buffer(weight, "full_parameter")
         lease.weights = weights
@@ -132,10 +142,12 @@ class Materializer:
         packed = pack_gradients(grads, specs, self.degree)
         source = self.comm.buffer(packed, f"fsdp_{bucket}_rs_input")
         starts, slot_len = offsets(specs)
-        output = packed.new_empty(slot_len)
+        # (a single member's slot is what it packed)
+        output = packed if self.degree == 1 and packed.is_cuda else packed.new_empty(slot_len)
         ticket = ready = None
         if self.degree == 1:
-            output.copy_(packed)
+            if output is not packed:
+                output.copy_(packed)
             if self.comm.streams:
                 here = self.comm.current_stream()
                 packed.record_stream(here)
@@ -174,7 +186,8 @@ class Materializer:
                                  buffer_id=state["source"].buffer_id)
         if self.degree > 1 and self.backend != "nccl":
             output.copy_(packed.narrow(0, self.rank * output.numel(), output.numel()))
-        output.div_(self.degree)  # the one FSDP average of every parameter
+        if self.degree > 1:
+            output.div_(self.degree)  # the one FSDP average of every parameter
         if self.comm.streams:
             output.record_stream(self.comm.current_stream())
         self.comm.retire(state["source"])
@@ -208,7 +221,9 @@ class Materializer:
             context = self.comm.stream_context(channel) if channel else _null()
             with context:
                 output, starts = self._consume_bucket(pending[bucket], bucket)
-                for i, start in zip(members, starts):
+                together = (tp.degree == 1 and _native_packing(output, [specs[i] for i in members])
+                            and runtime.commit_packed(unit, members, output))
+                for i, start in () if together else zip(members, starts):
                     spec = specs[i]
                     shard_grad = output.narrow(0, start, spec.fsdp_shard_numel)
                     if spec.tp_grad_reduce == "sum":

@@ -23,6 +23,7 @@ from shardtrain_b200.models.qwen2 import (
     Qwen2CausalLMOutput, apply_rotary, causal_attention, rotary_inverse_frequencies,
     rotary_tables, swiglu,
 )
+from shardtrain_b200.runtime import portable_kernels
 from shardtrain_b200.runtime.engine import TiedEmbeddingUnit, UnitState
 from shardtrain_b200.runtime.qwen2_operators import (
     Branch, ColumnProjection, EmbeddingFn, NormFn, RowLinear,
@@ -364,22 +365,25 @@ class PortableQwenExecutor:
         h = self.norm(unit, p + "input_layernorm.weight", x)
         q, k, v = self._column_group(unit, p + "self_attn.", ("q_proj", "k_proj", "v_proj"), h, "qkv")
         batch, seq, _ = q.shape
-
-        def heads(t, n):
-            return t.reshape(batch, seq, n, d).transpose(1, 2)
-
-        q, k, v = heads(q, runtime.local_heads), heads(k, runtime.local_kv_heads), heads(v, runtime.local_kv_heads)
         cos, sin = tables
         if cos.shape[-2] != seq:
             raise ValueError("QKV sequence length differs from global RoPE positions")
-        q, k = apply_rotary(q, k, cos, sin)
         cd = runtime.compute_dtype
-        mixed = causal_attention(q.to(cd), k.to(cd), v.to(cd), attention_mask)
-        mixed = mixed.transpose(1, 2).reshape(batch, seq, -1)
+        mixed = portable_kernels.attention(q, k, v, tables, attention_mask, d) if q.dtype == cd else None
+        if mixed is None:
+            def heads(t, n):
+                return t.reshape(batch, seq, n, d).transpose(1, 2)
+
+            q, k, v = (heads(q, runtime.local_heads), heads(k, runtime.local_kv_heads),
+                       heads(v, runtime.local_kv_heads))
+            q, k = apply_rotary(q, k, cos, sin)
+            mixed = causal_attention(q.to(cd), k.to(cd), v.to(cd), attention_mask)
+            mixed = mixed.transpose(1, 2).reshape(batch, seq, -1)
         x = x + self._row(unit, p + "self_attn.o_proj.weight", mixed)
         h = self.norm(unit, p + "post_attention_layernorm.weight", x)
         gate, up = self._column_group(unit, p + "mlp.", ("gate_proj", "up_proj"), h, "gate_up")
-        return x + self._row(unit, p + "mlp.down_proj.weight", swiglu(gate, up))
+        mixed = portable_kernels.swiglu(gate, up)
+        return x + self._row(unit, p + "mlp.down_proj.weight", swiglu(gate, up) if mixed is None else mixed)
 
     def final_norm(self, unit, x):
         return self.norm(unit, "model.norm.weight", x)

@@ -22,6 +22,12 @@ import torch
 from torch.autograd.function import once_differentiable
 from torch.nn import functional as F
 
+from shardtrain_b200 import ops as ops_module
+from shardtrain_b200.runtime.portable_kernels import usable
+
+
+NORM_COLUMNS = 8192     # csrc/api.h: kPortableNormCols
+
 
 def compact(x):
     """Contiguous tensor that owns exactly its elements (no oversized storage kept alive)."""
@@ -29,6 +35,22 @@ def compact(x):
     if value.untyped_storage().nbytes() != value.numel() * value.element_size():
         value = value.clone()
     return value
+
+
+def in_dtype(unit, weight, dtype):
+    """`weight` (a full parameter of the unit's current lease) in `dtype`.  The unit's parameters lie in
+    one flat buffer where a kernel unpacked them: the first request converts that buffer, once per lease."""
+    if weight.dtype == dtype:
+        return weight
+    lease = unit.lease
+    flat = lease.extras.get("flat") if lease is not None else None
+    if flat is None or weight.untyped_storage().data_ptr() != flat.untyped_storage().data_ptr():
+        return weight.to(dtype)
+    cast = lease.extras.get(("flat", dtype))
+    if cast is None:
+        cast = lease.extras[("flat", dtype)] = flat.detach().to(dtype)
+    at = weight.storage_offset() - flat.storage_offset()
+    return cast[at:at + weight.numel()].view(weight.shape)
 
 
 @dataclass
@@ -58,8 +80,8 @@ class ColumnProjection(torch.autograd.Function):
         source = tp.finish_gather(pending) if pending is not None else local
         outputs, cursor = [], 0
         for branch in branches:
-            w = weights[cursor].to(source.dtype)
-            b = weights[cursor + 1].to(source.dtype) if branch.bias is not None else None
+            w = in_dtype(unit, weights[cursor], source.dtype)
+            b = in_dtype(unit, weights[cursor + 1], source.dtype) if branch.bias is not None else None
             outputs.append(F.linear(source, w, b))
             cursor += 2 if branch.bias is not None else 1
         if pending is not None:
@@ -76,7 +98,7 @@ class ColumnProjection(torch.autograd.Function):
         (local,) = ctx.saved_tensors
         source = tp.gather(local, 1) if sp else local
         flat = source.reshape(-1, source.shape[-1])
-        dparams, dx = [], None
+        dparams, parts = [], []
         for grad, branch in zip(grads, ctx.branches):
             if grad is None:
                 raise RuntimeError("Unused Qwen projection branches are unsupported")
@@ -84,10 +106,13 @@ class ColumnProjection(torch.autograd.Function):
             g = grad.to(local.dtype)
             g2 = g.reshape(-1, g.shape[-1])
             dparams.append((g2.t() @ flat).to(weight.dtype))
-            part = (g @ weight.to(local.dtype)).to(torch.float32)
-            dx = part if dx is None else dx + part
+            parts.append(g @ in_dtype(unit, weight, local.dtype))
             if branch.bias is not None:
-                dparams.append(grad.float().sum(tuple(range(grad.ndim - 1))).to(weight.dtype))
+                dparams.append(grad.sum(tuple(range(grad.ndim - 1)), dtype=torch.float32).to(weight.dtype))
+        if len(parts) <= 3 and usable(*parts):
+            dx = ops_module.load().portable_sum(*parts, *([None] * (3 - len(parts))))
+        else:
+            dx = sum((p.to(torch.float32) for p in parts[1:]), parts[0].to(torch.float32))
         if sp:
             tp.retire_activation(source)
             dx = tp.reduce_scatter_sequence(dx)
@@ -106,7 +131,7 @@ class RowLinear(torch.autograd.Function):
         local = compact(x.to(runtime.compute_dtype))
         ctx.save_for_backward(local)
         handle.unit.prefetch_after_input(handle, "FWD")
-        partial = F.linear(local, weight.to(local.dtype))
+        partial = F.linear(local, in_dtype(handle.unit, weight, local.dtype))
         if replicated or tp.degree == 1:
             return partial
         return tp.reduce_scatter_sequence(partial) if sp else tp.sum(partial)
@@ -126,7 +151,7 @@ class RowLinear(torch.autograd.Function):
         weight = handle.weight()
         gc = g.to(local.dtype)
         dw = gc.reshape(-1, gc.shape[-1]).t() @ local.reshape(-1, local.shape[-1])
-        dx = gc @ weight.to(local.dtype)
+        dx = gc @ in_dtype(handle.unit, weight, local.dtype)
         if gathered:
             tp.retire_activation(g)
         return dx.to(ctx.input_dtype), dw.to(weight.dtype), None, None, None
@@ -137,6 +162,14 @@ class NormFn(torch.autograd.Function):
     def forward(ctx, x, weight, handle, eps):
         handle.unit.annotate("FWD")
         ctx.handle, ctx.input_dtype = handle, x.dtype
+        ctx.kernel = (x.dtype == torch.float32 and usable(x, weight) and x.numel() > 0
+                      and x.shape[-1] <= NORM_COLUMNS)
+        if ctx.kernel:
+            wide = compact(x)
+            out, inv = ops_module.load().portable_norm_fwd(wide, weight, eps)
+            ctx.save_for_backward(wide, inv)
+            handle.unit.prefetch_after_input(handle, "FWD")
+            return out
         wide = compact(x.float())
         inv = torch.rsqrt(wide.square().mean(-1, keepdim=True) + eps)
         normalized = (wide * inv).to(x.dtype)
@@ -150,9 +183,12 @@ class NormFn(torch.autograd.Function):
     def backward(ctx, grad):
         handle = ctx.handle
         handle.unit.annotate("BWD")
-        wide, inv, normalized = ctx.saved_tensors
         weight = handle.weight()
         handle.unit.prefetch_after_input(handle, "BWD")
+        if ctx.kernel:
+            wide, inv = ctx.saved_tensors
+            return (*ops_module.load().portable_norm_bwd(grad.contiguous(), wide, inv, weight), None, None)
+        wide, inv, normalized = ctx.saved_tensors
         scaled = grad.float() * weight.float()
         dx = inv * (scaled - wide * inv.square() * (scaled * wide).mean(-1, keepdim=True))
         dw = (grad.float() * normalized.float()).sum(tuple(range(grad.ndim - 1)))
