@@ -45,6 +45,14 @@ EVENT_DEFAULTS = dict(
 )
 
 
+# what a row takes over from the ticket it names, where it does not say it itself (and the ticket's group
+# members, as a list)
+TICKET_FIELDS = (("op_id", "op_id"), ("op_kind", "kind"), ("pg_id", "pg_id"),
+                 ("pg_local_seq", "pg_local_seq"), ("issue_stream", "issue_stream"),
+                 ("group_role", "group_role"), ("execution_mode", "execution_mode"),
+                 ("logical_cuda_stream", "logical_cuda_stream"),
+                 ("collective_cuda_stream", "collective_cuda_stream"),
+                 ("api_async_op", "api_async_op"), ("work_returned", "work_returned"))
 @dataclass
 class BufferLease:
     buffer_id: int
@@ -155,6 +163,7 @@ class CommunicationCoordinator:
         self._by_storage: dict[int, dict[int, BufferLease]] = {}
         self._storage_of: dict[int, int] = {}
         self._group_info: dict[int, tuple] = {}
+        self.read_environment()
         self._log_file = None
         self._log_written = 0
         # stream_id -> the registered Stream object, for current_stream() below
@@ -169,6 +178,10 @@ class CommunicationCoordinator:
                 streams={n: {"cuda_stream": s.cuda_stream, "torch_stream_id": s.stream_id}
                          for n, s in self.streams.items()},
             )
+
+    def read_environment(self):
+        """Whether rows are marked for an external profiler; asked again at every step boundary."""
+        self.nvtx = os.environ.get("SHARDTRAIN_NVTX") == "1"
 
     # ------------------------------------------------------------------ streams
     def current_stream(self):
@@ -245,29 +258,25 @@ class CommunicationCoordinator:
 
     @_locked
     def _record_event(self, event_type, **fields):
-        row = dict(step_id=self.step_id, rank=self.rank, unit_id=self.unit_id, phase=self.phase,
-                   materialization_generation=self.generation, CPU_timestamp=time.monotonic(),
-                   event_type=event_type, generation=self.generation, **EVENT_DEFAULTS)
-        row["group_role"] = self.group_role
-        row.update(fields)
-        ticket_id = next((row[k] for k in ("op_id", "consumer_ticket", "producer_ticket")
-                          if row[k] is not None), None)
+        row = {"step_id": self.step_id, "rank": self.rank, "unit_id": self.unit_id, "phase": self.phase,
+               "materialization_generation": self.generation, "CPU_timestamp": time.monotonic(),
+               "event_type": event_type, "generation": self.generation, **EVENT_DEFAULTS,
+               "group_role": self.group_role, **fields}
+        ticket_id = row["op_id"]
+        if ticket_id is None:
+            ticket_id = row["consumer_ticket"]
+            if ticket_id is None:
+                ticket_id = row["producer_ticket"]
         ticket = self._ticket_by_id(ticket_id)
         if ticket is not None:
-            inherited = dict(
-                op_id=ticket.op_id, op_kind=ticket.kind, pg_id=ticket.pg_id,
-                pg_local_seq=ticket.pg_local_seq, group_members=list(ticket.group_members),
-                issue_stream=ticket.issue_stream, group_role=ticket.group_role,
-                execution_mode=ticket.execution_mode,
-                logical_cuda_stream=ticket.logical_cuda_stream,
-                collective_cuda_stream=ticket.collective_cuda_stream,
-                api_async_op=ticket.api_async_op, work_returned=ticket.work_returned,
-            )
-            for key, value in inherited.items():
-                if row.get(key) is None:
-                    row[key] = value
+            get = row.get
+            for key, name in TICKET_FIELDS:
+                if get(key) is None:
+                    row[key] = getattr(ticket, name)
+            if get("group_members") is None:
+                row["group_members"] = list(ticket.group_members)
         self.events.append(row)
-        if self.streams and os.environ.get("SHARDTRAIN_NVTX") == "1":
+        if self.streams and self.nvtx:
             torch.cuda.nvtx.mark(
                 f"shardtrain/{event_type}/U{row['unit_id']}/{row['phase']}/step{row['step_id']}"
                 f"/op{row['op_id']}/pg{row['pg_id']}/{row['dependency_type']}"
@@ -502,7 +511,7 @@ class CommunicationCoordinator:
 
     @_locked
     def issue_kernel(self, pg_id, kind, group, launch, *, channel, after_streams=(),
-                     after_events=(), numel=0, leases=(), group_role=None):
+                     after_events=(), numel=0, leases=(), group_role=None, ready_event=None):
         """Submit a collective implemented by this package's own kernels.
 
         `launch()` enqueues the kernels; it runs with `channel`'s stream current, after that
@@ -511,7 +520,9 @@ class CommunicationCoordinator:
         recorded behind the kernels.  Ordering between GPUs is carried by flags in peer memory,
         so neither policy adds edges here; the per-communicator sequence is still recorded.
         `launch` None: the data is where it belongs already.  The ticket keeps its place in the
-        sequence and its event, and the log says that nothing ran (`launched` false, no elements).
+        sequence and its event, and the log says that nothing ran (`launched` false, no elements).  With
+        the log off such a ticket takes `ready_event` as its own and touches no stream: None where the
+        data was written on the stream that its readers use.
         """
         if launch is None:
             numel = 0
@@ -539,6 +550,9 @@ class CommunicationCoordinator:
                            group_members=list(members), group_role=ticket.group_role,
                            issue_stream=channel, backend="peer_kernel", launched=launch is not None,
                            output_buffer_ids=[l.buffer_id for l in leases])
+            if launch is None and not self.diagnostics_enabled:
+                ticket.ready_event = ready_event
+                return ticket
             for name in after_streams:
                 produced = torch.cuda.Event()
                 produced.record(self.streams[name])

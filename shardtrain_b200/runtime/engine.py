@@ -56,6 +56,10 @@ ENTERED_FROM = {
     "GRAD_REDUCING": {"BWD_ACTIVE"},
     "GRAD_READY": {"GRAD_REDUCING"},
 }
+def _always(unit):
+    return True
+
+
 DIRECTION = {"FWD": +1, "BWD": -1}      # which neighbour a phase prefetches
 
 
@@ -111,10 +115,11 @@ class UnitState:
         if self.lease is None:
             raise RuntimeError(f"Missing lease U{self.unit_id}")
         comm, lease = self.runtime.comm, self.lease
-        if comm.streams:
+        materializer = self.runtime.materializer
+        if comm.streams and getattr(materializer, "overwrites", _always)(self):
             lease.fullparam_last_consumer_event = torch.cuda.Event()
             lease.fullparam_last_consumer_event.record(comm.current_stream())
-        notify = getattr(self.runtime.materializer, "released", None)
+        notify = getattr(materializer, "released", None)
         if notify is not None:
             notify(self, lease.fullparam_last_consumer_event)
         for storage in lease.full_param_storages.values():
@@ -181,11 +186,23 @@ class UnitState:
         # the bridge node lives on the reduce-scatter stream when gradients reduce asynchronously,
         # so its backward (the reduction) is not serialised behind compute
         channel = "fsdp_rs" if runtime.async_grad_rs else "compute"
-        with runtime.comm.stream_context(channel):
-            weights = UnitMaterialize.apply(self, *(h.local_shard for h in self.handles))
-        if isinstance(weights, torch.Tensor):
-            weights = (weights,)
-        self.forward_weights = {h.spec.param_id: w for h, w in zip(self.handles, weights)}
+        if runtime.direct:
+            # the consumer's node re-materialises and reduces the unit itself; its edge to autograd is
+            # the unit's first shard
+            comm = runtime.comm
+            with comm.stream_context("compute"):
+                runtime.materializer.finish(self)
+            if self.lease.copy_out_ready_event is not None:
+                comm.wait_event(self.lease.copy_out_ready_event, dependency_type="DATA_DEP",
+                                stream=comm.streams[channel], consumer="materialize_outputs")
+            anchor = self.handles[0].local_shard
+            self.forward_weights = {h.spec.param_id: anchor for h in self.handles}
+        else:
+            with runtime.comm.stream_context(channel):
+                weights = UnitMaterialize.apply(self, *(h.local_shard for h in self.handles))
+            if isinstance(weights, torch.Tensor):
+                weights = (weights,)
+            self.forward_weights = {h.spec.param_id: w for h, w in zip(self.handles, weights)}
         self._enter("FWD_ACTIVE")
         runtime.comm.event("unit_forward")
         self._gather_neighbour("FWD", at="entry")
@@ -208,9 +225,20 @@ class UnitState:
         else:
             self._enter("FWD_RETAINED")
         runtime.comm.event(self.state)
-        return PreBackward.apply(output, self)
+        return output if runtime.direct else PreBackward.apply(output, self)
 
     # ------------------------------------------------------------------ backward
+    def reduce_direct(self, token):
+        """`ShardedRuntime.direct`: the unit's last consumer has written the gradients; reduce them where
+        the bridge node would have, on the stream it lives on."""
+        runtime = self.runtime
+        self.annotate("BWD")
+        comm = runtime.comm
+        with comm.stream_context("fsdp_rs" if runtime.async_grad_rs else "compute"):
+            if comm.diagnostics_enabled:
+                comm.event("bridge_backward_stream", cuda_stream=comm.current_stream().cuda_stream)
+            self.reduce((token,) * len(self.handles))
+
     def pre_backward(self):
         runtime = self.runtime
         if not runtime.active or self.backward_calls:
@@ -288,7 +316,7 @@ class TiedEmbeddingUnit(UnitState):
         self.annotate("FWD")
         self._enter("FWD_RETAINED")
         self.runtime.comm.event("tied_weight_retained", unit_id=self.unit_id)
-        return PreBackward.apply(output, self)
+        return output if self.runtime.direct else PreBackward.apply(output, self)
 
 
 class ShardedRuntime:
@@ -359,6 +387,12 @@ class ShardedRuntime:
         self.last_microstep = True
         self.retained_leases: dict[int, object] = {}
         self.fused = None            # FusedExecutor on sm_100a
+        # One member and the fused executor: no bridge nodes.  Each unit has one autograd node, which
+        # enters the unit's backward and submits its reduction itself; the order of all three is what
+        # autograd gave the three nodes.  (Two nodes and a token per parameter less, and no events for
+        # gathers and reductions that launch nothing: two layers of 256 at 4 x 256 tokens, bound by the
+        # host, went from 4.3 to 3.4 ms, 7 layers at 1.5B widths with 2 x 512 from 11.1 to 8.7.)
+        self.direct = False
         self.executor = None
         self.tp = None
         self.materializer = None
@@ -450,8 +484,9 @@ class ShardedRuntime:
                 event = torch.cuda.Event()
                 event.record(self.comm.current_stream())
             handle.grad_ready_event = event
-        self.comm.event("leaf_grad_committed", param_id=handle.spec.param_id,
-                        unit_id=handle.spec.unit_id)
+        if self.comm.diagnostics_enabled:
+            self.comm.event("leaf_grad_committed", param_id=handle.spec.param_id,
+                            unit_id=handle.spec.unit_id)
 
     @torch.no_grad()
     def commit_gradient(self, handle, shard_grad):
@@ -540,6 +575,7 @@ class ShardedRuntime:
             raise RuntimeError("Invalid step boundary or FAILED runtime")
         self.step_id, self.active, self.optimizer_ready = step_id, True, False
         self.comm.step_id = step_id
+        self.comm.read_environment()
         if not self.comm.streams or self.parameter_shards_ready_event is None:
             self.publish_parameter_shards_ready("step_entry")
         self.backward_prefetch_tokens.clear()
@@ -592,7 +628,8 @@ class ShardedRuntime:
                 self.comm.wait_event(event, dependency_type="DATA_DEP", consumer="optimizer",
                                      param_id=name)
             grad = handle.local_shard.grad
-            if grad is None or grad.shape != handle.local_shard.shape:
+            if grad is not handle.grad_shard and (
+                    grad is None or grad.shape != handle.local_shard.shape):
                 raise RuntimeError(f"Missing/invalid shard .grad {name}")
         self._check_gradients(allow_nonfinite)
         if self.comm.live_buffers and not self.retained_leases:

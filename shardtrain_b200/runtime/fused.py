@@ -301,8 +301,8 @@ class FusedExecutor:
         token_pool = torch.zeros(64 * max(1, len(rt.units)), dtype=torch.float32, device=rt.device)
         for unit in rt.units:
             plan = mat.plans[unit.unit_id] = build_plan(unit)
+            lo, hi = rt.plan.unit_ranges[unit.unit_id]
             if self._gradients_in_arena(unit, plan):
-                lo, hi = rt.plan.unit_ranges[unit.unit_id]
                 window = self.grad.narrow(0, lo, hi - lo)
                 plan.arena_slot = GradSlot(window, [window.data_ptr()])
             else:
@@ -312,14 +312,22 @@ class FusedExecutor:
                 # FSDP degree 1: a "gathered" matrix is the shard itself, and the shadow arena
                 # already holds it in bf16 at the offsets the kernels want -- the unit's weight
                 # buffer is a window of the shadow, only the FP32 vectors are still copied
-                lo = rt.plan.unit_ranges[unit.unit_id][0]
                 plan.full_bf16 = self.shadow.narrow(0, lo, max(plan.bf16_numel, 8))
                 keep = plan.gather_table[:, 4].bitwise_and(1).ne(0)
                 plan.gather_table = plan.gather_table[keep].contiguous()
             else:
                 plan.full_bf16 = torch.empty(max(plan.bf16_numel, 8), dtype=torch.bfloat16,
                                              device=rt.device)
-            plan.full_fp32 = torch.empty(max(plan.fp32_numel, 4), dtype=torch.float32, device=rt.device)
+            if plan.arena_slot is not None:
+                # a single member's vectors are read where the optimizer keeps them (`grad_offsets` are
+                # the arena's): like the matrices they change only after the unit's last reader
+                plan.full_fp32 = self.param.narrow(0, lo, hi - lo)
+                plan.param_offsets.update({n: plan.grad_offsets[n] for n in plan.fp32_names})
+                keep = plan.gather_table[:, 4].bitwise_and(1).eq(0)
+                plan.gather_table = plan.gather_table[keep].contiguous()
+            else:
+                plan.full_fp32 = torch.empty(max(plan.fp32_numel, 4), dtype=torch.float32,
+                                             device=rt.device)
             plan.weights = plan.views(plan.full_bf16, plan.full_fp32)
             base = 64 * unit.unit_id
             if len(unit.handles) > 64:
@@ -389,6 +397,7 @@ class FusedExecutor:
 
     def finish_registration(self):
         rt = self.runtime
+        rt.direct = self.reduce_peer.degree == 1 and rt.materializer.degree == 1
         self.hq, self.hkv = rt.local_heads, rt.local_kv_heads
         torch.cuda.synchronize(rt.device)
 
@@ -398,6 +407,11 @@ class FusedExecutor:
         return t
 
     # ------------------------------------------------------------------ runtime hooks
+    @property
+    def shards_dirty(self):
+        """Must the next gather wait for (or cast) shards that changed?"""
+        return self._shards_dirty or self.shards_clean_event is None
+
     def shards_written(self, shadow_current=False):
         """The FP32 shards changed.  `shadow_current`: every write went through a kernel that
         also wrote the bf16 shadow (the fused reduce-scatter + AdamW); otherwise the shadow is
@@ -610,6 +624,14 @@ class FusedExecutor:
         cos, sin, rows = self._rope_cache[key][:3]
         return cos, sin, rows, seq
 
+    def edge_gradient(self, unit):
+        """What a unit's node returns along its autograd edge: the token that makes the bridge node reduce
+        the unit, or nothing after reducing it here."""
+        if not self.runtime.direct:
+            return self.token_grad
+        unit.reduce_direct(self.token_grad)
+        return None
+
     # ------------------------------------------------------------------ unit math
     def embedding(self, unit, ids):
         handle = unit.handle("model.embed_tokens.weight")
@@ -619,6 +641,8 @@ class FusedExecutor:
     def layer(self, unit, index, x, tables, attention_mask):
         plan = self.runtime.materializer.plans[unit.unit_id]
         weights = [unit.forward_weight(n) for n in plan.names]
+        if self.runtime.direct:
+            del weights[1:]               # one edge per unit
         mask = self.key_mask_bits(attention_mask) if attention_mask is not None else None
         return FusedLayerFn.apply(x, self, unit, index, tables, mask, *weights)
 
@@ -670,6 +694,9 @@ class FusedEmbeddingFn(torch.autograd.Function):
     @once_differentiable
     def backward(ctx, grad):
         ex, unit = ctx.ex, ctx.unit
+        direct = ex.runtime.direct
+        if direct and not unit.tied:
+            unit.pre_backward()
         unit.annotate("BWD")
         (ids,) = ctx.saved_tensors
         handle = unit.handles[0]
@@ -683,6 +710,9 @@ class FusedEmbeddingFn(torch.autograd.Function):
         pad = ex.cfg.pad_token_id
         ex.ops.embedding_scatter_add(grad.reshape(-1, grad.shape[-1]).contiguous(),
                                      ids.reshape(-1).contiguous(), dw, -1 if pad is None else pad)
+        if direct:
+            unit.reduce_direct(ex.token_grad)
+            return None, None, None, None
         # a tied weight receives its gradient view from the head node; returning it twice would
         # make autograd add the two (identical) views
         return (None if unit.tied else ex.token_grad), None, None, None
@@ -708,6 +738,8 @@ class FusedNormFn(torch.autograd.Function):
     @once_differentiable
     def backward(ctx, grad):
         ex, unit = ctx.ex, ctx.unit
+        if ex.runtime.direct:
+            unit.pre_backward()
         unit.annotate("BWD")
         x2, inv = ctx.saved_tensors
         name = unit.handles[0].spec.param_id
@@ -722,7 +754,7 @@ class FusedNormFn(torch.autograd.Function):
         ex.ops.rmsnorm_bwd(dy, x2, weight, inv, None, dx, partial)
         dw = plan.grad_view(slot.local, name)
         ex.ops.colsum_f32(partial, dw, ex.accumulates(unit))
-        return dx.view(ctx.shape), ex.token_grad, None, None
+        return dx.view(ctx.shape), ex.edge_gradient(unit), None, None
 
 
 class FusedHeadLossFn(torch.autograd.Function):
@@ -759,6 +791,8 @@ class FusedHeadLossFn(torch.autograd.Function):
     def backward(ctx, grad):
         ex, unit, name = ctx.ex, ctx.unit, ctx.name
         ops = ex.ops
+        if ex.runtime.direct:
+            unit.pre_backward()
         unit.annotate("BWD")
         hidden2, target, lse = ctx.saved_tensors
         weight = unit.weight(name)
@@ -774,7 +808,9 @@ class FusedHeadLossFn(torch.autograd.Function):
         ops.gemm(logits, weight, dx, False, True, None, None, False, 1.0, 0)
         ex._head_dx = dx
         placeholder = torch.empty(ctx.hidden_shape, dtype=torch.bfloat16, device=hidden2.device)
-        return placeholder, ex.token_grad, None, None, None, None
+        # (a tied unit reduces in the embedding's backward)
+        edge = None if ex.runtime.direct and unit.tied else ex.edge_gradient(unit)
+        return placeholder, edge, None, None, None, None
 
 
 class FusedLayerFn(torch.autograd.Function):
@@ -851,6 +887,8 @@ class FusedLayerFn(torch.autograd.Function):
         ex, unit, index = ctx.ex, ctx.unit, ctx.index
         ops = ex.ops
         plan = ex.runtime.materializer.plans[unit.unit_id]
+        if ex.runtime.direct:
+            unit.pre_backward()
         unit.annotate("BWD")
         unit.weight(plan.names[0])  # state / generation check of the backward materialisation
         if ex.tp_degree > 1 and ex.runtime.sp:
@@ -887,7 +925,8 @@ class FusedLayerFn(torch.autograd.Function):
             ln2, gv["down"], gv["gate_up"], gv["ln2"], gv["o"], gv["bias"], gv["qkv"], gv["ln1"], cos,
             sin, positions, ctx.mask, ex.status, B, S, hq, hkv, ctx.replay, ex.accumulates(unit))
         ex._forward_open.discard(index)
-        return (dx.view(B, S, H), None, None, None, None, None, *([ex.token_grad] * len(plan.names)))
+        edges = ([ex.edge_gradient(unit)] if ex.runtime.direct else [ex.token_grad] * len(plan.names))
+        return (dx.view(B, S, H), None, None, None, None, None, *edges)
 
     @staticmethod
     def _backward_sp(ctx, dout, plan):

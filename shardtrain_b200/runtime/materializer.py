@@ -298,6 +298,14 @@ class PeerMaterializer:
 
         # a buffer may be re-gathered only after its last reader on the compute stream
         after = (plan.last_reader,) if plan.last_reader is not None else ()
+        if not table.numel() and not comm.diagnostics_enabled and not self.arenas.shards_dirty:
+            # Nothing to gather (a single member reads its shards and their shadow where they are) and the
+            # shadow is current: what a reader waits for is the event behind the last change.  (With the
+            # event log on every wait is queued and logged as it always was.)
+            lease.ag_ticket = comm.issue_kernel(
+                "fsdp", "fsdp_ag_cast", self.group, None, channel="fsdp_ag", leases=(lease.ag_storage,),
+                group_role="parameter_materialization", ready_event=self.arenas.shards_clean_event)
+            return lease
         lease.ag_ticket = comm.issue_kernel(
             "fsdp", "fsdp_ag_partial" if pull else "fsdp_ag_cast", self.group, launch,
             channel="fsdp_ag", after_events=after, numel=plan.shard_numel, leases=(lease.ag_storage,),
@@ -350,6 +358,10 @@ class PeerMaterializer:
         if ticket is not None:
             self.comm.consume(ticket, consumer=f"copy_out/U{unit.unit_id}")
             lease.copy_out_ready_event = ticket.ready_event
+
+    def overwrites(self, unit) -> bool:
+        """Will a later gather write the unit's buffers, so that it has to know their last reader?"""
+        return self.plans[unit.unit_id].gather_table.numel() > 0
 
     def released(self, unit, event):
         """Called when the unit's full parameters are given up; `event` marks the last reader."""

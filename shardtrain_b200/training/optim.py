@@ -50,10 +50,11 @@ class ArenaAdamW(_ArenaOptimizer):
         make = runtime.fused.state_arena if runtime.fused is not None else (
             lambda tag: torch.zeros(total, dtype=torch.float32, device=runtime.device))
         self.exp_avg, self.exp_avg_sq = make("exp_avg"), make("exp_avg_sq")
+        steps = torch.tensor(0.0)
         for h in runtime.registry.values():
             q = h.spec.fsdp_shard_numel
             self.state[h.local_shard] = {
-                "step": torch.tensor(0.0),
+                "step": steps,           # one counter for all leaves
                 "exp_avg": self.exp_avg.narrow(0, h.arena_offset, q),
                 "exp_avg_sq": self.exp_avg_sq.narrow(0, h.arena_offset, q),
             }
@@ -83,8 +84,9 @@ class ArenaAdamW(_ArenaOptimizer):
                 p.addcdiv_(m, (v.sqrt() / bc2 ** 0.5).add_(eps), value=-lr / bc1)
         self.arena_step += 1
         self.units_updated.clear()
-        for state in self.state.values():
-            state["step"] += 1
+        # (loaded state may hold a counter per leaf)
+        for counter in {id(state["step"]): state["step"] for state in self.state.values()}.values():
+            counter += 1
 
 
 class ArenaSGD(_ArenaOptimizer):
