@@ -186,6 +186,16 @@ cudaError_t launch_reduce_scatter_adamw(PeerPtrs full_grads, int degree, int ran
 // everything else keep the fixed-order peer loads.
 // `status` (both reductions): when the word already holds a failure code on entry the kernel
 // returns without touching gradients or parameters (the data it would reduce may be stale).
+// ------------------------------------------------------------------ a step's bookkeeping (step.cu)
+// target [batch, seq] contiguous (or null) = the next token's label, -100 after the last; *count (or null) =
+// how many are not -100
+cudaError_t launch_shift_targets(const int64_t* labels, int64_t row_stride, int64_t col_stride, int64_t batch,
+                                 int64_t seq, int64_t* target, int64_t* count, cudaStream_t s);
+cudaError_t launch_loss(const float* total, const int64_t* labels, float degree, float* loss, float* factor,
+                        cudaStream_t s);
+// out[5] = {gradients and loss finite, total / labels, count, padding flag, status}; clears flags[0..1]
+cudaError_t launch_step_metrics(int* flags, const float* total, const int64_t* labels, const int64_t* count,
+                                const int* status, double* out, cudaStream_t s);
 // ------------------------------------------------------------------ portable executor (portable.cu)
 enum class ScalarKind { f32, f16, bf16 };
 struct HeadTensors { void* p[3]; };      // q, k, v

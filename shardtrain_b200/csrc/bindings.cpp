@@ -476,6 +476,58 @@ void unpack_gathered(const Tensor& packed, int64_t slot, const Tensor& table, in
         "unpack_gathered");
 }
 
+// ---- a step's bookkeeping (step.cu)
+void need_labels(const Tensor& labels) {
+  TORCH_CHECK(labels.is_cuda() && labels.scalar_type() == at::kLong && labels.dim() == 2,
+              "labels must be an int64 [B, S] CUDA tensor");
+}
+Tensor shift_targets(const Tensor& labels) {
+  need_labels(labels);
+  const c10::cuda::CUDAGuard guard(labels.device());
+  Tensor target = at::empty(labels.sizes(), labels.options());
+  check(stb::launch_shift_targets(labels.data_ptr<int64_t>(), labels.stride(0), labels.stride(1),
+                                  labels.size(0), labels.size(1), target.data_ptr<int64_t>(), nullptr,
+                                  cur_stream()), "shift_targets");
+  return target;
+}
+Tensor count_targets(const Tensor& labels) {
+  need_labels(labels);
+  const c10::cuda::CUDAGuard guard(labels.device());
+  Tensor count = at::empty({}, labels.options());
+  check(stb::launch_shift_targets(labels.data_ptr<int64_t>(), labels.stride(0), labels.stride(1),
+                                  labels.size(0), labels.size(1), nullptr, count.data_ptr<int64_t>(),
+                                  cur_stream()), "count_targets");
+  return count;
+}
+void need_scalar(const Tensor& t, at::ScalarType type, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == type && t.numel() == 1, name, ": one CUDA value");
+}
+// total, labels -> loss (no dimensions) and the scale of its gradient [1]
+std::tuple<Tensor, Tensor> loss_of(const Tensor& total, const Tensor& labels, double degree) {
+  need_scalar(total, at::kFloat, "total");
+  need_scalar(labels, at::kLong, "labels");
+  const c10::cuda::CUDAGuard guard(total.device());
+  Tensor loss = at::empty({}, total.options()), factor = at::empty({1}, total.options());
+  check(stb::launch_loss(total.data_ptr<float>(), labels.data_ptr<int64_t>(), static_cast<float>(degree),
+                         loss.data_ptr<float>(), factor.data_ptr<float>(), cur_stream()), "loss");
+  return {loss, factor};
+}
+Tensor step_metrics(Tensor flags, const Tensor& total, const Tensor& labels, const Tensor& count,
+                    const Tensor& status) {
+  TORCH_CHECK(flags.is_cuda() && flags.scalar_type() == at::kInt && flags.numel() >= 2 && flags.is_contiguous() &&
+                  status.is_cuda() && status.scalar_type() == at::kInt && status.numel() >= 1,
+              "step_metrics: int32 flags and status");
+  need_scalar(total, at::kFloat, "total");
+  need_scalar(labels, at::kLong, "labels");
+  need_scalar(count, at::kLong, "count");
+  const c10::cuda::CUDAGuard guard(flags.device());
+  Tensor out = at::empty({5}, total.options().dtype(at::kDouble));
+  check(stb::launch_step_metrics(flags.data_ptr<int>(), total.data_ptr<float>(), labels.data_ptr<int64_t>(),
+                                 count.data_ptr<int64_t>(), status.data_ptr<int>(), out.data_ptr<double>(),
+                                 cur_stream()), "step_metrics");
+  return out;
+}
+
 // ---- portable executor (portable.cu).  Outputs are allocated here: a call is one trip from Python.
 stb::ScalarKind scalar_kind(const Tensor& t) {
   switch (t.scalar_type()) {
@@ -1120,6 +1172,10 @@ TORCH_LIBRARY(stb, m) {
   m.def("launch_count", &launch_count);
   m.def("unpack_gathered", &unpack_gathered);
   m.def("pack_gradients", &pack_gradients);
+  m.def("shift_targets", &shift_targets);
+  m.def("count_targets", &count_targets);
+  m.def("loss_of", &loss_of);
+  m.def("step_metrics", &step_metrics);
   m.def("portable_norm_fwd", &portable_norm_fwd);
   m.def("portable_norm_bwd", &portable_norm_bwd);
   m.def("portable_rotate", &portable_rotate);

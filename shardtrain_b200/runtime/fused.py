@@ -592,15 +592,17 @@ class FusedExecutor:
         indexed by the token's row.  Tables of caller-supplied positions are cached on the
         tensor's identity and version, so a batch that repeats them pays once; they are rebuilt
         in place when fresh positions arrive."""
-        seq = position_ids.shape[-1]
-        inv_freq = self.runtime.inv_freq.float()
         if default_positions:
+            seq = self.runtime.qwen_global_seq
             key = ("default", seq)
             if key not in self._rope_cache:
+                inv_freq = self.runtime.inv_freq.float()
                 pos = torch.arange(seq, device=self.runtime.device, dtype=torch.float32)
                 angle = pos[:, None] * inv_freq[None, :]
                 self._rope_cache[key] = (angle.cos().contiguous(), angle.sin().contiguous(), None)
         else:
+            seq = position_ids.shape[-1]
+            inv_freq = self.runtime.inv_freq.float()
             # One set of tables per shape of `position_ids`, at fixed addresses (they are part of
             # a layer's replay key), recomputed when another tensor or version arrives.
             shape = tuple(position_ids.shape)
@@ -763,7 +765,7 @@ class FusedHeadLossFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, hidden, weight, ex, unit, name, labels):
-        from shardtrain_b200.runtime.qwen2_adapter import finish_loss, shifted_labels
+        from shardtrain_b200.runtime.qwen2_adapter import finish_loss, native_labels, shifted_labels
 
         rt, ops = ex.runtime, ex.ops
         unit.annotate("FWD")
@@ -772,7 +774,11 @@ class FusedHeadLossFn(torch.autograd.Function):
         weight = unit.lease.weights[name]   # the `weight` argument is only the autograd edge token
         hidden2 = hidden.reshape(-1, h)
         rows, vocab = hidden2.shape[0], weight.shape[0]
-        target = shifted_labels(rt, labels).reshape(-1).contiguous()
+        native = native_labels(rt, labels)
+        if native and labels.shape[1] == rt.qwen_global_seq:
+            target = ops.shift_targets(labels).view(-1)
+        else:
+            target = shifted_labels(rt, labels).reshape(-1).contiguous()
         logits = ex.scratch("logits", (rows, vocab), torch.bfloat16)
         ops.gemm(hidden2, weight, logits, False, False, None, None, False, 1.0, 0)
         lse = torch.empty(rows, dtype=torch.float32, device=hidden.device)
@@ -780,8 +786,14 @@ class FusedHeadLossFn(torch.autograd.Function):
         ops.ce_fwd(logits, target, lse, per_row)
         total = torch.empty(1, dtype=torch.float32, device=hidden.device)
         ops.sum_f32(per_row, total, False)
-        loss = finish_loss(rt, total[0], target.ne(-100).sum())
-        ctx.factor = rt.materializer.degree / rt.qwen_denominator
+        labels_of_step = getattr(rt, "qwen_denominator_override", None)
+        if native and labels_of_step is not None and labels_of_step.dtype == torch.int64:
+            # (the trainer counted them over all micro-steps, at least one)
+            rt.qwen_denominator, rt.qwen_numerator = labels_of_step, total[0]
+            loss, ctx.factor = ops.loss_of(total, labels_of_step, float(rt.materializer.degree))
+        else:
+            loss = finish_loss(rt, total[0], target.ne(-100).sum())
+            ctx.factor = rt.materializer.degree / rt.qwen_denominator
         ctx.save_for_backward(hidden2, target, lse)
         ctx.hidden_shape = hidden.shape
         return loss

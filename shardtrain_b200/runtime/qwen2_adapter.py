@@ -449,6 +449,13 @@ def shifted_labels(runtime, labels):
     return sequence_input(runtime, F.pad(labels[:, 1:], (0, 1), value=-100))
 
 
+def native_labels(runtime, labels) -> bool:
+    """May the kernels of a step's bookkeeping read `labels`?  (One member; what they cannot read takes the
+    torch operators, and is accepted or refused as there.)"""
+    return (runtime.direct and labels.is_cuda and labels.dtype == torch.int64 and labels.ndim == 2
+            and labels.device == runtime.fused.grad.device)
+
+
 def qwen_loss(runtime, logits, labels):
     target = shifted_labels(runtime, labels)
     if target.shape != logits.shape[:2]:
@@ -485,8 +492,12 @@ def model_forward(runtime, model, input_ids, *, attention_mask=None, position_id
         first.embedding_complete()
     else:
         hidden = first.post_forward(hidden)
-    tables = ex.rotary(position_ids, default_positions) if hasattr(ex, "rotary") else rotary_tables(
-        position_ids.to(hidden.device), runtime.inv_freq, hidden.dtype)
+    if hasattr(ex, "rotary"):
+        tables = ex.rotary(position_ids, default_positions)
+    else:
+        if position_ids is None:
+            position_ids = torch.arange(runtime.qwen_global_seq, device=input_ids.device).unsqueeze(0)
+        tables = rotary_tables(position_ids.to(hidden.device), runtime.inv_freq, hidden.dtype)
     for index in range(len(layers)):
         unit = units[1 + index]
         unit.pre_forward()

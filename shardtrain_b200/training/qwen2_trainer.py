@@ -19,7 +19,7 @@ import torch
 import torch.distributed as dist
 from torch.nn import functional as F
 
-from shardtrain_b200.runtime.qwen2_adapter import sequence_input, sum_metric
+from shardtrain_b200.runtime.qwen2_adapter import native_labels, sequence_input, sum_metric
 from shardtrain_b200.training.optim import ArenaAdamW, ArenaSGD
 from shardtrain_b200.training.qwen2_precision import resolve_qwen_compute_dtype
 
@@ -107,8 +107,13 @@ class QwenTrainer:
         return finite
 
     def _read_metrics(self, reported, global_count):
-        finite = self._finite_vote(reported)
         fused = self.runtime.fused
+        if reported is None:       # one kernel forms (and clears) what the operators below do
+            self.runtime.comm.unit_id, self.runtime.comm.phase = None, "AMP"
+            return self._checked(fused.ops.step_metrics(
+                fused._flags, self.runtime.qwen_numerator, self.runtime.qwen_denominator, global_count,
+                fused.status))
+        finite = self._finite_vote(reported)
         padding = fused._flags[1] if fused is not None else torch.zeros((), device=finite.device)
         # the kernels' status word (bounded waits that expired, rejected arguments) rides along in
         # the same device-to-host read, so a silent peer fails this very step on the host
@@ -116,11 +121,16 @@ class QwenTrainer:
         packed = torch.stack([finite.to(torch.float64), reported.detach().to(torch.float64),
                               global_count.to(torch.float64), padding.to(torch.float64),
                               status.to(torch.float64)])
+        if fused is not None:
+            fused._flags.zero_()
+        return self._checked(packed)
+
+    def _checked(self, packed):
+        """{finite, loss, valid labels, padding, status} on the host: (finite, loss, valid labels)."""
         began = time.perf_counter()
         row = packed.cpu().tolist()          # the step's one device-to-host read
         self.blocked_seconds += time.perf_counter() - began
-        if fused is not None:
-            fused._flags.zero_()
+        if self.runtime.fused is not None:
             if row[4]:
                 from shardtrain_b200 import ops as ops_module
 
@@ -143,8 +153,12 @@ class QwenTrainer:
                 runtime.zero_grad()
                 runtime.comm.unit_id, runtime.comm.phase = None, "METRIC"
                 runtime.qwen_global_seq = input_ids.shape[1]
-                target = sequence_input(runtime, F.pad(labels[:, 1:], (0, 1), value=-100))
-                global_count = sum_metric(runtime, target.ne(-100).sum(), "lm_accum_valid_count")
+                native = native_labels(runtime, labels)
+                if native:
+                    global_count = runtime.fused.ops.count_targets(labels)
+                else:
+                    target = sequence_input(runtime, F.pad(labels[:, 1:], (0, 1), value=-100))
+                    global_count = sum_metric(runtime, target.ne(-100).sum(), "lm_accum_valid_count")
                 runtime.qwen_denominator_override = global_count.clamp_min(1)
                 for index in range(self.accumulation_steps):
                     lo, hi = index * micro, (index + 1) * micro
@@ -171,7 +185,7 @@ class QwenTrainer:
                     del out
                 runtime.qwen_numerator = total
                 runtime.comm.unit_id, runtime.comm.phase = None, "METRIC"
-                reported = runtime.qwen_reported_loss()
+                reported = None if native else runtime.qwen_reported_loss()
                 if self.scaler.is_enabled():
                     self.scaler.unscale_(self.optimizer)
                 finite, loss_value, valid = self._read_metrics(reported, global_count)
