@@ -327,6 +327,11 @@ struct AttnBwdCall {
   int key_bits_pitch;
 };
 cudaError_t launch_attention_bwd(const AttnBwdCall& c, int* status, cudaStream_t s);
+// Its three parts.  Both others read what delta writes and nothing of each other: dkv and dq may run side
+// by side.
+cudaError_t launch_attention_bwd_delta(const AttnBwdCall& c, cudaStream_t s);
+cudaError_t launch_attention_bwd_dkv(const AttnBwdCall& c, int* status, cudaStream_t s);
+cudaError_t launch_attention_bwd_dq(const AttnBwdCall& c, int* status, cudaStream_t s);
 int attention_bwd_parts(int batch, int seq, int hq, int hkv);
 
 }  // namespace stb

@@ -992,25 +992,26 @@ cudaError_t launch_attention_fwd(const AttnCall& c, int* status, cudaStream_t s)
   return cudaGetLastError();
 }
 
-cudaError_t launch_attention_bwd(const AttnBwdCall& c, int* status, cudaStream_t s) {
+namespace {
+// what dK/dV and dQ launch with, checked
+struct BwdLaunch {
+  CUtensorMap map_qkv, map_do;
+  BwdParams p;
+  int nblk;
+};
+cudaError_t prepare_bwd(const AttnBwdCall& c, int* status, BwdLaunch* out) {
   if (c.seq < 1 || c.hq % c.hkv) return cudaErrorInvalidValue;
   const int64_t rows = static_cast<int64_t>(c.batch) * c.seq;
   const int64_t width = static_cast<int64_t>(c.hq + 2 * c.hkv) * kD;
   const int64_t owidth = static_cast<int64_t>(c.hq) * kD;
-  CUtensorMap map_qkv, map_do;
-  if (!make_bf16_tensor_map(&map_qkv, c.qkv, rows, width, width, 64, kBlk) ||
-      !make_bf16_tensor_map(&map_do, c.dout, rows, owidth, owidth, 64, kBlk))
+  if (!make_bf16_tensor_map(&out->map_qkv, c.qkv, rows, width, width, 64, kBlk) ||
+      !make_bf16_tensor_map(&out->map_do, c.dout, rows, owidth, owidth, 64, kBlk))
     return cudaErrorInvalidValue;
   static cudaError_t attr1 = opt_in_smem(attention_dq_kernel, kDqSmem);
   static cudaError_t attr2 = opt_in_smem(attention_dkv_kernel, kDkvSmem);
   if (attr1 != cudaSuccess) return attr1;
   if (attr2 != cudaSuccess) return attr2;
-  const int64_t warps = rows * c.hq;
-  attention_delta_kernel<<<static_cast<int>((warps * 32 + 255) / 256), 256, 0, s>>>(
-      reinterpret_cast<const __nv_bfloat16*>(c.out), reinterpret_cast<const __nv_bfloat16*>(c.dout),
-      c.delta, c.batch, c.seq, c.hq);
-  count_launch();
-  const int nblk = (c.seq + kBlk - 1) / kBlk;
+  out->nblk = (c.seq + kBlk - 1) / kBlk;
   int parts = 1;
   if (c.dkv_accum != nullptr) {
     parts = attention_bwd_parts(c.batch, c.seq, c.hq, c.hkv);
@@ -1018,26 +1019,58 @@ cudaError_t launch_attention_bwd(const AttnBwdCall& c, int* status, cudaStream_t
     if (parts > 1 && c.dkv_accum_floats < need) return cudaErrorInvalidValue;
   }
   if (c.key_bits != nullptr &&
-      (c.key_bits_pitch < 4 * nblk || (c.key_bits_pitch % 4) ||
+      (c.key_bits_pitch < 4 * out->nblk || (c.key_bits_pitch % 4) ||
        (reinterpret_cast<uintptr_t>(c.key_bits) & 15)))
     return cudaErrorInvalidValue;
-  BwdParams p{c.lse, c.delta, reinterpret_cast<__nv_bfloat16*>(c.dqkv), c.key_mask, c.batch, c.seq,
-              c.hq, c.hkv, c.scale, status, parts > 1 ? c.dkv_accum : nullptr, parts,
-              c.key_bits, c.key_bits_pitch};
-  attention_dkv_kernel<<<static_cast<unsigned>(static_cast<int64_t>(nblk) * c.hkv * parts * c.batch),
-                         kBwdThreads, kDkvSmem, s>>>(map_qkv, map_do, p);
+  out->p = BwdParams{c.lse, c.delta, reinterpret_cast<__nv_bfloat16*>(c.dqkv), c.key_mask, c.batch, c.seq,
+                     c.hq, c.hkv, c.scale, status, parts > 1 ? c.dkv_accum : nullptr, parts,
+                     c.key_bits, c.key_bits_pitch};
+  return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t launch_attention_bwd_delta(const AttnBwdCall& c, cudaStream_t s) {
+  if (c.seq < 1 || c.hq % c.hkv) return cudaErrorInvalidValue;
+  const int64_t warps = static_cast<int64_t>(c.batch) * c.seq * c.hq;
+  attention_delta_kernel<<<static_cast<int>((warps * 32 + 255) / 256), 256, 0, s>>>(
+      reinterpret_cast<const __nv_bfloat16*>(c.out), reinterpret_cast<const __nv_bfloat16*>(c.dout),
+      c.delta, c.batch, c.seq, c.hq);
   count_launch();
-  attention_dq_kernel<<<static_cast<unsigned>(static_cast<int64_t>(nblk) * c.hq * c.batch), kBwdThreads,
-                        kDqSmem, s>>>(map_qkv, map_do, p);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_attention_bwd_dkv(const AttnBwdCall& c, int* status, cudaStream_t s) {
+  BwdLaunch l;
+  const cudaError_t e = prepare_bwd(c, status, &l);
+  if (e != cudaSuccess) return e;
+  attention_dkv_kernel<<<static_cast<unsigned>(static_cast<int64_t>(l.nblk) * c.hkv * l.p.parts * c.batch),
+                         kBwdThreads, kDkvSmem, s>>>(l.map_qkv, l.map_do, l.p);
   count_launch();
-  if (parts > 1) {
+  if (l.p.parts > 1) {
+    const int64_t rows = static_cast<int64_t>(c.batch) * c.seq;
     const int64_t work = rows * (2 * c.hkv * kD / 8);
     const int grid = static_cast<int>(std::min<int64_t>((work + 255) / 256, sm_count() * 8));
-    attention_dkv_finish_kernel<<<grid, 256, 0, s>>>(c.dkv_accum, parts, rows, c.hq, c.hkv,
+    attention_dkv_finish_kernel<<<grid, 256, 0, s>>>(c.dkv_accum, l.p.parts, rows, c.hq, c.hkv,
                                                      reinterpret_cast<__nv_bfloat16*>(c.dqkv));
     count_launch();
   }
   return cudaGetLastError();
+}
+
+cudaError_t launch_attention_bwd_dq(const AttnBwdCall& c, int* status, cudaStream_t s) {
+  BwdLaunch l;
+  const cudaError_t e = prepare_bwd(c, status, &l);
+  if (e != cudaSuccess) return e;
+  attention_dq_kernel<<<static_cast<unsigned>(static_cast<int64_t>(l.nblk) * c.hq * c.batch), kBwdThreads,
+                        kDqSmem, s>>>(l.map_qkv, l.map_do, l.p);
+  count_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_attention_bwd(const AttnBwdCall& c, int* status, cudaStream_t s) {
+  cudaError_t e = launch_attention_bwd_delta(c, s);
+  if (e == cudaSuccess) e = launch_attention_bwd_dkv(c, status, s);
+  return e != cudaSuccess ? e : launch_attention_bwd_dq(c, status, s);
 }
 
 namespace {

@@ -439,6 +439,69 @@ ReplayCache& replay_cache() {
   return cache;
 }
 
+// Work of a layer's sequence that nothing after it in the sequence reads (or only much later): a branch of
+// its graph while the sequence is being captured, the same launches in line otherwise.  `stream()` is
+// where the branch's kernels go; `join()` makes the sequence wait for them.  One second stream and two
+// events per device serve all captures: a branch holds their lock from its fork to its join.
+class Branch {
+ public:
+  explicit Branch(cudaStream_t main) : main_(main) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(main, &status) != cudaSuccess) cudaGetLastError();
+    if (status != cudaStreamCaptureStatusActive) return;
+    lock_ = std::unique_lock<std::mutex>(mutex());
+    Shared& shared = streams();
+    if (shared.side == nullptr) return;
+    if (cudaEventRecord(shared.fork, main) != cudaSuccess ||
+        cudaStreamWaitEvent(shared.side, shared.fork, 0) != cudaSuccess)
+      return;
+    side_ = shared.side;
+  }
+  cudaStream_t stream() const { return side_ != nullptr ? side_ : main_; }
+  void join() {
+    if (side_ == nullptr) return;
+    Shared& shared = streams();
+    ok(cudaEventRecord(shared.join, side_), "branch");
+    ok(cudaStreamWaitEvent(main_, shared.join, 0), "branch");
+    side_ = nullptr;
+    lock_.unlock();
+  }
+
+ private:
+  static std::mutex& mutex() {
+    static std::mutex m;
+    return m;
+  }
+  struct Shared {
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+  };
+  // per device (a process drives one; a second one gets its own)
+  static Shared& streams() {
+    static std::map<int, Shared> table;
+    int device = 0;
+    ok(cudaGetDevice(&device), "device");
+    Shared& s = table[device];
+    if (s.side == nullptr) {
+      int least = 0, greatest = 0;
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // creating is no part of the capture
+      ok(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+      const bool made = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
+                        cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) == cudaSuccess &&
+                        cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) == cudaSuccess &&
+                        cudaStreamCreateWithPriority(&s.side, cudaStreamNonBlocking, greatest) == cudaSuccess;
+      ok(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+      if (!made) {
+        cudaGetLastError();
+        s = Shared{};
+      }
+    }
+    return s;
+  }
+  cudaStream_t main_, side_ = nullptr;
+  std::unique_lock<std::mutex> lock_;
+};
+
 struct KeyBuilder {
   std::vector<int64_t> v;
   KeyBuilder& tag(int64_t t) { v.push_back(t); return *this; }
@@ -612,10 +675,12 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
                                inv2.data_ptr<float>(), d_out.data_ptr<float>(), t.d_mid.data_ptr<float>(),
                                t.partial.data_ptr<float>(), kNormPartialRows, M, H, st,
                                t.d_mid_b.data_ptr()), "rmsnorm_bwd");
+    Branch norm(st);
     ok(stb::launch_colsum_f32(t.partial.data_ptr<float>(), g_ln2.data_ptr<float>(), kNormPartialRows, H,
-                              accumulate, st), "colsum");
+                              accumulate, norm.stream()), "colsum");
     g.run(t.d_mid_b, attn, g_o, true, true, nullptr, nullptr, SeqPull{}, accumulate);    // dW o
     g.run(t.d_mid_b, w_o, t.d_attn, false, true, nullptr, nullptr);             // dX o
+    norm.join();
     stb::AttnBwdCall bc{};
     bc.qkv = qkv.data_ptr();
     bc.out = attn.data_ptr();
@@ -633,13 +698,19 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
     bc.hq = static_cast<int>(hq);
     bc.hkv = static_cast<int>(hkv);
     bc.scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(D)));
-    ok(stb::launch_attention_bwd(bc, g.status, st), "attention_bwd");
+    ok(stb::launch_attention_bwd_delta(bc, st), "attention_bwd");
+    Branch keys(st);                       // dK, dV next to dQ
+    ok(stb::launch_attention_bwd_dkv(bc, g.status, keys.stream()), "attention_bwd");
+    ok(stb::launch_attention_bwd_dq(bc, g.status, st), "attention_bwd");
+    keys.join();
     ok(stb::launch_rope(t.d_qkv.data_ptr(), cos.data_ptr<float>(), sin.data_ptr<float>(), pos, M, S, hq,
                         hkv, D, true, st), "rope inverse");
+    Branch bias(st);
     ok(stb::launch_colsum_bf16(t.d_qkv.data_ptr(), W, g_bias.data_ptr<float>(), M, W, accumulate,
-                               t.bias_partial.data_ptr<float>(), 64, st), "bias colsum");
+                               t.bias_partial.data_ptr<float>(), 64, bias.stream()), "bias colsum");
     g.run(t.d_qkv, h1, g_qkv, true, true, nullptr, nullptr, SeqPull{}, accumulate);      // dW q|k|v
     g.run(t.d_qkv, w_qkv, t.d_h1, false, true, nullptr, nullptr);               // dX q|k|v
+    bias.join();
     ok(stb::launch_rmsnorm_bwd(t.d_h1.data_ptr<float>(), x2.data_ptr<float>(), ln1.data_ptr<float>(),
                                inv1.data_ptr<float>(), t.d_mid.data_ptr<float>(), dx.data_ptr<float>(),
                                t.partial.data_ptr<float>(), kNormPartialRows, M, H, st), "rmsnorm_bwd");
