@@ -16,6 +16,22 @@ int sm_count();
 void count_launch();
 void count_launches(int64_t n);   // a replayed graph of n kernels
 int64_t launches_total();
+// A run of launches on one stream, each of which may be placed on the GPU while the one before it drains
+// (programmatic dependent launch): open one around launches that follow one another with nothing between
+// them.  Kernels of the run wait for their predecessor themselves (chain_wait) before they touch memory.
+// The first launch is an ordinary one; kernels that cannot wait are launched as ever, which also orders
+// what follows them.  Per thread; ends with the object.
+class LaunchChain {
+ public:
+  LaunchChain();
+  ~LaunchChain();
+  LaunchChain(const LaunchChain&) = delete;
+  LaunchChain& operator=(const LaunchChain&) = delete;
+};
+// May the next launch on `s` overlap the one before it?  Asked once per launch of a kernel that waits.
+bool chain_next(cudaStream_t s);
+// The next launch of the run follows more than the launch before it (an event): an ordinary one.
+void chain_break();
 
 // ------------------------------------------------------------------ GEMM (gemm_sm100.cu)
 struct GemmCall {

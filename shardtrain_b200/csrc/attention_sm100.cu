@@ -166,7 +166,6 @@ constexpr int kFwdSmem = 3 * kTile + 1024 + 128;
 
 __global__ void __launch_bounds__(kFwdThreads, 2)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
-  if (kernel_should_skip(p.status)) return;   // an earlier kernel already failed
   extern __shared__ uint8_t raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -204,10 +203,17 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
     tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
   }
+  chain_wait();                       // what is above ran under the kernel before
+  __shared__ int skip;
+  if (threadIdx.x == 0) skip = status_failed(p.status) ? 1 : 0;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  if (skip != 0) {                    // an earlier kernel already failed
+    if (warp == 1) tmem_dealloc(tmem, 256);
+    return;
+  }
   const uint32_t tS = tmem, tO = tmem + 128;
 
   if (warp == 0) {
@@ -233,6 +239,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
       __syncwarp();
       ++v_loads;
     }
+    if (elect_one()) chain_release();
     // q_full, k_full, -, v_full
     mbar_drain(bars + lane, lane == 0 ? 1 : lane == 1 ? k_loads : lane == 3 ? v_loads : 0, p.status);
   } else if (warp == 1) {
@@ -391,6 +398,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
 __global__ void attention_delta_kernel(const __nv_bfloat16* __restrict__ out,
                                        const __nv_bfloat16* __restrict__ dout,
                                        float* __restrict__ delta, int batch, int seq, int hq) {
+  chain_wait();
+  chain_release();
   const int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int64_t total = static_cast<int64_t>(batch) * seq * hq;
@@ -445,7 +454,6 @@ constexpr int kDqSmem = 7 * kTile + 1024 + 256;
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
                     const __grid_constant__ CUtensorMap map_do, BwdParams p) {
-  if (kernel_should_skip(p.status)) return;   // an earlier kernel already failed
   extern __shared__ uint8_t raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -485,10 +493,17 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  chain_wait();                       // what is above ran under the kernel before
+  __shared__ int skip;
+  if (threadIdx.x == 0) skip = status_failed(p.status) ? 1 : 0;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  if (skip != 0) {                    // an earlier kernel already failed
+    if (warp == 1) tmem_dealloc(tmem, 512);
+    return;
+  }
   const uint32_t tS = tmem, tdP = tmem + 256, tdQ = tmem + 384;   // S: two buffers
 
   if (warp == 0) {
@@ -516,6 +531,7 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
       __syncwarp();
       ++v_loads;
     }
+    if (elect_one()) chain_release();
     // q_full; k_full[3]; v_full[2]
     mbar_drain(bars + lane, lane == 0 ? 1 : lane >= 4 && lane < 7 ? ring_uses(k_loads, 3, lane - 4)
                             : lane == 10 || lane == 11 ? ring_uses(v_loads, 2, lane - 10) : 0, p.status);
@@ -673,7 +689,6 @@ constexpr int kDkvSmem = 6 * kTile + 2048 + 1024 + 256;
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
                      const __grid_constant__ CUtensorMap map_do, BwdParams p) {
-  if (kernel_should_skip(p.status)) return;   // an earlier kernel already failed
   extern __shared__ uint8_t raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -717,10 +732,17 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  chain_wait();                       // what is above ran under the kernel before
+  __shared__ int skip;
+  if (threadIdx.x == 0) skip = status_failed(p.status) ? 1 : 0;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  if (skip != 0) {                    // an earlier kernel already failed
+    if (warp == 1) tmem_dealloc(tmem, 512);
+    return;
+  }
   const uint32_t tST = tmem, tdPT = tmem + 128, tdV = tmem + 256, tdK = tmem + 384;
 
   if (warp == 0) {
@@ -744,6 +766,7 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
       __syncwarp();
       ++loads;
     }
+    if (elect_one()) chain_release();
     // kv_full; q_full[2]
     mbar_drain(bars + lane, lane == 0 ? 1 : lane == 6 || lane == 7 ? ring_uses(loads, 2, lane - 6) : 0, p.status);
   } else if (warp == 1) {
@@ -942,6 +965,8 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
 __global__ void attention_dkv_finish_kernel(const float* __restrict__ part, int parts,
                                             int64_t rows, int hq, int hkv,
                                             __nv_bfloat16* __restrict__ dqkv) {
+  chain_wait();
+  chain_release();
   const int64_t pwidth = static_cast<int64_t>(2 * hkv) * kD;     // floats per row of a plane
   const int64_t vec = pwidth / 8;
   const int64_t width = static_cast<int64_t>(hq + 2 * hkv) * kD;
@@ -987,7 +1012,7 @@ cudaError_t launch_attention_fwd(const AttnCall& c, int* status, cudaStream_t s)
   FwdParams p{reinterpret_cast<__nv_bfloat16*>(c.out), c.lse, c.key_mask, c.batch, c.seq, c.hq,
               c.hkv, c.scale, status, c.key_bits, c.key_bits_pitch};
   const int64_t grid = static_cast<int64_t>((c.seq + kBlk - 1) / kBlk) * c.hq * c.batch;
-  attention_fwd_kernel<<<static_cast<unsigned>(grid), kFwdThreads, kFwdSmem, s>>>(map, p);
+  launch_chained(attention_fwd_kernel, static_cast<unsigned>(grid), kFwdThreads, kFwdSmem, s, map, p);
   count_launch();
   return cudaGetLastError();
 }
@@ -1032,7 +1057,8 @@ cudaError_t prepare_bwd(const AttnBwdCall& c, int* status, BwdLaunch* out) {
 cudaError_t launch_attention_bwd_delta(const AttnBwdCall& c, cudaStream_t s) {
   if (c.seq < 1 || c.hq % c.hkv) return cudaErrorInvalidValue;
   const int64_t warps = static_cast<int64_t>(c.batch) * c.seq * c.hq;
-  attention_delta_kernel<<<static_cast<int>((warps * 32 + 255) / 256), 256, 0, s>>>(
+  launch_chained(
+      attention_delta_kernel, static_cast<int>((warps * 32 + 255) / 256), 256, 0, s,
       reinterpret_cast<const __nv_bfloat16*>(c.out), reinterpret_cast<const __nv_bfloat16*>(c.dout),
       c.delta, c.batch, c.seq, c.hq);
   count_launch();
@@ -1043,15 +1069,16 @@ cudaError_t launch_attention_bwd_dkv(const AttnBwdCall& c, int* status, cudaStre
   BwdLaunch l;
   const cudaError_t e = prepare_bwd(c, status, &l);
   if (e != cudaSuccess) return e;
-  attention_dkv_kernel<<<static_cast<unsigned>(static_cast<int64_t>(l.nblk) * c.hkv * l.p.parts * c.batch),
-                         kBwdThreads, kDkvSmem, s>>>(l.map_qkv, l.map_do, l.p);
+  launch_chained(attention_dkv_kernel,
+                 static_cast<unsigned>(static_cast<int64_t>(l.nblk) * c.hkv * l.p.parts * c.batch),
+                 kBwdThreads, kDkvSmem, s, l.map_qkv, l.map_do, l.p);
   count_launch();
   if (l.p.parts > 1) {
     const int64_t rows = static_cast<int64_t>(c.batch) * c.seq;
     const int64_t work = rows * (2 * c.hkv * kD / 8);
     const int grid = static_cast<int>(std::min<int64_t>((work + 255) / 256, sm_count() * 8));
-    attention_dkv_finish_kernel<<<grid, 256, 0, s>>>(c.dkv_accum, l.p.parts, rows, c.hq, c.hkv,
-                                                     reinterpret_cast<__nv_bfloat16*>(c.dqkv));
+    launch_chained(attention_dkv_finish_kernel, grid, 256, 0, s, c.dkv_accum, l.p.parts, rows, c.hq, c.hkv,
+                   reinterpret_cast<__nv_bfloat16*>(c.dqkv));
     count_launch();
   }
   return cudaGetLastError();
@@ -1061,8 +1088,8 @@ cudaError_t launch_attention_bwd_dq(const AttnBwdCall& c, int* status, cudaStrea
   BwdLaunch l;
   const cudaError_t e = prepare_bwd(c, status, &l);
   if (e != cudaSuccess) return e;
-  attention_dq_kernel<<<static_cast<unsigned>(static_cast<int64_t>(l.nblk) * c.hq * c.batch), kBwdThreads,
-                        kDqSmem, s>>>(l.map_qkv, l.map_do, l.p);
+  launch_chained(attention_dq_kernel, static_cast<unsigned>(static_cast<int64_t>(l.nblk) * c.hq * c.batch),
+                 kBwdThreads, kDqSmem, s, l.map_qkv, l.map_do, l.p);
   count_launch();
   return cudaGetLastError();
 }

@@ -78,6 +78,30 @@ __device__ __forceinline__ bool kernel_should_skip(const int* status) {
   return skip != 0;
 }
 
+// Chained launches (LaunchChain).  chain_wait: everything before this kernel is over and its writes are
+// visible; every thread calls it before it reads or writes global memory.  (So a kernel that is over
+// implies that all before it are.)  chain_release: this CTA does not mind the next kernel's CTAs being
+// placed from here on; they are when every CTA has said so or left.  A kernel that allocates TMEM says
+// so only when it has its own: the next one's CTAs may take what is left.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute overlap{};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = s;
+  config.attrs = &overlap;
+  config.numAttrs = chain_next(s) ? 1 : 0;
+  cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);     // (an error is the last error)
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -222,18 +246,12 @@ __device__ __forceinline__ void mbar_complete_tx(uint64_t* bar, uint32_t bytes) 
   asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
-// CTA-pair form of kernel_should_skip: both CTAs of the pair return the same answer (a status word
-// that changes between their reads must not let one of them wait for the other).
-__device__ __forceinline__ bool pair_should_skip(const int* status) {
-  __shared__ uint32_t skip;
-  if (threadIdx.x == 0) skip = status_failed(status) ? 1u : 0u;
-  cluster_sync();
+// The other CTA's copy of a shared-memory word (between cluster barriers that keep both CTAs alive).
+__device__ __forceinline__ uint32_t peer_word(const uint32_t* word) {
   uint32_t theirs;
   asm volatile("ld.shared::cluster.u32 %0, [%1];"
-               : "=r"(theirs) : "r"(cluster_addr(&skip, cluster_rank() ^ 1u)) : "memory");
-  const bool out = (skip | theirs) != 0;
-  cluster_sync();      // the peer has read this CTA's word: either may leave from here on
-  return out;
+               : "=r"(theirs) : "r"(cluster_addr(const_cast<uint32_t*>(word), cluster_rank() ^ 1u)) : "memory");
+  return theirs;
 }
 // TMA load into this CTA's shared memory that completes on a barrier of either CTA of the pair
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map,

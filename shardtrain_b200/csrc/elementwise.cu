@@ -6,6 +6,7 @@
 #include <math.h>
 
 #include "api.h"
+#include "common.cuh"
 
 namespace stb {
 
@@ -59,6 +60,8 @@ template <bool Y_FP32>
 __global__ void rmsnorm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                    void* __restrict__ y, float* __restrict__ inv_out, int cols,
                                    float eps) {
+  chain_wait();
+  chain_release();
   __shared__ float red[32];
   const int64_t row = blockIdx.x;
   const float* xr = x + row * cols;
@@ -132,6 +135,8 @@ __global__ void rmsnorm_bwd_kernel(const float* __restrict__ dy, const float* __
                                    const float* __restrict__ dres, float* __restrict__ dx,
                                    __nv_bfloat16* __restrict__ dx_bf16,
                                    float* __restrict__ dw_partial, int rows, int cols) {
+  chain_wait();
+  chain_release();
   extern __shared__ float sm[];  // cols floats of dw accumulation + 32 for reductions
   float* dw_acc = sm;
   float* red = sm + cols;
@@ -194,6 +199,8 @@ rmsnorm_bwd_rows_kernel(const float* __restrict__ dy, const float* __restrict__ 
                         const float* __restrict__ dres, float* __restrict__ dx,
                         __nv_bfloat16* __restrict__ dx_bf16, float* __restrict__ dw_partial,
                         int rows, int cols) {
+  chain_wait();
+  chain_release();
   constexpr bool kAhead = K <= 2;
   __shared__ float red[2][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -285,6 +292,8 @@ rmsnorm_bwd_rows_kernel(const float* __restrict__ dy, const float* __restrict__ 
 // groups stride over the rows, then combine through shared memory in a fixed order.
 __global__ void colsum_f32_kernel(const float* __restrict__ partial, float* __restrict__ out,
                                   int rows, int cols, int accumulate) {
+  chain_wait();
+  chain_release();
   __shared__ float part[8][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
@@ -312,6 +321,8 @@ __global__ void colsum_f32_kernel(const float* __restrict__ partial, float* __re
 // scratch[b, c] = sum over the rows handled by CTA row-group b of x[r, c] (bf16 input).
 __global__ void colsum_bf16_partial_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx,
                                            float* __restrict__ scratch, int rows, int cols) {
+  chain_wait();
+  chain_release();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
   if (c >= cols) return;
   float s0 = 0.f, s1 = 0.f;
@@ -344,6 +355,8 @@ template <int V>
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, const int* __restrict__ positions,
                             int rows, int seq, int hq, int hkv, int d, int inverse) {
+  chain_wait();
+  chain_release();
   const int half = d / 2;
   const int heads = hq + hkv;
   const int per_head = half / V, per_row = heads * per_head;
@@ -430,6 +443,8 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh,
                                   const __nv_bfloat16* __restrict__ gu,
                                   __nv_bfloat16* __restrict__ dgu, int rows, int inter) {
+  chain_wait();
+  chain_release();
   const int64_t n8 = static_cast<int64_t>(rows) * (inter / 8);
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -548,6 +563,8 @@ __global__ void embedding_scatter_add_kernel(const float* __restrict__ dx,
 
 __global__ void cast_f32_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                      int64_t n) {
+  chain_wait();
+  chain_release();
   const int64_t n4 = n / 4;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -709,10 +726,10 @@ cudaError_t launch_rmsnorm_fwd(const float* x, const float* w, void* y, float* i
   if (cols % 4) return cudaErrorInvalidValue;
   const int threads = cols >= 1024 ? 256 : 128;
   if (y_fp32) {
-    rmsnorm_fwd_kernel<true><<<rows, threads, 0, s>>>(x, w, y, inv, cols, eps);
+    launch_chained(rmsnorm_fwd_kernel<true>, rows, threads, 0, s, x, w, y, inv, cols, eps);
     count_launch();
   } else {
-    rmsnorm_fwd_kernel<false><<<rows, threads, 0, s>>>(x, w, y, inv, cols, eps);
+    launch_chained(rmsnorm_fwd_kernel<false>, rows, threads, 0, s, x, w, y, inv, cols, eps);
     count_launch();
   }
   return cudaGetLastError();
@@ -742,23 +759,23 @@ cudaError_t launch_rmsnorm_bwd(const float* dy, const float* x, const float* w, 
   const bool wide = (reinterpret_cast<uintptr_t>(dw_partial) & 15) == 0;
   switch (wide ? (cols + 1023) / 1024 : 0) {
     case 1:
-      rmsnorm_bwd_rows_kernel<1><<<partial_rows, 256, 0, s>>>(dy, x, w, inv, dres_in, dx_out, copy,
+      launch_chained(rmsnorm_bwd_rows_kernel<1>, partial_rows, 256, 0, s, dy, x, w, inv, dres_in, dx_out, copy,
                                                               dw_partial, rows, cols);
       break;
     case 2:
-      rmsnorm_bwd_rows_kernel<2><<<partial_rows, 256, 0, s>>>(dy, x, w, inv, dres_in, dx_out, copy,
+      launch_chained(rmsnorm_bwd_rows_kernel<2>, partial_rows, 256, 0, s, dy, x, w, inv, dres_in, dx_out, copy,
                                                               dw_partial, rows, cols);
       break;
     case 3:
-      rmsnorm_bwd_rows_kernel<3><<<partial_rows, 256, 0, s>>>(dy, x, w, inv, dres_in, dx_out, copy,
+      launch_chained(rmsnorm_bwd_rows_kernel<3>, partial_rows, 256, 0, s, dy, x, w, inv, dres_in, dx_out, copy,
                                                               dw_partial, rows, cols);
       break;
     case 4:
-      rmsnorm_bwd_rows_kernel<4><<<partial_rows, 256, 0, s>>>(dy, x, w, inv, dres_in, dx_out, copy,
+      launch_chained(rmsnorm_bwd_rows_kernel<4>, partial_rows, 256, 0, s, dy, x, w, inv, dres_in, dx_out, copy,
                                                               dw_partial, rows, cols);
       break;
     default:     // wider rows than the registers hold, or partial sums off a 16-byte boundary
-      rmsnorm_bwd_kernel<<<partial_rows, 256, (cols + 32) * sizeof(float), s>>>(
+      launch_chained(rmsnorm_bwd_kernel, partial_rows, 256, (cols + 32) * sizeof(float), s, 
           dy, x, w, inv, dres_in, dx_out, copy, dw_partial, rows, cols);
   }
   count_launch();
@@ -767,7 +784,7 @@ cudaError_t launch_rmsnorm_bwd(const float* dy, const float* x, const float* w, 
 
 cudaError_t launch_colsum_f32(const float* partial, float* out, int rows, int cols,
                               bool accumulate, cudaStream_t s) {
-  colsum_f32_kernel<<<(cols + 31) / 32, dim3(32, 8), 0, s>>>(partial, out, rows, cols, accumulate);
+  launch_chained(colsum_f32_kernel, (cols + 31) / 32, dim3(32, 8), 0, s, partial, out, rows, cols, accumulate);
   count_launch();
   return cudaGetLastError();
 }
@@ -776,10 +793,10 @@ cudaError_t launch_colsum_bf16(const void* x, int64_t ldx, float* out, int rows,
                                bool accumulate, float* scratch, int scratch_rows, cudaStream_t s) {
   if (cols % 2 || scratch_rows < 1) return cudaErrorInvalidValue;
   dim3 grid((cols / 2 + 127) / 128, scratch_rows);
-  colsum_bf16_partial_kernel<<<grid, 128, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), ldx,
+  launch_chained(colsum_bf16_partial_kernel, grid, 128, 0, s, reinterpret_cast<const __nv_bfloat16*>(x), ldx,
                                                   scratch, rows, cols);
   count_launch();
-  colsum_f32_kernel<<<(cols + 31) / 32, dim3(32, 8), 0, s>>>(scratch, out, scratch_rows, cols,
+  launch_chained(colsum_f32_kernel, (cols + 31) / 32, dim3(32, 8), 0, s, scratch, out, scratch_rows, cols,
                                                              accumulate);
   count_launch();
   return cudaGetLastError();
@@ -795,10 +812,10 @@ cudaError_t launch_rope(void* qkv, const float* cos, const float* sin, const int
   const int64_t work = static_cast<int64_t>(rows) * (hq + hkv) * (d / (wide ? 16 : 4));
   const int grid = static_cast<int>((work + 255) / 256);
   if (wide)
-    rope_kernel<8><<<grid, 256, 0, s>>>(reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions, rows,
+    launch_chained(rope_kernel<8>, grid, 256, 0, s, reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions, rows,
                                         seq, hq, hkv, d, inverse);
   else
-    rope_kernel<2><<<grid, 256, 0, s>>>(reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions, rows,
+    launch_chained(rope_kernel<2>, grid, 256, 0, s, reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions, rows,
                                         seq, hq, hkv, d, inverse);
   count_launch();
   return cudaGetLastError();
@@ -817,7 +834,7 @@ cudaError_t launch_swiglu_bwd(const void* dh, const void* gu, void* dgu, int row
                               cudaStream_t s) {
   if (inter % 8) return cudaErrorInvalidValue;
   const int64_t work = static_cast<int64_t>(rows) * (inter / 8);
-  swiglu_bwd_kernel<<<grid_for(work, 256, sm_count() * 16), 256, 0, s>>>(
+  launch_chained(swiglu_bwd_kernel, grid_for(work, 256, sm_count() * 16), 256, 0, s, 
       reinterpret_cast<const __nv_bfloat16*>(dh), reinterpret_cast<const __nv_bfloat16*>(gu),
       reinterpret_cast<__nv_bfloat16*>(dgu), rows, inter);
   count_launch();
@@ -856,7 +873,7 @@ cudaError_t launch_embedding_scatter_add(const float* dx, const int64_t* ids, fl
 }
 
 cudaError_t launch_cast_f32_to_bf16(const float* x, void* y, int64_t n, cudaStream_t s) {
-  cast_f32_bf16_kernel<<<grid_for(n / 4 + 1, 256, sm_count() * 16), 256, 0, s>>>(
+  launch_chained(cast_f32_bf16_kernel, grid_for(n / 4 + 1, 256, sm_count() * 16), 256, 0, s, 
       x, reinterpret_cast<__nv_bfloat16*>(y), n);
   count_launch();
   return cudaGetLastError();

@@ -113,6 +113,27 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 void count_launches(int64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 int64_t launches_total() { return g_launches.load(std::memory_order_relaxed); }
 
+namespace {
+struct ChainState {
+  int depth = 0;
+  bool begun = false;               // a kernel of the run was launched on `stream`
+  cudaStream_t stream = nullptr;
+};
+thread_local ChainState t_chain;
+}  // namespace
+LaunchChain::LaunchChain() {
+  if (t_chain.depth++ == 0) t_chain.begun = false;
+}
+LaunchChain::~LaunchChain() { --t_chain.depth; }
+void chain_break() { t_chain.begun = false; }
+bool chain_next(cudaStream_t s) {
+  if (t_chain.depth == 0) return false;
+  const bool follows = t_chain.begun && t_chain.stream == s;
+  t_chain.begun = true;
+  t_chain.stream = s;
+  return follows;
+}
+
 int sm_count() {
   static int n = [] {
     int dev = 0, v = 0;
@@ -318,8 +339,8 @@ cudaError_t launch_variant(const GemmCall& c, int* status, cudaStream_t stream) 
     attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   });
   if (attr_err != cudaSuccess) return attr_err;
-  kernel<<<grid, kGemmThreads, smem, stream>>>(ta, tb, tc, tc_up, tc_h, ep, sp, c.M, c.N, c.K,
-                                               status);
+  launch_chained(kernel, grid, kGemmThreads, smem, stream, ta, tb, tc, tc_up, tc_h, ep, sp, c.M, c.N, c.K,
+                 status);
   count_launch();
   return cudaGetLastError();
 }

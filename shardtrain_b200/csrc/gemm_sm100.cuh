@@ -150,9 +150,6 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
   using S = GemmSmem<BN, B_MN, PAIR>;
   static_assert(!(PULL && PAIR), "the pulling GEMM runs one CTA per tile");
   constexpr int STAGES = S::kStages;
-  // an earlier kernel recorded a failure (a peer that never signalled, a wait that expired): the
-  // operands may be stale, skip the work -- uniformly, before any barrier or TMEM exists
-  if (PAIR ? pair_should_skip(status) : kernel_should_skip(status)) return;
   // position in the pair, and the index / stride of the CTA (or pair) over the work units
   const int rank = PAIR ? static_cast<int>(cluster_rank()) : 0;
   const int first_unit = PAIR ? blockIdx.x / 2 : blockIdx.x;
@@ -242,6 +239,10 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
       tmem_relinquish();
     }
   }
+  // from here on memory is touched; what is above ran under the kernel before
+  chain_wait();
+  __shared__ uint32_t skip;
+  if (threadIdx.x == 0) skip = status_failed(status) ? 1u : 0u;
   tc_fence_before_sync();
   if constexpr (PAIR)
     cluster_sync();      // both CTAs' barriers exist before either signals the other's
@@ -249,6 +250,9 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
     __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr;
+  // An earlier kernel recorded a failure (a peer that never signalled, a wait that expired): the operands
+  // may be stale, there is no work.  Both CTAs of a pair find the same, whenever the word changed.
+  const int total_units = (skip | (PAIR ? peer_word(&skip) : 0u)) != 0 ? 0 : sp.total_units;
   // the barriers of rank 0 that both CTAs of a pair signal
   auto leader_bar = [&](uint64_t* bar) { return PAIR ? cluster_addr(bar, 0) : smem_u32(bar); };
   auto load = [&](void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
@@ -289,7 +293,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
         bool ok = true;
         uint64_t ready_tiles = 0;   // PULL: row tiles of A whose groups were all seen landed
         (void)ready_tiles;
-        for (int unit = first_unit; unit < sp.total_units && ok; unit += unit_stride) {
+        for (int unit = first_unit; unit < total_units && ok; unit += unit_stride) {
           int tile, kb0, kb1, part, m0, n0;
           unit_work(unit, tile, kb0, kb1, part);
           tile_origin(tile, m0, n0);
@@ -372,6 +376,9 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
             __syncwarp();
           }
         }
+        // every operand is on its way: the next kernel's CTAs may come (earlier they would sit next to this
+        // one for its whole life, where the optimizer's sweep runs)
+        if (elect_one()) chain_release();
         if constexpr (PAIR) {
           // Rank 0's commits arrive at the empty barriers of both CTAs, and no later barrier tells that
           // they have (a commit's arrival is ordered behind its MMAs, not behind other commits').  Each
@@ -404,7 +411,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
         const uint64_t desc_b0 = make_smem_desc_sw128(smem_u32(tiles) + S::kABytes, B_MN ? 8192 : 16, 1024);
         int it = 0, local = 0;      // k-blocks and tiles committed so far
         bool ok = true;
-        for (int unit = first_unit; unit < sp.total_units; unit += unit_stride, ++local) {
+        for (int unit = first_unit; unit < total_units; unit += unit_stride, ++local) {
           int tile, kb0, kb1, part;
           unit_work(unit, tile, kb0, kb1, part);
           const int ab = local & 1;
@@ -462,7 +469,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
     const int seq = pull.degree * pull.seq_local;
     const int chunks_per_row = (K * 2) / 16;               // 16-byte pieces of a row (K % 8 == 0)
     const int groups = (M + kPullRows - 1) / kPullRows;
-    for (int g = blockIdx.x; g < groups; g += gridDim.x) {
+    for (int g = total_units != 0 ? blockIdx.x : groups; g < groups; g += gridDim.x) {
       const int row0 = g * kPullRows;
       const int rows = min(kPullRows, M - row0);
       const int total = rows * chunks_per_row;
@@ -506,7 +513,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
     int sbuf = 0;          // staged store: which of this warp's staging buffers is written next
     bool ok = true;
     int* last_flag = reinterpret_cast<int*>(tmem_ptr + 2);   // shared: "this CTA reduces the tile"
-    for (int unit = first_unit; unit < sp.total_units; unit += unit_stride, ++local) {
+    for (int unit = first_unit; unit < total_units; unit += unit_stride, ++local) {
       int tile, kb0, kb1, part, m0, n0;
       unit_work(unit, tile, kb0, kb1, part);
       tile_origin(tile, m0, n0);

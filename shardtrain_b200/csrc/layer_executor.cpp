@@ -456,6 +456,7 @@ class Branch {
         cudaStreamWaitEvent(shared.side, shared.fork, 0) != cudaSuccess)
       return;
     side_ = shared.side;
+    stb::chain_break();
   }
   cudaStream_t stream() const { return side_ != nullptr ? side_ : main_; }
   void join() {
@@ -463,6 +464,7 @@ class Branch {
     Shared& shared = streams();
     ok(cudaEventRecord(shared.join, side_), "branch");
     ok(cudaStreamWaitEvent(main_, shared.join, 0), "branch");
+    stb::chain_break();
     side_ = nullptr;
     lock_.unlock();
   }
@@ -555,6 +557,7 @@ std::vector<Tensor> layer_forward(const Tensor& x2, const Tensor& w_qkv, const T
             at::empty({M, H}, f32),     at::empty({M, inter}, bf)};
   };
   auto launch = [&](std::vector<Tensor>& b) {
+    const stb::LaunchChain chain;
     Tensor &h1 = b[0], &inv1 = b[1], &qkv = b[2], &attn = b[3], &lse = b[4], &x_mid = b[5];
     Tensor &h2 = b[6], &inv2 = b[7], &gu = b[8], &out = b[9], &hm = b[10];
     ok(stb::launch_rmsnorm_fwd(x2.data_ptr<float>(), ln1.data_ptr<float>(), h1.data_ptr(),
@@ -663,6 +666,7 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
 
   auto alloc = [&]() -> std::vector<Tensor> { return {at::empty({M, H}, f32)}; };
   auto launch = [&](std::vector<Tensor>& b) {
+    const stb::LaunchChain chain;
     Tensor& dx = b[0];
     ok(stb::launch_cast_f32_to_bf16(d_out.data_ptr<float>(), t.d_out_b.data_ptr(), M * H, st), "cast");
     g.run(t.d_out_b, hm, g_down, true, true, nullptr, nullptr, SeqPull{}, accumulate);   // dW down
