@@ -9,6 +9,9 @@ re-materialised (reference: `src/sharded_runtime/runtime/bridge.py:9-47`).
 
 The reduced shard gradients are committed into the persistent gradient arena by the unit itself
 (`UnitState.reduce`), so this node returns no gradient for the shard leaves.
+
+With one member on the sm_100a executor neither node exists (`ShardedRuntime.direct`): the unit's own node
+does what they do, at the same points.
 """
 
 from __future__ import annotations
