@@ -230,6 +230,9 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
       }
     }
   }
+  // A pair allocates together, in the TMEM of both: not before both CTAs run.  (In a chain this is over
+  // before the kernel ahead is.)
+  if constexpr (PAIR) cluster_sync();
   if (warp == 1) {
     if constexpr (PAIR) {
       tmem_alloc_pair(tmem_ptr, S::kTmemCols);
