@@ -395,9 +395,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
 }
 
 // delta[b, h, s] = sum_d dO[b, s, h, d] * O[b, s, h, d]   (one warp per (row, head))
-__global__ void attention_delta_kernel(const __nv_bfloat16* __restrict__ out,
-                                       const __nv_bfloat16* __restrict__ dout,
-                                       float* __restrict__ delta, int batch, int seq, int hq) {
+__global__ void attention_delta_kernel(const __nv_bfloat16* out, const __nv_bfloat16* dout, float* delta,
+                                       int batch, int seq, int hq) {
   chain_wait();
   chain_release();
   const int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -962,9 +961,8 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
 }
 
 // dqkv[row, K|V columns] = bf16(sum over parts of the fp32 partial planes), fixed order.
-__global__ void attention_dkv_finish_kernel(const float* __restrict__ part, int parts,
-                                            int64_t rows, int hq, int hkv,
-                                            __nv_bfloat16* __restrict__ dqkv) {
+__global__ void attention_dkv_finish_kernel(const float* part, int parts, int64_t rows, int hq, int hkv,
+                                            __nv_bfloat16* dqkv) {
   chain_wait();
   chain_release();
   const int64_t pwidth = static_cast<int64_t>(2 * hkv) * kD;     // floats per row of a plane

@@ -83,6 +83,9 @@ __device__ __forceinline__ bool kernel_should_skip(const int* status) {
 // implies that all before it are.)  chain_release: this CTA does not mind the next kernel's CTAs being
 // placed from here on; they are when every CTA has said so or left.  A kernel that allocates TMEM says
 // so only when it has its own: the next one's CTAs may take what is left.
+// A chained kernel begins before its predecessor's last stores.  `__restrict__` would tell the compiler
+// that nobody else writes the data while the kernel runs (it may then load it through the read-only path,
+// or above chain_wait), so only what nothing in a chain writes carries it: weights and rotary tables.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -57,9 +57,8 @@ __device__ __forceinline__ float2 unpack2(uint32_t u) {
 // ------------------------------------------------------------------ RMSNorm
 // One CTA per row; x fp32 -> y = (x * rsqrt(mean(x^2)+eps)) * w, rounded once to the output type.
 template <bool Y_FP32>
-__global__ void rmsnorm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                   void* __restrict__ y, float* __restrict__ inv_out, int cols,
-                                   float eps) {
+__global__ void rmsnorm_fwd_kernel(const float* x, const float* __restrict__ w, void* y, float* inv_out,
+                                   int cols, float eps) {
   chain_wait();
   chain_release();
   __shared__ float red[32];
@@ -130,11 +129,9 @@ __global__ void slot_sum_rmsnorm_kernel(const float* __restrict__ slots, int n_s
 // dx = inv * (g*w - x * inv^2 * mean(g*w*x)) (+ incoming residual gradient), and optionally a bf16
 // copy of it; d(weight) partial per CTA = sum over its rows of g * (x*inv).  Rows are strided over
 // CTAs; thread t owns columns 4 t + 1024 k, whatever the width.
-__global__ void rmsnorm_bwd_kernel(const float* __restrict__ dy, const float* __restrict__ x,
-                                   const float* __restrict__ w, const float* __restrict__ inv,
-                                   const float* __restrict__ dres, float* __restrict__ dx,
-                                   __nv_bfloat16* __restrict__ dx_bf16,
-                                   float* __restrict__ dw_partial, int rows, int cols) {
+__global__ void rmsnorm_bwd_kernel(const float* dy, const float* x, const float* __restrict__ w,
+                                   const float* inv, const float* dres, float* dx, __nv_bfloat16* dx_bf16,
+                                   float* dw_partial, int rows, int cols) {
   chain_wait();
   chain_release();
   extern __shared__ float sm[];  // cols floats of dw accumulation + 32 for reductions
@@ -194,11 +191,9 @@ __global__ void rmsnorm_bwd_kernel(const float* __restrict__ dy, const float* __
 // -> reduction -> load per row: 35 us at 4096 x 1536, 107 us at 8192 x 3584; now 31 and 92 us.
 template <int K>
 __global__ void __launch_bounds__(256, 4)
-rmsnorm_bwd_rows_kernel(const float* __restrict__ dy, const float* __restrict__ x,
-                        const float* __restrict__ w, const float* __restrict__ inv,
-                        const float* __restrict__ dres, float* __restrict__ dx,
-                        __nv_bfloat16* __restrict__ dx_bf16, float* __restrict__ dw_partial,
-                        int rows, int cols) {
+rmsnorm_bwd_rows_kernel(const float* dy, const float* x, const float* __restrict__ w, const float* inv,
+                        const float* dres, float* dx, __nv_bfloat16* dx_bf16, float* dw_partial, int rows,
+                        int cols) {
   chain_wait();
   chain_release();
   constexpr bool kAhead = K <= 2;
@@ -290,8 +285,7 @@ rmsnorm_bwd_rows_kernel(const float* __restrict__ dy, const float* __restrict__ 
 // out[c] (+)= sum_r partial[r, c]; deterministic order.
 // out[c] = sum_r partial[r, c].  A CTA covers 32 columns with 8 row groups (blockDim 32 x 8): the
 // groups stride over the rows, then combine through shared memory in a fixed order.
-__global__ void colsum_f32_kernel(const float* __restrict__ partial, float* __restrict__ out,
-                                  int rows, int cols, int accumulate) {
+__global__ void colsum_f32_kernel(const float* partial, float* out, int rows, int cols, int accumulate) {
   chain_wait();
   chain_release();
   __shared__ float part[8][33];
@@ -319,8 +313,8 @@ __global__ void colsum_f32_kernel(const float* __restrict__ partial, float* __re
 }
 
 // scratch[b, c] = sum over the rows handled by CTA row-group b of x[r, c] (bf16 input).
-__global__ void colsum_bf16_partial_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx,
-                                           float* __restrict__ scratch, int rows, int cols) {
+__global__ void colsum_bf16_partial_kernel(const __nv_bfloat16* x, int64_t ldx, float* scratch, int rows,
+                                           int cols) {
   chain_wait();
   chain_release();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
@@ -352,7 +346,7 @@ __global__ void colsum_bf16_partial_kernel(const __nv_bfloat16* __restrict__ x, 
 // (the backward pass is the transposed rotation).
 // V elements of each half per thread: 8 (16-byte accesses) where d and the base allow it, else 2.
 template <int V>
-__global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ cos_t,
+__global__ void rope_kernel(__nv_bfloat16* qkv, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, const int* __restrict__ positions,
                             int rows, int seq, int hq, int hkv, int d, int inverse) {
   chain_wait();
@@ -440,9 +434,8 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu,
 }
 
 // d(gate) = dh * up * (sig + gate*sig*(1-sig)), d(up) = dh * silu(gate).
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh,
-                                  const __nv_bfloat16* __restrict__ gu,
-                                  __nv_bfloat16* __restrict__ dgu, int rows, int inter) {
+__global__ void swiglu_bwd_kernel(const __nv_bfloat16* dh, const __nv_bfloat16* gu, __nv_bfloat16* dgu,
+                                  int rows, int inter) {
   chain_wait();
   chain_release();
   const int64_t n8 = static_cast<int64_t>(rows) * (inter / 8);
@@ -561,18 +554,22 @@ __global__ void embedding_scatter_add_kernel(const float* __restrict__ dx,
     atomicAdd(dw + id * cols + c, dx[row * cols + c]);
 }
 
-__global__ void cast_f32_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y,
-                                     int64_t n) {
+__global__ void cast_f32_bf16_kernel(const float* x, __nv_bfloat16* y, int64_t n) {
   chain_wait();
   chain_release();
-  const int64_t n4 = n / 4;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const float4 v = *reinterpret_cast<const float4*>(x + i * 4);
-    uint2 pk;
-    pk.x = pack2(v.x, v.y);
-    pk.y = pack2(v.z, v.w);
-    *reinterpret_cast<uint2*>(y + i * 4) = pk;
+  const int64_t n4 = n / 4, stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  // four loads in flight per thread before the first store (the compiler may not move a load of x over a
+  // store to y by itself: 8192 x 3584 takes 46 us one by one, 35 like this)
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += 4 * stride) {
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * stride < n4) v[u] = *reinterpret_cast<const float4*>(x + (i + u * stride) * 4);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * stride < n4)
+        *reinterpret_cast<uint2*>(y + (i + u * stride) * 4) =
+            make_uint2(pack2(v[u].x, v[u].y), pack2(v[u].z, v[u].w));
   }
   if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {
     const int64_t i = n4 * 4 + threadIdx.x;

@@ -143,7 +143,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
                                                        const CUtensorMap& tma_c_h,
                                                        const GemmEpilogue& ep, const GemmSplit& sp,
                                                        const GemmPull& pull, int M, int N, int K,
-                                                       int* __restrict__ status) {
+                                                       int* status) {
   // Persistent: each CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...  The accumulator is
   // double buffered in TMEM (2 x BN columns) so the epilogue of one tile overlaps the MMAs of the
   // next; the shared-memory operand pipeline runs across tile boundaries without draining.
@@ -929,7 +929,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
                          const __grid_constant__ CUtensorMap tma_c,
                          const __grid_constant__ CUtensorMap tma_c_up,
                          const __grid_constant__ CUtensorMap tma_c_h, GemmEpilogue ep, GemmSplit sp,
-                         int M, int N, int K, int* __restrict__ status) {
+                         int M, int N, int K, int* status) {
   gemm_bf16_tcgen05_body<BN, A_MN, B_MN, false, false>(tma_a, tma_b, tma_c, tma_c_up, tma_c_h, ep, sp,
                                                 GemmPull{}, M, N, K, status);
 }
@@ -942,7 +942,7 @@ gemm_pair_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
                               const __grid_constant__ CUtensorMap tma_c,
                               const __grid_constant__ CUtensorMap tma_c_up,
                               const __grid_constant__ CUtensorMap tma_c_h, GemmEpilogue ep,
-                              GemmSplit sp, int M, int N, int K, int* __restrict__ status) {
+                              GemmSplit sp, int M, int N, int K, int* status) {
   gemm_bf16_tcgen05_body<BN, A_MN, B_MN, false, true>(tma_a, tma_b, tma_c, tma_c_up, tma_c_h, ep, sp,
                                                       GemmPull{}, M, N, K, status);
 }
@@ -956,7 +956,7 @@ gemm_pull_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
                               const __grid_constant__ CUtensorMap tma_c_up,
                               const __grid_constant__ CUtensorMap tma_c_h, GemmEpilogue ep,
                               GemmSplit sp, GemmPull pull, int M, int N, int K,
-                              int* __restrict__ status) {
+                              int* status) {
   gemm_bf16_tcgen05_body<BN, false, B_MN, true, false>(tma_a, tma_b, tma_c, tma_c_up, tma_c_h, ep, sp, pull,
                                                 M, N, K, status);
 }
