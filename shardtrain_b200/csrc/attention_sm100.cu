@@ -160,7 +160,7 @@ __device__ __forceinline__ void load_key_bits(const uint32_t* bits, int pitch, c
 // for TMEM loads and barriers.  At 1 x 8192 a block takes 2300 to 3200 clocks of an SM (1.4 to 1.965
 // GHz); its exponentials need 1024, its products 1024.
 // Measured on B200 (12 heads): 1 x 8192, causal, 1576 us before (one CTA per SM, MMAs issued from
-// one lane, P through shared memory) and 274 us now; 8 x 512: 100 and 33 us.
+// one lane, P through shared memory) and 269 us now; 8 x 512: 100 and 31 us.
 // smem: Q | K | V | barriers
 constexpr int kFwdSmem = 3 * kTile + 1024 + 128;
 
@@ -203,14 +203,14 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map, FwdParams p) {
     tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
   }
-  chain_wait();                       // what is above ran under the kernel before
-  __shared__ int skip;
-  if (threadIdx.x == 0) skip = status_failed(p.status) ? 1 : 0;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  if (skip != 0) {                    // an earlier kernel already failed
+  chain_wait();                       // what is above ran under the kernel before
+  // (asked in a step of its own: together with the barrier above, the loops below were compiled slower,
+  // 1 x 8192 in 299 instead of 269 us)
+  if (kernel_should_skip(p.status)) { // an earlier kernel already failed
     if (warp == 1) tmem_dealloc(tmem, 256);
     return;
   }
@@ -492,14 +492,12 @@ attention_dq_kernel(const __grid_constant__ CUtensorMap map_qkv,
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  chain_wait();                       // what is above ran under the kernel before
-  __shared__ int skip;
-  if (threadIdx.x == 0) skip = status_failed(p.status) ? 1 : 0;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  if (skip != 0) {                    // an earlier kernel already failed
+  chain_wait();                       // what is above ran under the kernel before
+  if (kernel_should_skip(p.status)) { // an earlier kernel already failed
     if (warp == 1) tmem_dealloc(tmem, 512);
     return;
   }
@@ -731,14 +729,12 @@ attention_dkv_kernel(const __grid_constant__ CUtensorMap map_qkv,
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  chain_wait();                       // what is above ran under the kernel before
-  __shared__ int skip;
-  if (threadIdx.x == 0) skip = status_failed(p.status) ? 1 : 0;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  if (skip != 0) {                    // an earlier kernel already failed
+  chain_wait();                       // what is above ran under the kernel before
+  if (kernel_should_skip(p.status)) { // an earlier kernel already failed
     if (warp == 1) tmem_dealloc(tmem, 512);
     return;
   }
