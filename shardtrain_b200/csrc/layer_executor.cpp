@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "api.h"
+#include "branch.h"
 
 namespace {
 
@@ -439,70 +440,45 @@ ReplayCache& replay_cache() {
   return cache;
 }
 
-// Work of a layer's sequence that nothing after it in the sequence reads (or only much later): a branch of
-// its graph while the sequence is being captured, the same launches in line otherwise.  `stream()` is
-// where the branch's kernels go; `join()` makes the sequence wait for them.  One second stream and two
-// events per device serve all captures: a branch holds their lock from its fork to its join.
-class Branch {
- public:
-  explicit Branch(cudaStream_t main) : main_(main) {
+// The CUDA runtime as branch.h asks for it.
+struct CudaBranches {
+  using Stream = cudaStream_t;
+  using Event = cudaEvent_t;
+  static bool capturing(Stream s) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(main, &status) != cudaSuccess) cudaGetLastError();
-    if (status != cudaStreamCaptureStatusActive) return;
-    lock_ = std::unique_lock<std::mutex>(mutex());
-    Shared& shared = streams();
-    if (shared.side == nullptr) return;
-    if (cudaEventRecord(shared.fork, main) != cudaSuccess ||
-        cudaStreamWaitEvent(shared.side, shared.fork, 0) != cudaSuccess)
-      return;
-    side_ = shared.side;
-    stb::chain_break();
+    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) cudaGetLastError();
+    return status == cudaStreamCaptureStatusActive;
   }
-  cudaStream_t stream() const { return side_ != nullptr ? side_ : main_; }
-  void join() {
-    if (side_ == nullptr) return;
-    Shared& shared = streams();
-    ok(cudaEventRecord(shared.join, side_), "branch");
-    ok(cudaStreamWaitEvent(main_, shared.join, 0), "branch");
-    stb::chain_break();
-    side_ = nullptr;
-    lock_.unlock();
+  static int device() {
+    int d = 0;
+    ok(cudaGetDevice(&d), "device");
+    return d;
   }
-
- private:
-  static std::mutex& mutex() {
-    static std::mutex m;
-    return m;
+  // Creating is no part of the capture: a call that a capture of this thread would not allow.
+  template <class F>
+  static bool outside_capture(F&& create) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    ok(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+    const bool made = create();
+    ok(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+    return made;
   }
-  struct Shared {
-    cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-  };
-  // per device (a process drives one; a second one gets its own)
-  static Shared& streams() {
-    static std::map<int, Shared> table;
-    int device = 0;
-    ok(cudaGetDevice(&device), "device");
-    Shared& s = table[device];
-    if (s.side == nullptr) {
+  static bool make_event(Event* e) {
+    return outside_capture([&] { return cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess; });
+  }
+  static bool make_stream(Stream* s) {
+    return outside_capture([&] {
       int least = 0, greatest = 0;
-      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // creating is no part of the capture
-      ok(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
-      const bool made = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
-                        cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) == cudaSuccess &&
-                        cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) == cudaSuccess &&
-                        cudaStreamCreateWithPriority(&s.side, cudaStreamNonBlocking, greatest) == cudaSuccess;
-      ok(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
-      if (!made) {
-        cudaGetLastError();
-        s = Shared{};
-      }
-    }
-    return s;
+      return cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
+             cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, greatest) == cudaSuccess;
+    });
   }
-  cudaStream_t main_, side_ = nullptr;
-  std::unique_lock<std::mutex> lock_;
+  static bool record(Event e, Stream s) { return cudaEventRecord(e, s) == cudaSuccess; }
+  static bool wait(Stream s, Event e) { return cudaStreamWaitEvent(s, e, 0) == cudaSuccess; }
+  static void clear_error() { cudaGetLastError(); }
+  static void chain_break() { stb::chain_break(); }
 };
+using Branch = stb::Branch<CudaBranches>;
 
 struct KeyBuilder {
   std::vector<int64_t> v;
