@@ -3,65 +3,77 @@
 // second stream cannot be made or the fork fails.  `stream()` is where the branch's kernels go; `join()`
 // makes the sequence wait for them.
 //
-// `Api` is the CUDA runtime (or a stand-in on the host): Stream, Event, capturing, device, make_stream,
-// make_event, record, wait, clear_error, chain_break; record and wait say whether they succeeded.
+// A stream that forked from a capture belongs to it until that capture ENDS, not until the join: nobody
+// else may use it in between.  So whoever captures owns the second stream (SideStreams, under the lock of
+// the replay cache) and hands it to the sequence.  A sequence that was given none runs in line, also
+// when it finds its stream in a capture that somebody else began.
+//
+// `Api` is the CUDA runtime (or a stand-in on the host): Stream, Event, device, make_stream, make_event,
+// drop_event, record, wait, clear_error, chain_break; those that can fail say whether they succeeded.
 #pragma once
 
 #include <map>
-#include <mutex>
 #include <stdexcept>
 
 namespace stb {
 
-// One second stream and two events per device serve all captures: a branch holds their lock from its
-// fork to its join, and none when it runs in line.
+template <class Api>
+struct SideStream {
+  typename Api::Stream stream{};
+  typename Api::Event fork{}, join{};
+};
+
+// The second streams of one owner, per device (a process drives one; a second one gets its own).  Whoever
+// uses them holds the owner's lock from the begin of a capture to its end.
+template <class Api>
+class SideStreams {
+ public:
+  // null where it cannot be made; tried again the next time
+  SideStream<Api>* get() {
+    SideStream<Api>& s = table_[Api::device()];
+    if (s.stream != typename Api::Stream{}) return &s;
+    SideStream<Api> made{};
+    const bool fork = Api::make_event(&made.fork), join = fork && Api::make_event(&made.join);
+    if (join && Api::make_stream(&made.stream)) {
+      s = made;
+      return &s;
+    }
+    if (join) Api::drop_event(made.join);
+    if (fork) Api::drop_event(made.fork);
+    Api::clear_error();
+    return nullptr;
+  }
+
+ private:
+  std::map<int, SideStream<Api>> table_;
+};
+
 template <class Api>
 class Branch {
  public:
   using Stream = typename Api::Stream;
-  using Event = typename Api::Event;
-  explicit Branch(Stream main) : main_(main) {
-    if (!Api::capturing(main)) return;
-    lock_ = std::unique_lock<std::mutex>(mutex());
-    Shared& shared = streams();
-    if (shared.side != Stream{} && Api::record(shared.fork, main) && Api::wait(shared.side, shared.fork)) {
-      side_ = shared.side;
+  // `side`: of the capture that `main` is in; null outside one
+  Branch(Stream main, SideStream<Api>* side) : main_(main) {
+    if (side == nullptr) return;
+    if (Api::record(side->fork, main) && Api::wait(side->stream, side->fork)) {
+      side_ = side;
       Api::chain_break();
     } else {
       Api::clear_error();
-      lock_.unlock();
     }
   }
-  Stream stream() const { return side_ != Stream{} ? side_ : main_; }
+  Stream stream() const { return side_ != nullptr ? side_->stream : main_; }
   void join() {
-    if (side_ == Stream{}) return;
-    Shared& shared = streams();
-    if (!Api::record(shared.join, side_) || !Api::wait(main_, shared.join))
+    if (side_ == nullptr) return;
+    if (!Api::record(side_->join, side_->stream) || !Api::wait(main_, side_->join))
       throw std::runtime_error("shardtrain_b200: a branch of a launch sequence could not be joined");
     Api::chain_break();
-    side_ = Stream{};
-    lock_.unlock();
+    side_ = nullptr;
   }
 
  private:
-  struct Shared {
-    Stream side{};
-    Event fork{}, join{};
-  };
-  static std::mutex& mutex() {
-    static std::mutex m;
-    return m;
-  }
-  // per device (a process drives one; a second one gets its own)
-  static Shared& streams() {
-    static std::map<int, Shared> table;
-    Shared& s = table[Api::device()];
-    if (s.side == Stream{} && !(Api::make_event(&s.fork) && Api::make_event(&s.join) && Api::make_stream(&s.side)))
-      s = Shared{};
-    return s;
-  }
-  Stream main_, side_{};
-  std::unique_lock<std::mutex> lock_;
+  Stream main_;
+  SideStream<Api>* side_ = nullptr;
 };
 
 }  // namespace stb

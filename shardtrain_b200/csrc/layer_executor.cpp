@@ -272,6 +272,43 @@ SpLink make_link(cudaStream_t st, int* status, c10::ArrayRef<int64_t> pads, int6
   return l;
 }
 
+// The CUDA runtime as branch.h asks for it.
+struct CudaBranches {
+  using Stream = cudaStream_t;
+  using Event = cudaEvent_t;
+  static int device() {
+    int d = 0;
+    ok(cudaGetDevice(&d), "device");
+    return d;
+  }
+  // Creating is no part of the capture: a call that a capture of this thread would not allow.
+  template <class F>
+  static bool outside_capture(F&& create) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    ok(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+    const bool made = create();
+    ok(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+    return made;
+  }
+  static bool make_event(Event* e) {
+    return outside_capture([&] { return cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess; });
+  }
+  static bool make_stream(Stream* s) {
+    return outside_capture([&] {
+      int least = 0, greatest = 0;
+      return cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
+             cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, greatest) == cudaSuccess;
+    });
+  }
+  static void drop_event(Event e) { cudaEventDestroy(e); }
+  static bool record(Event e, Stream s) { return cudaEventRecord(e, s) == cudaSuccess; }
+  static bool wait(Stream s, Event e) { return cudaStreamWaitEvent(s, e, 0) == cudaSuccess; }
+  static void clear_error() { cudaGetLastError(); }
+  static void chain_break() { stb::chain_break(); }
+};
+using Branch = stb::Branch<CudaBranches>;
+using Side = stb::SideStream<CudaBranches>;
+
 // ---------------------------------------------------------------------------------------------
 // Replay of launch sequences (CUDA graphs).
 //
@@ -302,7 +339,8 @@ struct ReplayEntry {
 
 class ReplayCache {
  public:
-  // `alloc()` -> the tensors the sequence writes and returns; `launch(buffers)` issues the kernels.
+  // `alloc()` -> the tensors the sequence writes and returns; `launch(buffers, side)` issues the kernels,
+  // with a second stream for branches (branch.h) while they are captured here, else null.
   template <class Alloc, class Launch>
   std::vector<Tensor> run(std::vector<int64_t> key, cudaStream_t st, Alloc&& alloc, Launch&& launch) {
     std::lock_guard<std::mutex> lock(mu_);
@@ -315,7 +353,7 @@ class ReplayCache {
       e->buffers = alloc();
       for (const Tensor& b : e->buffers) e->bytes += static_cast<int64_t>(b.nbytes());
       bytes_ += e->bytes;
-      launch(e->buffers);
+      launch(e->buffers, nullptr);
       return e->buffers;
     }
     e->used = ++tick_;
@@ -329,7 +367,7 @@ class ReplayCache {
       ok(cudaGraphLaunch(e->exec, st), "graph launch");
     } else {
       e->refuse = true;
-      launch(e->buffers);
+      launch(e->buffers, nullptr);
     }
     return e->buffers;
   }
@@ -407,13 +445,14 @@ class ReplayCache {
   template <class Launch>
   void capture(ReplayEntry* e, cudaStream_t st, Launch&& launch) {
     const int64_t before = stb::launches_total();
+    Side* const side = sides_.get();       // (mu_ is held until the capture has ended)
     if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       cudaGetLastError();
       return;
     }
     bool threw = false;
     try {
-      launch(e->buffers);
+      launch(e->buffers, side);
     } catch (...) {
       threw = true;           // the kernel-by-kernel launch that follows reports the error
     }
@@ -429,6 +468,7 @@ class ReplayCache {
 
   static constexpr size_t kMaxEntries = 1024;
   std::mutex mu_;
+  stb::SideStreams<CudaBranches> sides_;
   std::unordered_map<uint64_t, std::vector<std::unique_ptr<ReplayEntry>>> table_;
   size_t entries_ = 0;
   int64_t bytes_ = 0;
@@ -439,46 +479,6 @@ ReplayCache& replay_cache() {
   static ReplayCache cache;
   return cache;
 }
-
-// The CUDA runtime as branch.h asks for it.
-struct CudaBranches {
-  using Stream = cudaStream_t;
-  using Event = cudaEvent_t;
-  static bool capturing(Stream s) {
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) cudaGetLastError();
-    return status == cudaStreamCaptureStatusActive;
-  }
-  static int device() {
-    int d = 0;
-    ok(cudaGetDevice(&d), "device");
-    return d;
-  }
-  // Creating is no part of the capture: a call that a capture of this thread would not allow.
-  template <class F>
-  static bool outside_capture(F&& create) {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    ok(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
-    const bool made = create();
-    ok(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
-    return made;
-  }
-  static bool make_event(Event* e) {
-    return outside_capture([&] { return cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess; });
-  }
-  static bool make_stream(Stream* s) {
-    return outside_capture([&] {
-      int least = 0, greatest = 0;
-      return cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
-             cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, greatest) == cudaSuccess;
-    });
-  }
-  static bool record(Event e, Stream s) { return cudaEventRecord(e, s) == cudaSuccess; }
-  static bool wait(Stream s, Event e) { return cudaStreamWaitEvent(s, e, 0) == cudaSuccess; }
-  static void clear_error() { cudaGetLastError(); }
-  static void chain_break() { stb::chain_break(); }
-};
-using Branch = stb::Branch<CudaBranches>;
 
 struct KeyBuilder {
   std::vector<int64_t> v;
@@ -532,7 +532,7 @@ std::vector<Tensor> layer_forward(const Tensor& x2, const Tensor& w_qkv, const T
             at::empty({M, H}, bf),      at::empty({M}, f32),          at::empty({M, 2 * inter}, bf),
             at::empty({M, H}, f32),     at::empty({M, inter}, bf)};
   };
-  auto launch = [&](std::vector<Tensor>& b) {
+  auto launch = [&](std::vector<Tensor>& b, Side*) {
     const stb::LaunchChain chain;
     Tensor &h1 = b[0], &inv1 = b[1], &qkv = b[2], &attn = b[3], &lse = b[4], &x_mid = b[5];
     Tensor &h2 = b[6], &inv2 = b[7], &gu = b[8], &out = b[9], &hm = b[10];
@@ -555,7 +555,7 @@ std::vector<Tensor> layer_forward(const Tensor& x2, const Tensor& w_qkv, const T
   };
   if (!replay) {
     std::vector<Tensor> b = alloc();
-    launch(b);
+    launch(b, nullptr);
     return b;
   }
   KeyBuilder k;
@@ -641,7 +641,7 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
   BackwardScratch& t = replay ? shared_backward_scratch(x2, B, S, H, W, inter, hq, hkv, parts, st) : own;
 
   auto alloc = [&]() -> std::vector<Tensor> { return {at::empty({M, H}, f32)}; };
-  auto launch = [&](std::vector<Tensor>& b) {
+  auto launch = [&](std::vector<Tensor>& b, Side* side) {
     const stb::LaunchChain chain;
     Tensor& dx = b[0];
     ok(stb::launch_cast_f32_to_bf16(d_out.data_ptr<float>(), t.d_out_b.data_ptr(), M * H, st), "cast");
@@ -655,7 +655,7 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
                                inv2.data_ptr<float>(), d_out.data_ptr<float>(), t.d_mid.data_ptr<float>(),
                                t.partial.data_ptr<float>(), kNormPartialRows, M, H, st,
                                t.d_mid_b.data_ptr()), "rmsnorm_bwd");
-    Branch norm(st);
+    Branch norm(st, side);
     ok(stb::launch_colsum_f32(t.partial.data_ptr<float>(), g_ln2.data_ptr<float>(), kNormPartialRows, H,
                               accumulate, norm.stream()), "colsum");
     g.run(t.d_mid_b, attn, g_o, true, true, nullptr, nullptr, SeqPull{}, accumulate);    // dW o
@@ -679,13 +679,13 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
     bc.hkv = static_cast<int>(hkv);
     bc.scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(D)));
     ok(stb::launch_attention_bwd_delta(bc, st), "attention_bwd");
-    Branch keys(st);                       // dK, dV next to dQ
+    Branch keys(st, side);                       // dK, dV next to dQ
     ok(stb::launch_attention_bwd_dkv(bc, g.status, keys.stream()), "attention_bwd");
     ok(stb::launch_attention_bwd_dq(bc, g.status, st), "attention_bwd");
     keys.join();
     ok(stb::launch_rope(t.d_qkv.data_ptr(), cos.data_ptr<float>(), sin.data_ptr<float>(), pos, M, S, hq,
                         hkv, D, true, st), "rope inverse");
-    Branch bias(st);
+    Branch bias(st, side);
     ok(stb::launch_colsum_bf16(t.d_qkv.data_ptr(), W, g_bias.data_ptr<float>(), M, W, accumulate,
                                t.bias_partial.data_ptr<float>(), 64, bias.stream()), "bias colsum");
     g.run(t.d_qkv, h1, g_qkv, true, true, nullptr, nullptr, SeqPull{}, accumulate);      // dW q|k|v
@@ -699,7 +699,7 @@ Tensor layer_backward(const Tensor& d_out, const Tensor& x2, const Tensor& inv1,
   };
   if (!replay) {
     std::vector<Tensor> b = alloc();
-    launch(b);
+    launch(b, nullptr);
     return b[0];
   }
   KeyBuilder k;
