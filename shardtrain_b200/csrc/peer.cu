@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "api.h"
 #include "common.cuh"
@@ -161,10 +162,14 @@ __global__ void gather_params_kernel(PeerPtrs shards, ShadowPtrs shadows, int us
 // shape.  A CTA takes ONE tile and leaves: a kernel of the compute stream (higher priority) that needs
 // whole SMs can be placed only when the CTAs in its way have left, and with CTAs that lived for a sixth
 // of the sweep every layer's gate|up dW GEMM (pairs of CTAs) stood still for that long -- 65 us at the
-// 1.5B widths, 380 us twice a layer at the 7B widths.  A thread keeps 128 bytes of loads in flight, the
-// first of them issued before the status word is known.  Alone, in place: 46.8 M elements 217 us (6470
-// GB/s; 248 us before), 233 M 1038 us (1187), the check alone 33 us (84); tiles of 2048 and 8192
-// elements ran the training steps no faster.
+// 1.5B widths, 380 us twice a layer at the 7B widths.  The loads of a round are in flight together, the
+// first of them before the status word is known: with AdamW and one member 128 bytes a thread, for the
+// check alone 32, with several members 32 from each of four and then the 96 of p, m and v (before the sum
+// they would spill).  One member with AdamW, alone, in place: 46.8 M elements 217 us (6470 GB/s; 248 us
+// before), 233 M 1038 us (1187); the check alone 33 us for 46.8 M (84).  Tiles of 2048 and 8192 elements
+// ran the training steps no faster.
+// The vectors of a layer are shorter than a tile: 20 of 1536 elements take 9.2 us with one member (11.3
+// with the elements of a vector one after the other), five odd segments 13.2 with four members (19).
 constexpr int kRsThreads = 256;
 constexpr int kRsGroups = 2;                                     // float4 groups a thread loads at once
 constexpr int kRsRound = kRsThreads * 4 * kRsGroups;
@@ -227,103 +232,102 @@ __global__ void __launch_bounds__(kRsThreads, 4)
   int bad = 0, pad_bad = 0;
   const int64_t base = static_cast<int64_t>(blockIdx.x - tab.first[seg]) * kRsTile;
   const int64_t end = min(base + kRsTile, sg.q);
-  if (vec && base + kRsTile <= valid) {
-    // whole tile: 16-byte accesses, every load of a round in flight before the first use.  p, m and v
-    // stream past (nobody reads them again in this step): they should not push GEMM operands out of L2
-#pragma unroll 1
-    for (int64_t i = base + threadIdx.x * 4; i < base + kRsTile; i += kRsRound) {
-      const int64_t e = sg.shard_off + i;
-      float4 g[kRsGroups], pv[kRsGroups], mv[kRsGroups], vv[kRsGroups];
-      auto load_state = [&] {
+  // G times four elements from i on, all of them data: 16-byte accesses, every load in flight before the
+  // first use.  p, m and v stream past (nobody reads them again in this step): they should not push GEMM
+  // operands out of L2
+  auto vectors = [&](auto count, int64_t i) {
+    constexpr int G = decltype(count)::value;
+    const int64_t e = sg.shard_off + i;
+    float4 g[G], pv[G], mv[G], vv[G];
+    auto load_state = [&] {
 #pragma unroll
-        for (int u = 0; u < kRsGroups; ++u) {
-          pv[u] = __ldcs(reinterpret_cast<const float4*>(p + e + u * kRsThreads * 4));
-          mv[u] = __ldcs(reinterpret_cast<const float4*>(m + e + u * kRsThreads * 4));
-          vv[u] = __ldcs(reinterpret_cast<const float4*>(v + e + u * kRsThreads * 4));
-        }
-      };
-      if (ADAMW && LOCAL) load_state();
-      if (LOCAL) {
-        const float* src = full.p[0] + sg.full_off + i;
-#pragma unroll
-        for (int u = 0; u < kRsGroups; ++u)
-          g[u] = *reinterpret_cast<const float4*>(src + u * kRsThreads * 4);
-      } else if (multicast != nullptr && !replicated) {
-        // NVLS: one load through the multicast address of the gradient slot; the NVSwitch reads
-        // the same 16 bytes of every member's slot, adds them and returns the sum, so only
-        // 1 / F of the gradient enters this GPU instead of (F - 1) / F
-#pragma unroll
-        for (int u = 0; u < kRsGroups; ++u)
-          asm volatile("multimem.ld_reduce.relaxed.sys.global.add.v4.f32 {%0, %1, %2, %3}, [%4];"
-                       : "=f"(g[u].x), "=f"(g[u].y), "=f"(g[u].z), "=f"(g[u].w)
-                       : "l"(multicast + sg.full_off + lo + i + u * kRsThreads * 4)
-                       : "memory");
-      } else {
-#pragma unroll
-        for (int u = 0; u < kRsGroups; ++u) g[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        // rotate the peer order by rank so the ranks do not all hit one peer at once
-        for (int d = 0; d < n_src; ++d) {
-          const int src = ((first + d) % n_src) * stride + offset;
-          const float* from = full.p[src] + sg.full_off + lo + i;
-#pragma unroll
-          for (int u = 0; u < kRsGroups; ++u) {
-            const float4 t = *reinterpret_cast<const float4*>(from + u * kRsThreads * 4);
-            g[u].x += t.x; g[u].y += t.y; g[u].z += t.z; g[u].w += t.w;
-          }
-        }
+      for (int u = 0; u < G; ++u) {
+        pv[u] = __ldcs(reinterpret_cast<const float4*>(p + e + u * kRsThreads * 4));
+        mv[u] = __ldcs(reinterpret_cast<const float4*>(m + e + u * kRsThreads * 4));
+        vv[u] = __ldcs(reinterpret_cast<const float4*>(v + e + u * kRsThreads * 4));
       }
-      if (skip) return;
-      if (ADAMW && !LOCAL) load_state();       // (before the sum they would spill)
+    };
+    if (ADAMW && LOCAL) load_state();
+    if (LOCAL) {
+      const float* src = full.p[0] + sg.full_off + i;
 #pragma unroll
-      for (int u = 0; u < kRsGroups; ++u) {
-        const int64_t eu = e + u * kRsThreads * 4;
-        g[u].x *= scale; g[u].y *= scale; g[u].z *= scale; g[u].w *= scale;
-        if (accumulate) {
-          const float4 o = *reinterpret_cast<const float4*>(gshard + eu);
-          g[u].x += o.x; g[u].y += o.y; g[u].z += o.z; g[u].w += o.w;
-        }
-        if (!in_place) *reinterpret_cast<float4*>(gshard + eu) = g[u];
-        bad |= !(isfinite(g[u].x) && isfinite(g[u].y) && isfinite(g[u].z) && isfinite(g[u].w));
-        if (ADAMW) {
-          adamw_update(pv[u].x, mv[u].x, vv[u].x, g[u].x, a, step_size, inv_bc2_sqrt);
-          adamw_update(pv[u].y, mv[u].y, vv[u].y, g[u].y, a, step_size, inv_bc2_sqrt);
-          adamw_update(pv[u].z, mv[u].z, vv[u].z, g[u].z, a, step_size, inv_bc2_sqrt);
-          adamw_update(pv[u].w, mv[u].w, vv[u].w, g[u].w, a, step_size, inv_bc2_sqrt);
-          __stcs(reinterpret_cast<float4*>(p + eu), pv[u]);
-          __stcs(reinterpret_cast<float4*>(m + eu), mv[u]);
-          __stcs(reinterpret_cast<float4*>(v + eu), vv[u]);
-          if (shadow != nullptr)                     // compute-dtype copy for the next gather
-            *reinterpret_cast<uint2*>(shadow + eu) =
-                make_uint2(pk2(pv[u].x, pv[u].y), pk2(pv[u].z, pv[u].w));
+      for (int u = 0; u < G; ++u)
+        g[u] = *reinterpret_cast<const float4*>(src + u * kRsThreads * 4);
+    } else if (multicast != nullptr && !replicated) {
+      // NVLS: one load through the multicast address of the gradient slot; the NVSwitch reads
+      // the same 16 bytes of every member's slot, adds them and returns the sum, so only
+      // 1 / F of the gradient enters this GPU instead of (F - 1) / F
+#pragma unroll
+      for (int u = 0; u < G; ++u)
+        asm volatile("multimem.ld_reduce.relaxed.sys.global.add.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(g[u].x), "=f"(g[u].y), "=f"(g[u].z), "=f"(g[u].w)
+                     : "l"(multicast + sg.full_off + lo + i + u * kRsThreads * 4)
+                     : "memory");
+    } else {
+#pragma unroll
+      for (int u = 0; u < G; ++u) g[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      // rotate the peer order by rank so the ranks do not all hit one peer at once
+#pragma unroll 4
+      for (int d = 0; d < n_src; ++d) {
+        const int src = ((first + d) % n_src) * stride + offset;
+        const float* from = full.p[src] + sg.full_off + lo + i;
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+          const float4 t = *reinterpret_cast<const float4*>(from + u * kRsThreads * 4);
+          g[u].x += t.x; g[u].y += t.y; g[u].z += t.z; g[u].w += t.w;
         }
       }
     }
-  } else {
-    // the last tile of a segment, or one that is not aligned
     if (skip) return;
+    if (ADAMW && !LOCAL) load_state();       // (before the sum they would spill)
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      const int64_t eu = e + u * kRsThreads * 4;
+      g[u].x *= scale; g[u].y *= scale; g[u].z *= scale; g[u].w *= scale;
+      if (accumulate) {
+        const float4 o = *reinterpret_cast<const float4*>(gshard + eu);
+        g[u].x += o.x; g[u].y += o.y; g[u].z += o.z; g[u].w += o.w;
+      }
+      if (!in_place) *reinterpret_cast<float4*>(gshard + eu) = g[u];
+      bad |= !(isfinite(g[u].x) && isfinite(g[u].y) && isfinite(g[u].z) && isfinite(g[u].w));
+      if (ADAMW) {
+        adamw_update(pv[u].x, mv[u].x, vv[u].x, g[u].x, a, step_size, inv_bc2_sqrt);
+        adamw_update(pv[u].y, mv[u].y, vv[u].y, g[u].y, a, step_size, inv_bc2_sqrt);
+        adamw_update(pv[u].z, mv[u].z, vv[u].z, g[u].z, a, step_size, inv_bc2_sqrt);
+        adamw_update(pv[u].w, mv[u].w, vv[u].w, g[u].w, a, step_size, inv_bc2_sqrt);
+        __stcs(reinterpret_cast<float4*>(p + eu), pv[u]);
+        __stcs(reinterpret_cast<float4*>(m + eu), mv[u]);
+        __stcs(reinterpret_cast<float4*>(v + eu), vv[u]);
+        if (shadow != nullptr)                     // compute-dtype copy for the next gather
+          *reinterpret_cast<uint2*>(shadow + eu) =
+              make_uint2(pk2(pv[u].x, pv[u].y), pk2(pv[u].z, pv[u].w));
+      }
+    }
+  };
+  if (vec && base + kRsTile <= valid) {
+#pragma unroll 1
+    for (int64_t i = base + threadIdx.x * 4; i < base + kRsTile; i += kRsRound)
+      vectors(std::integral_constant<int, kRsGroups>{}, i);
+  } else {
+    // The last tile of a segment (and so every segment that is shorter than a tile), or one that is not
+    // aligned: element by element only what 16-byte accesses cannot reach.
     const int step = vec ? 4 : 1;
+#pragma unroll 1
     for (int64_t i = base + threadIdx.x * step; i < end; i += kRsThreads * step) {
-      const bool quad = vec && i + 3 < valid;
+      if (vec && i + 3 < valid) {
+        vectors(std::integral_constant<int, 1>{}, i);
+        continue;
+      }
+      if (skip) break;
 #pragma unroll 1
       for (int j = 0; j < step; ++j) {
         const int64_t e = sg.shard_off + i + j;
         float acc = 0.f;
-        if (i + j < valid) {
-          if (!LOCAL && quad && multicast != nullptr && !replicated) {
-            // the switch adds 16 bytes at a time; each of the four elements takes its own part
-            float4 t;
-            asm volatile("multimem.ld_reduce.relaxed.sys.global.add.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
-                         : "l"(multicast + sg.full_off + lo + i)
-                         : "memory");
-            acc = j == 0 ? t.x : j == 1 ? t.y : j == 2 ? t.z : t.w;
-          } else {
-            for (int d = 0; d < n_src; ++d) {
-              const int src = ((first + d) % n_src) * stride + offset;
-              acc += full.p[src][sg.full_off + lo + i + j];
-            }
+        if (i + j < valid)
+          for (int d = 0; d < n_src; ++d) {
+            const int src = ((first + d) % n_src) * stride + offset;
+            acc += full.p[src][sg.full_off + lo + i + j];
           }
-        }
         float g = acc * scale;
         if (accumulate) g += gshard[e];
         if (!in_place) gshard[e] = g;              // padding stays exactly zero: acc is 0 there
