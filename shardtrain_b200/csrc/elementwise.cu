@@ -757,23 +757,23 @@ cudaError_t launch_rmsnorm_bwd(const float* dy, const float* x, const float* w, 
   switch (wide ? (cols + 1023) / 1024 : 0) {
     case 1:
       launch_chained(rmsnorm_bwd_rows_kernel<1>, partial_rows, 256, 0, s, dy, x, w, inv, dres_in, dx_out, copy,
-                                                              dw_partial, rows, cols);
+                     dw_partial, rows, cols);
       break;
     case 2:
       launch_chained(rmsnorm_bwd_rows_kernel<2>, partial_rows, 256, 0, s, dy, x, w, inv, dres_in, dx_out, copy,
-                                                              dw_partial, rows, cols);
+                     dw_partial, rows, cols);
       break;
     case 3:
       launch_chained(rmsnorm_bwd_rows_kernel<3>, partial_rows, 256, 0, s, dy, x, w, inv, dres_in, dx_out, copy,
-                                                              dw_partial, rows, cols);
+                     dw_partial, rows, cols);
       break;
     case 4:
       launch_chained(rmsnorm_bwd_rows_kernel<4>, partial_rows, 256, 0, s, dy, x, w, inv, dres_in, dx_out, copy,
-                                                              dw_partial, rows, cols);
+                     dw_partial, rows, cols);
       break;
     default:     // wider rows than the registers hold, or partial sums off a 16-byte boundary
-      launch_chained(rmsnorm_bwd_kernel, partial_rows, 256, (cols + 32) * sizeof(float), s, 
-          dy, x, w, inv, dres_in, dx_out, copy, dw_partial, rows, cols);
+      launch_chained(rmsnorm_bwd_kernel, partial_rows, 256, (cols + 32) * sizeof(float), s, dy, x, w, inv,
+                     dres_in, dx_out, copy, dw_partial, rows, cols);
   }
   count_launch();
   return cudaGetLastError();
@@ -791,10 +791,10 @@ cudaError_t launch_colsum_bf16(const void* x, int64_t ldx, float* out, int rows,
   if (cols % 2 || scratch_rows < 1) return cudaErrorInvalidValue;
   dim3 grid((cols / 2 + 127) / 128, scratch_rows);
   launch_chained(colsum_bf16_partial_kernel, grid, 128, 0, s, reinterpret_cast<const __nv_bfloat16*>(x), ldx,
-                                                  scratch, rows, cols);
+                 scratch, rows, cols);
   count_launch();
   launch_chained(colsum_f32_kernel, (cols + 31) / 32, dim3(32, 8), 0, s, scratch, out, scratch_rows, cols,
-                                                             accumulate);
+                 accumulate);
   count_launch();
   return cudaGetLastError();
 }
@@ -809,11 +809,11 @@ cudaError_t launch_rope(void* qkv, const float* cos, const float* sin, const int
   const int64_t work = static_cast<int64_t>(rows) * (hq + hkv) * (d / (wide ? 16 : 4));
   const int grid = static_cast<int>((work + 255) / 256);
   if (wide)
-    launch_chained(rope_kernel<8>, grid, 256, 0, s, reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions, rows,
-                                        seq, hq, hkv, d, inverse);
+    launch_chained(rope_kernel<8>, grid, 256, 0, s, reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions,
+                   rows, seq, hq, hkv, d, inverse);
   else
-    launch_chained(rope_kernel<2>, grid, 256, 0, s, reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions, rows,
-                                        seq, hq, hkv, d, inverse);
+    launch_chained(rope_kernel<2>, grid, 256, 0, s, reinterpret_cast<__nv_bfloat16*>(qkv), cos, sin, positions,
+                   rows, seq, hq, hkv, d, inverse);
   count_launch();
   return cudaGetLastError();
 }
@@ -831,9 +831,9 @@ cudaError_t launch_swiglu_bwd(const void* dh, const void* gu, void* dgu, int row
                               cudaStream_t s) {
   if (inter % 8) return cudaErrorInvalidValue;
   const int64_t work = static_cast<int64_t>(rows) * (inter / 8);
-  launch_chained(swiglu_bwd_kernel, grid_for(work, 256, sm_count() * 16), 256, 0, s, 
-      reinterpret_cast<const __nv_bfloat16*>(dh), reinterpret_cast<const __nv_bfloat16*>(gu),
-      reinterpret_cast<__nv_bfloat16*>(dgu), rows, inter);
+  launch_chained(swiglu_bwd_kernel, grid_for(work, 256, sm_count() * 16), 256, 0, s,
+                 reinterpret_cast<const __nv_bfloat16*>(dh), reinterpret_cast<const __nv_bfloat16*>(gu),
+                 reinterpret_cast<__nv_bfloat16*>(dgu), rows, inter);
   count_launch();
   return cudaGetLastError();
 }
@@ -870,8 +870,8 @@ cudaError_t launch_embedding_scatter_add(const float* dx, const int64_t* ids, fl
 }
 
 cudaError_t launch_cast_f32_to_bf16(const float* x, void* y, int64_t n, cudaStream_t s) {
-  launch_chained(cast_f32_bf16_kernel, grid_for(n / 4 + 1, 256, sm_count() * 16), 256, 0, s, 
-      x, reinterpret_cast<__nv_bfloat16*>(y), n);
+  launch_chained(cast_f32_bf16_kernel, grid_for(n / 4 + 1, 256, sm_count() * 16), 256, 0, s, x,
+                 reinterpret_cast<__nv_bfloat16*>(y), n);
   count_launch();
   return cudaGetLastError();
 }

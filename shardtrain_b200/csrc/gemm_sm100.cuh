@@ -313,7 +313,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
               const uint64_t t0 = global_ns();
               for (uint32_t spin = 0;; ++spin) {
                 uint32_t seen[kGemmBM / kPullRows];
-  #pragma unroll
+#pragma unroll
                 for (int g = 0; g < kGemmBM / kPullRows; ++g) {
                   seen[g] = pull.epoch;
                   if (g < g_count)
@@ -321,7 +321,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
                                  : "=r"(seen[g]) : "l"(pull.flags + g_first + g) : "memory");
                 }
                 bool all = true;
-  #pragma unroll
+#pragma unroll
                 for (int g = 0; g < kGemmBM / kPullRows; ++g) all = all && seen[g] == pull.epoch;
                 if (__all_sync(0xffffffffu, all)) break;
                 if ((spin & 63u) == 63u &&
@@ -355,7 +355,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
               if constexpr (!A_MN) {
                 load(sa, &tma_a, &full_bar[s], kb * kGemmBK, m0);
               } else {
-  #pragma unroll
+#pragma unroll
                 for (int c = 0; c < kGemmBM / 64; ++c)
                   load(sa + c * 8192, &tma_a, &full_bar[s], m0 + c * 64, kb * kGemmBK);
               }
@@ -371,7 +371,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
                   load(sb, &tma_b, &full_bar[s], kb * kGemmBK, n0 + rank * S::kBRows);
                 }
               } else {
-  #pragma unroll
+#pragma unroll
                 for (int c = 0; c < S::kBLoad / 64; ++c)
                   load(sb + c * 8192, &tma_b, &full_bar[s], n0 + rank * S::kBRows + c * 64, kb * kGemmBK);
               }
@@ -433,7 +433,7 @@ __device__ __forceinline__ void gemm_bf16_tcgen05_body(const CUtensorMap& tma_a,
             const uint64_t da_s = desc_a0 + s * (S::kStageBytes >> 4);
             const uint64_t db_s = desc_b0 + s * (S::kStageBytes >> 4);
             if (elect_one()) {
-  #pragma unroll
+#pragma unroll
               for (int k = 0; k < kGemmBK / 16; ++k) {
                 const uint64_t da = da_s + k * ((A_MN ? 2048 : 32) >> 4);
                 const uint64_t db = db_s + k * ((B_MN ? 2048 : 32) >> 4);

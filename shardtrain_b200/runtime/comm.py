@@ -53,6 +53,8 @@ TICKET_FIELDS = (("op_id", "op_id"), ("op_kind", "kind"), ("pg_id", "pg_id"),
                  ("logical_cuda_stream", "logical_cuda_stream"),
                  ("collective_cuda_stream", "collective_cuda_stream"),
                  ("api_async_op", "api_async_op"), ("work_returned", "work_returned"))
+
+
 @dataclass
 class BufferLease:
     buffer_id: int

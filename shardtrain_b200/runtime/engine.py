@@ -56,11 +56,11 @@ ENTERED_FROM = {
     "GRAD_REDUCING": {"BWD_ACTIVE"},
     "GRAD_READY": {"GRAD_REDUCING"},
 }
+DIRECTION = {"FWD": +1, "BWD": -1}      # which neighbour a phase prefetches
+
+
 def _always(unit):
     return True
-
-
-DIRECTION = {"FWD": +1, "BWD": -1}      # which neighbour a phase prefetches
 
 
 class UnitState:
